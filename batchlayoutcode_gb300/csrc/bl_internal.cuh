@@ -172,12 +172,8 @@ struct Scratch {
   double *energy = nullptr;        // per-iteration energies (device)
   DevStatus *status = nullptr;
   // minibatch sweep
-  float2 *partials = nullptr;
+  void *partials = nullptr;  // control words, exchange, partial forces
   size_t partials_bytes = 0;
-  int *cursor = nullptr;  // per (block, vertex) neighbour cursor start
-  int cursor_grid = 0;
-  int *cursor_full = nullptr;  // the same for the full sorted rows (algo 7)
-  int cursor_full_grid = 0;
   // algo 5, first phase: repulsion sources per vertex as (vertex, count) pairs
   long long *walk_off = nullptr;  // n + 1
   int2 *walk_pairs = nullptr;
@@ -291,7 +287,6 @@ void bl_time_end(bl_ctx *ctx, const char *kernel);
 
 // ---- kernels drivers (smu.cu, bh.cu, reduce.cu) ----------------------------
 namespace bl {
-int ensure_minibatch_scratch(bl_ctx *ctx, int batch, int grid);
 int minibatch_run(bl_ctx *ctx, int model, int batch, int iterations, double step0,
                   double decay, bool converged, double engt, long long max_loops,
                   double *energy_out, long long *loops_out);

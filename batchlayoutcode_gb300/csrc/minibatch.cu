@@ -11,18 +11,35 @@
 // the neighbours matched by the sorted-CSR cursor (kindex, :758-762) plus
 // repulsion -d/|d|^2 over every other vertex with |d| > 0.
 //
-// GB300 design: one persistent cooperative kernel runs every iteration and
-// batch.  Each block owns a contiguous slice of source vertices kept in shared
-// memory for the whole run (8 B per vertex, float2).  For batch c every block
-// sweeps its slice against the batch's targets with a branch-free inner loop
-// (repulsion for all pairs; 7 FP32 instructions per pair, one MUFU rcp), and
-// writes one FP32 partial force per target.  After a grid barrier the block(s)
-// whose slice holds batch c sum the partials in FP64 in a fixed order, correct
-// the neighbour pairs (remove their repulsion, add the model's attraction --
-// the decomposition the reference's own algo 7 uses, :553-579), move the
-// vertices and refresh their shared-memory copy.  Blocks that do not own
-// batch c go straight on to batch c+1: the only values that changed are batch
-// c's own positions, which live in the owners' slices.
+// GB300 design: one persistent cooperative kernel, one 1,024-thread block per
+// SM, runs every iteration and batch without a grid barrier.  Batches are
+// numbered through the run (q = 0, 1, ...).  The sequential chain (a batch's
+// forces need the batch before it moved) only touches the pairs with the last
+// few batches, so two kinds of blocks share the work:
+//
+// * Sweepers own a contiguous slice of the source vertices in shared memory
+//   and add up, for batch q, the repulsion of their sources except those in
+//   the `lag` (two) batches before q, which may still be moving: one FP32
+//   partial force per target, stored to global memory.  They need only batch
+//   q - lag - 1 to have moved, so they run up to `lag` batches ahead of the
+//   chain.  Two 512-thread teams take alternate batches, so one team's waits,
+//   partial sums and stores overlap the other's sweep.
+// * Movers (the first M blocks) each move a fixed share of every batch.
+//   Three teams work side by side: P adds up the sweepers' partials, N the
+//   neighbour corrections (remove the repulsion, add the model's attraction
+//   -- the decomposition the reference's own algo 7 uses, :553-579), and the
+//   critical team the pairs with the last `lag` batches; it receives the batch
+//   before as 8-byte words {coordinate, batch tag} the other movers write (one
+//   L2 hop, no barrier), moves its share and publishes it the same way.
+//
+// So a batch costs max(sweep, chain) instead of their sum and a grid barrier
+// (one barrier per batch, the form before this one, in brackets).  Bound of
+// the sweep: the MUFU reciprocal, 16 a clock and SM; its loop runs at 14.9
+// pairs a clock, 6.8 us a batch at 100,000 vertices and batch 256 (10.8, of
+// which 6.9 the sweep).  Bound of the chain: instruction latency of about 400
+// dependent instructions and one L2 round trip, 2.9 us a batch at 4,096
+// vertices (5.2), 3.5 at 20,000 and batch 200 (5.4); 31,000 and batch 512 5.9
+// (12.3).  Every sum has a fixed order, so results are deterministic.
 //
 // Algorithmic work: 10 flops per ordered pair (2 sub, 3 for |d|^2, 1 rcp,
 // 2 FMA x 2 components counted as 4), n*n pairs per iteration.
@@ -32,6 +49,7 @@
 #include <cfloat>
 #include <climits>
 #include <cmath>
+#include <cstddef>
 #include <mutex>
 
 #include "../../include/batchlayout_gb300.h"
@@ -40,48 +58,53 @@
 namespace bl {
 namespace {
 
-constexpr int kThreads = 512;
-constexpr int kGroups = 4;                     // source sub-slices per block
-constexpr int kGroup = kThreads / kGroups;     // 128 threads per group
-constexpr int kChunk = 2 * kGroup;             // 256 targets per sweep pass
-constexpr int kWarps = kThreads / 32;
+constexpr int kThreads = 1024;
+constexpr int kTeam = 512;                  // sweeper team
+constexpr int kGroups = 4;                  // source groups of a team
+constexpr int kGroup = kTeam / kGroups;     // 128 threads, two targets each
+constexpr int kChunk = 2 * kGroup;          // targets per pass of a team
+constexpr int kCWarps = 16;                 // mover: critical team
+constexpr int kNWarps = 7;                  // mover: neighbours
+constexpr int kPWarps = 8;                  // mover: sweepers' partials (and one warp that watches for them)
+constexpr int kRows = 16;                   // sums per target that N and P leave (row kNWarps stays zero)
+constexpr int kMoveTile = 32;               // targets a mover handles at a time
+constexpr int kPartLoads = 5;               // partials a P lane loads at a time
+constexpr int kMaxMovers = 32;
+constexpr int kMaxLag = 2;
+constexpr int kExchange = 4;                // exchange slots (two would do)
+constexpr int kNear = 16;                   // staged neighbours in the batch before
+constexpr unsigned int kNearMore = 0x80000000u;
 constexpr int kMaxBatch = 4096;
 
-// Block partial forces are summed across blocks as 64-bit fixed-point
-// integers (units of 2^-28): integer addition is exact and associative, so
-// the total does not depend on the order of the atomics and stays
-// deterministic.  A partial beyond +-2^34 (forces of ~1e10, coincident
-// vertices) is reported as an error instead of wrapping.
-// Every buffer of accumulators has kAccCopies copies; block s adds into copy
-// s % kAccCopies, so fewer blocks queue on one address at the same time, and
-// the owners add the copies up (integer sums: exact in any order).
-constexpr int kAccCopies = 8;
-constexpr float kFixScale = 268435456.0f;        // 2^28
-constexpr double kFixInv = 1.0 / 268435456.0;    // 2^-28
-constexpr float kFixLimit = 17179869184.0f;      // 2^34
+// A force component beyond +-2^34 (coincident-but-for-rounding vertices) or
+// not a number is reported as an error instead of moving the vertex.
+constexpr float kForceLimit = 17179869184.0f;  // 2^34
 
-__device__ __forceinline__ void acc_add(long long *dst, float v, DevStatus *st) {
-  if (!(fabsf(v) < kFixLimit)) {
-    dev_record_error(st, DEV_FORCE_RANGE);
-    return;
-  }
-  atomicAdd(reinterpret_cast<unsigned long long *>(dst), (unsigned long long)__float2ll_rn(v * kFixScale));
-}
+// Control words of a launch (zero before it).
+struct MbControl {
+  unsigned int moved;   // movers that finished a batch, over all batches
+  unsigned int stop;    // converged runs: the movers ended
+  unsigned int ready;   // movers whose first loads are done
+  unsigned int pad;
+  unsigned int arrive[kMaxLag + 2];  // sweepers that stored a batch's partials, per slot
+  // energy per mover, tagged by iteration: {low word, tag}, {high word, tag}
+  alignas(16) ulonglong2 energy[2][kMaxMovers];
+};
+static_assert(offsetof(MbControl, energy) % 16 == 0 && alignof(MbControl) == 16, "16-byte accesses");
 
 struct MinibatchArgs {
-  int n, batch, nbatches, model, grid;
-  double W;
+  int n, batch, nbatches, model, lag, movers, sweepers;
+  int late;  // the movers' early teams start on a batch one batch later (one buffer instead of two)
+  float W;
   const int *eff_rowptr, *eff_colids;
-  // cursor[s * n + i]: neighbours of i below the first vertex of block s's
-  // slice (null: found by binary search)
-  const int *cursor;
   float2 *pos;
   double2 *force;
   double *e;
-  long long *acc;         // [2][kAccCopies][batch][2] fixed-point force sums (2^-28 units)
-  double *energy;         // energy per iteration (device)
-  double *energy_parts;   // [grid]
-  long long *loops;       // iterations run (device, 1 value)
+  float2 *part;             // [lag + 1][sweepers][batch rounded up to even] partial forces
+  ulonglong2 *exchange;     // [kExchange][batch] new positions {x, tag}, {y, tag}
+  MbControl *ctl;
+  double *energy;           // energy of the last iteration (device)
+  long long *loops;         // iterations run (device, 1 value)
   DevStatus *st;
   int iterations;
   double step0, decay;
@@ -90,380 +113,1029 @@ struct MinibatchArgs {
   long long max_loops;
 };
 
-// The reference's kindex cursor (algorithms.cpp:746,758-762) restricted to
-// this block's slice: the target's matched neighbours inside [slo, shi) are
-// staged in shared memory (up to kNbCap, slice-local indices) with the
-// batch's targets, so stepping the cursor reads shared memory; a target with
-// more neighbours in the slice continues from global memory.
-constexpr int kNbCap = 16;
+// ---- waits and named barriers ------------------------------------------------
 
-struct NbList {
-  int *ids;    // [kChunk][kNbCap] slice-local ids
-  int *meta;   // [kChunk][2]: number of neighbours in the slice, first CSR index
+__device__ __forceinline__ void bar_sync(int id, int count) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int count) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void red_add(unsigned int *p, unsigned int v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Bounded poll step: false when the wait has to end (time-out, or an error
+// recorded elsewhere).
+struct Poll {
+  unsigned long long t0;
+  unsigned int polls;
+  __device__ __forceinline__ Poll() : t0(0), polls(0) {}
+  __device__ __forceinline__ bool again(DevStatus *st) {
+    if ((++polls & 63u) == 0u) {
+      if (ld_volatile_u32(&st->code) != 0u) return false;
+      const unsigned long long t = dev_globaltimer();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > kBarrierTimeoutNs) {
+        dev_record_error(st, DEV_TIMEOUT_GRID_BARRIER);
+        return false;
+      }
+    }
+    return true;
+  }
 };
 
-// Stage the neighbours of targets [base, base + cnt) (cnt <= kChunk) that lie
-// in [slo, shi).  One thread per target.
-__device__ __forceinline__ void stage_neighbours(const MinibatchArgs &a, NbList L, int s, int base, int cnt,
-                                                 int slo, int shi, int sbase) {
-  for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-    const int i = base + t;
-    const int r0 = a.eff_rowptr[i], r1 = a.eff_rowptr[i + 1];
-    int k0, k1;
-    if (a.cursor) {
-      k0 = r0 + a.cursor[(size_t)s * a.n + i];
-      k1 = (s + 1 < a.grid) ? r0 + a.cursor[(size_t)(s + 1) * a.n + i] : r1;
-    } else {  // lower bounds of slo and shi in the sorted neighbour list
-      int lo = r0, hi = r1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(&a.eff_colids[mid]) < slo) lo = mid + 1;
-        else hi = mid;
-      }
-      k0 = lo;
-      hi = r1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(&a.eff_colids[mid]) < shi) lo = mid + 1;
-        else hi = mid;
-      }
-      k1 = lo;
-    }
-    const int m = min(k1 - k0, kNbCap);
-    for (int q = 0; q < m; q++) L.ids[t * kNbCap + q] = __ldg(&a.eff_colids[k0 + q]) - sbase;
-    L.meta[2 * t] = k1 - k0;
-    L.meta[2 * t + 1] = k0;
-  }
+// counters are monotone modulo 2^32
+__device__ __forceinline__ bool reached(unsigned int v, unsigned int target) { return (int)(v - target) >= 0; }
+
+__device__ __forceinline__ bool wait_count(const unsigned int *p, unsigned int target, DevStatus *st) {
+  Poll w;
+#pragma unroll 1
+  while (!reached(ld_acquire_gpu(p), target))
+    if (!w.again(st)) return false;
+  return true;
 }
 
-struct Cursor {
-  int ptr, cnt, k0, next;
-  const int *ids;
-};
-
-__device__ __forceinline__ int cursor_at(const MinibatchArgs &a, const Cursor &c, int sbase) {
-  if (c.ptr >= c.cnt) return INT_MAX;
-  if (c.ptr < kNbCap) return c.ids[c.ptr];
-  return __ldg(&a.eff_colids[c.k0 + c.ptr]) - sbase;  // beyond the staged ones
+__device__ __forceinline__ unsigned long long tagged(float v, unsigned int tag) {
+  return (unsigned long long)__float_as_uint(v) | ((unsigned long long)tag << 32);
 }
 
-// Cursor of target t positioned at the group's first source `from` (slice-local).
-__device__ __forceinline__ void cursor_init(Cursor &c, const MinibatchArgs &a, NbList L, int t, int from,
-                                            int sbase) {
-  c.ids = L.ids + t * kNbCap;
-  c.cnt = L.meta[2 * t];
-  c.k0 = L.meta[2 * t + 1];
-  c.ptr = 0;
-  c.next = cursor_at(a, c, sbase);
-  // bounded by the neighbours inside the slice
-  while (c.next < from) {
-    c.ptr++;
-    c.next = cursor_at(a, c, sbase);
-  }
+__device__ __forceinline__ ulonglong2 ld_relaxed_pair(const ulonglong2 *p) {
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
 }
 
-// For each matched neighbour q of the target with ga <= q < gb: remove the
-// repulsion the sweep added (identical FP32 operations) and add the model's
-// attraction -- the reference applies attraction instead of repulsion to
-// these pairs (algorithms.cpp:758-768).
-template <int kRep>
-__device__ __noinline__ void correct_neighbours(const MinibatchArgs &a, Cursor c, int ga, int gb,
-                                                const float2 *slice, float2 pi, int sbase, float &fx, float &fy) {
-  // bounded by the target's neighbours inside the slice
-  for (int q = c.next; q < gb; q = c.next) {
-    if (q >= ga) {
-      const float2 pj = slice[q];
-      const float dx = pj.x - pi.x, dy = pj.y - pi.y;
-      const float d2 = fmaf(dx, dx, fmaf(dy, dy, kTinyD2));
-      const float r = (kRep == REP_UNIT) ? rsqrt_approx(d2) : rcp_approx(d2);
-      fx = fmaf(dx, r, fx);
-      fy = fmaf(dy, r, fy);
-      attract_pair(a.model, (float)a.W, pj.x, pj.y, pi.x, pi.y, fx, fy);
-    }
-    c.ptr++;
-    c.next = cursor_at(a, c, sbase);
-  }
+__device__ __forceinline__ void st_relaxed_pair(ulonglong2 *p, unsigned long long x, unsigned long long y) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
 }
 
-// Slice of sources owned by block s: [lo, hi).
-__device__ __forceinline__ void slice_of(int n, int grid, int s, int &lo, int &hi) {
-  lo = (int)(((long long)n * s) / grid);
-  hi = (int)(((long long)n * (s + 1)) / grid);
-}
+// ---- packed FP32 pairs -----------------------------------------------------------
+//
+// Two sources at a time through the packed FP32 instructions (the same
+// operations per lane as the scalar form; half the issue slots, which leaves
+// room for the reciprocals: 4,307 against 3,788 pairs per ns on 152 SMs with
+// 656 sources and 256 targets each).  Sharing one reciprocal between two
+// pairs was slower (3,209-3,980): the extra products cost more than the
+// shared unit saves.
 
-__device__ double block_sum(double v, double *red) {
-  // fixed-order tree: warp xor-shuffle, then warp 0 over the warp sums
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (w == 0) {
-    t = (l < kWarps) ? red[l] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) red[0] = t;
-  __syncthreads();
-  const double r = red[0];
-  __syncthreads();
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
   return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+template <int kRep>
+__device__ __forceinline__ float rep_scale(float d2) {
+  return kRep == REP_UNIT ? rsqrt_approx(d2) : rcp_approx(d2);
+}
+
+// A target and its packed force sums.
+struct Target {
+  unsigned long long x, y, fx, fy;
+  __device__ __forceinline__ void set(float2 p) {
+    x = pack2(p.x, p.x);
+    y = pack2(p.y, p.y);
+    fx = fy = 0ull;  // two +0
+  }
+  // repulsion of the source pair q = (x0, x1, y0, y1)
+  template <int kRep>
+  __device__ __forceinline__ void pair(float4 q) {
+    const unsigned long long dx = sub2(x, pack2(q.x, q.y)), dy = sub2(y, pack2(q.z, q.w));
+    const unsigned long long d2 = fma2(dx, dx, fma2(dy, dy, pack2(kTinyD2, kTinyD2)));
+    float a, b;
+    unpack2(d2, a, b);
+    const unsigned long long r = pack2(rep_scale<kRep>(a), rep_scale<kRep>(b));
+    fx = fma2(dx, r, fx);
+    fy = fma2(dy, r, fy);
+  }
+  // repulsion of one source
+  template <int kRep>
+  __device__ __forceinline__ void single(float sx, float sy) {
+    float px, py, t, ax, bx, ay, by;
+    unpack2(x, px, t);
+    unpack2(y, py, t);
+    unpack2(fx, ax, bx);
+    unpack2(fy, ay, by);
+    rep_law_pair<kRep>(sx, sy, px, py, ax, ay);
+    fx = pack2(ax, bx);
+    fy = pack2(ay, by);
+  }
+  __device__ __forceinline__ float2 sum() const {
+    float ax, bx, ay, by;
+    unpack2(fx, ax, bx);
+    unpack2(fy, ay, by);
+    return make_float2(ax + bx, ay + by);
+  }
+};
+
+// Points in shared memory, two per float4 (x0, x1, y0, y1).
+__device__ __forceinline__ void put_point(float4 *a, int k, float2 p) {
+  float *f = reinterpret_cast<float *>(a + (k >> 1)) + (k & 1);
+  f[0] = p.x;
+  f[2] = p.y;
+}
+__device__ __forceinline__ float2 get_point(const float4 *a, int k) {
+  const float *f = reinterpret_cast<const float *>(a + (k >> 1)) + (k & 1);
+  return make_float2(f[0], f[2]);
+}
+
+// Targets of a batch that one mover moves (even, so that pairs of partials
+// load as float4).
+__host__ __device__ __forceinline__ int mover_share(int batch, int movers) {
+  return 2 * ((batch + 2 * movers - 1) / (2 * movers));
+}
+
+// Sources of sweeper s: [lo, hi), lo even.
+__device__ __forceinline__ void slice_of(int n, int sweepers, int s, int &lo, int &hi) {
+  const long long half = (n + 1) / 2;
+  lo = 2 * (int)(half * s / sweepers);
+  hi = min(n, 2 * (int)(half * (s + 1) / sweepers));
+}
+
+// ---- sweeper -----------------------------------------------------------------------
+
+// Slice-local sources [a, b) on two targets.
+template <int kRep>
+__device__ __forceinline__ void sweep_range(const float4 *slice, int a, int b, Target &t0, Target &t1) {
+  if (a >= b) return;
+  if (a & 1) {
+    const float2 q = get_point(slice, a);
+    t0.single<kRep>(q.x, q.y);
+    t1.single<kRep>(q.x, q.y);
+    a++;
+  }
+  const int p1 = b >> 1;
+#pragma unroll 4
+  for (int p = a >> 1; p < p1; p++) {
+    const float4 q = slice[p];
+    t0.pair<kRep>(q);
+    t1.pair<kRep>(q);
+  }
+  if ((b & 1) && a < b) {
+    const float2 q = get_point(slice, b - 1);
+    t0.single<kRep>(q.x, q.y);
+    t1.single<kRep>(q.x, q.y);
+  }
+}
+
+// Part g of kGroups of [a, b), cut at even sources.
+__device__ __forceinline__ int cut(int a, int b, int g) {
+  if (g == 0) return a;
+  if (g == kGroups) return b;
+  return max(a, (a + (int)((long long)(b - a) * g / kGroups)) & ~1);
+}
+
+template <int kRep>
+__device__ __forceinline__ void sweeper(const MinibatchArgs &a, unsigned char *smem) {
+  const int s = (int)blockIdx.x - a.movers;
+  int slo, shi;
+  slice_of(a.n, a.sweepers, s, slo, shi);
+  const int len = shi - slo;
+  float4 *slice = reinterpret_cast<float4 *>(smem);
+  const int tid = threadIdx.x % kTeam, team = threadIdx.x / kTeam;
+  float2 *gsum = reinterpret_cast<float2 *>(slice + (len + 1) / 2) + team * kGroups * kChunk;
+  __shared__ int s_go[2];
+  const int grp = tid / kGroup, gl = tid % kGroup;
+#pragma unroll 1
+  for (int k = threadIdx.x; k < len; k += kThreads) put_point(slice, k, __ldcg(&a.pos[slo + k]));
+  __syncthreads();
+  const int nb = a.nbatches, B = a.batch, slots = a.lag + 1, stride = (B + 1) & ~1;
+  const unsigned int M = (unsigned int)a.movers;
+  long long left = (a.converged ? LLONG_MAX : (long long)a.iterations * nb) - team;
+  // next batch whose new positions this team takes over into the slice
+  // (batch numbers modulo 2^32)
+  unsigned int fresh = 0;
+  int fresh_b = 0;
+  int b = team % nb, slot = team % slots;
+  // the first targets of the team's next batch are loaded ahead when they
+  // cannot move before the current one is done
+  const bool ahead = nb >= a.lag + 3;
+  float2 p0 = make_float2(0.f, 0.f), p1 = p0;
+  bool have = false;
+  bool started = false;  // a batch has to have moved
+  for (unsigned int q = (unsigned int)team; left > 0; q += 2, left -= 2) {
+    const unsigned int need = q - (unsigned int)a.lag;  // batches that have moved
+    started = started || (int)need > 0;
+    if (tid == 0) {
+      int go = 1;
+      const unsigned int target = need * M;
+      if (started) {
+        Poll w;
+#pragma unroll 1
+        while (!reached(ld_acquire_gpu(&a.ctl->moved), target)) {
+          if ((a.converged && ld_volatile_u32(&a.ctl->stop) != 0u) || !w.again(a.st)) {
+            go = 0;
+            break;
+          }
+        }
+      }
+      s_go[team] = go;
+    }
+    bar_sync(1 + team, kTeam);
+    if (!s_go[team]) return;
+    // the batches up to q - lag - 1 have moved: their new positions into the slice
+    bool changed = false;
+#pragma unroll 1
+    for (; started && fresh != need; fresh++) {
+      const int lo = fresh_b * B;
+      const int f0 = max(slo, lo), f1 = min(shi, min(a.n, lo + B));
+#pragma unroll 1
+      for (int i = f0 + tid; i < f1; i += kTeam) put_point(slice, i - slo, __ldcg(&a.pos[i]));
+      changed |= f0 < f1;
+      if (++fresh_b == nb) fresh_b = 0;
+    }
+    const int base = b * B, cnt = min(B, a.n - base);
+    if (!have) {
+      p0 = gl < cnt ? __ldcg(&a.pos[base + gl]) : make_float2(0.f, 0.f);
+      p1 = gl + kGroup < cnt ? __ldcg(&a.pos[base + gl + kGroup]) : make_float2(0.f, 0.f);
+    }
+    if (changed) bar_sync(1 + team, kTeam);
+    // this team's next batch
+    int nxt = b + 2;
+    while (nxt >= nb) nxt -= nb;
+    // allowed sources: all but batches b - lag .. b - 1 (cyclically)
+    const int e = b - a.lag;
+    int a0, a1, c0 = 0, c1 = 0;
+    if (e >= 0) {
+      a0 = 0;
+      a1 = min(len, e * B - slo);
+      c0 = max(0, base - slo);
+      c1 = len;
+      if (a.lag == 0) {
+        a1 = len;
+        c0 = len;
+      }
+    } else {
+      a0 = max(0, base - slo);
+      a1 = min(len, (nb + e) * B - slo);
+    }
+    const int ga0 = cut(a0, max(a0, a1), grp), ga1 = cut(a0, max(a0, a1), grp + 1);
+    const int gc0 = cut(c0, max(c0, c1), grp), gc1 = cut(c0, max(c0, c1), grp + 1);
+    float2 *out = a.part + ((size_t)slot * a.sweepers + s) * stride;
+    for (int t0 = 0; t0 < cnt; t0 += kChunk) {
+      Target u, v;
+      u.set(p0);
+      v.set(p1);
+      // the next targets: of this batch, else of the team's next one
+      {
+        const bool more = t0 + kChunk < cnt;
+        const int nbase = more ? base + t0 + kChunk : nxt * B;
+        const int ncnt = more ? cnt - t0 - kChunk : min(B, a.n - nbase);
+        if (more || ahead) {
+          if (gl < ncnt) p0 = __ldcg(&a.pos[nbase + gl]);
+          if (gl + kGroup < ncnt) p1 = __ldcg(&a.pos[nbase + gl + kGroup]);
+        }
+      }
+      sweep_range<kRep>(slice, ga0, ga1, u, v);
+      sweep_range<kRep>(slice, gc0, gc1, u, v);
+      if (t0 > 0) bar_sync(1 + team, kTeam);  // gsum of the chunk before is read
+      gsum[grp * kChunk + gl] = u.sum();
+      gsum[grp * kChunk + gl + kGroup] = v.sum();
+      bar_sync(1 + team, kTeam);
+      if (tid < kChunk && t0 + tid < cnt) {
+        float2 f = gsum[tid];
+#pragma unroll
+        for (int g = 1; g < kGroups; g++) {
+          const float2 w = gsum[g * kChunk + tid];
+          f.x += w.x;
+          f.y += w.y;
+        }
+        __stcg(&out[t0 + tid], f);
+      }
+    }
+    have = ahead;
+    bar_sync(1 + team, kTeam);
+    if (tid == 0) {
+      __threadfence();
+      red_add(&a.ctl->arrive[slot], 1u);
+    }
+    b = nxt;
+    slot += 2;
+    while (slot >= slots) slot -= slots;
+  }
+}
+
+// ---- mover --------------------------------------------------------------------------
+
+// The model's attraction of neighbour pj on pi with the pair's repulsion (the
+// same FP32 operations) taken back (algorithms.cpp:758-768).
+template <int kRep>
+__device__ __forceinline__ float2 neighbour_force(int model, float W, float2 pj, float2 pi) {
+  const float dx = pj.x - pi.x, dy = pj.y - pi.y;
+  const float r = rep_scale<kRep>(fmaf(dx, dx, fmaf(dy, dy, kTinyD2)));
+  float fx = dx * r, fy = dy * r;
+  attract_pair(model, W, pj.x, pj.y, pi.x, pi.y, fx, fy);
+  return make_float2(fx, fy);
+}
+
+// Float-float sums of (x, y) in packed form.
+struct Sum2 {
+  unsigned long long hi, lo;
+  __device__ __forceinline__ void add(unsigned long long t) {  // Knuth's TwoSum, as ff_add
+    const unsigned long long sum = add2(hi, t);
+    const unsigned long long bb = sub2(sum, hi);
+    const unsigned long long err = add2(sub2(hi, sub2(sum, bb)), sub2(t, bb));
+    hi = sum;
+    lo = add2(lo, err);
+  }
+  __device__ __forceinline__ void add(float x, float y) { add(pack2(x, y)); }
+};
+
+struct MoverSmem {
+  float4 *ring;        // [lag + 1][pairs]: positions of the last batches, slot = q % (lag + 1)
+  ulonglong2 *rows;    // [2, 1 when late][chunks][kRows][kMoveTile]: N's and P's sums, float-float
+  float4 *moved;       // [2][share]: the forces of the share {hi x, hi y, lo x, lo y}
+  float2 *tile;        // [tiles][stride]: positions of batches q .. q + 2 (q + 1 when late) before they move
+  int *near;           // [2][share][kNear]: neighbours in the batch before (unless late)
+  unsigned int *mask;  // [2][share]: which of them are set
+  int pairs, stride, share, chunks, tiles;
+};
+
+constexpr int kBarC = 1, kBarRing = 2, kBarEarly = 4, kBarPub = 6;
+constexpr int kCThreads = kCWarps * 32;
+constexpr int kEarlyThreads = kCThreads + (kNWarps + kPWarps) * 32;  // C with N and P
+
+struct MoverFlags {
+  volatile int fail;           // a wait ran out or a force left the range
+  volatile unsigned int end;   // batches from this one on do not exist (0: not known yet)
+  volatile unsigned int seen;  // batches whose partials all sweepers have stored
+  volatile int last[2];        // by parity of the batch: 1 no batch follows, 2 not even this one
+  volatile double step;
+  volatile float stepf;
+  volatile double energy;  // of the iteration before
+  volatile int settled;    // converged runs: the energy changed by no more than engt
+  volatile long long loop;  // iterations finished
+  volatile int last_loop;   // this iteration is the last one
+  double e_lane[32];       // this iteration's energy so far, per lane of the warp that adds it up
+};
+
+__device__ __forceinline__ ulonglong2 *rows_of(const MinibatchArgs &a, const MoverSmem &S, int par, int ch) {
+  return S.rows + ((a.late ? 0 : par * S.chunks) + ch) * (kRows * kMoveTile);
+}
+
+// The critical team's signal that batch q - 2 (q - 1 when late) is in the
+// ring, which also means that the sums of that batch are used up; false: there
+// is no batch q.
+__device__ __forceinline__ bool ring_ready(const MinibatchArgs &a, MoverFlags &F, int par, bool first) {
+  if (a.late) {
+    bar_sync(kBarRing + par, kEarlyThreads);
+  } else if (!first) {
+    bar_sync(kBarRing + (par ^ 1), kEarlyThreads);
+    return F.last[par ^ 1] == 0;
+  }
+  return true;
+}
+
+// One warp: announces in shared memory which batches' partials are complete,
+// a round trip ahead of the team that reads them.
+__device__ __forceinline__ void mover_watch(const MinibatchArgs &a, MoverFlags &F) {
+  if ((threadIdx.x & 31) != 0) return;
+  unsigned int q = 0, round = 1;
+  for (int slot = 0;; q++) {
+    Poll p;
+#pragma unroll 1
+    while (!reached(ld_acquire_gpu(&a.ctl->arrive[slot]), round * (unsigned int)a.sweepers)) {
+      const unsigned int end = F.end;
+      if ((end != 0u && reached(q, end)) || F.fail) return;
+      if (!p.again(a.st)) {
+        F.fail = 1;
+        return;
+      }
+    }
+    __threadfence_block();
+    F.seen = q + 1u;
+    if (++slot > a.lag) {
+      slot = 0;
+      round++;
+    }
+  }
+}
+
+// Team P: the sweepers' partials of the share, and the positions of batch
+// q + 2 (q + 1 when late) before it moves: N starts on a batch when the
+// critical team has finished the second (first) batch before it.
+__device__ __forceinline__ void mover_partials(const MinibatchArgs &a, const MoverSmem &S, MoverFlags &F, int m) {
+  const int pt = (int)threadIdx.x - (kCWarps + kNWarps + 1) * 32, w = pt >> 5, lane = pt & 31;
+  const int nb = a.nbatches, B = a.batch, slots = a.lag + 1;
+  const bool closed = nb == slots;  // every batch is in the ring
+  const int t0 = m * S.share;
+  int b = 0, slot = 0, tslot = 0, par = 0;
+  unsigned int q = 0;
+  for (bool first = true;; first = false) {
+    const int cnt = min(B, a.n - b * B), t1 = min(cnt, t0 + S.share);
+    int fb = b + S.tiles / 2;
+    if (fb >= nb) fb -= nb;
+    const int nbase = fb * B, ncnt = min(B, a.n - nbase);
+    if (lane == 0) {  // the watching warp bounds this wait
+#pragma unroll 1
+      while (!reached(F.seen, q + 1u)) {
+        const unsigned int end = F.end;
+        if ((end != 0u && reached(q, end)) || F.fail) break;
+      }
+    }
+    __syncwarp();
+    __threadfence_block();
+#pragma unroll 1
+    for (int ch = 0; ch < S.chunks; ch++) {
+      // lane: targets 2 (lane % 16) and the next of sweepers 2 w + lane / 16 + 16 k
+      const int t = t0 + ch * kMoveTile + 2 * (lane & 15);
+      const float2 *col = a.part + (size_t)slot * a.sweepers * S.stride + t;
+      float2 nt[2];
+      if (ch == 0) {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          const int x = pt + k * kPWarps * 32;
+          nt[k] = x < ncnt && !closed ? __ldcg(&a.pos[nbase + x]) : make_float2(0.f, 0.f);
+        }
+      }
+      Sum2 f0 = {0ull, 0ull}, f1 = {0ull, 0ull};
+#pragma unroll 1
+      for (int s0 = w * 2 + (lane >> 4); s0 < a.sweepers; s0 += 2 * kPWarps * kPartLoads) {
+        float4 v[kPartLoads];
+#pragma unroll
+        for (int k = 0; k < kPartLoads; k++) {
+          v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (t < t1 && s0 + 2 * kPWarps * k < a.sweepers)
+            v[k] = __ldcg(reinterpret_cast<const float4 *>(&col[(size_t)(s0 + 2 * kPWarps * k) * S.stride]));
+        }
+#pragma unroll
+        for (int k = 0; k < kPartLoads; k++) {
+          f0.add(v[k].x, v[k].y);
+          f1.add(v[k].z, v[k].w);
+        }
+      }
+      __syncwarp();
+      // the other half-warp's sweepers: lanes 0-15 keep the first target, 16-31 the second
+      const bool up = lane & 16;
+      Sum2 keep = up ? f1 : f0;
+      const unsigned long long gh = __shfl_xor_sync(0xffffffffu, up ? f0.hi : f1.hi, 16);
+      const unsigned long long gl = __shfl_xor_sync(0xffffffffu, up ? f0.lo : f1.lo, 16);
+      keep.add(gh);
+      keep.lo = add2(keep.lo, gl);
+      if (ch == 0) {
+        if (!ring_ready(a, F, par, first)) return;
+        if (!closed) {
+          float2 *dst = S.tile + ((tslot + S.tiles / 2) & (S.tiles - 1)) * S.stride;
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            const int x = pt + k * kPWarps * 32;
+            if (x < ncnt) dst[x] = nt[k];
+          }
+#pragma unroll 1
+          for (int x = pt + 2 * kPWarps * 32; x < ncnt; x += kPWarps * 32) dst[x] = __ldcg(&a.pos[nbase + x]);
+        }
+      }
+      rows_of(a, S, par, ch)[(kNWarps + 1 + w) * kMoveTile + 2 * (lane & 15) + (lane >> 4)] =
+          make_ulonglong2(keep.hi, keep.lo);
+    }
+    bar_arrive(kBarEarly + par, kEarlyThreads);
+    if (a.late && F.last[par]) return;
+    q++;
+    if (++b == nb) b = 0;
+    par ^= 1;
+    if (++slot == slots) slot = 0;
+    tslot = (tslot + 1) & (S.tiles - 1);
+  }
+}
+
+// Team N: the neighbour corrections of the share, those in batch q - 1 staged
+// for the critical team (unless late: the ring holds it then).  What
+// it reads from global memory moved before batch q - lag - 1, which the
+// sweepers saw before they stored the partials of batch q - 1: it waits for
+// the watching warp to have seen those (long since).
+template <int kRep>
+__device__ __forceinline__ void mover_neighbours(const MinibatchArgs &a, const MoverSmem &S, MoverFlags &F, int m) {
+  const int w = (int)(threadIdx.x >> 5) - kCWarps, lane = threadIdx.x & 31;
+  const int nb = a.nbatches, B = a.batch, slots = a.lag + 1;
+  const bool closed = nb == slots;
+  const float W = a.W, inv_b = 1.0f / (float)B;
+  const int t0 = m * S.share;
+  int b = 0, slot = 0, tslot = 0, par = 0;
+  // the next batch's row of this thread's first target
+  int r0 = 0, r1 = 0;
+  if (t0 + lane < min(min(B, a.n), t0 + S.share)) {
+    r0 = __ldg(&a.eff_rowptr[t0 + lane]);
+    r1 = __ldg(&a.eff_rowptr[t0 + lane + 1]);
+  }
+  unsigned int q = 0;
+  for (bool first = true;; first = false, q++) {
+    const int base = b * B, cnt = min(B, a.n - base);
+    const int t1 = min(cnt, t0 + S.share);
+    const int nbb = b + 1 == nb ? 0 : b + 1;
+    const int nbase = nbb * B, ncnt = min(B, a.n - nbase);
+    // batches q - slots .. q (cyclically) start at these ids
+    const int w0 = (b - slots) * B, w1 = (nb + b - slots) * B;
+#pragma unroll 1
+    for (int ch = 0; ch < S.chunks; ch++) {
+      const int t = t0 + ch * kMoveTile + lane;
+      const bool valid = t < t1;
+      if (ch > 0 && valid) {
+        r0 = __ldg(&a.eff_rowptr[base + t]);
+        r1 = __ldg(&a.eff_rowptr[base + t + 1]);
+      }
+      int e = r0 + w;
+      int j0 = valid && e < r1 ? __ldg(&a.eff_colids[e]) : -1;
+      if (ch == 0) {
+        if (!ring_ready(a, F, par, first)) return;
+        if (lane == 0)
+#pragma unroll 1
+          while (!reached(F.seen, q) && !F.fail) {
+          }
+        __syncwarp();
+        __threadfence_block();
+      }
+      auto target_at = [&](int x) {
+        return closed ? get_point(S.ring + slot * S.pairs, x) : S.tile[tslot * S.stride + x];
+      };
+      const float2 p = valid ? target_at(t) : make_float2(0.f, 0.f);
+      Sum2 f = {0ull, 0ull};
+#pragma unroll 1
+      while (j0 >= 0) {
+        const int e1 = e + kNWarps;
+        const int j1 = e1 < r1 ? __ldg(&a.eff_colids[e1]) : -1;
+        // batch q - d holds j0 as its vertex jt; d > slots: further back
+        int d = slots + 1, jt = 0;
+        int rel = j0 - w0;
+        if (rel < 0 || rel >= (slots + 1) * B) rel = b < slots ? j0 - w1 : -1;
+        if (rel >= 0) {
+          const int k = (int)(((float)rel + 0.5f) * inv_b);  // exact: rel < 2^16
+          d = slots - k;
+          jt = rel - k * B;
+        }
+        if (d == 1 && !a.late) {  // the batch before: the critical team's
+          const int x = (e - r0) & (kNear - 1), t2 = par * S.share + (t - t0);
+          S.near[t2 * kNear + x] = jt;
+          const unsigned int old = atomicOr(&S.mask[t2], 1u << x);
+          if ((old >> x) & 1u) atomicOr(&S.mask[t2], kNearMore);
+        } else {
+          float2 pj;
+          if (d > slots) {
+            pj = __ldcg(&a.pos[j0]);
+          } else if (d == 0) {
+            pj = target_at(jt);
+          } else {
+            int ss = slot - d;
+            if (ss < 0) ss += slots;
+            pj = get_point(S.ring + ss * S.pairs, jt);
+          }
+          const float2 v = neighbour_force<kRep>(a.model, W, pj, p);
+          f.add(v.x, v.y);
+        }
+        j0 = j1;
+        e = e1;
+      }
+      if (ch + 1 == S.chunks) {  // the next batch's row
+        const bool more = t0 + lane < min(ncnt, t0 + S.share);
+        r0 = more ? __ldg(&a.eff_rowptr[nbase + t0 + lane]) : 0;
+        r1 = more ? __ldg(&a.eff_rowptr[nbase + t0 + lane + 1]) : 0;
+      }
+      rows_of(a, S, par, ch)[w * kMoveTile + lane] = make_ulonglong2(f.hi, f.lo);
+    }
+    bar_arrive(kBarEarly + par, kEarlyThreads);
+    if (a.late && F.last[par]) return;
+    b = nbb;
+    par ^= 1;
+    if (++slot == slots) slot = 0;
+    tslot = (tslot + 1) & (S.tiles - 1);
+  }
+}
+
+// A half-warp's sum over the neighbours of vertex i in the batch at `pbase`
+// when there are more than were staged: the row again.
+template <int kRep>
+__device__ __noinline__ float2 near_row(const MinibatchArgs &a, const float4 *prev, int pbase, int i, float2 pi) {
+  const int r1 = __ldg(&a.eff_rowptr[i + 1]), pcnt = min(a.batch, a.n - pbase);
+  float2 f = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int e = __ldg(&a.eff_rowptr[i]) + ((int)threadIdx.x & 15); e < r1; e += 16) {
+    const int jt = __ldg(&a.eff_colids[e]) - pbase;
+    if (jt < 0 || jt >= pcnt) continue;
+    const float2 g = neighbour_force<kRep>(a.model, a.W, get_point(prev, jt), pi);
+    f.x += g.x;
+    f.y += g.y;
+  }
+  return f;
+}
+
+// The step when |f|^2 is outside the FP32 range.
+__device__ __noinline__ float2 step_fp64(float2 p, float hx, float hy, float lx, float ly, double step) {
+  const double dx = (double)hx + (double)lx, dy = (double)hy + (double)ly;
+  const double mag = sqrt(dx * dx + dy * dy);
+  return make_float2((float)((double)p.x + (dx / mag) * step), (float)((double)p.y + (dy / mag) * step));
+}
+
+// One thread's part of the movers' energy exchange: publishes this mover's
+// energy of iteration `loop` and, when asked, adds up all of them in order.
+__device__ __noinline__ double exchange_energy(const MinibatchArgs &a, MoverFlags &F, int m, long long loop, double v,
+                                               bool total) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+  const unsigned long long tag = (unsigned long long)(unsigned int)(loop + 1);
+  ulonglong2 *ce = a.ctl->energy[loop & 1];
+  st_relaxed_pair(&ce[m], (bits & 0xffffffffull) | (tag << 32), (bits >> 32) | (tag << 32));
+  double tot = 0.0;
+#pragma unroll 1
+  for (int k = 0; total && k < a.movers; k++) {
+    Poll p;
+    ulonglong2 x = ld_relaxed_pair(&ce[k]);
+#pragma unroll 1
+    while ((x.x >> 32) != tag || (x.y >> 32) != tag) {
+      if (!p.again(a.st)) {
+        F.fail = 1;
+        break;
+      }
+      x = ld_relaxed_pair(&ce[k]);
+    }
+    tot += __longlong_as_double((long long)((x.x & 0xffffffffull) | (x.y << 32)));
+  }
+  return tot;
+}
+
+// The FP64 forces and |f|^2 of a mover's share (one warp) and, at the end of
+// an iteration, its energy: lanes in a fixed tree, movers in order.
+__device__ __noinline__ void mover_outputs(const MinibatchArgs &a, const MoverSmem &S, MoverFlags &F, int m, int par,
+                                           int base, int count, bool iteration_end) {
+  const int lane = threadIdx.x & 31, t0 = m * S.share;
+  double e_sum = F.e_lane[lane];
+#pragma unroll 1
+  for (int t = lane; t < count; t += 32) {
+    const float4 f = S.moved[par * S.share + t];
+    const double dx = (double)f.x + (double)f.z, dy = (double)f.y + (double)f.w;
+    const double e = dx * dx + dy * dy;
+    a.force[base + t0 + t] = make_double2(dx, dy);
+    a.e[base + t0 + t] = e;
+    e_sum += e;
+  }
+  if (iteration_end) {
+    for (int o = 16; o > 0; o >>= 1) e_sum += __shfl_xor_sync(0xffffffffu, e_sum, o);
+    if (lane == 0) {
+      const double tot = exchange_energy(a, F, m, F.loop, e_sum, a.converged || m == 0);
+      if (m == 0) a.energy[0] = tot;
+      F.settled = !(fabs(F.energy - tot) / F.energy > a.engt) ? 1 : 0;
+      F.energy = tot;
+    }
+    e_sum = 0.0;
+  }
+  F.e_lane[lane] = e_sum;
+}
+
+// Critical team: the pairs with the last batches, the move, its publication.
+// While the batch before is on its way from the other movers, the team adds
+// the pairs with the older ones.  The last warp also announces the moved
+// batch to the sweepers and turns the share's forces into the FP64 outputs,
+// in full warps (the FP64 pipe is charged by the warp instruction), off the
+// other warps' path.
+template <int kRep>
+__device__ __forceinline__ void mover_critical(const MinibatchArgs &a, const MoverSmem &S, MoverFlags &F, int m) {
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int nb = a.nbatches, B = a.batch, slots = a.lag + 1;
+  const bool closed = nb == slots;
+  const int t0 = m * S.share;
+  bool stop = false, started = false;
+  int b = 0, slot = 0, tslot = 0;
+  for (unsigned int q = 0;; q++) {
+    const int par = (int)(q & 1);
+    const int base = b * B;
+    const int t1 = min(min(B, a.n - base), t0 + S.share);
+    int last = 0;
+#pragma unroll 1
+    for (int ch = 0; ch < S.chunks; ch++) {
+      const int ta = t0 + ch * kMoveTile + 2 * w;
+      auto target_at = [&](int t) {
+        return t >= t1 ? make_float2(0.f, 0.f)
+                       : closed ? get_point(S.ring + slot * S.pairs, t) : S.tile[tslot * S.stride + t];
+      };
+      Target u, v;  // (without a lag no pair is added)
+      u.set(target_at(ta));
+      v.set(target_at(ta + 1));
+#pragma unroll 1
+      for (int d = max(a.lag, 1); d >= 1; d--) {  // batch q - d
+        int sb = b - d, ss = slot - d;
+        if (sb < 0) sb += nb;
+        if (ss < 0) ss += slots;
+        float4 *src = S.ring + ss * S.pairs;
+        const int scnt = min(B, a.n - sb * B);
+        if (d == 1 && ch == 0) {
+          // the batch before, from the other movers into the ring
+          if (started && !stop) {
+            const ulonglong2 *ex = a.exchange + (size_t)((q - 1) & (kExchange - 1)) * B;
+#pragma unroll 1
+            for (int t = tid; t < scnt; t += kCThreads) {
+              Poll p;
+              ulonglong2 x = ld_relaxed_pair(&ex[t]);
+#pragma unroll 1
+              while ((unsigned int)(x.x >> 32) != q || (unsigned int)(x.y >> 32) != q) {
+                if (!p.again(a.st)) {
+                  F.fail = 1;
+                  break;
+                }
+                x = ld_relaxed_pair(&ex[t]);
+              }
+              put_point(src, t, make_float2(__uint_as_float((unsigned int)x.x), __uint_as_float((unsigned int)x.y)));
+            }
+          }
+          if (tid == kCThreads - 1) {
+            if (!started && !wait_count(&a.ctl->ready, (unsigned int)a.movers, a.st)) F.fail = 1;
+            const int l = (stop || F.fail) ? 2 : (F.last_loop && b == nb - 1) ? 1 : 0;
+            F.last[par] = l;
+            if (l) F.end = q + 1u;
+          }
+          bar_sync(kBarC, kCThreads);
+          last = F.last[par];
+          bar_arrive(kBarRing + par, kEarlyThreads);
+          if (last == 2) {  // the early teams finish the batch they are in
+            bar_sync(kBarEarly + par, kEarlyThreads);
+            return;
+          }
+        }
+        if (a.lag >= 1 && ta < t1) {
+          // one source pair a lane, the warp's two targets
+#pragma unroll 4
+          for (int k = lane; k < (scnt >> 1); k += 32) {
+            const float4 x = src[k];
+            u.pair<kRep>(x);
+            v.pair<kRep>(x);
+          }
+          if ((scnt & 1) && lane == 0) {
+            const float2 x = get_point(src, scnt - 1);
+            u.single<kRep>(x.x, x.y);
+            v.single<kRep>(x.x, x.y);
+          }
+        }
+      }
+      if (ch == 0) bar_sync(kBarEarly + par, kEarlyThreads);
+      if (ta >= t1) continue;  // a small share leaves warps without targets
+      // lanes 0-15 go on with the first target, 16-31 with the second
+      const int up = lane >> 4, t = ta + up;
+      const float2 pi = target_at(t);
+      float fx, fy;
+      {
+        const float2 fu = u.sum(), fv = v.sum();
+        fx = (up ? fv.x : fu.x) + __shfl_xor_sync(0xffffffffu, up ? fu.x : fv.x, 16);
+        fy = (up ? fv.y : fu.y) + __shfl_xor_sync(0xffffffffu, up ? fu.y : fv.y, 16);
+      }
+      // neighbours in the batch before
+      if (!a.late) {
+        const int x = par * S.share + (t - t0);
+        const unsigned int mask = t < t1 ? S.mask[x] : 0u;
+        if (__any_sync(0xffffffffu, mask != 0u)) {
+          const float4 *prev = S.ring + (slot == 0 ? slots - 1 : slot - 1) * S.pairs;
+          const int pbase = b == 0 ? (nb - 1) * B : base - B;
+          if (mask & kNearMore) {
+            const float2 g = near_row<kRep>(a, prev, pbase, base + t, pi);
+            fx += g.x;
+            fy += g.y;
+          } else if ((mask >> (lane & 15)) & 1u) {
+            const float2 g = neighbour_force<kRep>(a.model, a.W, get_point(prev, S.near[x * kNear + (lane & 15)]), pi);
+            fx += g.x;
+            fy += g.y;
+          }
+          __syncwarp();
+          if ((lane & 15) == 0 && mask != 0u) S.mask[x] = 0u;  // for batch q + 2
+        }
+      }
+      // with N's and P's sums (a row per lane), a fixed tree over the 16 lanes
+      Sum2 s;
+      {
+        const ulonglong2 row = rows_of(a, S, par, ch)[(lane & 15) * kMoveTile + 2 * w + up];
+        s.hi = row.x;
+        s.lo = row.y;
+      }
+      s.add(fx, fy);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        const unsigned long long h = __shfl_down_sync(0xffffffffu, s.hi, o, 16);
+        const unsigned long long l = __shfl_down_sync(0xffffffffu, s.lo, o, 16);
+        s.add(h);
+        s.lo = add2(s.lo, l);
+      }
+      if ((lane & 15) == 0 && t < t1) {
+        float hx, hy, lx, ly;
+        unpack2(s.hi, hx, hy);
+        unpack2(s.lo, lx, ly);
+        fx = hx + lx;
+        fy = hy + ly;
+        float2 np = pi;
+        const float m2 = fmaf(fx, fx, fy * fy);
+        if (m2 >= 1.17549435e-38f && m2 <= 3.0e38f) {
+          const float rm = rsqrt_approx(m2), stepf = F.stepf;
+          np.x = fmaf(stepf, fx * rm, pi.x);
+          np.y = fmaf(stepf, fy * rm, pi.y);
+        } else if (fx != 0.f || fy != 0.f) {
+          np = step_fp64(pi, hx, hy, lx, ly, F.step);
+        }
+        st_relaxed_pair(&a.exchange[(size_t)(q & (kExchange - 1)) * B + t], tagged(np.x, q + 1u), tagged(np.y, q + 1u));
+        __stcg(&a.pos[base + t], np);
+        if (!(fabsf(fx) < kForceLimit) || !(fabsf(fy) < kForceLimit)) {
+          dev_record_error(a.st, DEV_FORCE_RANGE);
+          F.fail = 1;
+        }
+        S.moved[par * S.share + (t - t0)] = make_float4(hx, hy, lx, ly);
+      }
+    }
+    // the last warp learns that the share is stored
+    if (w < kCWarps - 1) {
+      bar_arrive(kBarPub, kCThreads);
+    } else {
+      bar_sync(kBarPub, kCThreads);
+      if (lane == 0) {
+        __threadfence();
+        red_add(&a.ctl->moved, 1u);
+      }
+      if (a.converged || F.last_loop) mover_outputs(a, S, F, m, par, base, t1 - t0, b == nb - 1);
+    }
+    if (b == nb - 1) {  // end of an iteration
+      bar_sync(kBarC, kCThreads);
+      const long long loop = F.loop + 1;
+      if (a.converged && (F.settled || loop >= a.max_loops)) {
+        stop = true;
+        F.end = q + 1u;
+        if (m == 0 && tid == 0) atomicExch(&a.ctl->stop, 1u);
+      }
+      bar_sync(kBarC, kCThreads);
+      if (tid == kCThreads - 1) {
+        F.loop = loop;
+        F.last_loop = !a.converged && loop == a.iterations - 1;
+        F.step = F.step * a.decay;
+        F.stepf = (float)F.step;
+        if (m == 0) *a.loops = loop;
+      }
+    }
+    if (last) return;
+    started = true;
+    if (++b == nb) b = 0;
+    if (++slot == slots) slot = 0;
+    tslot = (tslot + 1) & (S.tiles - 1);
+  }
+}
+
+template <int kRep>
+__device__ __forceinline__ void mover(const MinibatchArgs &a, unsigned char *smem) {
+  __shared__ MoverFlags F;
+  __shared__ MoverSmem S;
+  const int m = (int)blockIdx.x, B = a.batch, slots = a.lag + 1, nb = a.nbatches;
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    S.pairs = (B + 1) / 2;
+    S.stride = 2 * S.pairs;
+    S.share = mover_share(B, a.movers);
+    S.chunks = (S.share + kMoveTile - 1) / kMoveTile;
+    S.tiles = a.late ? 2 : 4;
+    S.ring = reinterpret_cast<float4 *>(smem);
+    S.rows = reinterpret_cast<ulonglong2 *>(S.ring + slots * S.pairs);
+    S.moved = reinterpret_cast<float4 *>(S.rows + (a.late ? 1 : 2) * S.chunks * kRows * kMoveTile);
+    S.tile = reinterpret_cast<float2 *>(S.moved + 2 * S.share);
+    S.mask = reinterpret_cast<unsigned int *>(S.tile + S.tiles * S.stride);
+    S.near = reinterpret_cast<int *>(S.mask + 2 * S.share);
+    F.fail = 0;
+    F.end = 0;
+    F.seen = 0;
+    F.last[0] = F.last[1] = 0;
+    F.step = a.step0;
+    F.stepf = (float)a.step0;
+    F.energy = 0.0;
+    F.settled = 0;
+    F.loop = 0;
+    F.last_loop = !a.converged && a.iterations == 1;
+  }
+  if (tid < 32) F.e_lane[tid] = 0.0;
+  __syncthreads();
+  // batches -1 .. -slots (the run's first batch has them before it), the first targets
+#pragma unroll 1
+  for (int d = 1; d <= slots; d++) {
+    const int sb = nb - d;
+    const int cnt = min(B, a.n - sb * B);
+#pragma unroll 1
+    for (int t = tid; t < cnt; t += kThreads) put_point(S.ring + (slots - d) * S.pairs, t, __ldcg(&a.pos[sb * B + t]));
+  }
+  if (nb > slots)  // else every batch is in the ring
+#pragma unroll 1
+    for (int k = 0; k < S.tiles / 2; k++)
+#pragma unroll 1
+      for (int t = tid; t < min(B, a.n - k * B); t += kThreads) S.tile[k * S.stride + t] = __ldcg(&a.pos[k * B + t]);
+#pragma unroll 1
+  for (int t = tid; t < 2 * S.share; t += kThreads) S.mask[t] = 0u;
+#pragma unroll 1
+  for (int k = tid; k < (a.late ? 1 : 2) * S.chunks * kMoveTile; k += kThreads)
+    S.rows[(k / kMoveTile * kRows + kNWarps) * kMoveTile + k % kMoveTile] = make_ulonglong2(0ull, 0ull);
+  __syncthreads();
+  // no mover moves a vertex before every mover has its first positions
+  if (tid == 0) red_add(&a.ctl->ready, 1u);
+  if (tid < kCThreads) mover_critical<kRep>(a, S, F, m);
+  else if (tid < kCThreads + kNWarps * 32) mover_neighbours<kRep>(a, S, F, m);
+  else if (tid < kCThreads + (kNWarps + 1) * 32) mover_watch(a, F);
+  else mover_partials(a, S, F, m);
 }
 
 template <int kRep>
 __global__ void __launch_bounds__(kThreads, 1) minibatch_kernel(MinibatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int s = blockIdx.x;
-  int slo, shi;
-  slice_of(a.n, a.grid, s, slo, shi);
-  const int sbase = slo & ~1;  // even so that pairs of sources load as float4
-  const int slen = shi - sbase;
-  float2 *slice = reinterpret_cast<float2 *>(smem_raw);
-  const int slen_pad = (slen + 3) & ~3;
-  float2 *gsum = slice + slen_pad;              // [kGroups-1][kChunk]
-  float2 *tbuf = gsum + (kGroups - 1) * kChunk;  // [2][batch]: targets of this and the next batch
-  int *nbmem = reinterpret_cast<int *>(tbuf + 2 * a.batch);  // [2][kChunk * (kNbCap + 2)]
-  auto nblist = [&](unsigned int b) {
-    NbList L;
-    L.ids = nbmem + b * (kChunk * (kNbCap + 2));
-    L.meta = L.ids + kChunk * kNbCap;
-    return L;
-  };
-  __shared__ double red[kWarps];
-
-  const int tid = threadIdx.x;
-  const int grp = tid / kGroup, gl = tid % kGroup;
-
-  for (int k = tid; k < slen; k += kThreads) slice[k] = __ldcg(&a.pos[sbase + k]);
-  // group sub-ranges of [slo, shi) in slice-local indices
-  const int la = slo - sbase, lb = shi - sbase;
-  const int ga = la + (int)((long long)(lb - la) * grp / kGroups);
-  const int gb = la + (int)((long long)(lb - la) * (grp + 1) / kGroups);
-  __syncthreads();
-
-  unsigned int epoch = 0;
-  double step = a.step0;
-  double e_prev = DBL_MAX, e_cur = 0.0;
-  long long loop = 0;
-  bool ok = true;
-  bool prefetched = false;
-  unsigned int seq = 0;  // batches processed in this launch
-
-  while (ok) {
-    if (a.converged) {
-      if (!(fabs(e_prev - e_cur) / e_prev > a.engt) || loop >= a.max_loops) break;
-    } else if (loop >= a.iterations) {
-      break;
-    }
-    const bool need_energy = a.converged || (loop == a.iterations - 1);
-    for (int c = 0; c < a.nbatches && ok; c++, seq++) {
-      const int base = c * a.batch;
-      const int cnt = min(a.batch, a.n - base);
-      // buffers alternate by the batch's position in the whole run, so the
-      // last batch of an iteration and the first of the next never share one
-      const int buf = (int)(seq & 1u);
-      float2 *tpos = tbuf + buf * a.batch;
-      // the targets of batch c are normally prefetched during batch c-1;
-      // the first batch of the run, and every batch when there is only one,
-      // loads them here
-      if (!prefetched) {
-        for (int t = tid; t < cnt; t += kThreads) tpos[t] = __ldcg(&a.pos[base + t]);
-        if (cnt <= kChunk) stage_neighbours(a, nblist(buf), s, base, cnt, slo, shi, sbase);
-      }
-      __syncthreads();
-      // ---- sweep: partial force of this block's slice on every target ----
-      // repulsion for every source, attraction instead for the target's
-      // matched neighbours (found by a sorted cursor, rare), as in the
-      // reference's j loop
-      for (int c0 = 0; c0 < cnt; c0 += kChunk) {
-        const int t0 = c0 + gl, t1 = t0 + kGroup;
-        const bool v0 = t0 < cnt, v1 = t1 < cnt;
-        const float2 p0 = v0 ? tpos[t0] : make_float2(0.f, 0.f);
-        const float2 p1 = v1 ? tpos[t1] : make_float2(0.f, 0.f);
-        NbList L = nblist(buf);
-        if (cnt > kChunk) {  // several chunks: stage this chunk's neighbours now
-          __syncthreads();
-          stage_neighbours(a, L, s, base + c0, min(kChunk, cnt - c0), slo, shi, sbase);
-          __syncthreads();
-        }
-        Cursor c0r, c1r;
-        c0r.next = c1r.next = INT_MAX;
-        c0r.ptr = c0r.cnt = c1r.ptr = c1r.cnt = 0;
-        if (v0) cursor_init(c0r, a, L, gl, ga, sbase);
-        if (v1) cursor_init(c1r, a, L, gl + kGroup, ga, sbase);
-        float fx0a = 0.f, fy0a = 0.f, fx0b = 0.f, fy0b = 0.f;
-        float fx1a = 0.f, fy1a = 0.f, fx1b = 0.f, fy1b = 0.f;
-        // branch-free repulsion over the group's sources ...
-        int k = ga;
-        if ((k & 1) && k < gb) {
-          const float2 q = slice[k];
-          rep_law_pair<kRep>(q.x, q.y, p0.x, p0.y, fx0a, fy0a);
-          rep_law_pair<kRep>(q.x, q.y, p1.x, p1.y, fx1a, fy1a);
-          k++;
-        }
-#pragma unroll 4
-        for (; k + 1 < gb; k += 2) {
-          const float4 q = *reinterpret_cast<const float4 *>(&slice[k]);
-          rep_law_pair<kRep>(q.x, q.y, p0.x, p0.y, fx0a, fy0a);
-          rep_law_pair<kRep>(q.z, q.w, p0.x, p0.y, fx0b, fy0b);
-          rep_law_pair<kRep>(q.x, q.y, p1.x, p1.y, fx1a, fy1a);
-          rep_law_pair<kRep>(q.z, q.w, p1.x, p1.y, fx1b, fy1b);
-        }
-        if (k < gb) {
-          const float2 q = slice[k];
-          rep_law_pair<kRep>(q.x, q.y, p0.x, p0.y, fx0b, fy0b);
-          rep_law_pair<kRep>(q.x, q.y, p1.x, p1.y, fx1b, fy1b);
-        }
-        // ... then the matched neighbours in [ga, gb): take their repulsion
-        // back (same FP32 formula) and add the model's attraction instead
-        if (v0) correct_neighbours<kRep>(a, c0r, ga, gb, slice, p0, sbase, fx0b, fy0b);
-        if (v1) correct_neighbours<kRep>(a, c1r, ga, gb, slice, p1, sbase, fx1b, fy1b);
-        const float2 r0 = make_float2(fx0a + fx0b, fy0a + fy0b);
-        const float2 r1 = make_float2(fx1a + fx1b, fy1a + fy1b);
-        if (grp > 0) {
-          gsum[(grp - 1) * kChunk + gl] = r0;
-          gsum[(grp - 1) * kChunk + gl + kGroup] = r1;
-        }
-        __syncthreads();
-        if (grp == 0) {
-          float2 o0 = r0, o1 = r1;
-#pragma unroll
-          for (int g = 0; g < kGroups - 1; g++) {
-            const float2 u0 = gsum[g * kChunk + gl], u1 = gsum[g * kChunk + gl + kGroup];
-            o0.x += u0.x; o0.y += u0.y;
-            o1.x += u1.x; o1.y += u1.y;
-          }
-          long long *A = a.acc + ((size_t)buf * kAccCopies + s % kAccCopies) * a.batch * 2;
-          if (t0 < cnt) {
-            acc_add(&A[2 * t0], o0.x, a.st);
-            acc_add(&A[2 * t0 + 1], o0.y, a.st);
-          }
-          if (t1 < cnt) {
-            acc_add(&A[2 * t1], o1.x, a.st);
-            acc_add(&A[2 * t1 + 1], o1.y, a.st);
-          }
-        }
-        __syncthreads();
-      }
-      // announce this block's partials, then prefetch the next batch's targets
-      // and cursors while the other blocks arrive: its vertices do not move
-      // before it, and the cursors depend on the graph only.  Positions are
-      // read through L2: other blocks moved them.
-      grid_arrive(a.st, epoch);
-      {
-        const int cn = (c + 1 < a.nbatches) ? c + 1 : 0;
-        prefetched = (cn != c);  // a single batch moves itself: reload after the update
-        if (prefetched) {
-          const int nbase = cn * a.batch;
-          const int ncnt = min(a.batch, a.n - nbase);
-          float2 *ntpos = tbuf + (int)((seq + 1u) & 1u) * a.batch;
-          for (int t = tid; t < ncnt; t += kThreads) ntpos[t] = __ldcg(&a.pos[nbase + t]);
-          if (ncnt <= kChunk) stage_neighbours(a, nblist((seq + 1u) & 1u), s, nbase, ncnt, slo, shi, sbase);
-        }
-      }
-      ok = grid_wait(a.st, epoch);
-      if (!ok) break;
-      // ---- owners: read the summed force, update, clear the accumulator -----
-      const int olo = max(slo, base), ohi = min(shi, base + cnt);
-      if (olo < ohi) {
-        long long *A = a.acc + (size_t)buf * kAccCopies * a.batch * 2;
-        const float stepf = (float)step;
-        for (int i = olo + tid; i < ohi; i += kThreads) {
-          const int t = i - base;
-          longlong2 v = make_longlong2(0, 0);
-#pragma unroll
-          for (int k = 0; k < kAccCopies; k++) {
-            long long *Ak = A + (size_t)k * a.batch * 2;
-            const longlong2 u = __ldcg(reinterpret_cast<const longlong2 *>(&Ak[2 * t]));
-            // cleared for the batch after next, which reuses this buffer
-            *reinterpret_cast<longlong2 *>(&Ak[2 * t]) = make_longlong2(0, 0);
-            v.x += u.x;
-            v.y += u.y;
-          }
-          const double dfx = (double)v.x * kFixInv, dfy = (double)v.y * kFixInv;
-          const float2 pi = tpos[t];
-          const float fx = (float)dfx, fy = (float)dfy;
-          float2 np = pi;
-          const float m2 = fmaf(fx, fx, fy * fy);
-          if (m2 >= 1.17549435e-38f && m2 <= 3.0e38f) {
-            const float rm = rsqrt_approx(m2);
-            np.x = fmaf(stepf, fx * rm, pi.x);
-            np.y = fmaf(stepf, fy * rm, pi.y);
-          } else if (fx != 0.f || fy != 0.f) {  // |f|^2 outside the FP32 range
-            const double mag = sqrt(dfx * dfx + dfy * dfy);
-            np.x = (float)((double)pi.x + (dfx / mag) * step);
-            np.y = (float)((double)pi.y + (dfy / mag) * step);
-          }
-          a.pos[i] = np;
-          slice[i - sbase] = np;
-          a.force[i] = make_double2(dfx, dfy);
-          a.e[i] = dfx * dfx + dfy * dfy;
-        }
-      }
-      // owner warps still read tpos and write the slice: finish before the
-      // next batch reloads tpos and sweeps the slice
-      __syncthreads();
-    }
-    if (!ok) break;
-    if (need_energy) {
-      ok = grid_barrier(a.st, epoch);
-      if (!ok) break;
-      double v = 0.0;
-      for (int i = slo + tid; i < shi; i += kThreads) v += __ldcg(&a.e[i]);
-      v = block_sum(v, red);
-      if (tid == 0) a.energy_parts[s] = v;
-      ok = grid_barrier(a.st, epoch);
-      if (!ok) break;
-      double tot = 0.0;
-      if (tid == 0)
-        for (int q = 0; q < a.grid; q++) tot += __ldcg(&a.energy_parts[q]);
-      if (tid == 0) red[0] = tot;
-      __syncthreads();
-      tot = red[0];
-      __syncthreads();
-      e_prev = e_cur;
-      e_cur = tot;
-      if (s == 0 && tid == 0) a.energy[0] = tot;
-    }
-    step = step * a.decay;
-    loop++;
+  if (a.converged && (!(1.0 > a.engt) || a.max_loops < 1)) {  // (DBL_MAX - 0) / DBL_MAX > engt before the first loop
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.loops = 0;
+    return;
   }
-  if (s == 0 && tid == 0) *a.loops = loop;
+  if ((int)blockIdx.x < a.movers) mover<kRep>(a, smem_raw);
+  else sweeper<kRep>(a, smem_raw);
 }
 
-// cursor[s * n + i] = number of matched neighbours of i below slice_lo(s)
-__global__ void cursor_table_kernel(const int *__restrict__ rowptr, const int *__restrict__ colids, int n,
-                                    int grid, int *cursor) {
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= (long long)n * grid) return;
-  const int s = (int)(gid / n), i = (int)(gid % n);
-  int slo, shi;
-  slice_of(n, grid, s, slo, shi);
-  int lo = rowptr[i], hi = rowptr[i + 1];
-  const int k0 = lo;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (colids[mid] < slo) lo = mid + 1;
-    else hi = mid;
+// ---- launch shape ---------------------------------------------------------------------
+
+struct MinibatchShape {
+  int movers = 1, sweepers = 1, lag = 0, late = 1;
+  size_t smem = 0, part_bytes = 0, exchange_bytes = 0;
+  // scratch: control words and exchange (zero before a launch), then partials
+  size_t control_bytes() const { return ((sizeof(MbControl) + 255) / 256) * 256 + exchange_bytes; }
+  void carve(void *base, MinibatchArgs &a) const {
+    unsigned char *p = static_cast<unsigned char *>(base);
+    a.ctl = reinterpret_cast<MbControl *>(p);
+    a.exchange = reinterpret_cast<ulonglong2 *>(p + ((sizeof(MbControl) + 255) / 256) * 256);
+    a.part = reinterpret_cast<float2 *>(p + control_bytes());
+    a.lag = lag;
+    a.late = late;
+    a.movers = movers;
+    a.sweepers = sweepers;
   }
-  cursor[gid] = lo - k0;
+};
+
+// Blocks and shared memory for `movers` movers and a lag.
+MinibatchShape shape_of(int n, int batch, int num_sms, int movers, int lag) {
+  MinibatchShape s;
+  const int nb = (n + batch - 1) / batch;
+  s.movers = movers;
+  s.sweepers = std::max(1, std::min(num_sms - movers, (n + 63) / 64));
+  s.lag = std::min(lag, nb - 1);
+  if (s.lag > 0 && nb == s.lag + 2) s.lag--;  // every batch in the ring, or the next two outside it
+  const size_t slice = (size_t)(2 * (((n + 1) / 2 + s.sweepers - 1) / s.sweepers) + 2);
+  const size_t sweeper = slice * sizeof(float2) + 16 + (size_t)2 * kGroups * kChunk * sizeof(float2);
+  const size_t share = (size_t)mover_share(batch, s.movers), stride = (size_t)(batch + 1) / 2 * 2;
+  const size_t chunks = (share + kMoveTile - 1) / kMoveTile;
+  s.late = s.lag == 0 || chunks > 2 ? 1 : 0;
+  const size_t mover = (s.lag + 1) * (stride / 2) * sizeof(float4) +
+                       (s.late ? 1 : 2) * chunks * kRows * kMoveTile * sizeof(ulonglong2) +
+                       2 * share * sizeof(float4) + (s.late ? 2 : 4) * stride * sizeof(float2) +
+                       2 * share * (s.late ? 1 : kNear + 1) * sizeof(int);
+  s.smem = std::max(sweeper, mover);
+  s.part_bytes = (size_t)(s.lag + 1) * s.sweepers * stride * sizeof(float2);
+  s.exchange_bytes = (size_t)kExchange * batch * sizeof(ulonglong2);
+  return s;
+}
+
+// The number of movers with the smallest time per batch, the larger of the
+// chain's (2.6 us and the pairs of a share with the `lag` batches before at
+// 15,600 a us) and the sweep's (28,500 pairs a us and SM, and 1 us).
+// Measured, us per batch with 8 / 16 / 32 movers: 4,096 vertices, batch 256
+// 4.0 / 3.2 / 2.9; 100,000, batch 256 6.8 / 7.1 / 7.9; 31,000, batch 512
+// 9.1 / 5.8 / 6.1; 30,000, batch 1,000 21.5 / 12.0 / 9.8; 90,000, batch 1,000
+// 25.1 / 24.5 / 26.8.  A lag of 2 was best or within 3 % everywhere (4,096
+// vertices 1 / 2 / 3 / 4: 3.7 / 2.9 / 3.1 / 3.3; 31,000: 7.8 / 5.8 / 5.9 /
+// 6.6); a smaller one where shared memory does not hold the batches.  False
+// when a slice does not fit a block's shared memory.
+bool minibatch_shape(int n, int batch, int num_sms, int smem_optin, MinibatchShape &s) {
+  // the largest graph taken: 3.5 million vertices at batch 256, 2.3 million at 4,096
+  if ((((n + num_sms - 1) / num_sms + 5) & ~3) * 8LL + 16LL * batch + 44032 > smem_optin) return false;
+  bool found = false;
+  for (int lag = 2; lag >= 0 && !found; lag--) {
+    double best = 0.0;
+    for (int movers = kMaxMovers; movers >= 1; movers /= 2) {
+      if (movers > 1 && (movers > (batch + 7) / 8 || movers > num_sms / 4)) continue;
+      const int share = mover_share(batch, movers);
+      if (movers < 16 && share > kMoveTile && movers < num_sms / 4) continue;  // several passes a batch
+      const MinibatchShape t = shape_of(n, batch, num_sms, movers, lag);
+      if (t.smem + 1024 > (size_t)smem_optin) continue;
+      const double chain = 2.6 + (double)std::max(t.lag, 1) * batch * share / 15600.0;
+      const double sweep = 1.0 + (double)batch * n / (28500.0 * t.sweepers);
+      const double us = t.lag == 0 ? chain + sweep : std::max(chain, sweep);
+      if (!found || us < best) {
+        best = us;
+        s = t;
+        found = true;
+      }
+    }
+  }
+  return found;
 }
 
 }  // namespace
-
-int ensure_minibatch_scratch(bl_ctx *ctx, int batch, int grid) {
-  (void)grid;
-  const size_t need = (size_t)2 * kAccCopies * batch * 2 * sizeof(long long);
-  if (ctx->s.partials_bytes < need) {
-    if (ctx->s.partials) cudaFree(ctx->s.partials);
-    ctx->s.partials = nullptr;
-    ctx->s.partials_bytes = 0;
-    BL_CUDA(ctx, cudaMalloc(&ctx->s.partials, need));
-    ctx->s.partials_bytes = need;
-  }
-  return 0;
-}
 
 int minibatch_run(bl_ctx *ctx, int model, int batch, int iterations, double step0,
                   double decay, bool converged, double engt, long long max_loops,
@@ -487,64 +1159,42 @@ int minibatch_run(bl_ctx *ctx, int model, int batch, int iterations, double step
   const bool full_rows = model == MODEL_SD;
   if (full_rows)
     if (int rc = ensure_sorted_csr(ctx)) return rc;
-  const int *nb_rowptr = full_rows ? ctx->g.srt_rowptr : ctx->g.eff_rowptr;
-  const int *nb_colids = full_rows ? ctx->g.srt_colids : ctx->g.eff_colids;
-  // the cursor table belongs to one neighbour set; the full rows share the
-  // cursor-matched set's table when the two sets are the same arrays
-  const bool own_table = full_rows && nb_colids != ctx->g.eff_colids;
-  int *&cursor = own_table ? ctx->s.cursor_full : ctx->s.cursor;
-  int &cursor_grid = own_table ? ctx->s.cursor_full_grid : ctx->s.cursor_grid;
-  void (*kernel)(MinibatchArgs) = unit_rep ? minibatch_kernel<REP_UNIT> : minibatch_kernel<REP_INV>;
-  int grid = std::min(ctx->num_sms, std::max(1, (n + 127) / 128));
   int dev_smem_optin = 0;
   cudaDeviceGetAttribute(&dev_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-  auto smem_for = [&](int g) {
-    const int slice_max = (n + g - 1) / g + 2;
-    return (size_t)(((slice_max + 3) & ~3) + (kGroups - 1) * kChunk + 2 * batch) * sizeof(float2) +
-           (size_t)2 * kChunk * (kNbCap + 2) * sizeof(int);
-  };
-  while (smem_for(grid) + 1024 > (size_t)dev_smem_optin && grid < ctx->num_sms) grid++;
-  const size_t smem = smem_for(grid);
-  if (smem + 1024 > (size_t)dev_smem_optin)
+  MinibatchShape sh;
+  if (!minibatch_shape(n, batch, ctx->num_sms, dev_smem_optin, sh))
     return bl_fail(ctx, -5, "graph too large for the shared-memory source slices of the minibatch path");
-  BL_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  void (*kernel)(MinibatchArgs) = unit_rep ? minibatch_kernel<REP_UNIT> : minibatch_kernel<REP_INV>;
+  const int grid = sh.movers + sh.sweepers;
+  BL_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
   int occ = 0;
-  BL_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kThreads, smem));
+  BL_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kThreads, sh.smem));
   if (occ < 1 || grid > occ * ctx->num_sms)
     return bl_fail(ctx, -5, "minibatch kernel cannot be co-resident");
-  if (int rc = ensure_minibatch_scratch(ctx, batch, grid)) return rc;
-  if (cursor_grid != grid) {
-    if (cursor) cudaFree(cursor);
-    cursor = nullptr;
-    cursor_grid = 0;
-    BL_CUDA(ctx, cudaMalloc(&cursor, (size_t)n * grid * sizeof(int)));
-    const long long total = (long long)n * grid;
-    cursor_table_kernel<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(nb_rowptr, nb_colids, n, grid,
-                                                                                cursor);
-    BL_CUDA(ctx, cudaGetLastError());
-    ctx->launches++;
-    cursor_grid = grid;
+  const size_t need = sh.control_bytes() + sh.part_bytes;
+  if (ctx->s.partials_bytes < need) {
+    if (ctx->s.partials) cudaFree(ctx->s.partials);
+    ctx->s.partials = nullptr;
+    ctx->s.partials_bytes = 0;
+    BL_CUDA(ctx, cudaMalloc(&ctx->s.partials, need));
+    ctx->s.partials_bytes = need;
   }
   BL_CUDA(ctx, cudaMemsetAsync(ctx->s.status, 0, sizeof(DevStatus), ctx->stream));
-  BL_CUDA(ctx, cudaMemsetAsync(ctx->s.partials, 0, (size_t)2 * kAccCopies * batch * 2 * sizeof(long long),
-                               ctx->stream));
+  BL_CUDA(ctx, cudaMemsetAsync(ctx->s.partials, 0, sh.control_bytes(), ctx->stream));
 
   MinibatchArgs a;
   a.n = n;
   a.batch = batch;
   a.nbatches = (n + batch - 1) / batch;
   a.model = attract;
-  a.grid = grid;
-  a.W = ctx->weight;
-  a.eff_rowptr = nb_rowptr;
-  a.eff_colids = nb_colids;
-  a.cursor = cursor;
+  a.W = (float)ctx->weight;
+  a.eff_rowptr = full_rows ? ctx->g.srt_rowptr : ctx->g.eff_rowptr;
+  a.eff_colids = full_rows ? ctx->g.srt_colids : ctx->g.eff_colids;
   a.pos = ctx->pos;
   a.force = ctx->force;
   a.e = ctx->e;
-  a.acc = reinterpret_cast<long long *>(ctx->s.partials);
+  sh.carve(ctx->s.partials, a);
   a.energy = ctx->s.energy;
-  a.energy_parts = ctx->s.energy_parts;
   a.loops = reinterpret_cast<long long *>(ctx->s.energy + 1);
   a.st = ctx->s.status;
   a.iterations = iterations;
@@ -555,14 +1205,17 @@ int minibatch_run(bl_ctx *ctx, int model, int batch, int iterations, double step
   a.max_loops = max_loops;
   void *args[] = {&a};
   bl_time_begin(ctx, "minibatch_kernel");
-  BL_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(kThreads), args, smem,
+  BL_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(kThreads), args, sh.smem,
                                            ctx->stream));
   bl_time_end(ctx, "minibatch_kernel");
   ctx->launches++;
   double host[2];
+  DevStatus st;
   BL_CUDA(ctx, cudaMemcpyAsync(host, ctx->s.energy, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  BL_CUDA(ctx, cudaMemcpyAsync(&st, ctx->s.status, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
   BL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (int rc = bl_check_status(ctx)) return rc;
+  if (st.code != DEV_OK)
+    if (int rc = bl_check_status(ctx)) return rc;
   long long loops;
   memcpy(&loops, &host[1], sizeof(loops));
   if (energy_out) *energy_out = host[0];
@@ -580,12 +1233,12 @@ int minibatch_run(bl_ctx *ctx, int model, int batch, int iterations, double step
 // that forbid allocation after start-up, or code that enqueues work on a
 // stream another component owns.  bl_minibatch_iteration_noalloc runs the
 // same minibatch kernel as bl_minibatch_iteration, but every scratch buffer
-// it needs (partial forces, energy partials, the device status word) lives
+// it needs (partial forces, control words, the device status word) lives
 // in the fixed array below, so the call allocates nothing.  The caller passes
 // its inputs and outputs as device pointers.
 //
 // Limits: batch <= 256 and at most 160 blocks (one per SM); the scratch is a
-// fixed 768 KiB (force accumulators, energy partials, status word).
+// fixed 1 MiB (partial forces of the batches in flight, control words, status).
 // The array exists once per device for the lifetime of the process and every
 // call on that device shares it: calls that overlap on the GPU (different
 // streams, or host threads that do not serialise) race and give wrong
@@ -598,12 +1251,11 @@ namespace {
 
 constexpr int kNoAllocMaxBatch = 256;
 constexpr int kNoAllocMaxGrid = 160;
-constexpr size_t kNoAllocPartialBytes = (size_t)2 * kNoAllocMaxBatch * kNoAllocMaxGrid * sizeof(float2);
-constexpr size_t kNoAllocBytes = 768 * 1024;
-static_assert((size_t)2 * kAccCopies * kNoAllocMaxBatch * 2 * sizeof(long long) <= kNoAllocPartialBytes,
-              "no-alloc accumulators too small");
-static_assert(kNoAllocPartialBytes + kNoAllocMaxGrid * sizeof(double) + 4 * sizeof(double) +
-                      sizeof(DevStatus) <= kNoAllocBytes,
+constexpr int kNoAllocMaxLag = kMaxLag;
+constexpr size_t kNoAllocBytes = 1024 * 1024;
+static_assert(256 + ((sizeof(MbControl) + 255) / 256) * 256 + (size_t)kExchange * kNoAllocMaxBatch * sizeof(ulonglong2) +
+                      (size_t)(kNoAllocMaxLag + 1) * kNoAllocMaxGrid * kNoAllocMaxBatch * sizeof(float2) <=
+                  kNoAllocBytes,
               "no-alloc scratch too small");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -641,51 +1293,39 @@ extern "C" int bl_minibatch_iteration_noalloc(int n, const int *d_rowptr, const 
   int num_sms = 0, smem_optin = 0;
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-  // same block count and shared-memory sizing as the context path
-  int grid = std::min(num_sms, std::max(1, (n + 127) / 128));
-  auto smem_for = [&](int g) {
-    const int slice_max = (n + g - 1) / g + 2;
-    return (size_t)(((slice_max + 3) & ~3) + (kGroups - 1) * kChunk + 2 * batch) * sizeof(float2) +
-           (size_t)2 * kChunk * (kNbCap + 2) * sizeof(int);
-  };
-  while (smem_for(grid) + 1024 > (size_t)smem_optin && grid < num_sms) grid++;
-  if (grid > kNoAllocMaxGrid) return BL_ERR_TOO_LARGE;  // scratch holds 160 blocks of partials
-  const size_t smem = smem_for(grid);
-  if (smem + 1024 > (size_t)smem_optin) return BL_ERR_TOO_LARGE;
-  if (cudaFuncSetAttribute(minibatch_kernel<REP_INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+  // same blocks and shared-memory sizing as the context path
+  MinibatchShape sh;
+  if (!minibatch_shape(n, batch, std::min(num_sms, kNoAllocMaxGrid), smem_optin, sh)) return BL_ERR_TOO_LARGE;
+  const int grid = sh.movers + sh.sweepers;
+  if (cudaFuncSetAttribute(minibatch_kernel<REP_INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem) !=
       cudaSuccess)
     return BL_ERR_CUDA;
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, minibatch_kernel<REP_INV>, kThreads, smem) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, minibatch_kernel<REP_INV>, kThreads, sh.smem) !=
+          cudaSuccess ||
       occ < 1 || grid > occ * num_sms)
     return BL_ERR_TOO_LARGE;
-  // carve the scratch: force accumulators | energy parts | energy + loops | status
-  float2 *partials = reinterpret_cast<float2 *>(base);
-  double *energy_parts = reinterpret_cast<double *>(base + kNoAllocPartialBytes);
-  double *energy = energy_parts + kNoAllocMaxGrid;
-  DevStatus *status = reinterpret_cast<DevStatus *>(energy + 4);
+  // the scratch: status | energy + loops | control words, exchange, partials.
+  // The first two and the control words and exchange start at zero; every
+  // other value is written before it is read.
+  DevStatus *status = reinterpret_cast<DevStatus *>(base);
+  double *energy = reinterpret_cast<double *>(base + sizeof(DevStatus));
+  unsigned char *scratch = base + 256;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // the status word (barrier counter, error code) and the force accumulators
-  // must start at zero; every other scratch value is written before it is read
-  if (cudaMemsetAsync(status, 0, sizeof(DevStatus), st) != cudaSuccess) return BL_ERR_CUDA;
-  if (cudaMemsetAsync(partials, 0, (size_t)2 * kAccCopies * batch * 2 * sizeof(long long), st) != cudaSuccess)
-    return BL_ERR_CUDA;
+  if (cudaMemsetAsync(base, 0, 256 + sh.control_bytes(), st) != cudaSuccess) return BL_ERR_CUDA;
   MinibatchArgs a;
   a.n = n;
   a.batch = batch;
   a.nbatches = (n + batch - 1) / batch;
   a.model = model;
-  a.grid = grid;
-  a.W = weight;
+  a.W = (float)weight;
   a.eff_rowptr = d_rowptr;
   a.eff_colids = d_colids;
-  a.cursor = nullptr;
   a.pos = reinterpret_cast<float2 *>(d_xy);
   a.force = reinterpret_cast<double2 *>(d_force);
   a.e = d_vertex_energy;
-  a.acc = reinterpret_cast<long long *>(partials);
+  sh.carve(scratch, a);
   a.energy = energy;
-  a.energy_parts = energy_parts;
   a.loops = reinterpret_cast<long long *>(energy + 1);
   a.st = status;
   a.iterations = 1;
@@ -695,7 +1335,7 @@ extern "C" int bl_minibatch_iteration_noalloc(int n, const int *d_rowptr, const 
   a.engt = 0.0;
   a.max_loops = 0;
   void *args[] = {&a};
-  if (cudaLaunchCooperativeKernel((const void *)minibatch_kernel<REP_INV>, dim3(grid), dim3(kThreads), args, smem,
+  if (cudaLaunchCooperativeKernel((const void *)minibatch_kernel<REP_INV>, dim3(grid), dim3(kThreads), args, sh.smem,
                                   st) !=
       cudaSuccess)
     return BL_ERR_CUDA;

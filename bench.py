@@ -186,7 +186,7 @@ def allpairs_fraction(B, torch, device: int, flush, iterations: int = 3) -> dict
     g, xy = load_workload("chunglu100k")
     with B.Algorithms(g.rowptr, g.colids, device=device) as a:
         a.nCoordinates = xy
-        a.run_resident(2, 1, 256, 1.2, 1.0, want_energy=True)  # warm-up (builds the cursor table)
+        a.run_resident(2, 1, 256, 1.2, 1.0, want_energy=True)  # warm-up
         a.kernel_time("minibatch_kernel")
         step = 0.999
         for _ in range(iterations):

@@ -360,7 +360,7 @@ int bl_wait_selftest(bl_ctx *ctx, int site, int complete);
  * they run -- services that reserve all GPU memory up front in their own pool,
  * real-time loops that forbid allocation after start-up, code enqueuing on a
  * stream another component owns.  It allocates nothing: its scratch is a fixed
- * 768 KiB device array inside the library, which limits batch to 256 and the
+ * 1 MiB device array inside the library, which limits batch to 256 and the
  * launch to 160 blocks (larger requests return BL_ERR_TOO_LARGE).
  * Device pointers, all caller-owned, on the current device:
  *   d_rowptr[n+1], d_colids   neighbour lists the minibatch cursor matches,
