@@ -10,15 +10,22 @@
 //   f[12]     log2(1 + deg), f[13] 1 / (1 + deg),
 //   f[14]     mean of log2(1 + deg) over the neighbours,
 //   f[15]     log2(n) / 20.
-// Hop distances come from one multi-source BFS on the device (a 16-bit
-// visited mask per vertex, one level per grid-barrier step, the vertices of
-// the level's frontier push their new source bits to their neighbours, which
-// join the next frontier list the first time a bit reaches them); all graphs
-// of a training set run in the same BFS, each with its own pivots.  The work
-// of a level is its frontier (the 1M-vertex random geometric graph has 1,430
-// levels), and a block gathers its new frontier vertices in shared memory and
-// reserves room for them in the global list with one atomic per level.  Distances to pivots that a vertex cannot
-// reach count as one more than the pivot's largest finite distance.
+// Hop distances.  A graph with rows of at most 64 entries gets one block per
+// pivot, which runs that breadth-first search by itself, the frontier and (up
+// to 1.3 million vertices) the visited bits in shared memory, one block barrier
+// a level: the graphs this engine lays out are mostly mesh-like, with hundreds
+// to thousands of levels and frontiers of hundreds of vertices, where a level
+// is a chain of round trips (400,000-vertex random geometric graph: 8.8 ms
+// with one grid barrier a level over the whole device, 2.6 ms this way).
+// Graphs with longer rows, and all graphs when a frontier outgrows a block's
+// queue, take the device-wide form: one multi-source BFS over their pivots (a
+// 16-bit visited mask per vertex, one level per grid-barrier step, the
+// vertices of the level's frontier push their new source bits to their
+// neighbours, which join the next frontier list the first time a bit reaches
+// them); a block gathers its new frontier vertices in shared memory and
+// reserves room for them in the global list with one atomic per level.
+// Distances to pivots that a vertex cannot reach count as one more than the
+// pivot's largest finite distance.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -35,24 +42,21 @@ namespace {
 constexpr int kP = kPivots;
 constexpr unsigned short kUnreached = 0xFFFF;
 
-__global__ void bfs_init_kernel(int n, unsigned int *visited, unsigned int *fr0, unsigned int *fr1,
-                                unsigned short *dist) {
+__global__ void bfs_init_kernel(int n, unsigned int *visited, unsigned int *fr0, unsigned int *fr1) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n) return;
   visited[v] = 0u;
   fr0[v] = 0u;
   fr1[v] = 0u;
-#pragma unroll
-  for (int s = 0; s < kP; s++) dist[(size_t)v * kP + s] = kUnreached;
 }
 
 // pivots[g * 16 + s]: global vertex of pivot s of graph g; the distinct pivot
-// vertices form the frontier list of level 0
-__global__ void bfs_seed_kernel(int count, const int *pivots, unsigned int *visited, unsigned int *fr0,
-                                unsigned short *dist, int *wl0, unsigned int *cnt) {
+// vertices of the listed graphs form the frontier list of level 0
+__global__ void bfs_seed_kernel(int count, const int *list, const int *pivots, unsigned int *visited,
+                                unsigned int *fr0, unsigned short *dist, int *wl0, unsigned int *cnt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  const int p = pivots[i], s = i % kP;
+  const int s = i % kP, p = pivots[list[i / kP] * kP + s];
   atomicOr(&visited[p], 1u << s);
   dist[(size_t)p * kP + s] = 0;
   if (atomicOr(&fr0[p], 1u << s) == 0u) wl0[atomicAdd(&cnt[0], 1u)] = p;
@@ -128,6 +132,152 @@ __global__ void __launch_bounds__(512) msbfs_kernel(BfsArgs a) {
     for (unsigned int k = threadIdx.x; k < mine; k += blockDim.x) a.wl[nbuf][s_base + k] = s_buf[k];
     if (!grid_barrier(a.st, epoch)) return;
   }
+}
+
+// ---- one block per (graph, pivot) --------------------------------------------
+
+constexpr int kBlockThreads = 1024;
+// vertices of a frontier; a level of 8,192 vertices costs one block about
+// what a level costs the whole device (10 us)
+constexpr int kBlockQueue = 8192;
+constexpr int kBlockEdges = 8;  // row entries a lane loads at a time, two lanes a row
+// longest row taken: the level waits for the longest row of its frontier
+constexpr int kBlockRow = 64;
+
+struct BlockBfsArgs {
+  const int *rowptr, *colids;
+  const int *voff;    // [graphs + 1]
+  const int *pivots;  // [graphs * 16]
+  const int *list;    // graph of each 16 blocks
+  unsigned short *dist;
+  int *wide;  // set when a frontier outgrows the queue
+  int bits;   // visited bits that fit in shared memory
+};
+
+struct BlockBfsSmem {
+  int queue[2][kBlockQueue];
+  int count[3];  // frontier sizes, rotating by level
+};
+
+__device__ __forceinline__ void prefetch_l1(const void *p) {
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
+// Bound by latency: per level one L2 round trip for the row entries (the row
+// pointers are prefetched when a vertex is found), the shared-memory tests and
+// appends of a row's entries side by side, one block barrier.
+template <bool kBits>
+__device__ __forceinline__ void bfs_block(const BlockBfsArgs &a, BlockBfsSmem &S, unsigned int *vis, int v0, int n,
+                                          int pivot, int s) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const unsigned int lt = (1u << lane) - 1u;
+  if (kBits)
+    for (int k = tid; k < (n + 31) / 32; k += kBlockThreads) vis[k] = 0u;
+  __syncthreads();
+  if (tid == 0) {
+    if (kBits) vis[pivot >> 5] = 1u << (pivot & 31);
+    a.dist[(size_t)(v0 + pivot) * kP + s] = 0;
+    S.queue[0][0] = pivot;
+    S.count[0] = 1;
+    S.count[1] = S.count[2] = 0;
+  }
+  __syncthreads();
+  unsigned short *const dist = a.dist + (size_t)v0 * kP + s;
+  int cur = 0, nxt = 1, third = 2;
+  // every vertex enters the frontier once: at most n levels
+  for (int L = 1; L <= n; L++) {
+    const int count = S.count[cur];
+    if (count == 0) return;
+    if (count > kBlockQueue) {  // every thread sees the same count
+      if (tid == 0) atomicExch(a.wide, 1);
+      return;
+    }
+    if ((L & 63) == 0) {  // another block gave up
+      if (__syncthreads_or(tid == 0 && ld_volatile_u32(reinterpret_cast<const unsigned int *>(a.wide)) != 0u)) return;
+    }
+    if (tid == 0) S.count[third] = 0;  // read as `cur` one level ago, appended to in the next one
+    const int *q = S.queue[(L - 1) & 1];
+    int *out = S.queue[L & 1];
+    const unsigned short d = (unsigned short)min(L, 65534);
+    for (int i0 = 0; i0 < 2 * count; i0 += kBlockThreads) {
+      const int idx = (i0 + tid) >> 1;
+      int e = 0, e1 = 0;
+      if (idx < count) {
+        const int u = v0 + q[idx];
+        e = __ldg(&a.rowptr[u]) + (tid & 1);
+        e1 = __ldg(&a.rowptr[u + 1]);
+      }
+      while (__any_sync(0xffffffffu, e < e1)) {
+        int v[kBlockEdges];
+        unsigned int fresh = 0;
+#pragma unroll
+        for (int k = 0; k < kBlockEdges; k++) v[k] = e + 2 * k < e1 ? __ldg(&a.colids[e + 2 * k]) - v0 : -1;
+        if (kBits) {
+          unsigned int old[kBlockEdges];
+#pragma unroll
+          for (int k = 0; k < kBlockEdges; k++) old[k] = v[k] >= 0 ? vis[v[k] >> 5] : 0xffffffffu;
+#pragma unroll
+          for (int k = 0; k < kBlockEdges; k++)
+            if (((old[k] >> (v[k] & 31)) & 1u) == 0u) old[k] = atomicOr(&vis[v[k] >> 5], 1u << (v[k] & 31));
+#pragma unroll
+          for (int k = 0; k < kBlockEdges; k++)
+            if (((old[k] >> (v[k] & 31)) & 1u) == 0u) {
+              fresh |= 1u << k;
+              dist[(size_t)v[k] * kP] = d;
+            }
+        } else {
+          unsigned short old[kBlockEdges];
+#pragma unroll
+          for (int k = 0; k < kBlockEdges; k++) {
+            old[k] = 0;
+            if (v[k] >= 0) old[k] = atomicCAS(&dist[(size_t)v[k] * kP], kUnreached, d);
+          }
+#pragma unroll
+          for (int k = 0; k < kBlockEdges; k++)
+            if (old[k] == kUnreached) fresh |= 1u << k;
+        }
+        // appended to the next frontier, one shared atomic a warp
+        unsigned int b[kBlockEdges];
+        int total = 0;
+#pragma unroll
+        for (int k = 0; k < kBlockEdges; k++) {
+          b[k] = __ballot_sync(0xffffffffu, (fresh >> k) & 1u);
+          total += __popc(b[k]);
+        }
+        if (total) {
+          int slot = 0;
+          if (lane == 0) slot = atomicAdd(&S.count[nxt], total);
+          slot = __shfl_sync(0xffffffffu, slot, 0);
+#pragma unroll
+          for (int k = 0; k < kBlockEdges; k++) {
+            const int x = slot + __popc(b[k] & lt);
+            if (((fresh >> k) & 1u) && x < kBlockQueue) {
+              out[x] = v[k];
+              prefetch_l1(&a.rowptr[v0 + v[k]]);
+            }
+            slot += __popc(b[k]);
+          }
+        }
+        e += 2 * kBlockEdges;
+      }
+    }
+    __syncthreads();
+    const int t = cur;
+    cur = nxt;
+    nxt = third;
+    third = t;
+  }
+}
+
+__global__ void __launch_bounds__(kBlockThreads, 1) bfs_block_kernel(BlockBfsArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  BlockBfsSmem &S = *reinterpret_cast<BlockBfsSmem *>(smem_raw);
+  unsigned int *vis = reinterpret_cast<unsigned int *>(smem_raw + sizeof(BlockBfsSmem));
+  const int g = a.list[blockIdx.x / kP], s = blockIdx.x % kP;
+  const int v0 = a.voff[g], n = a.voff[g + 1] - v0;
+  const int pivot = a.pivots[g * kP + s] - v0;
+  if (n <= a.bits) bfs_block<true>(a, S, vis, v0, n, pivot, s);
+  else bfs_block<false>(a, S, vis, v0, n, pivot, s);
 }
 
 // ---- pivot MDS of one graph (vertices [v0, v1)) ---------------------------
@@ -358,30 +508,38 @@ void jacobi_eigen(int m, std::vector<double> A, std::vector<double> &lam, std::v
 }
 
 // Features of the graphs [voff[g], voff[g+1]) of a block-diagonal device CSR.
-int compute_features(bl_ctx *ctx, int num_graphs, const int *voff, int n, const int *d_rowptr, const int *d_colids,
-                     const int *pivots, float *d_features, unsigned short *d_dist) {
+// max_row[g]: the graph's longest row.
+int compute_features(bl_ctx *ctx, int num_graphs, const int *voff, int n, const int *max_row, const int *d_rowptr,
+                     const int *d_colids, const int *pivots, float *d_features, unsigned short *d_dist) {
   cudaStream_t st = ctx->stream;
   const int P = num_graphs * kP;
   unsigned int *visited = nullptr, *fr0 = nullptr, *fr1 = nullptr, *cnt = nullptr;
-  int *d_piv = nullptr, *d_maxd = nullptr, *d_ipart = nullptr, *wl0 = nullptr, *wl1 = nullptr;
+  int *d_piv = nullptr, *d_maxd = nullptr, *d_ipart = nullptr, *wl0 = nullptr, *wl1 = nullptr, *d_voff = nullptr;
   double *d_dpart = nullptr, *d_colmean = nullptr, *d_V = nullptr;
   const int kBlocks = 256;
   int rc = 0;
   auto cleanup = [&]() {
     cudaFree(visited); cudaFree(fr0); cudaFree(fr1); cudaFree(cnt); cudaFree(wl0); cudaFree(wl1);
-    cudaFree(d_piv); cudaFree(d_maxd);
+    cudaFree(d_piv); cudaFree(d_maxd); cudaFree(d_voff);
     cudaFree(d_ipart); cudaFree(d_dpart); cudaFree(d_colmean); cudaFree(d_V);
   };
   auto ck = [&](cudaError_t e, const char *w) {
     if (e != cudaSuccess && !rc) rc = bl_cuda_fail(ctx, e, w);
     return rc == 0;
   };
-  ck(cudaMalloc(&visited, sizeof(unsigned int) * n), "cudaMalloc");
-  ck(cudaMalloc(&fr0, sizeof(unsigned int) * n), "cudaMalloc");
-  ck(cudaMalloc(&fr1, sizeof(unsigned int) * n), "cudaMalloc");
-  ck(cudaMalloc(&cnt, 3 * sizeof(unsigned int)), "cudaMalloc");
-  ck(cudaMalloc(&wl0, sizeof(int) * n), "cudaMalloc");
-  ck(cudaMalloc(&wl1, sizeof(int) * n), "cudaMalloc");
+  // graphs by the form of their search: blocks first
+  std::vector<int> list;
+  for (int k = 0; k < 2; k++)
+    for (int g = 0; g < num_graphs; g++)
+      if ((max_row[g] <= kBlockRow) == (k == 0)) list.push_back(g);
+  int nblock = 0, largest = 0;
+  for (int g = 0; g < num_graphs; g++)
+    if (max_row[g] <= kBlockRow) {
+      nblock++;
+      largest = std::max(largest, voff[g + 1] - voff[g]);
+    }
+  ck(cudaMalloc(&cnt, 4 * sizeof(unsigned int)), "cudaMalloc");
+  ck(cudaMalloc(&d_voff, sizeof(int) * (2 * num_graphs + 1)), "cudaMalloc");
   ck(cudaMalloc(&d_piv, sizeof(int) * P), "cudaMalloc");
   ck(cudaMalloc(&d_maxd, sizeof(int) * kP), "cudaMalloc");
   ck(cudaMalloc(&d_ipart, sizeof(int) * kBlocks * kP), "cudaMalloc");
@@ -393,12 +551,47 @@ int compute_features(bl_ctx *ctx, int num_graphs, const int *voff, int n, const 
     return rc;
   }
   ck(cudaMemcpyAsync(d_piv, pivots, sizeof(int) * P, cudaMemcpyHostToDevice, st), "H2D");
-  ck(cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned int), st), "memset");
-  bfs_init_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, visited, fr0, fr1, d_dist);
-  bfs_seed_kernel<<<(P + 255) / 256, 256, 0, st>>>(P, d_piv, visited, fr0, d_dist, wl0, cnt);
-  ck(cudaMemsetAsync(&ctx->s.status->barrier, 0, sizeof(unsigned int), st), "memset");
-  ctx->launches += 2;
-  {
+  int *d_list = d_voff + num_graphs + 1;
+  ck(cudaMemcpyAsync(d_voff, voff, sizeof(int) * (num_graphs + 1), cudaMemcpyHostToDevice, st), "H2D");
+  ck(cudaMemcpyAsync(d_list, list.data(), sizeof(int) * num_graphs, cudaMemcpyHostToDevice, st), "H2D");
+  ck(cudaMemsetAsync(cnt, 0, 4 * sizeof(unsigned int), st), "memset");  // list lengths, then the give-up flag
+  ck(cudaMemsetAsync(d_dist, 0xff, sizeof(unsigned short) * kP * (size_t)n, st), "memset");
+  if (!rc && nblock > 0) {
+    int optin = 0, wide = 0;
+    ck(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device), "attribute");
+    const int room = (optin - 1024 - (int)sizeof(BlockBfsSmem)) / 4;  // words of visited bits
+    const int words = std::min(room, (largest + 31) / 32);
+    const size_t smem = sizeof(BlockBfsSmem) + 4 * (size_t)words;
+    ck(cudaFuncSetAttribute(bfs_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attribute");
+    BlockBfsArgs b{d_rowptr, d_colids, d_voff, d_piv, d_list, d_dist, reinterpret_cast<int *>(cnt + 3), 32 * words};
+    bl_time_begin(ctx, "msbfs_kernel");
+    if (!rc) bfs_block_kernel<<<nblock * kP, kBlockThreads, smem, st>>>(b);
+    bl_time_end(ctx, "msbfs_kernel");
+    ctx->launches++;
+    ck(cudaGetLastError(), "BFS launch");
+    ck(cudaMemcpyAsync(&wide, cnt + 3, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H");
+    ck(cudaStreamSynchronize(st), "BFS");
+    if (!rc && wide) {  // a frontier outgrew a block's queue: every graph device-wide, from the start
+      nblock = 0;
+      ck(cudaMemsetAsync(d_dist, 0xff, sizeof(unsigned short) * kP * (size_t)n, st), "memset");
+    }
+  }
+  if (!rc && nblock < num_graphs) {
+    ck(cudaMalloc(&visited, sizeof(unsigned int) * n), "cudaMalloc");
+    ck(cudaMalloc(&fr0, sizeof(unsigned int) * n), "cudaMalloc");
+    ck(cudaMalloc(&fr1, sizeof(unsigned int) * n), "cudaMalloc");
+    ck(cudaMalloc(&wl0, sizeof(int) * n), "cudaMalloc");
+    ck(cudaMalloc(&wl1, sizeof(int) * n), "cudaMalloc");
+    if (rc) {
+      cleanup();
+      return rc;
+    }
+    const int seeds = (num_graphs - nblock) * kP;
+    bfs_init_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, visited, fr0, fr1);
+    bfs_seed_kernel<<<(seeds + 255) / 256, 256, 0, st>>>(seeds, d_list + nblock, d_piv, visited, fr0, d_dist, wl0,
+                                                         cnt);
+    ck(cudaMemsetAsync(&ctx->s.status->barrier, 0, sizeof(unsigned int), st), "memset");
+    ctx->launches += 2;
     int occ = 0;
     ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, msbfs_kernel, 512, 0), "occupancy");
     if (!rc && occ < 1) rc = bl_fail(ctx, BL_ERR_TOO_LARGE, "BFS kernel cannot be resident");
@@ -478,6 +671,8 @@ int bl_learned_features(bl_ctx *ctx, int n, const int *rowptr, const int *colids
   const long long nnz = rowptr[n];
   for (int v = 0; v < n; v++)
     if (rowptr[v + 1] < rowptr[v]) return bl_fail(ctx, BL_ERR_ARG, "rowptr decreases");
+  int max_row = 0;
+  for (int v = 0; v < n; v++) max_row = std::max(max_row, rowptr[v + 1] - rowptr[v]);
   for (long long e = 0; e < nnz; e++)
     if (colids[e] < 0 || colids[e] >= n) return bl_fail(ctx, BL_ERR_ARG, "colid out of range");
   int piv[kPivots];
@@ -510,7 +705,7 @@ int bl_learned_features(bl_ctx *ctx, int n, const int *rowptr, const int *colids
     if (nnz) ck(cudaMemcpy(d_ci, colids, sizeof(int) * nnz, cudaMemcpyHostToDevice), "H2D");
   }
   const int voff[2] = {0, n};
-  if (!rc) rc = compute_features(ctx, 1, voff, n, d_rp, d_ci, piv, d_f, d_d);
+  if (!rc) rc = compute_features(ctx, 1, voff, n, &max_row, d_rp, d_ci, piv, d_f, d_d);
   if (!rc) ck(cudaMemcpy(features, d_f, sizeof(float) * kFeat * (size_t)n, cudaMemcpyDeviceToHost), "D2H");
   if (!rc && dist) ck(cudaMemcpy(dist, d_d, sizeof(unsigned short) * kPivots * (size_t)n, cudaMemcpyDeviceToHost), "D2H");
   cudaFree(d_rp);

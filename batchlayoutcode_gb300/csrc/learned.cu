@@ -161,7 +161,9 @@ int learned_init(bl_ctx *ctx, const float *params, const double *scale_model, in
   int piv[kPivots];
   choose_pivots(n, (uint64_t)seed, piv);
   const int voff[2] = {0, n};
-  int rc = compute_features(ctx, 1, voff, n, ctx->g.rowptr, ctx->g.colids, piv, d_f, d_d);
+  int max_row = 0;
+  for (int v = 0; v < n; v++) max_row = std::max(max_row, ctx->h_rowptr[v + 1] - ctx->h_rowptr[v]);
+  int rc = compute_features(ctx, 1, voff, n, &max_row, ctx->g.rowptr, ctx->g.colids, piv, d_f, d_d);
   if (!rc) {
     f32_to_bf16_kernel<<<(int)((16LL * n + 255) / 256), 256, 0, ctx->stream>>>(d_f, mpnn_input(ctx), 16LL * n);
     ctx->launches++;
@@ -254,6 +256,7 @@ int bl_learned_train(bl_ctx *ctx, int num_graphs, const int *vertex_offset, cons
   gci.reserve((size_t)edge_offset[num_graphs]);
   std::vector<int> piv((size_t)num_graphs * kPivots);
   std::vector<double> logn(num_graphs), logd(num_graphs);
+  std::vector<int> max_row(num_graphs, 0);
   grp[0] = 0;
   for (int g = 0; g < num_graphs; g++) {
     const int v0 = vertex_offset[g], v1 = vertex_offset[g + 1], n = v1 - v0;
@@ -263,6 +266,7 @@ int bl_learned_train(bl_ctx *ctx, int num_graphs, const int *vertex_offset, cons
     if (rp[0] != 0 || rp[n] != m) return bl_fail(ctx, BL_ERR_ARG, "rowptr does not match edge_offset");
     for (int v = 0; v < n; v++) {
       if (rp[v + 1] < rp[v]) return bl_fail(ctx, BL_ERR_ARG, "rowptr decreases");
+      max_row[g] = std::max(max_row[g], rp[v + 1] - rp[v]);
       for (int e = rp[v]; e < rp[v + 1]; e++) {
         const int c = colids[e0 + e];
         if (c < 0 || c >= n) return bl_fail(ctx, BL_ERR_ARG, "colid out of range");
@@ -297,7 +301,8 @@ int bl_learned_train(bl_ctx *ctx, int num_graphs, const int *vertex_offset, cons
     ck(cudaMemcpy(d_rp, grp.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice), "H2D");
     ck(cudaMemcpy(d_ci, gci.data(), sizeof(int) * gci.size(), cudaMemcpyHostToDevice), "H2D");
   }
-  if (!rc) rc = compute_features(ctx, num_graphs, vertex_offset, N, d_rp, d_ci, piv.data(), d_f, d_d);
+  if (!rc)
+    rc = compute_features(ctx, num_graphs, vertex_offset, N, max_row.data(), d_rp, d_ci, piv.data(), d_f, d_d);
   std::vector<float> feat, target, vw;
   std::vector<double> logsig(num_graphs);
   if (!rc) {
