@@ -167,7 +167,7 @@ int learned_init(bl_ctx *ctx, const float *params, const double *scale_model, in
   if (!rc) {
     f32_to_bf16_kernel<<<(int)((16LL * n + 255) / 256), 256, 0, ctx->stream>>>(d_f, mpnn_input(ctx), 16LL * n);
     ctx->launches++;
-    rc = mpnn_forward(ctx, n, ctx->g.rowptr, ctx->g.colids, false);
+    rc = mpnn_forward(ctx, n, max_row, ctx->g.rowptr, ctx->g.colids, false);
   }
   if (!rc) {
     residual_start_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(mpnn_output(ctx), d_f, n, ctx->pos);
@@ -362,10 +362,11 @@ int bl_learned_train(bl_ctx *ctx, int num_graphs, const int *vertex_offset, cons
     f32_to_bf16_kernel<<<(int)((16LL * N + 255) / 256), 256, 0, ctx->stream>>>(d_f, mpnn_input(ctx), 16LL * N);
     ctx->launches++;
   }
+  const int longest = *std::max_element(max_row.begin(), max_row.end());
   for (int e = 0; e < epochs && !rc; e++) {
     const double lr_e = lr * 0.5 * (1.0 + std::cos(M_PI * e / std::max(epochs, 1)));
-    rc = mpnn_forward(ctx, N, d_rp, d_ci, true);
-    if (!rc) rc = mpnn_backward(ctx, N, d_rp, d_ci);
+    rc = mpnn_forward(ctx, N, longest, d_rp, d_ci, true);
+    if (!rc) rc = mpnn_backward(ctx, N, longest, d_rp, d_ci);
     double loss = 0.0;
     if (!rc && loss_history) rc = mpnn_loss(ctx, N, &loss);
     if (!rc && loss_history) loss_history[e] = loss;

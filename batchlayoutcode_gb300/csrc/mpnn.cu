@@ -8,8 +8,9 @@
 //   xy = h_3 Wo^T + bo.
 // Activations and weights are BF16, products accumulate in FP32 in tensor
 // memory.  Every layer is one persistent kernel over tiles of 128 vertices:
-// each thread gathers its vertex's row and the mean of its neighbours' rows
-// straight into the shared-memory A tile (K-major core matrices), one thread
+// groups of lanes, one lane per 16 bytes of a row, gather the vertices' rows
+// and the mean of their neighbours' rows straight into the shared-memory A tile
+// (K-major core matrices), one thread
 // issues the 128 x 64 x 16 tcgen05.mma steps, and the epilogue reads the
 // accumulator rows back with tcgen05.ld, adds the bias, applies ReLU and
 // writes the BF16 output row (and, for the last layer, the readout, the loss
@@ -78,9 +79,20 @@ __device__ __forceinline__ bool tile_mma_wait(uint64_t *mbar, uint32_t phase, in
   return *s_ok != 0;
 }
 
+// Rows longer than this are loaded by all groups of a block, a chunk at a time
+// through shared memory, and summed from there in row order: one group alone
+// would keep its tile waiting (a row of 2,000 neighbours, 500 us).  In a graph
+// with such rows the tiles take vertices ntiles apart, so that hubs with
+// neighbouring ids do not share a tile.  Forward pass of 380,000 power-law
+// vertices 2.8 -> 0.65 ms, an epoch over 12 graphs (208,000 vertices) 1.9 ->
+// 0.9 ms.
+constexpr int kLongRow = 64;
+constexpr int kLongChunk = 32;  // rows a chunk
+
 // ---- forward layer ------------------------------------------------------------
 struct FwdArgs {
   int n;
+  int spread;  // tile t takes vertices t, t + tiles, ... instead of 128 in a row
   const int *rowptr, *colids;
   const __nv_bfloat16 *hin;   // n x DIN
   __nv_bfloat16 *hout;        // n x 64
@@ -108,6 +120,8 @@ __global__ void __launch_bounds__(kT) mpnn_fwd_kernel(FwdArgs a) {
   __shared__ uint32_t tmem_base;
   __shared__ int s_ok;
   __shared__ double s_red[kT / 32];
+  __shared__ int s_nlong, s_long[kT];
+  __shared__ __align__(16) __nv_bfloat16 s_rows[kLongChunk][DIN];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int idx = tid; idx < 64 * (K / 8); idx += kT) {
     const int o = idx / (K / 8), c = idx % (K / 8);
@@ -125,40 +139,117 @@ __global__ void __launch_bounds__(kT) mpnn_fwd_kernel(FwdArgs a) {
   uint32_t phase = 0;
   double loss = 0.0;
   const int ntiles = (a.n + kT - 1) / kT;
+  // LPR lanes per row; group gr holds rows gr * LPR .. of the tile, lane gl the
+  // 16-byte chunk gl of each
+  constexpr int LPR = DIN / 8, CPL = 8 / LPR, kGroups = kT / LPR;
+  const int gl = tid % LPR, gr = tid / LPR, gbase = lane - gl;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int v = tile * kT + tid;
+    auto vertex = [&](int row) { return a.spread ? tile + row * ntiles : tile * kT + row; };
+    const int v = vertex(tid);
+    int e0 = 0, e1 = 0;
     if (v < a.n) {
-      const uint4 *hv = reinterpret_cast<const uint4 *>(a.hin + (size_t)v * DIN);
+      e0 = a.rowptr[v];
+      e1 = a.rowptr[v + 1];
+    }
+    if (tid == 0) s_nlong = 0;
+    __syncthreads();
+    const int deg = e1 - e0;
+    if (deg > kLongRow) s_long[atomicAdd(&s_nlong, 1)] = tid;
+    // the rows' first neighbour ids, one round trip for all of the group's rows
+    int first[LPR][CPL];
 #pragma unroll
-      for (int c = 0; c < DIN / 8; c++) *reinterpret_cast<uint4 *>(sA + tc::kmajor_offset(tid, c * 8, K)) = hv[c];
-      float acc[DIN];
+    for (int i = 0; i < LPR; i++) {
+      const int b0 = __shfl_sync(0xffffffffu, e0, gbase + i), b1 = __shfl_sync(0xffffffffu, e1, gbase + i);
 #pragma unroll
-      for (int k = 0; k < DIN; k++) acc[k] = 0.f;
-      const int e0 = a.rowptr[v], e1 = a.rowptr[v + 1];
-      for (int e = e0; e < e1; e++) {
-        const uint4 *hu = reinterpret_cast<const uint4 *>(a.hin + (size_t)a.colids[e] * DIN);
+      for (int j = 0; j < CPL; j++) {
+        const int e = b0 + gl + j * LPR;
+        first[i][j] = e < b1 && b1 - b0 <= kLongRow ? __ldg(&a.colids[e]) : 0;
+      }
+    }
 #pragma unroll
-        for (int c = 0; c < DIN / 8; c++) {
+    for (int i = 0; i < LPR; i++) {
+      const int row = gr * LPR + i, u = vertex(row);
+      const int b0 = __shfl_sync(0xffffffffu, e0, gbase + i), b1 = __shfl_sync(0xffffffffu, e1, gbase + i);
+      uint4 own = make_uint4(0, 0, 0, 0);
+      if (u < a.n) own = reinterpret_cast<const uint4 *>(a.hin + (size_t)u * DIN)[gl];
+      float acc[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) acc[k] = 0.f;
+      const int len = b1 - b0 <= kLongRow ? b1 - b0 : 0;
+      for (int d = 0; __any_sync(0xffffffffu, d < len); d += 8) {
+        int col[CPL];
+#pragma unroll
+        for (int j = 0; j < CPL; j++) {
+          col[j] = first[i][j];
+          if (d > 0) {
+            const int e = d + gl + j * LPR;
+            col[j] = e < len ? __ldg(&a.colids[b0 + e]) : 0;
+          }
+        }
+        uint4 q[8];  // eight rows in flight, summed in row order
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const int c = __shfl_sync(0xffffffffu, col[k / LPR], gbase + k % LPR);
+          q[k] = d + k < len ? reinterpret_cast<const uint4 *>(a.hin + (size_t)c * DIN)[gl] : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          if (d + k >= len) continue;
           float f[8];
-          bf16x8_to_f32(hu[c], f);
+          bf16x8_to_f32(q[k], f);
 #pragma unroll
-          for (int i = 0; i < 8; i++) acc[8 * c + i] += f[i];
+          for (int x = 0; x < 8; x++) acc[x] += f[x];
         }
       }
-      const float inv = (e1 > e0) ? 1.0f / (float)(e1 - e0) : 0.0f;
+      *reinterpret_cast<uint4 *>(sA + tc::kmajor_offset(row, gl * 8, K)) = own;
+      if (b1 - b0 <= kLongRow) {
+        const float inv = (b1 > b0) ? 1.0f / (float)(b1 - b0) : 0.0f;
 #pragma unroll
-      for (int c = 0; c < DIN / 8; c++) {
-        float f[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) f[i] = acc[8 * c + i] * inv;
-        const uint4 q = f32_to_bf16x8(f);
-        *reinterpret_cast<uint4 *>(sA + tc::kmajor_offset(tid, DIN + c * 8, K)) = q;
-        if (a.agg) *reinterpret_cast<uint4 *>(a.agg + (size_t)v * DIN + c * 8) = q;
+        for (int x = 0; x < 8; x++) acc[x] *= inv;
+        const uint4 m = f32_to_bf16x8(acc);
+        *reinterpret_cast<uint4 *>(sA + tc::kmajor_offset(row, DIN + gl * 8, K)) = m;
+        if (a.agg && u < a.n) *reinterpret_cast<uint4 *>(a.agg + (size_t)u * DIN + gl * 8) = m;
       }
-    } else {
+    }
+    __syncthreads();
+    // long rows: each group loads RPG rows of a chunk, one thread per feature
+    // adds them in row order while the next chunk is on its way
+    constexpr int RPG = kLongChunk / kGroups > 0 ? kLongChunk / kGroups : 1, kChunk = kLongChunk;
+    for (int x = 0; x < s_nlong; x++) {
+      const int row = s_long[x], u = vertex(row);
+      const int b0 = a.rowptr[u], b1 = a.rowptr[u + 1];
+      uint4 q[RPG];
+      auto load = [&](int e) {
 #pragma unroll
-      for (int c = 0; c < K / 8; c++)
-        *reinterpret_cast<uint4 *>(sA + tc::kmajor_offset(tid, c * 8, K)) = make_uint4(0, 0, 0, 0);
+        for (int k = 0; k < RPG; k++) {
+          const int y = e + gr * RPG + k;
+          q[k] = gr * RPG + k < kChunk && y < b1 ? reinterpret_cast<const uint4 *>(a.hin + (size_t)__ldg(&a.colids[y]) * DIN)[gl]
+                        : make_uint4(0, 0, 0, 0);
+        }
+      };
+      float sum = 0.f;
+      load(b0);
+      for (int e = b0; e < b1; e += kChunk) {
+#pragma unroll
+        for (int k = 0; k < RPG; k++)
+          if (gr * RPG + k < kChunk) *reinterpret_cast<uint4 *>(&s_rows[gr * RPG + k][gl * 8]) = q[k];
+        __syncthreads();
+        load(e + kChunk);
+        if (tid < DIN) {
+          const int m = min(kChunk, b1 - e);
+#pragma unroll 8
+          for (int k = 0; k < m; k++) sum += __bfloat162float(s_rows[k][tid]);
+        }
+        __syncthreads();
+      }
+      if (tid < DIN) s_rows[0][tid] = __float2bfloat16_rn(sum * (1.0f / (float)(b1 - b0)));
+      __syncthreads();
+      if (tid < LPR) {
+        const uint4 m = *reinterpret_cast<const uint4 *>(&s_rows[0][tid * 8]);
+        *reinterpret_cast<uint4 *>(sA + tc::kmajor_offset(row, DIN + tid * 8, K)) = m;
+        if (a.agg) *reinterpret_cast<uint4 *>(a.agg + (size_t)u * DIN + tid * 8) = m;
+      }
+      __syncthreads();
     }
     tc::fence_smem_to_async();
     __syncthreads();
@@ -478,35 +569,108 @@ __global__ void __launch_bounds__(kT) mpnn_dgrad_kernel(DgradArgs a) {
   if (warp == 0) tc::tmem_dealloc(tmem, N);
 }
 
-// dz_prev(v) = (P(v) + sum_{u in N(v)} G(u)) * [h_prev(v) > 0], 4 features a thread
-__global__ void mpnn_gather_kernel(int n, const int *__restrict__ rowptr, const int *__restrict__ colids,
-                                   const float *__restrict__ P, const float *__restrict__ G,
-                                   const __nv_bfloat16 *__restrict__ hprev, float *__restrict__ dz) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)n * 16) return;
-  const int v = (int)(t >> 4), c = (int)(t & 15);
-  float4 s = reinterpret_cast<const float4 *>(P + (size_t)v * 64)[c];
-  for (int e = rowptr[v]; e < rowptr[v + 1]; e++) {
-    const float4 g = reinterpret_cast<const float4 *>(G + (size_t)colids[e] * 64)[c];
+// dz_prev(v) = (P(v) + sum_{u in N(v)} G(u)) * [h_prev(v) > 0]: 16 lanes a
+// vertex, 4 features a lane, eight neighbours' rows in flight, summed in row
+// order; a row of more than kLongRow as in the forward pass.
+constexpr int kGatherVerts = 16, kGatherChunk = 64;
+__global__ void __launch_bounds__(kGatherVerts * 16) mpnn_gather_kernel(
+    int n, int spread, const int *__restrict__ rowptr, const int *__restrict__ colids, const float *__restrict__ P,
+    const float *__restrict__ G, const __nv_bfloat16 *__restrict__ hprev, float *__restrict__ dz) {
+  __shared__ int s_nlong, s_long[kGatherVerts];
+  __shared__ float4 s_rows[kGatherChunk][16];
+  const int grp = threadIdx.x >> 4, c = threadIdx.x & 15, lane = threadIdx.x & 31;
+  auto vertex = [&](int g) { return spread ? (int)blockIdx.x + g * (int)gridDim.x : (int)blockIdx.x * kGatherVerts + g; };
+  const int v = vertex(grp);
+  if (threadIdx.x == 0) s_nlong = 0;
+  __syncthreads();
+  auto finish = [&](int u, float4 s) {
+    const __nv_bfloat16 *h = hprev + (size_t)u * 64 + 4 * c;
+    s.x = __bfloat162float(h[0]) > 0.f ? s.x : 0.f;
+    s.y = __bfloat162float(h[1]) > 0.f ? s.y : 0.f;
+    s.z = __bfloat162float(h[2]) > 0.f ? s.z : 0.f;
+    s.w = __bfloat162float(h[3]) > 0.f ? s.w : 0.f;
+    reinterpret_cast<float4 *>(dz + (size_t)u * 64)[c] = s;
+  };
+  auto add = [](float4 &s, const float4 &g) {
     s.x += g.x;
     s.y += g.y;
     s.z += g.z;
     s.w += g.w;
+  };
+  int b0 = 0, len = 0;
+  if (v < n) {
+    b0 = rowptr[v];
+    len = rowptr[v + 1] - b0;
   }
-  const __nv_bfloat16 *h = hprev + (size_t)v * 64 + 4 * c;
-  s.x = __bfloat162float(h[0]) > 0.f ? s.x : 0.f;
-  s.y = __bfloat162float(h[1]) > 0.f ? s.y : 0.f;
-  s.z = __bfloat162float(h[2]) > 0.f ? s.z : 0.f;
-  s.w = __bfloat162float(h[3]) > 0.f ? s.w : 0.f;
-  reinterpret_cast<float4 *>(dz + (size_t)v * 64)[c] = s;
+  const bool is_long = len > kLongRow;
+  if (is_long && c == 0) s_long[atomicAdd(&s_nlong, 1)] = grp;
+  const int todo = is_long ? 0 : len;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (v < n) s = reinterpret_cast<const float4 *>(P + (size_t)v * 64)[c];
+  for (int d = 0; __any_sync(0xffffffffu, d < todo); d += 16) {
+    const int col = d + c < todo ? __ldg(&colids[b0 + d + c]) : 0;
+#pragma unroll
+    for (int h = 0; h < 16; h += 8) {
+      float4 g[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const int u = __shfl_sync(0xffffffffu, col, (lane & 16) + h + k);
+        if (d + h + k < todo) g[k] = reinterpret_cast<const float4 *>(G + (size_t)u * 64)[c];
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (d + h + k < todo) add(s, g[k]);
+    }
+  }
+  if (v < n && !is_long) finish(v, s);
+  __syncthreads();
+  constexpr int RPG = kGatherChunk / kGatherVerts;
+  for (int x = 0; x < s_nlong; x++) {
+    const int u = vertex(s_long[x]);
+    const int r0 = rowptr[u], r1 = rowptr[u + 1];
+    float4 g[RPG];
+    auto load = [&](int e) {
+#pragma unroll
+      for (int k = 0; k < RPG; k++) {
+        const int y = e + grp * RPG + k;
+        if (y < r1) g[k] = reinterpret_cast<const float4 *>(G + (size_t)__ldg(&colids[y]) * 64)[c];
+      }
+    };
+    load(r0);
+    float4 t = reinterpret_cast<const float4 *>(P + (size_t)u * 64)[c];
+    for (int e = r0; e < r1; e += kGatherChunk) {
+#pragma unroll
+      for (int k = 0; k < RPG; k++) s_rows[grp * RPG + k][c] = g[k];
+      __syncthreads();
+      load(e + kGatherChunk);
+      if (grp == 0) {
+        const int m = min(kGatherChunk, r1 - e);
+#pragma unroll 8
+        for (int k = 0; k < m; k++) add(t, s_rows[k][c]);
+      }
+      __syncthreads();
+    }
+    if (grp == 0) finish(u, t);
+  }
 }
 
-// sum of per-block partials in block order: out[i] = sum_b part[b * len + i]
-__global__ void mpnn_reduce_kernel(const float *__restrict__ part, int blocks, int len, float *__restrict__ out) {
+// sum of per-block partials in block order: out[i] = sum_b part[b * len + i];
+// 32 loads in flight (608 partials one after another took 41 us)
+__global__ void __launch_bounds__(64) mpnn_reduce_kernel(const float *__restrict__ part, int blocks, int len,
+                                                         float *__restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= len) return;
   float s = 0.f;
-  for (int b = 0; b < blocks; b++) s += part[(size_t)b * len + i];
+  const float *p = part + i;
+  int b = 0;
+  for (; b + 32 <= blocks; b += 32, p += (size_t)32 * len) {
+    float v[32];
+#pragma unroll
+    for (int k = 0; k < 32; k++) v[k] = __ldg(p + (size_t)k * len);
+#pragma unroll
+    for (int k = 0; k < 32; k++) s += v[k];
+  }
+  for (; b < blocks; b++, p += len) s += __ldg(p);
   out[i] = s;
 }
 
@@ -639,14 +803,15 @@ int sync_weights(bl_ctx *ctx) {
 }  // namespace
 
 // Forward over a graph already on the device (n vertices, CSR rowptr/colids,
-// features in m.x).  With `train`, keeps the aggregates, computes the loss
+// features in m.x, longest row max_row).  With `train`, keeps the aggregates, computes the loss
 // against m.target/m.vweight and its gradient dxy.
-int mpnn_forward(bl_ctx *ctx, int n, const int *d_rowptr, const int *d_colids, bool train) {
+int mpnn_forward(bl_ctx *ctx, int n, int max_row, const int *d_rowptr, const int *d_colids, bool train) {
   MpnnState &m = *ctx->mpnn;
   cudaStream_t st = ctx->stream;
   const int grid = std::min(m.grid, std::max(1, nblk(n, kT)));
   FwdArgs a{};
   a.n = n;
+  a.spread = max_row > kLongRow ? 1 : 0;
   a.rowptr = d_rowptr;
   a.colids = d_colids;
   a.st = ctx->s.status;
@@ -679,13 +844,13 @@ int mpnn_forward(bl_ctx *ctx, int n, const int *d_rowptr, const int *d_colids, b
 }
 
 // Backward after a training forward: gradient of the loss into m.grad.
-int mpnn_backward(bl_ctx *ctx, int n, const int *d_rowptr, const int *d_colids) {
+int mpnn_backward(bl_ctx *ctx, int n, int max_row, const int *d_rowptr, const int *d_colids) {
   MpnnState &m = *ctx->mpnn;
   cudaStream_t st = ctx->stream;
   const int grid = std::min(m.grid, std::max(1, nblk(n, kT)));
   TopArgs t{n, m.dxy, m.h[2], m.params + kOffWo, m.dz, m.part};
   mpnn_top_kernel<<<grid, kT, 0, st>>>(t);
-  mpnn_reduce_kernel<<<1, 256, 0, st>>>(m.part, grid, 130, m.grad + kOffWo);
+  mpnn_reduce_kernel<<<nblk(130, 64), 64, 0, st>>>(m.part, grid, 130, m.grad + kOffWo);
   ctx->launches += 2;
   for (int l = 2; l >= 0; l--) {
     const int din = l == 0 ? 16 : 64;
@@ -693,14 +858,14 @@ int mpnn_backward(bl_ctx *ctx, int n, const int *d_rowptr, const int *d_colids) 
     WgradArgs w{n, l == 0 ? m.x : m.h[l - 1], m.agg[l], m.dz, m.part, ctx->s.status};
     if (l == 0) mpnn_wgrad_kernel<16><<<grid, kT, kT * kT * 2 + 64 * kT * 2, st>>>(w);
     else mpnn_wgrad_kernel<64><<<grid, kT, kT * kT * 2 + 64 * kT * 2, st>>>(w);
-    mpnn_reduce_kernel<<<nblk(len, 256), 256, 0, st>>>(m.part, grid, len, m.grad + kOffW[l]);
+    mpnn_reduce_kernel<<<nblk(len, 64), 64, 0, st>>>(m.part, grid, len, m.grad + kOffW[l]);
     ctx->launches += 2;
     BL_CUDA(ctx, cudaGetLastError());
     if (l > 0) {
       DgradArgs d{n, d_rowptr, m.dz, m.wbf + kOffW[l], m.P, m.G, ctx->s.status};
       mpnn_dgrad_kernel<64><<<grid, kT, kT * 64 * 2 + 128 * 64 * 2, st>>>(d);
-      mpnn_gather_kernel<<<nblk((long long)n * 16, 256), 256, 0, st>>>(n, d_rowptr, d_colids, m.P, m.G, m.h[l - 1],
-                                                                      m.dz);
+      mpnn_gather_kernel<<<nblk(n, kGatherVerts), kGatherVerts * 16, 0, st>>>(
+          n, max_row > kLongRow ? 1 : 0, d_rowptr, d_colids, m.P, m.G, m.h[l - 1], m.dz);
       ctx->launches += 2;
       BL_CUDA(ctx, cudaGetLastError());
     }
@@ -791,6 +956,8 @@ int bl_mpnn_run(bl_ctx *ctx, int n, const int *rowptr, const int *colids, const 
   const long long nnz = rowptr[n];
   for (int v = 0; v < n; v++)
     if (rowptr[v + 1] < rowptr[v]) return bl_fail(ctx, BL_ERR_ARG, "rowptr decreases");
+  int max_row = 0;
+  for (int v = 0; v < n; v++) max_row = std::max(max_row, rowptr[v + 1] - rowptr[v]);
   for (long long e = 0; e < nnz; e++)
     if (colids[e] < 0 || colids[e] >= n) return bl_fail(ctx, BL_ERR_ARG, "colid out of range");
   if (int rc = ensure_mpnn(ctx, n)) return rc;
@@ -816,8 +983,8 @@ int bl_mpnn_run(bl_ctx *ctx, int n, const int *rowptr, const int *colids, const 
       cudaMemcpyAsync(m.target, target, sizeof(float) * 2 * (size_t)n, cudaMemcpyHostToDevice, st);
       cudaMemcpyAsync(m.vweight, vweight, sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, st);
     }
-    rc = mpnn_forward(ctx, n, d_rp, d_ci, target != nullptr);
-    if (!rc && target) rc = mpnn_backward(ctx, n, d_rp, d_ci);
+    rc = mpnn_forward(ctx, n, max_row, d_rp, d_ci, target != nullptr);
+    if (!rc && target) rc = mpnn_backward(ctx, n, max_row, d_rp, d_ci);
     if (!rc && (e = cudaStreamSynchronize(st)) != cudaSuccess) fail(e, "mpnn kernels");
     if (!rc) rc = bl_check_status(ctx);
     if (!rc) {

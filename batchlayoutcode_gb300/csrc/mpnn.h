@@ -16,8 +16,8 @@ constexpr int kMpnnParams = 64 * 32 + 64 + 2 * (64 * 128 + 64) + 2 * 64 + 2;
 
 int mpnn_prepare(bl_ctx *ctx, int n);
 int mpnn_set_params_device(bl_ctx *ctx, const float *h_params);
-int mpnn_forward(bl_ctx *ctx, int n, const int *d_rowptr, const int *d_colids, bool train);
-int mpnn_backward(bl_ctx *ctx, int n, const int *d_rowptr, const int *d_colids);
+int mpnn_forward(bl_ctx *ctx, int n, int max_row, const int *d_rowptr, const int *d_colids, bool train);
+int mpnn_backward(bl_ctx *ctx, int n, int max_row, const int *d_rowptr, const int *d_colids);
 int mpnn_loss(bl_ctx *ctx, int n, double *loss);
 int mpnn_adam_step(bl_ctx *ctx, double lr);
 // device buffers of the prepared network: BF16 input features (n x 16),
