@@ -174,7 +174,7 @@ void free_ctx(bl_ctx *c) {
   fr(s.perm); fr(s.perm_alt); fr(s.hist); fr(s.bbox); fr(s.frame); fr(s.spos); fr(s.bparent);
   fr(s.bchild); fr(s.brange); fr(s.bdelta); fr(s.qkids); fr(s.qpar); fr(s.qnchild); fr(s.span); fr(s.span_stage); fr(s.ztab); fr(s.chain); fr(s.qcen); fr(s.qbelow); fr(s.startcnt);
   fr(s.startbase); fr(s.nodes); fr(s.nodes_c64); fr(s.nodes_lvl); fr(s.rep);
-  fr(s.stats); fr(s.pos_alt); fr(s.f0); fr(s.runs); fr(s.bnode); fr(s.walk_off); fr(s.walk_pairs);
+  fr(s.stats); fr(s.pos_alt); fr(s.f0); fr(s.runs); fr(s.bnode); fr(s.pairs); fr(s.walk_off); fr(s.walk_pairs);
   fr(s.term_off); fr(s.terms); fr(s.term_tgt); fr(s.greedy_share); fr(s.greedy_pos);
   for (auto &ls : c->schedules) {
     fr(ls.order);
@@ -361,7 +361,7 @@ bl_ctx *bl_algorithms_create(int device, int n, long long nnz, const int *rowptr
   if ((e = cudaMalloc(&ctx->s.energy, 16 * sizeof(double))) != cudaSuccess) return bad(e, "cudaMalloc");
   if ((e = cudaMalloc(&ctx->s.status, sizeof(DevStatus))) != cudaSuccess) return bad(e, "cudaMalloc");
   if ((e = cudaMalloc(&ctx->s.bbox, 8 * sizeof(unsigned int))) != cudaSuccess) return bad(e, "cudaMalloc");
-  if ((e = cudaMalloc(&ctx->s.frame, 4 * sizeof(double))) != cudaSuccess) return bad(e, "cudaMalloc");
+  if ((e = cudaMalloc(&ctx->s.frame, 16 * sizeof(double))) != cudaSuccess) return bad(e, "cudaMalloc");
   if ((e = cudaMalloc(&ctx->s.stats, 2 * sizeof(unsigned long long))) != cudaSuccess) return bad(e, "cudaMalloc");
   cudaMemset(ctx->pos, 0, m * sizeof(float2));
   cudaMemset(ctx->force, 0, m * sizeof(double2));

@@ -8,9 +8,9 @@
 //   1. bbox of the positions; Morton frame {minX, minY, MAXMIN} and 64-bit keys
 //      (y-major interleave of the two 32-bit quantised coordinates, quantised
 //      in FP64 exactly as the reference: (uint32)(4294967295.0*(x-minX)/MAXMIN)).
-//   2. stable LSD radix sort of (key, vertex) pairs on the high 32 bits (4
-//      passes of 8 bits), then each run of equal high halves sorted on its
-//      own (they are rare).
+//   2. stable LSD radix sort of the keys on the high 32 bits (4 passes of 8
+//      bits), then each run of equal high halves sorted on its own (they are
+//      rare); 1 and 2 are one cooperative launch.
 //   3. binary radix tree over the sorted keys (Karras 2012), then a bottom-up
 //      pass that merges the x-bit level into the y-bit level of the same
 //      digit, giving exactly the reference quadtree without its single-child
@@ -44,284 +44,323 @@ namespace {
 constexpr int kQuadLevels = 33;  // quad levels 0..31, 32 for runs of identical keys
 
 
-// ---- stable LSD radix sort, 8-bit digits ------------------------------------
+// ---- box, keys and order: one cooperative launch --------------------------------
 //
-// Each digit pass is three kernels without any inter-block waiting: the tile
-// digit counts (hist[d * ntiles + tile]), one block that turns every digit
-// row into exclusive offsets across tiles and scans the digit totals, and the
-// scatter, which ranks its tile's keys stably and writes them to
-// digit offset + row offset + rank.  Tiles are 2,048 keys (one wave of four
-// 256-thread blocks per SM for a million keys; 1,024-key tiles took 1.3
-// waves and 6 % longer); warp w of a block owns keys [w*256, (w+1)*256) of
-// its tile and ranks them with warp-private counters, so no block barrier
-// sits inside the ranking loop.
-constexpr int kRsThreads = 256;
-constexpr int kRsItems = 8;
-constexpr int kRsTile = kRsThreads * kRsItems;
-constexpr int kRsWarps = kRsThreads / 32;
+// Bounding box of the positions (MortonCode.h:42-58), the FP64 frame
+// {minX, minY, MAXMIN, 1/MAXMIN}, the high half of every point's 64-bit Morton
+// key, and a stable LSD radix sort of (high half, vertex) words on it (four
+// 8-bit digits).  The points are cut into tiles of r * 512 (r such that one
+// tile per resident block covers them where r <= 16 does); a block takes tiles
+// b, b + grid, ...  Per digit pass:
+//   - a tile's keys are ranked stably: warp w owns r * 32 consecutive keys and
+//     counts with warp-private counters, so no block barrier sits in the
+//     ranking; the keys are placed in shared memory grouped by digit (with
+//     more than one tile a block, then written back where they were read);
+//     the tile's digit counts go to hist[tile][256] and are added to the
+//     totals of the tile's group (16 groups);
+//   - grid barrier;
+//   - a tile's offset of a digit = the digit's global offset + the groups
+//     before + the tiles before in its group: 16 + tiles / 16 loads a thread,
+//     all independent, in place of a scan over all tiles;
+//   - the grouped keys are written out, each digit's run of the tile as whole
+//     sectors;
+//   - grid barrier.
+// Bound by the nine barriers and the L2 round trips between them at small
+// sizes (2 us of the 3 us a half pass takes at 100,000 points) and by the
+// ranking's shared-memory traffic at large ones (9,000 of a pass's 25,000
+// cycles at a million).  As sixteen launches (frame and keys, three a digit
+// pass, two for the runs, a gather) the stage up to the sorted positions took
+// 104 us at 4,000 points, 103 at 100,000, 160 at 1,000,000 and 346 at
+// 3,000,000; it takes 43, 51, 90 and 206.  One cluster of 16 blocks that keeps
+// everything in shared memory took 26 us at 4,000 but 97 at 100,000.
+constexpr int kSortThreads = 512;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kSortItems = 16;
+constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr int kSortGroups = 16;
 
-__global__ void __launch_bounds__(kRsThreads) rs_count_kernel(const u64 *__restrict__ keys, int n, int shift,
-                                                              int ntiles, unsigned int *hist) {
-  __shared__ unsigned int cnt[kRsWarps][256];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-#pragma unroll
-  for (int w = 0; w < kRsWarps; w++) cnt[w][tid] = 0;
+__device__ __forceinline__ unsigned int hi32(u64 k) { return (unsigned int)(k >> 32); }
+
+struct SortSmem {
+  u64 key[kSortTile];                     // a tile's words grouped by digit
+  unsigned short rank[kSortTile];         // of a key among its warp's and its digit's
+  unsigned int wcnt[kSortWarps][256];     // per-warp digit counts, then offsets within the digit
+  // first key of each digit: position in the tile; global position less that
+  unsigned int base[256], loc[256];
+  unsigned int ws[kSortWarps];
+  unsigned int box[kSortWarps][4];
+  KeyFrame frame;
+  unsigned int ok;
+};
+
+struct SortArgs {
+  const float2 *pos;
+  int n, items, ntiles, group;  // keys per thread, tiles, tiles per group
+  // all bits set before the launch: {min x, ~max x, min y, ~max y} as ordered
+  // integers, barrier arrivals
+  unsigned int *ctl;
+  double *frame;
+  KeyFrame *kframe;
+  double inv_theta2;
+  float *ztab;
+  u64 *pairs0, *pairs1;  // (high half << 32) | vertex; a pass reads one and writes the other
+  unsigned int *hist;    // [tiles][256]
+  unsigned int *gtot;    // [4 passes][kSortGroups][256]
+  int *runs;             // count of the long runs (cleared)
+  int *zero0, *zero1;    // cleared for the tree kernels
+  int nzero0, nzero1;
+  DevStatus *st;
+};
+
+// Grid barrier `k` (1, 2, ...) of a launch; false when the kernel has to end.
+__device__ __forceinline__ bool sort_barrier(const SortArgs &a, SortSmem &S, unsigned int k) {
   __syncthreads();
-  const int wbase = blockIdx.x * kRsTile + warp * (kRsItems * 32);
-#pragma unroll 4
-  for (int r = 0; r < kRsItems; r++) {
-    const int idx = wbase + r * 32 + lane;
-    if (idx < n) atomicAdd(&cnt[warp][(unsigned int)(keys[idx] >> shift) & 255u], 1u);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicSub(&a.ctl[4], 1u);
+    const unsigned int target = 0xffffffffu - k * gridDim.x;
+    const unsigned long long t0 = dev_globaltimer();
+    unsigned int ok = 1, polls = 0;
+    while (ld_acquire_gpu(&a.ctl[4]) > target) {
+      if ((++polls & 127u) == 0u) {
+        if (ld_volatile_u32(&a.st->code) != 0u) {
+          ok = 0;
+          break;
+        }
+        if (dev_globaltimer() - t0 > kBarrierTimeoutNs) {
+          dev_record_error(a.st, DEV_TIMEOUT_GRID_BARRIER);
+          ok = 0;
+          break;
+        }
+      }
+    }
+    S.ok = ok;
   }
   __syncthreads();
-  unsigned int tot = 0;
-#pragma unroll
-  for (int w = 0; w < kRsWarps; w++) tot += cnt[w][tid];
-  hist[(size_t)tid * ntiles + blockIdx.x] = tot;
+  return S.ok != 0u;
 }
 
-// Block d turns digit row d (ntiles contiguous counts) into exclusive
-// offsets across tiles, 256 tiles at a time, and stores the row total.
-__global__ void __launch_bounds__(256) rs_rowscan_kernel(unsigned int *hist, int ntiles,
-                                                         unsigned int *row_total) {
-  __shared__ unsigned int ws[8];
-  __shared__ unsigned int carry;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  unsigned int *row = hist + (size_t)blockIdx.x * ntiles;
-  if (tid == 0) carry = 0;
-  __syncthreads();
-  for (int c0 = 0; c0 < ntiles; c0 += 256) {
-    const int b = c0 + tid;
-    const unsigned int v = (b < ntiles) ? row[b] : 0u;
-    unsigned int x = v;
+// Lanes of the warp with the same digit (256: none).  Eight ballots: with
+// a __match_any_sync the ranking of a million keys took 16,600 cycles a pass,
+// so it takes 12,000 with the placing.
+__device__ __forceinline__ unsigned int digit_peers(unsigned int d) {
+  unsigned int peers = __ballot_sync(0xffffffffu, d < 256u);
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    const bool one = (d >> b) & 1u;
+    const unsigned int m = __ballot_sync(0xffffffffu, one);
+    peers &= one ? m : ~m;
+  }
+  return peers;
+}
+
+// Exclusive scan over the first 256 threads; every thread of the block calls it.
+__device__ __forceinline__ unsigned int sort_scan256(unsigned int v, SortSmem &S) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned int x = v;
+  if (tid < 256) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
-    if (lane == 31) ws[w] = x;
-    __syncthreads();
-    unsigned int wpre = 0, total = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const unsigned int t = ws[k];
-      if (k < w) wpre += t;
-      total += t;
-    }
-    const unsigned int base = carry;
-    if (b < ntiles) row[b] = base + wpre + x - v;
-    __syncthreads();
-    if (tid == 0) carry = base + total;
-    __syncthreads();
+    if (lane == 31) S.ws[warp] = x;
   }
-  if (tid == 0) row_total[blockIdx.x] = carry;
+  __syncthreads();
+  unsigned int pre = 0;
+  if (tid < 256)
+    for (int w = 0; w < warp; w++) pre += S.ws[w];
+  __syncthreads();
+  return pre + x - v;
 }
 
-// Exclusive scan of one value per thread over a 256-thread block (ws: 8
-// words of shared scratch); every thread calls it.
-__device__ __forceinline__ unsigned int rs_block_scan256(unsigned int v, unsigned int *ws) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  unsigned int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) ws[warp] = x;
-  __syncthreads();
-  unsigned int wpre = 0;
-#pragma unroll
-  for (int k = 0; k < kRsWarps; k++)
-    if (k < warp) wpre += ws[k];
-  __syncthreads();
-  return wpre + x - v;
-}
-
-// The tile's keys are ranked (stably: warp order, then lane order within a
-// warp's 32-key rows), placed in shared memory grouped by digit, and written
-// out from there: consecutive threads write consecutive keys of a digit's
-// run, so each run of the tile reaches L2 as whole sectors rather than as one
-// partial sector per key.
-__global__ void __launch_bounds__(kRsThreads) rs_scatter_kernel(
-    const u64 *__restrict__ kin, const int *__restrict__ vin, u64 *__restrict__ kout, int *__restrict__ vout,
-    int n, int shift, int ntiles, const unsigned int *__restrict__ hist, const unsigned int *__restrict__ row_total) {
-  __shared__ unsigned int s_cnt[kRsWarps][256];  // per-warp counts, then per-warp offsets within the digit
-  __shared__ unsigned int s_base[256];            // global position of the tile's first key of each digit
-  __shared__ unsigned int s_loc[256];             // position of the tile's first key of each digit in the tile
-  __shared__ unsigned int s_ws[kRsWarps];
-  __shared__ u64 s_key[kRsTile];
-  __shared__ int s_val[kRsTile];
+// A tile of the pass's input grouped by digit in S.key (stable), the first
+// position of each digit in S.loc; returns the digit counts to threads
+// 0..255.
+__device__ __forceinline__ unsigned int sort_rank_tile(const SortArgs &a, SortSmem &S, const u64 *in, int shift,
+                                                       int tile) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-#pragma unroll
-  for (int w = 0; w < kRsWarps; w++) s_cnt[w][tid] = 0;
-  // digit offset = exclusive scan of the 256 row totals (every block does it)
-  s_base[tid] = rs_block_scan256(row_total[tid], s_ws) + hist[(size_t)tid * ntiles + blockIdx.x];
-  const int wbase = blockIdx.x * kRsTile + warp * (kRsItems * 32);
   const unsigned int lt = (1u << lane) - 1u;
-  u64 key[kRsItems];
-  int val[kRsItems];
-  unsigned int rd[kRsItems];  // rank within the warp's keys (low 16 bits) | digit << 16, digit 256 = none
 #pragma unroll
-  for (int r = 0; r < kRsItems; r++) {
-    const int idx = wbase + r * 32 + lane;
-    const bool valid = idx < n;
-    key[r] = valid ? kin[idx] : 0ull;
-    val[r] = valid ? vin[idx] : 0;
-    const unsigned int d = valid ? ((unsigned int)(key[r] >> shift) & 255u) : 256u;
-    const unsigned int peers = __match_any_sync(0xffffffffu, d);
-    const unsigned int leader = __ffs(peers) - 1;
-    unsigned int old = 0;
-    if (d < 256u) old = s_cnt[warp][d];
-    __syncwarp();
-    if (d < 256u && lane == leader) s_cnt[warp][d] = old + __popc(peers);
-    __syncwarp();
-    rd[r] = (old + __popc(peers & lt)) | (d << 16);
+  for (int k = 0; k < 256 / 32; k++) S.wcnt[warp][k * 32 + lane] = 0u;
+  __syncwarp();
+  const int first = warp * a.items * 32, i0 = tile * a.items * kSortThreads + first;
+  for (int r0 = 0; r0 < a.items; r0 += 4) {
+    unsigned int dg[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {  // four loads in flight
+      const int i = i0 + (r0 + q) * 32 + lane;
+      dg[q] = r0 + q < a.items && i < a.n ? ((unsigned int)(__ldcg(&in[i]) >> shift) & 255u) : 256u;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (r0 + q >= a.items) break;
+      const unsigned int d = dg[q];
+      const unsigned int peers = digit_peers(d);
+      unsigned int old = 0;
+      if (d < 256u) old = S.wcnt[warp][d];
+      __syncwarp();
+      if (d < 256u && (peers & lt) == 0u) S.wcnt[warp][d] = old + __popc(peers);
+      __syncwarp();
+      S.rank[first + (r0 + q) * 32 + lane] = (unsigned short)(old + __popc(peers & lt));
+    }
   }
   __syncthreads();
   unsigned int run = 0;
+  if (tid < 256) {
 #pragma unroll
-  for (int w = 0; w < kRsWarps; w++) {
-    const unsigned int c = s_cnt[w][tid];
-    s_cnt[w][tid] = run;
-    run += c;
-  }
-  s_loc[tid] = rs_block_scan256(run, s_ws);  // its barriers also publish s_cnt
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < kRsItems; r++) {
-    const unsigned int d = rd[r] >> 16;
-    if (d < 256u) {
-      const unsigned int p = s_loc[d] + s_cnt[warp][d] + (rd[r] & 0xffffu);
-      s_key[p] = key[r];
-      s_val[p] = val[r];
+    for (int w = 0; w < kSortWarps; w++) {
+      const unsigned int c = S.wcnt[w][tid];
+      S.wcnt[w][tid] = run;
+      run += c;
     }
   }
+  const unsigned int loff = sort_scan256(run, S);
+  if (tid < 256) S.loc[tid] = loff;
   __syncthreads();
-  const int cnt = min(kRsTile, n - (int)blockIdx.x * kRsTile);
-  for (int p = tid; p < cnt; p += kRsThreads) {
-    const u64 k = s_key[p];
-    const unsigned int d = (unsigned int)(k >> shift) & 255u;
-    const unsigned int g = s_base[d] + ((unsigned int)p - s_loc[d]);
-    if (g < (unsigned int)n) {
-      kout[g] = k;
-      vout[g] = s_val[p];
-    }
-  }
-}
-
-// ---- frame and keys: one cooperative launch ---------------------------------
-//
-// Bounding box of the positions (MortonCode.h:42-58), the FP64 frame
-// {minX, minY, MAXMIN, 1/MAXMIN} and the 64-bit Morton key of every point,
-// together with the tile digit counts of the first sort pass (bits
-// shift..shift+7), so that pass starts at its row scan.  Block b handles
-// sort tiles b, b + grid, ...; one grid barrier separates the box from the
-// keys.  box[0..3] = {min x, ~max x, min y, ~max y} in the order-preserving
-// integer form of the floats and box[4] the arrivals, all reset to
-// 0xffffffff before the launch: every slot only decreases.
-__global__ void __launch_bounds__(kRsThreads, 8) frame_keys_kernel(const float2 *__restrict__ pos, int n, int ntiles,
-                                                                unsigned int *box, double *frame, u64 *keys,
-                                                                int *vals, int shift, unsigned int *hist,
-                                                                double inv_theta2, float *ztab, DevStatus *st) {
-  __shared__ unsigned int s_box[kRsWarps][4];
-  __shared__ unsigned int cnt[kRsWarps][256];
-  __shared__ double s_frame[4];
-  __shared__ unsigned int s_ok;
-  if (!block_status_ok(st)) return;  // every block sees the same value: no barrier is left waiting
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  unsigned int mnx = 0xffffffffu, mxx = 0u, mny = 0xffffffffu, mxy = 0u;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  for (int r0 = 0; r0 < a.items; r0 += 4) {
+    u64 k[4];
 #pragma unroll
-    for (int r = 0; r < kRsItems; r++) {
-      const int idx = tile * kRsTile + r * kRsThreads + tid;
-      if (idx < n) {
-        const float2 p = pos[idx];
-        const unsigned int ux = f2ord(p.x), uy = f2ord(p.y);
-        mnx = min(mnx, ux); mxx = max(mxx, ux);
-        mny = min(mny, uy); mxy = max(mxy, uy);
+    for (int q = 0; q < 4; q++) {
+      const int i = i0 + (r0 + q) * 32 + lane;
+      if (r0 + q < a.items && i < a.n) k[q] = __ldcg(&in[i]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int i = i0 + (r0 + q) * 32 + lane;
+      if (r0 + q < a.items && i < a.n) {
+        const unsigned int d = (unsigned int)(k[q] >> shift) & 255u;
+        S.key[S.loc[d] + S.wcnt[warp][d] + S.rank[first + (r0 + q) * 32 + lane]] = k[q];
       }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    mnx = min(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-    mxx = max(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-    mny = min(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-    mxy = max(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+  return run;
+}
+
+__global__ void __launch_bounds__(kSortThreads, 2) morton_sort_kernel(SortArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SortSmem &S = *reinterpret_cast<SortSmem *>(smem_raw);
+  if (!block_status_ok(a.st)) return;  // every block sees the same value: no barrier is left waiting
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tsize = a.items * kSortThreads;
+  const bool single = a.ntiles <= (int)gridDim.x;  // one tile a block: its ranks stay
+  unsigned int nbar = 0;
+  // box
+  unsigned int bb[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+  for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
+#pragma unroll 4
+    for (int r = 0; r < a.items; r++) {
+      const int i = tile * tsize + r * kSortThreads + tid;
+      if (i < a.n) {
+        const float2 p = a.pos[i];
+        const unsigned int ux = f2ord(p.x), uy = f2ord(p.y);
+        bb[0] = min(bb[0], ux);
+        bb[1] = min(bb[1], ~ux);
+        bb[2] = min(bb[2], uy);
+        bb[3] = min(bb[3], ~uy);
+      }
+    }
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    bb[c] = __reduce_min_sync(0xffffffffu, bb[c]);
+    if (lane == 0) S.box[warp][c] = bb[c];
   }
-  if (lane == 0) {
-    s_box[warp][0] = mnx;
-    s_box[warp][1] = ~mxx;
-    s_box[warp][2] = mny;
-    s_box[warp][3] = ~mxy;
-  }
+  // what this launch and the tree kernels count from zero
+  const int gid = blockIdx.x * kSortThreads + tid, gsz = gridDim.x * kSortThreads;
+  for (int k = gid; k < 4 * kSortGroups * 256; k += gsz) a.gtot[k] = 0u;
+  for (int k = gid; k < a.nzero0; k += gsz) a.zero0[k] = 0;
+  for (int k = gid; k < a.nzero1; k += gsz) a.zero1[k] = 0;
+  if (gid == 0) a.runs[0] = 0;
   __syncthreads();
   if (tid < 4) {
     unsigned int v = 0xffffffffu;
 #pragma unroll
-    for (int w = 0; w < kRsWarps; w++) v = min(v, s_box[w][tid]);
-    atomicMin(&box[tid], v);
+    for (int w = 0; w < kSortWarps; w++) v = min(v, S.box[w][tid]);
+    atomicMin(&a.ctl[tid], v);
   }
-  __syncthreads();
+  if (!sort_barrier(a, S, ++nbar)) return;
   if (tid == 0) {
-    __threadfence();
-    atomicSub(&box[4], 1u);
-    const unsigned int target = 0xffffffffu - gridDim.x;  // every block arrived
-    const unsigned long long t0 = dev_globaltimer();
-    unsigned int ok = 1, polls = 0;
-    while (ld_acquire_gpu(&box[4]) > target) {
-      if ((++polls & 127u) == 0u && dev_globaltimer() - t0 > kBarrierTimeoutNs) {
-        dev_record_error(st, DEV_TIMEOUT_GRID_BARRIER);
-        ok = 0;
-        break;
-      }
+    unsigned int box[4];
+    box[0] = ld_volatile_u32(&a.ctl[0]);
+    box[1] = ~ld_volatile_u32(&a.ctl[1]);
+    box[2] = ld_volatile_u32(&a.ctl[2]);
+    box[3] = ~ld_volatile_u32(&a.ctl[3]);
+    double minX, minY, maxmin;
+    frame_from_bbox(box, minX, minY, maxmin);
+    S.frame = key_frame(minX, minY, maxmin);
+    if (blockIdx.x == 0) {
+      a.frame[0] = minX;
+      a.frame[1] = minY;
+      a.frame[2] = maxmin;
+      a.frame[3] = S.frame.inv;
+      *a.kframe = S.frame;
     }
-    if (ok) {
-      unsigned int bb[4];
-      bb[0] = ld_volatile_u32(&box[0]);
-      bb[1] = ~ld_volatile_u32(&box[1]);
-      bb[2] = ld_volatile_u32(&box[2]);
-      bb[3] = ~ld_volatile_u32(&box[3]);
-      double minX, minY, maxmin;
-      frame_from_bbox(bb, minX, minY, maxmin);
-      s_frame[0] = minX;
-      s_frame[1] = minY;
-      s_frame[2] = maxmin;
-      s_frame[3] = (maxmin > 0.0) ? 1.0 / maxmin : 0.0;
-      if (blockIdx.x == 0) {
-        for (int k = 0; k < 4; k++) frame[k] = s_frame[k];
-      }
-    }
-    s_ok = ok;
   }
   __syncthreads();
-  if (!s_ok) return;
-  const double minX = s_frame[0], minY = s_frame[1], maxmin = s_frame[2], inv = s_frame[3];
-  // the records' z by quad level: D^2 / theta^2 with D = MAXMIN / 2^level
-  if (blockIdx.x == 0 && tid < kQuadLevels) ztab[tid] = bh_record_z(ldexp(maxmin, -tid), inv_theta2);
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-#pragma unroll
-    for (int w = 0; w < kRsWarps; w++) cnt[w][tid] = 0;
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < kRsItems; r++) {
-      const int idx = tile * kRsTile + r * kRsThreads + tid;
-      if (idx < n) {
-        const u64 key = morton_key(pos[idx], minX, minY, maxmin, inv);
-        keys[idx] = key;
-        vals[idx] = idx;
-        atomicAdd(&cnt[warp][(unsigned int)(key >> shift) & 255u], 1u);
+  const KeyFrame &frame = S.frame;
+  // keys; the records' z by quad level: D^2 / theta^2 with D = MAXMIN / 2^level
+  if (blockIdx.x == 0 && tid < kQuadLevels) a.ztab[tid] = bh_record_z(ldexp(frame.maxmin, -tid), a.inv_theta2);
+  for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
+#pragma unroll 2
+    for (int r = 0; r < a.items; r++) {
+      const int i = tile * tsize + r * kSortThreads + tid;
+      if (i < a.n)
+        __stcg(&a.pairs1[i], ((u64)morton_halves(a.pos[i], frame).y << 32) | (unsigned int)i);
+    }
+  __syncthreads();  // a block ranks its own tiles' keys
+  for (int pass = 0; pass < 4; pass++) {
+    const int shift = 32 + 8 * pass;
+    unsigned int *gt = a.gtot + pass * kSortGroups * 256;
+    u64 *in = (pass & 1) ? a.pairs0 : a.pairs1, *out = (pass & 1) ? a.pairs1 : a.pairs0;
+    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
+      const unsigned int mine = sort_rank_tile(a, S, in, shift, tile);
+      if (tid < 256) {
+        __stcg(&a.hist[(size_t)tile * 256 + tid], mine);
+        if (mine) atomicAdd(&gt[(tile / a.group) * 256 + tid], mine);
+      }
+      if (!single) {  // back to where the tile's keys were read
+        __syncthreads();
+        const int cnt = min(tsize, a.n - tile * tsize);
+        for (int x = tid; x < cnt; x += kSortThreads) __stcg(&in[tile * tsize + x], S.key[x]);
+        __syncthreads();
       }
     }
-    __syncthreads();
-    unsigned int tot = 0;
+    if (!sort_barrier(a, S, ++nbar)) return;
+    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
+      unsigned int all = 0, before = 0;
+      if (tid < 256) {
+        const int g = tile / a.group;
 #pragma unroll
-    for (int w = 0; w < kRsWarps; w++) tot += cnt[w][tid];
-    hist[(size_t)tid * ntiles + tile] = tot;
-    __syncthreads();
+        for (int q = 0; q < kSortGroups; q++) {
+          const unsigned int c = __ldcg(&gt[q * 256 + tid]);
+          all += c;
+          if (q < g) before += c;
+        }
+#pragma unroll 8
+        for (int t = g * a.group; t < tile; t++) before += __ldcg(&a.hist[(size_t)t * 256 + tid]);
+      }
+      if (!single) {
+        const unsigned int mine = tid < 256 ? __ldcg(&a.hist[(size_t)tile * 256 + tid]) : 0u;
+        const unsigned int loff = sort_scan256(mine, S);
+        if (tid < 256) S.loc[tid] = loff;
+      }
+      const unsigned int goff = sort_scan256(all, S);
+      if (tid < 256) S.base[tid] = goff + before - S.loc[tid];
+      __syncthreads();
+      const int cnt = min(tsize, a.n - tile * tsize);
+#pragma unroll 4
+      for (int x = tid; x < cnt; x += kSortThreads) {
+        const u64 k = single ? S.key[x] : __ldcg(&in[tile * tsize + x]);
+        const unsigned int g = S.base[(unsigned int)(k >> shift) & 255u] + (unsigned int)x;
+        if (g < (unsigned int)a.n) __stcg(&out[g], k);
+      }
+      if (!single) __syncthreads();
+    }
+    if (pass < 3 && !sort_barrier(a, S, ++nbar)) return;
   }
 }
 
-// ---- the low 32 bits: only inside runs of equal high halves ---------------------
+// ---- sorted keys, vertices and positions; the low 32 bits -----------------------
 //
 // The four LSD passes on bits 32..63 leave the keys ordered by their high
 // halves and, within a run of equal high halves, by vertex id (the passes are
@@ -332,49 +371,9 @@ __global__ void __launch_bounds__(kRsThreads, 8) frame_keys_kernel(const float2 
 // longer ones by one block each (bitonic network in shared memory up to
 // kRunCap keys, beyond that stable 8-bit LSD passes through global memory).
 // The result is the stable order of the full 64-bit keys.
+constexpr int kRunThreads = 512;
 constexpr int kRunShort = 32;
 constexpr int kRunCap = 2048;
-constexpr int kRunThreads = 512;
-
-__device__ __forceinline__ unsigned int hi32(u64 k) { return (unsigned int)(k >> 32); }
-
-// One thread per position; a run's first position sorts a short run or
-// queues a long one (runs[0] = count, then start, length pairs; runs_cap
-// exceeds n / (kRunShort + 1), the most long runs there can be).
-__global__ void run_fix_kernel(u64 *__restrict__ keys, int *__restrict__ vals, int n, int *runs, int runs_cap,
-                               DevStatus *st) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const unsigned int h = hi32(keys[k]);
-  if (k > 0 && hi32(keys[k - 1]) == h) return;        // not a run start
-  if (k + 1 >= n || hi32(keys[k + 1]) != h) return;   // a run of one
-  int len = 2;
-  while (k + len < n && hi32(keys[k + len]) == h && len <= kRunShort) len++;  // bounded scan
-  if (len <= kRunShort) {
-    // insertion sort by (key, vertex id); already in vertex-id order
-    for (int a = k + 1; a < k + len; a++) {
-      const u64 ka = keys[a];
-      const int va = vals[a];
-      int b = a - 1;
-      while (b >= k && (keys[b] > ka || (keys[b] == ka && vals[b] > va))) {
-        keys[b + 1] = keys[b];
-        vals[b + 1] = vals[b];
-        b--;
-      }
-      keys[b + 1] = ka;
-      vals[b + 1] = va;
-    }
-    return;
-  }
-  while (k + len < n && hi32(keys[k + len]) == h) len++;  // the whole run
-  const int slot = atomicAdd(&runs[0], 1);
-  if (slot < runs_cap) {
-    runs[1 + 2 * slot] = k;
-    runs[2 + 2 * slot] = len;
-  } else {
-    dev_record_error(st, DEV_BAD_INDEX);  // cannot happen (see runs_cap)
-  }
-}
 
 struct RunSmem {
   union {
@@ -412,107 +411,172 @@ __device__ __forceinline__ unsigned int run_scan256(unsigned int x, RunSmem &S) 
   return pre + inc - x;
 }
 
-// One block per queued run (grid-stride over the queue).
-__global__ void __launch_bounds__(kRunThreads) run_sort_kernel(u64 *__restrict__ keys, int *__restrict__ vals,
-                                                               u64 *__restrict__ kalt, int *__restrict__ valt,
-                                                               const int *runs, int runs_cap) {
-  __shared__ RunSmem S;
+// The run [start, start + len) sorted by one block.
+__device__ __noinline__ void sort_run(u64 *keys, int *vals, u64 *kalt, int *valt, int start, int len, RunSmem &S) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int count = min(runs[0], runs_cap);
-  for (int r = blockIdx.x; r < count; r += gridDim.x) {
-    const int start = runs[1 + 2 * r], len = runs[2 + 2 * r];
-    if (len <= kRunCap) {
-      int m = 2;
-      while (m < len) m <<= 1;
-      for (int q = tid; q < m; q += kRunThreads) {
-        S.u.b.k[q] = q < len ? keys[start + q] : ~0ull;
-        S.u.b.v[q] = q < len ? vals[start + q] : INT_MAX;
-      }
-      __syncthreads();
-      for (int size = 2; size <= m; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-          for (int i = tid; i < (m >> 1); i += kRunThreads) {
-            const int lo = ((i & ~(stride - 1)) << 1) | (i & (stride - 1));
-            const int hi = lo + stride;
-            const bool up = (lo & size) == 0;
-            const u64 ka = S.u.b.k[lo], kb = S.u.b.k[hi];
-            const int va = S.u.b.v[lo], vb = S.u.b.v[hi];
-            if ((ka > kb || (ka == kb && va > vb)) == up) {
-              S.u.b.k[lo] = kb;
-              S.u.b.k[hi] = ka;
-              S.u.b.v[lo] = vb;
-              S.u.b.v[hi] = va;
-            }
-          }
-          __syncthreads();
-        }
-      }
-      for (int q = tid; q < len; q += kRunThreads) {
-        keys[start + q] = S.u.b.k[q];
-        vals[start + q] = S.u.b.v[q];
-      }
-      __syncthreads();
-      continue;
+  if (len <= kRunCap) {
+    int m = 2;
+    while (m < len) m <<= 1;
+    for (int q = tid; q < m; q += kRunThreads) {
+      S.u.b.k[q] = q < len ? keys[start + q] : ~0ull;
+      S.u.b.v[q] = q < len ? vals[start + q] : INT_MAX;
     }
-    // a long run: four stable 8-bit passes on the low 32 bits through
-    // global memory (keys <-> the same range of kalt), chunk by chunk
-    const unsigned int lt = (1u << lane) - 1u;
-    for (int pass = 0; pass < 4; pass++) {
-      const u64 *ks = (pass & 1) ? kalt + start : keys + start;
-      const int *vs = (pass & 1) ? valt + start : vals + start;
-      u64 *kd = (pass & 1) ? keys + start : kalt + start;
-      int *vd = (pass & 1) ? vals + start : valt + start;
-      const int shift = 8 * pass;
-      if (tid < 256) S.u.c.carry[tid] = 0;
+    __syncthreads();
+    for (int size = 2; size <= m; size <<= 1) {
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (int i = tid; i < (m >> 1); i += kRunThreads) {
+          const int lo = ((i & ~(stride - 1)) << 1) | (i & (stride - 1));
+          const int hi = lo + stride;
+          const bool up = (lo & size) == 0;
+          const u64 ka = S.u.b.k[lo], kb = S.u.b.k[hi];
+          const int va = S.u.b.v[lo], vb = S.u.b.v[hi];
+          if ((ka > kb || (ka == kb && va > vb)) == up) {
+            S.u.b.k[lo] = kb;
+            S.u.b.k[hi] = ka;
+            S.u.b.v[lo] = vb;
+            S.u.b.v[hi] = va;
+          }
+        }
+        __syncthreads();
+      }
+    }
+    for (int q = tid; q < len; q += kRunThreads) {
+      keys[start + q] = S.u.b.k[q];
+      vals[start + q] = S.u.b.v[q];
+    }
+    __syncthreads();
+    return;
+  }
+  // a long run: four stable 8-bit passes on the low 32 bits through
+  // global memory (keys <-> the same range of kalt), chunk by chunk
+  const unsigned int lt = (1u << lane) - 1u;
+  for (int pass = 0; pass < 4; pass++) {
+    const u64 *ks = (pass & 1) ? kalt + start : keys + start;
+    const int *vs = (pass & 1) ? valt + start : vals + start;
+    u64 *kd = (pass & 1) ? keys + start : kalt + start;
+    int *vd = (pass & 1) ? vals + start : valt + start;
+    const int shift = 8 * pass;
+    if (tid < 256) S.u.c.carry[tid] = 0;
+    __syncthreads();
+    for (int q = tid; q < len; q += kRunThreads) atomicAdd(&S.u.c.carry[(unsigned int)(ks[q] >> shift) & 255u], 1u);
+    __syncthreads();
+    const unsigned int pre = run_scan256(tid < 256 ? S.u.c.carry[tid] : 0u, S);
+    if (tid < 256) {
+      S.u.c.base[tid] = pre;
+      S.u.c.carry[tid] = 0;
+    }
+    __syncthreads();
+    for (int c0 = 0; c0 < len; c0 += kRunThreads) {  // one key per thread and chunk
+      for (int q = tid; q < (kRunThreads / 32) * 256; q += kRunThreads) (&S.u.c.cnt[0][0])[q] = 0;
       __syncthreads();
-      for (int q = tid; q < len; q += kRunThreads) atomicAdd(&S.u.c.carry[(unsigned int)(ks[q] >> shift) & 255u], 1u);
+      const int q = c0 + tid;
+      const bool valid = q < len;
+      const u64 key = valid ? ks[q] : 0ull;
+      const int val = valid ? vs[q] : 0;
+      const unsigned int d = valid ? ((unsigned int)(key >> shift) & 255u) : 256u;
+      const unsigned int peers = __match_any_sync(0xffffffffu, d);
+      const unsigned int rank = __popc(peers & lt);
+      if (d < 256u && lane == __ffs(peers) - 1) S.u.c.cnt[warp][d] = __popc(peers);
       __syncthreads();
-      const unsigned int pre = run_scan256(tid < 256 ? S.u.c.carry[tid] : 0u, S);
       if (tid < 256) {
-        S.u.c.base[tid] = pre;
-        S.u.c.carry[tid] = 0;
+        unsigned int run = 0;
+        for (int w = 0; w < kRunThreads / 32; w++) {
+          const unsigned int c = S.u.c.cnt[w][tid];
+          S.u.c.cnt[w][tid] = run;
+          run += c;
+        }
+        S.u.c.tot[tid] = run;
       }
       __syncthreads();
-      for (int c0 = 0; c0 < len; c0 += kRunThreads) {  // one key per thread and chunk
-        for (int q = tid; q < (kRunThreads / 32) * 256; q += kRunThreads) (&S.u.c.cnt[0][0])[q] = 0;
-        __syncthreads();
-        const int q = c0 + tid;
-        const bool valid = q < len;
-        const u64 key = valid ? ks[q] : 0ull;
-        const int val = valid ? vs[q] : 0;
-        const unsigned int d = valid ? ((unsigned int)(key >> shift) & 255u) : 256u;
-        const unsigned int peers = __match_any_sync(0xffffffffu, d);
-        const unsigned int rank = __popc(peers & lt);
-        if (d < 256u && lane == __ffs(peers) - 1) S.u.c.cnt[warp][d] = __popc(peers);
-        __syncthreads();
-        if (tid < 256) {
-          unsigned int run = 0;
-          for (int w = 0; w < kRunThreads / 32; w++) {
-            const unsigned int c = S.u.c.cnt[w][tid];
-            S.u.c.cnt[w][tid] = run;
-            run += c;
-          }
-          S.u.c.tot[tid] = run;
-        }
-        __syncthreads();
-        if (d < 256u) {
-          const unsigned int p = S.u.c.base[d] + S.u.c.carry[d] + S.u.c.cnt[warp][d] + rank;
-          kd[p] = key;
-          vd[p] = val;
-        }
-        __syncthreads();
-        if (tid < 256) S.u.c.carry[tid] += S.u.c.tot[tid];
-        __syncthreads();
+      if (d < 256u) {
+        const unsigned int p = S.u.c.base[d] + S.u.c.carry[d] + S.u.c.cnt[warp][d] + rank;
+        kd[p] = key;
+        vd[p] = val;
       }
+      __syncthreads();
+      if (tid < 256) S.u.c.carry[tid] += S.u.c.tot[tid];
+      __syncthreads();
     }
-    // four passes end where they started (keys/vals)
+  }
+  // four passes end where they started (keys/vals)
+}
+
+// One thread per sorted position: full key, vertex and position, from the
+// position that is fetched by vertex anyway (the sort carries high halves
+// only).  A thread of a kernel of its own, not of the sort: the random 8-byte
+// fetches need many of them in flight, and beside the sort's 200 KB of shared
+// memory the first-level cache leaves few: there a million points took 27 us,
+// here 9.
+__global__ void __launch_bounds__(256) morton_emit_kernel(const float2 *__restrict__ pos, int n,
+                                                          const u64 *__restrict__ pairs, const KeyFrame *__restrict__ frame,
+                                                          u64 *__restrict__ keys, int *__restrict__ vals,
+                                                          float2 *__restrict__ spos, int *runs, int runs_cap,
+                                                          DevStatus *st) {
+  if (!block_status_ok(st)) return;
+  const int k = blockIdx.x * 256 + threadIdx.x;
+  if (k >= n) return;
+  const KeyFrame &F = *frame;
+  const u64 w = pairs[k];
+  const unsigned int h = hi32(w);
+  const unsigned int before = k > 0 ? hi32(pairs[k - 1]) : ~h, after = k + 1 < n ? hi32(pairs[k + 1]) : ~h;
+  const float2 p = pos[(unsigned int)w];
+  int len = 1;
+  if (before == h || after == h) {  // in a run
+    int first = k;
+    while (first > 0 && k - first < kRunShort && hi32(pairs[first - 1]) == h) first--;
+    len = k + 1 - first;
+    while (first + len < n && len <= kRunShort && hi32(pairs[first + len]) == h) len++;
+    if (len <= kRunShort) {
+      if (first != k) return;  // the run's first thread writes all of it
+    } else if (before != h) {
+      while (k + len < n && hi32(pairs[k + len]) == h) len++;  // the whole run
+      const int slot = atomicAdd(&runs[0], 1);
+      if (slot < runs_cap) {
+        runs[1 + 2 * slot] = k;
+        runs[2 + 2 * slot] = len;
+      } else {
+        dev_record_error(st, DEV_BAD_INDEX);  // cannot happen (see runs_cap)
+      }
+      len = 1;
+    } else {
+      len = 1;
+    }
+  }
+  keys[k] = ((u64)h << 32) | morton_halves(p, F).x;
+  vals[k] = (int)(unsigned int)w;
+  spos[k] = p;
+  // a short run: insertion by (key, vertex id); the rest arrive in vertex order
+  for (int x = k + 1; x < k + len; x++) {
+    const unsigned int vx = (unsigned int)pairs[x];
+    const float2 px = pos[vx];
+    const u64 kx = ((u64)h << 32) | morton_halves(px, F).x;
+    int b = x - 1;
+    for (; b >= k && keys[b] > kx; b--) {
+      keys[b + 1] = keys[b];
+      vals[b + 1] = vals[b];
+      spos[b + 1] = spos[b];
+    }
+    keys[b + 1] = kx;
+    vals[b + 1] = (int)vx;
+    spos[b + 1] = px;
   }
 }
 
-__global__ void gather_kernel(const float2 *__restrict__ pos, const int *__restrict__ perm, int n,
-                              float2 *__restrict__ spos) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) spos[k] = pos[perm[k]];
+// The queued long runs, one block each, and their positions.
+__global__ void __launch_bounds__(kRunThreads) run_sort_kernel(u64 *keys, int *vals, u64 *kalt, int *valt,
+                                                               const int *runs, int runs_cap,
+                                                               const float2 *__restrict__ pos, float2 *spos,
+                                                               DevStatus *st) {
+  __shared__ RunSmem S;
+  const int nruns = min(runs[0], runs_cap);
+  if ((int)blockIdx.x >= nruns || !block_status_ok(st)) return;
+  for (int q = blockIdx.x; q < nruns; q += gridDim.x) {
+    const int start = runs[1 + 2 * q], len = runs[2 + 2 * q];
+    __syncthreads();
+    sort_run(keys, vals, kalt, valt, start, len, S);
+    __syncthreads();
+    for (int k = threadIdx.x; k < len; k += kRunThreads) spos[start + k] = pos[vals[start + k]];
+  }
 }
 
 // ---- binary radix tree (Karras 2012) ----------------------------------------
@@ -599,7 +663,7 @@ struct TreeArgs {
   // level])
   unsigned long long *chain_mask;
   int *chain_node;
-  const float *ztab;  // the records' z = D^2 / theta^2 by quad level (frame_keys_kernel)
+  const float *ztab;  // the records' z = D^2 / theta^2 by quad level (morton_sort_kernel)
   float4 *nodes;
   double2 *nodes_c64;
   unsigned char *nodes_lvl;
@@ -1618,15 +1682,13 @@ int ensure_bh_scratch(bl_ctx *ctx) {
   fr(s.bparent); fr(s.bchild); fr(s.brange); fr(s.bdelta); fr(s.qkids); fr(s.qpar); fr(s.qnchild);
   fr(s.span); fr(s.span_stage); fr(s.ztab); fr(s.chain); fr(s.qcen);
   fr(s.qbelow); fr(s.startcnt); fr(s.startbase); fr(s.nodes); fr(s.nodes_c64);
-  fr(s.nodes_lvl); fr(s.rep); fr(s.f0); fr(s.pos_alt); fr(s.runs); fr(s.bnode);
-  const size_t nb = (n + kRsTile - 1) / kRsTile;
-  s.hist_entries = 256 * std::max<size_t>(nb, 1) + 256;
+  fr(s.nodes_lvl); fr(s.rep); fr(s.f0); fr(s.pos_alt); fr(s.runs); fr(s.bnode); fr(s.pairs);
   const size_t m = std::max<size_t>(n, 2);
   BL_CUDA(ctx, cudaMalloc(&s.keys, m * 8));
   BL_CUDA(ctx, cudaMalloc(&s.keys_alt, m * 8));
   BL_CUDA(ctx, cudaMalloc(&s.perm, m * 4));
   BL_CUDA(ctx, cudaMalloc(&s.perm_alt, m * 4));
-  BL_CUDA(ctx, cudaMalloc(&s.hist, s.hist_entries * 4));
+  BL_CUDA(ctx, cudaMalloc(&s.pairs, 2 * m * 8));
   BL_CUDA(ctx, cudaMalloc(&s.spos, m * sizeof(float2)));
   BL_CUDA(ctx, cudaMalloc(&s.bparent, 2 * m * sizeof(int)));
   BL_CUDA(ctx, cudaMalloc(&s.bchild, m * sizeof(int2)));
@@ -1657,10 +1719,22 @@ int ensure_bh_scratch(bl_ctx *ctx) {
   BL_CUDA(ctx, cudaMalloc(&s.pos_alt, m * sizeof(float2)));
   s.runs_cap = (int)(m / (kRunShort + 1) + 1);  // runs longer than kRunShort: at most n / (kRunShort + 1)
   BL_CUDA(ctx, cudaMalloc(&s.runs, (2 * (size_t)s.runs_cap + 1) * sizeof(int)));
+  // the sort's tiles: one a resident block where 16 keys a thread are enough
+  // (they then stay in shared memory between the ranking and the scatter),
+  // else an even number of tiles a block
+  BL_CUDA(ctx, cudaFuncSetAttribute(morton_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(SortSmem)));
   int occ = 0;
-  BL_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, frame_keys_kernel, kRsThreads, 0));
-  if (occ < 1) return bl_fail(ctx, -5, "frame/key kernel cannot be resident");
-  s.fk_grid = ctx->num_sms * occ;
+  BL_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, morton_sort_kernel, kSortThreads,
+                                                             sizeof(SortSmem)));
+  if (occ < 1) return bl_fail(ctx, -5, "sort kernel cannot be resident");
+  const int resident = ctx->num_sms * occ;
+  const long long per_wave = (long long)resident * kSortThreads;
+  const int waves = (int)((m + per_wave * kSortItems - 1) / (per_wave * kSortItems));
+  s.sort_items = (int)((m + per_wave * waves - 1) / (per_wave * waves));
+  s.sort_tiles = nblk((long long)m, s.sort_items * kSortThreads);
+  s.sort_grid = std::min(s.sort_tiles, resident);
+  BL_CUDA(ctx, cudaMalloc(&s.hist, ((size_t)s.sort_tiles + 4 * kSortGroups) * 256 * sizeof(unsigned int)));
   // set here, outside any stream capture of the iteration
   BL_CUDA(ctx, cudaFuncSetAttribute(centroid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sizeof(CenSmem)));
@@ -1678,31 +1752,9 @@ int bh_build(bl_ctx *ctx, const float2 *pos, double theta, int attract_batch) {
   Scratch &s = ctx->s;
   cudaStream_t st = ctx->stream;
   if (n < 2) return 0;
-  const int nb = nblk(n, kRsTile);
-  unsigned long long *kin = s.keys, *kout = s.keys_alt;
-  int *vin = s.perm, *vout = s.perm_alt;
-  // hist layout: [256 digits x ntiles counts][256 digit-row totals]
-  unsigned int *digit_off = s.hist + (size_t)256 * nb;
-  bl_time_begin(ctx, "frame_morton");
-  // box and barrier slots to 0xffffffff; then the frame, the keys and the
-  // digit counts of the first pass (bits 32..39) in one cooperative launch
-  BL_CUDA(ctx, cudaMemsetAsync(s.bbox, 0xff, 5 * sizeof(unsigned int), st));
-  {
-    const int grid = std::min(nb, s.fk_grid);
-    int shift = 32;
-    int nn = n;
-    int ntiles = nb;
-    double inv_theta2 = 1.0 / (theta * theta);
-    void *args[] = {(void *)&pos, &nn, &ntiles, &s.bbox, &s.frame, &s.keys, &s.perm, &shift, &s.hist,
-                    &inv_theta2, &s.ztab, &s.status};
-    BL_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)frame_keys_kernel, dim3(grid), dim3(kRsThreads), args, 0,
-                                             st));
-    ctx->launches++;
-  }
-  bl_time_end(ctx, "frame_morton");
+  const int ncb = nblk(n, kCenSpan);  // centroid blocks
   // the walk's attraction part (for the iteration that follows) needs no
-  // tree: on the second stream (lower priority) beside the single-wave sort
-  // passes; before the frame kernel it slowed that cooperative launch
+  // tree: on the second stream (lower priority) beside the sort
   if (attract_batch > 0) {
     const bool side = ctx->side && ctx->ev_fork && ctx->ev_join;
     if (side) {
@@ -1713,36 +1765,48 @@ int bh_build(bl_ctx *ctx, const float2 *pos, double theta, int attract_batch) {
         n, ctx->g.rowptr, ctx->g.colids, pos, attract_batch, (float)ctx->weight, s.f0);
     ctx->launches++;
   }
-  bl_time_begin(ctx, "radix_sort");
-  bl_time_begin(ctx, "lsd_passes");
-  // bits 32..63 by four LSD passes, then the runs of equal high halves
-  for (int pass = 4; pass < 8; pass++) {
-    if (pass > 4) {  // the first pass's counts come with the keys
-      rs_count_kernel<<<nb, kRsThreads, 0, st>>>(kin, n, 8 * pass, nb, s.hist);
-      ctx->launches++;
-    }
-    rs_rowscan_kernel<<<256, 256, 0, st>>>(s.hist, nb, digit_off);
-    rs_scatter_kernel<<<nb, kRsThreads, 0, st>>>(kin, vin, kout, vout, n, 8 * pass, nb, s.hist, digit_off);
-    std::swap(kin, kout);
-    std::swap(vin, vout);
-    ctx->launches += 2;
+  bl_time_begin(ctx, "morton_sort");
+  BL_CUDA(ctx, cudaMemsetAsync(s.bbox, 0xff, 5 * sizeof(unsigned int), st));
+  {
+    SortArgs a;
+    a.pos = pos;
+    a.n = n;
+    a.items = s.sort_items;
+    a.ntiles = s.sort_tiles;
+    a.group = (s.sort_tiles + kSortGroups - 1) / kSortGroups;
+    a.ctl = s.bbox;
+    a.frame = s.frame;
+    a.kframe = reinterpret_cast<KeyFrame *>(s.frame + 4);
+    a.inv_theta2 = 1.0 / (theta * theta);
+    a.ztab = s.ztab;
+    a.pairs0 = s.pairs;
+    a.pairs1 = s.pairs + std::max(n, 2);
+    a.hist = s.hist;
+    a.gtot = s.hist + (size_t)s.sort_tiles * 256;
+    a.runs = s.runs;
+    // span_cnt, the block totals and the boundary chains' level masks
+    a.zero0 = s.span;
+    a.nzero0 = kQuadLevels + ncb + 1;
+    a.zero1 = reinterpret_cast<int *>(s.chain);
+    a.nzero1 = 2 * ncb;
+    a.st = s.status;
+    void *args[] = {&a};
+    BL_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)morton_sort_kernel, dim3(s.sort_grid), dim3(kSortThreads),
+                                             args, sizeof(SortSmem), st));
+    ctx->launches++;
   }
-  bl_time_end(ctx, "lsd_passes");
-  // 4 passes: the data is back in keys/perm
-  BL_CUDA(ctx, cudaMemsetAsync(s.runs, 0, sizeof(int), st));
-  run_fix_kernel<<<nblk(n, 256), 256, 0, st>>>(s.keys, s.perm, n, s.runs, s.runs_cap, s.status);
-  run_sort_kernel<<<ctx->num_sms, kRunThreads, 0, st>>>(s.keys, s.perm, s.keys_alt, s.perm_alt, s.runs, s.runs_cap);
-  ctx->launches += 2;
-  bl_time_end(ctx, "radix_sort");
-  bl_time_begin(ctx, "gather_tree");
-  gather_kernel<<<nblk(n, 256), 256, 0, st>>>(pos, s.perm, n, s.spos);
+  morton_emit_kernel<<<nblk(n, 256), 256, 0, st>>>(pos, n, s.pairs + std::max(n, 2),
+                                                   reinterpret_cast<const KeyFrame *>(s.frame + 4), s.keys, s.perm, s.spos,
+                                                   s.runs, s.runs_cap, s.status);
+  ctx->launches++;
+  run_sort_kernel<<<std::min(s.runs_cap, ctx->num_sms), kRunThreads, 0, st>>>(
+      s.keys, s.perm, s.keys_alt, s.perm_alt, s.runs, s.runs_cap, pos, s.spos, s.status);
+  ctx->launches++;
+  bl_time_end(ctx, "morton_sort");
+  bl_time_begin(ctx, "radix_tree");
   radix_tree_kernel<<<nblk(n - 1, 256), 256, 0, st>>>(s.keys, n, s.bchild, s.brange, s.bdelta, s.bparent,
                                                        reinterpret_cast<int *>(s.bnode));
-  bl_time_end(ctx, "gather_tree");
-  const int ncb = nblk(n, kCenSpan);  // centroid blocks
-  // span_cnt, the block totals and the boundary chains' level masks to 0
-  BL_CUDA(ctx, cudaMemsetAsync(s.span, 0, (kQuadLevels + ncb + 1) * sizeof(int), st));
-  BL_CUDA(ctx, cudaMemsetAsync(s.chain, 0, (size_t)ncb * sizeof(unsigned long long), st));
+  bl_time_end(ctx, "radix_tree");
   TreeArgs t;
   t.n = n;
   t.spos = s.spos;
@@ -1889,7 +1953,7 @@ int bh_iteration(bl_ctx *ctx, int batch, double theta, double step, bool want_en
 
 // ---- CUDA-graph replay of the iteration ------------------------------------
 // One Barnes-Hut iteration without the energy read-back is a fixed sequence
-// of about 45 launches and memsets on fixed buffers; only the positions
+// of about 15 launches and memsets on fixed buffers; only the positions
 // alternate between two buffers and STEP changes.  It is captured once per
 // parity of the position buffers and replayed, STEP being set on the sweep's
 // kernel node before each replay.

@@ -96,7 +96,7 @@ struct BhShared {
   unsigned int box[4];
   int wsum[kBWarps];
   int lvl_off[kMaxBfsLevels + 2];
-  double frame[4];
+  KeyFrame frame;
   int trivial;
 };
 
@@ -313,18 +313,14 @@ __device__ void layout_bh(const BatchedArgs &a, int g, BhShared &S, double *red)
     if (tid == 0) {
       double minX, minY, maxmin;
       frame_from_bbox(S.box, minX, minY, maxmin);
-      S.frame[0] = minX;
-      S.frame[1] = minY;
-      S.frame[2] = maxmin;
-      S.frame[3] = (maxmin > 0.0) ? 1.0 / maxmin : 0.0;
+      S.frame = key_frame(minX, minY, maxmin);
     }
     __syncthreads();
-    const double maxmin = S.frame[2];
+    const double maxmin = S.frame.maxmin;
     // 2. keys
     {
-      const double minX = S.frame[0], minY = S.frame[1], inv = S.frame[3];
       for (int k = tid; k < n; k += kBThreads) {
-        kin[k] = morton_key(pos[k], minX, minY, maxmin, inv);
+        kin[k] = morton_key(pos[k], S.frame);
         vin[k] = k;
       }
     }

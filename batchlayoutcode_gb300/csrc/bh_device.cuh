@@ -24,16 +24,6 @@ __device__ __forceinline__ float ord2f(unsigned int u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-__device__ __forceinline__ u64 spread32(unsigned int v) {
-  u64 x = v;
-  x = (x | (x << 16)) & 0x0000FFFF0000FFFFull;
-  x = (x | (x << 8)) & 0x00FF00FF00FF00FFull;
-  x = (x | (x << 4)) & 0x0F0F0F0F0F0F0F0Full;
-  x = (x | (x << 2)) & 0x3333333333333333ull;
-  x = (x | (x << 1)) & 0x5555555555555555ull;
-  return x;
-}
-
 // float -> double without the conversion instruction (exact; the bits are
 // rebiased and shifted): normal floats and +-0; subnormal, infinite and NaN
 // floats take the conversion.
@@ -84,15 +74,37 @@ __device__ __forceinline__ void frame_from_bbox(const unsigned int *bbox, double
   maxmin = (ry < rx) ? rx : ry;  // std::max(y-range, x-range)
 }
 
+// The frame as the keys need it: FP64 for the exact form, and the same scale
+// 4294967295 / maxmin as a pair of floats (0 where it leaves 2^-60 .. 2^60:
+// every key then takes the exact form).
+struct KeyFrame {
+  double minX, minY, maxmin, inv;
+  float fx, fy;  // minX, minY: positions are floats, so these are exact
+  float ch, cl;
+};
+
+__device__ __forceinline__ KeyFrame key_frame(double minX, double minY, double maxmin) {
+  KeyFrame f;
+  f.minX = minX;
+  f.minY = minY;
+  f.maxmin = maxmin;
+  f.inv = maxmin > 0.0 ? 1.0 / maxmin : 0.0;
+  f.fx = (float)minX;
+  f.fy = (float)minY;
+  const double c = maxmin > 0.0 ? 4294967295.0 / maxmin : 0.0;
+  const bool ok = c > 0x1p-60 && c < 0x1p60;
+  f.ch = ok ? (float)c : 0.0f;
+  f.cl = ok ? (float)(c - (double)f.ch) : 0.0f;
+  return f;
+}
+
 // (uint32)(4294967295.0 * (v - mn) / maxmin), MortonCode.h:62-67, no contraction.
 // The quotient is formed with the reciprocal (one multiply); its error is a
 // couple of ulp, so unless it lies within 8 ulp of an integer its truncation
 // equals the truncation of the correctly rounded quotient.  Otherwise the
-// exact division decides.  The truncation and the distance to the nearest
-// integers are read from the bits of the quotient with integer operations:
-// the FP64 pipe (a small fraction of the FP32 rate on this part) only sees
-// the subtraction and the two products.
-__device__ __forceinline__ unsigned int quantise(float v, double mn, double maxmin, double inv) {
+// exact division decides.
+static_assert(sizeof(KeyFrame) <= 12 * sizeof(double), "kept behind the four words of the frame");
+static __device__ __noinline__ unsigned int quantise_exact(float v, double mn, double maxmin, double inv) {
   if (!(maxmin > 0.0)) return 0u;
   const double a = __dmul_rn(4294967295.0, __dsub_rn(f2d_int(v), mn));
   const double qf = __dmul_rn(a, inv);
@@ -107,9 +119,52 @@ __device__ __forceinline__ unsigned int quantise(float v, double mn, double maxm
   return __double2uint_rz(__ddiv_rn(a, maxmin));  // near an integer, below 1 or out of range
 }
 
-// 64-bit Morton key, y bit above x bit of every digit (MortonCode.h:83-97).
-__device__ __forceinline__ u64 morton_key(float2 p, double minX, double minY, double maxmin, double inv) {
-  return (spread32(quantise(p.y, minY, maxmin, inv)) << 1) | spread32(quantise(p.x, minX, maxmin, inv));
+// The same value from FP32 pairs where those decide it.  d = v - mn is exact
+// as a sum of two floats (Knuth's two-sum); the product with the scale's pair
+// is p + e with an error of at most 2^-45 p (the FMA residual of the leading
+// product is exact; two rounded terms of at most 3 * 2^-24 p, the dropped
+// product of the low parts and the rounding of cl are each of the order of
+// 2^-48 p), so at most 2^-13 for p < 2^32; adding the fraction of p to e
+// rounds by at most 2^-15, and the reference's own three roundings by 2^-19.
+// Unless the fraction is within 2^-11 of an integer the truncation is
+// therefore the reference's; there (two points in 1,000), below 1 and at the
+// upper end the FP64 form decides.  FP64 runs at 2 lanes a cycle and SM on
+// this part: with three FP64 operations a coordinate the keys of a million
+// points took 19 us, so they take 5.
+__device__ __forceinline__ unsigned int quantise(float v, float mn, double mnd, const KeyFrame &f) {
+  const float d = __fsub_rn(v, mn);
+  const float t = __fsub_rn(d, v);
+  const float dl = __fsub_rn(__fsub_rn(v, __fsub_rn(d, t)), __fadd_rn(mn, t));
+  const float p = __fmul_rn(d, f.ch);
+  const float e = __fmaf_rn(d, f.cl, __fmaf_rn(dl, f.ch, __fmaf_rn(d, f.ch, -p)));
+  if (p >= 1.0f && p < 4294967040.0f) {
+    const unsigned int ip = __float2uint_rz(p);
+    const float fr = __fadd_rn(__fsub_rn(p, __uint2float_rn(ip)), e);  // ip has at most 24 bits: exact
+    const float fi = floorf(fr);
+    const float ff = __fsub_rn(fr, fi);
+    if (ff > 0x1p-11f && ff < 1.0f - 0x1p-11f) return ip + (unsigned int)(int)fi;
+  }
+  return quantise_exact(v, mnd, f.maxmin, f.inv);
+}
+
+// Bit b of the low 16 bits to bit 2b.
+__device__ __forceinline__ unsigned int spread16(unsigned int v) {
+  v = (v | (v << 8)) & 0x00ff00ffu;
+  v = (v | (v << 4)) & 0x0f0f0f0fu;
+  v = (v | (v << 2)) & 0x33333333u;
+  return (v | (v << 1)) & 0x55555555u;
+}
+
+// Halves of the 64-bit Morton key, y bit above x bit of every digit
+// (MortonCode.h:83-97): each comes from 16 bits of either coordinate, so all
+// the bit spreading is 32 bits wide.
+__device__ __forceinline__ uint2 morton_halves(float2 p, const KeyFrame &f) {  // {low, high}
+  const unsigned int qy = quantise(p.y, f.fy, f.minY, f), qx = quantise(p.x, f.fx, f.minX, f);
+  return make_uint2((spread16(qy & 0xffffu) << 1) | spread16(qx & 0xffffu), (spread16(qy >> 16) << 1) | spread16(qx >> 16));
+}
+__device__ __forceinline__ u64 morton_key(float2 p, const KeyFrame &f) {
+  const uint2 h = morton_halves(p, f);
+  return ((u64)h.y << 32) | h.x;
 }
 
 // x / c for the child count c of a quad node, correctly rounded like the

@@ -189,14 +189,14 @@ struct Scratch {
   size_t bh_n = 0;
   unsigned long long *keys = nullptr, *keys_alt = nullptr;
   int *perm = nullptr, *perm_alt = nullptr;
-  unsigned int *hist = nullptr;  // radix histograms / offsets
-  int fk_grid = 0;               // resident blocks of the frame/key kernel
+  unsigned long long *pairs = nullptr;  // sort: two buffers of (high key half, vertex) words
+  unsigned int *hist = nullptr;  // sort: digit counts per tile, then per group and pass
+  int sort_items = 0, sort_tiles = 0, sort_grid = 0;  // keys a thread, tiles, blocks
   int4 *bnode = nullptr;         // packed binary radix nodes for the chain walk
   int *runs = nullptr;           // runs of equal high key halves: count, (start, length) pairs, overflow
   int runs_cap = 0;
-  size_t hist_entries = 0;
-  unsigned int *bbox = nullptr;  // frame/key kernel: box (ordered-uint floats) and arrivals
-  double *frame = nullptr;       // minX, minY, MAXMIN
+  unsigned int *bbox = nullptr;  // sort: box (ordered-uint floats), arrivals
+  double *frame = nullptr;  // {minX, minY, MAXMIN, 1 / MAXMIN}, then the key constants
   float2 *spos = nullptr;        // positions in Morton order
   int *bparent = nullptr;        // binary radix tree: parent of node (internal i, leaf n-1+k)
   int2 *bchild = nullptr;        // children of internal node (encoded: >= 0 internal, < 0 leaf ~k)
