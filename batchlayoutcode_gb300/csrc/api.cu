@@ -178,7 +178,7 @@ void free_ctx(bl_ctx *c) {
   fr(s.term_off); fr(s.terms); fr(s.term_tgt); fr(s.greedy_share); fr(s.greedy_pos);
   for (auto &ls : c->schedules) {
     fr(ls.order);
-    fr(ls.d_offsets);
+    fr(ls.d_groups);
     fr(ls.early_off);
     fr(ls.early_col);
   }

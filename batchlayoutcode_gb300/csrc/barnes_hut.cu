@@ -1442,15 +1442,71 @@ struct TraverseArgs {
 // FR attraction (algorithms.cpp:1056-1058) of the neighbours of v that have
 // not moved before v in the iteration (same or later batch), float-float, by
 // vertex id.  It needs no tree, so it runs on the second stream beside the
-// tree's spanning passes; the walk then adds minus the repulsion.
-__global__ void __launch_bounds__(256) unmoved_attraction_kernel(int n, const int *__restrict__ rowptr,
-                                                                 const int *__restrict__ colids,
-                                                                 const float2 *pold, int batch, float W,
-                                                                 float4 *f0) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < n) f0[v] = bh_unmoved_attraction(v, rowptr, colids, pold, batch, W);
+// sort and the tree; the walk then adds minus the repulsion.
+// A thread takes a row of up to kHubRow neighbours, a warp a longer one: its
+// lanes fetch 32 neighbours at once and form the factors, which every lane
+// then multiplies and adds in CSR order, so the sum is the thread's bit for bit.  A thread alone
+// is bound by its fetches (two dependent L2 round trips per four neighbours):
+// with the longest row at 633 neighbours of 100,003 vertices the
+// kernel took 155 us, longer than the sort and the tree beside it; so 49.  The vertices with long rows often have
+// neighbouring ids, so a block takes groups of 8 vertices from all over the
+// range (8 keep the rows' offsets and the results in whole sectors) and its
+// warps share the long rows among them.
+constexpr int kHubRow = 32;
+constexpr int kAttractThreads = 256;
+
+__device__ __forceinline__ float4 hub_unmoved_attraction(int v, const int *__restrict__ rowptr,
+                                                         const int *__restrict__ colids, const float2 *pold, int batch,
+                                                         float W) {
+  const int lane = threadIdx.x & 31;
+  const float2 pv = pold[v];
+  const int batch_lo = (v / batch) * batch, e0 = rowptr[v], e1 = rowptr[v + 1];
+  auto column = [&](int e) { return e < e1 ? colids[e] : -1; };
+  auto position = [&](int j) { return j >= batch_lo ? pold[j] : pv; };
+  float hx = 0.f, lx = 0.f, hy = 0.f, ly = 0.f;
+  int j = column(e0 + lane), jn = e1 - e0 > 32 ? column(e0 + 32 + lane) : -1;
+  float2 p = position(j);
+  for (int e = e0; e < e1; e += 32) {  // positions one chunk ahead, columns two
+    const float2 pn = position(jn);
+    const int j2 = e1 - e > 64 ? column(e + 64 + lane) : -1;
+    const float dx = p.x - pv.x, dy = p.y - pv.y;
+    const float sc = W * sqrtf(fmaf(dx, dx, dy * dy));
+    const unsigned int m = __ballot_sync(0xffffffffu, j >= batch_lo);  // past the row's end j is -1
+#pragma unroll 8
+    for (int q = 0; q < 32; q++) {
+      const float x = __shfl_sync(0xffffffffu, dx, q), y = __shfl_sync(0xffffffffu, dy, q);
+      const float s = __shfl_sync(0xffffffffu, sc, q);
+      if ((m >> q) & 1u) {  // the products here, as in bh_attract: the sums take them unrounded
+        ff_add(hx, lx, x * s);
+        ff_add(hy, ly, y * s);
+      }
+    }
+    j = jn;
+    jn = j2;
+    p = pn;
+  }
+  return make_float4(hx, hy, lx, ly);
 }
 
+__global__ void __launch_bounds__(kAttractThreads) unmoved_attraction_kernel(int n, const int *__restrict__ rowptr,
+                                                                             const int *__restrict__ colids,
+                                                                             const float2 *pold, int batch, float W,
+                                                                             float4 *f0) {
+  __shared__ int hub[kAttractThreads];
+  __shared__ int nhub;
+  if (threadIdx.x == 0) nhub = 0;
+  __syncthreads();
+  const long long v = 8ll * ((threadIdx.x >> 3) * (long long)gridDim.x + blockIdx.x) + (threadIdx.x & 7);
+  if (v < n) {
+    if (rowptr[v + 1] - rowptr[v] <= kHubRow) f0[v] = bh_unmoved_attraction((int)v, rowptr, colids, pold, batch, W);
+    else hub[atomicAdd(&nhub, 1)] = (int)v;
+  }
+  __syncthreads();
+  for (int h = threadIdx.x >> 5; h < nhub; h += kAttractThreads / 32) {
+    const float4 f = hub_unmoved_attraction(hub[h], rowptr, colids, pold, batch, W);
+    if ((threadIdx.x & 31) == 0) f0[hub[h]] = f;
+  }
+}
 
 // 128 threads per block: measured 1.5 % faster than 256 and 512 on the 1M
 // graph (finer blocks, smaller tail); 64 is no better.
@@ -1486,11 +1542,11 @@ __global__ void __launch_bounds__(kTravThreads) traverse_kernel(TraverseArgs a) 
 }
 
 struct SweepArgs {
-  const int *order;      // vertices grouped by dependency level
-  const int *level_off;  // levels + 1 offsets into order
+  const int *order;        // vertices grouped by dependency level
+  const int *group_start;  // groups + 1 offsets into order
   const int *early_off;  // per level-order slot: earlier-batch neighbours
   const int *early_col;
-  int levels;
+  int groups;
   const float4 *f0;      // attraction of unmoved neighbours minus repulsion (float-float)
   float4 *f0out;         // the same array: the final float-float force when write_out
   const float2 *pold;
@@ -1502,6 +1558,7 @@ struct SweepArgs {
 };
 
 constexpr int kSweepThreads = 1024;
+constexpr unsigned int kSweepSleep = 100;  // ns
 
 // A new position not yet written: both coordinates NaN, all bits set
 // (no layout coordinate is NaN).  pnew is filled with it before the sweep.
@@ -1521,27 +1578,6 @@ __device__ __forceinline__ void st_relaxed_u64(float2 *p, float2 v) {
 
 __device__ __forceinline__ float2 unpack_pos(unsigned long long b) {
   return make_float2(__uint_as_float((unsigned int)b), __uint_as_float((unsigned int)(b >> 32)));
-}
-
-// The new position of neighbour c, which an earlier dependency level writes:
-// the 8-byte word is the position and its own ready flag (a single-copy
-// atomic 64-bit access), so one load both tests and reads it.  The wait is
-// bounded; false when it ran out or another thread recorded an error.
-__device__ __forceinline__ bool wait_moved(const SweepArgs &a, int c, unsigned long long &b) {
-  if (b != kUnmoved) return true;
-  const unsigned long long t0 = dev_globaltimer();
-  for (unsigned int polls = 1;; polls++) {
-    __nanosleep(100);  // fewer polls queued at L2 while the writer works
-    b = ld_relaxed_u64(&a.pnew[c]);
-    if (b != kUnmoved) return true;
-    if ((polls & 63u) == 0u) {
-      if (ld_volatile_u32(&a.st->code) != 0u) return false;
-      if (dev_globaltimer() - t0 > kBarrierTimeoutNs) {
-        dev_record_error(a.st, DEV_TIMEOUT_SWEEP);
-        return false;
-      }
-    }
-  }
 }
 
 // A vertex's data that does not change during the sweep: its slot in the
@@ -1566,38 +1602,70 @@ __device__ __forceinline__ void sweep_load(const SweepArgs &a, int t, SweepVerte
   for (int q = 0; q < 4; q++) v.c[q] = (v.e0 + q < v.e1) ? a.early_col[v.e0 + q] : 0;
 }
 
-// Adds the attraction of the neighbours that moved earlier in this iteration
-// (earlier batches, their new positions, each waited for) to f0, then the
-// unit-step update (algorithms.cpp:1056-1066).  FP32 terms, float-float sum,
-// FP32 unit vector.  False when a wait gave up.
-__device__ __forceinline__ bool sweep_vertex(const SweepArgs &a, const SweepVertex &v) {
+// The vertices of a warp (one a lane, has: the lane has one): adds the
+// attraction of the neighbours that moved earlier in this iteration (earlier
+// batches, their new positions) to f0, then the unit-step update
+// (algorithms.cpp:1056-1066).  FP32 terms, float-float sum in neighbour
+// order, FP32 unit vector.
+// A neighbour's new position, which an earlier dependency level writes, is an
+// 8-byte word that is its own ready flag (a single-copy atomic 64-bit access):
+// one load both tests and reads it.  The warp stays converged: in every round
+// each lane loads the words of its next four neighbours (only the first while
+// it waits for that one), takes those that are there and, with the last,
+// publishes its own position.  So a row of many moved neighbours costs a round
+// trip per four of them, all lanes at once; a lane that waited alone and then
+// loaded its neighbours one by one held up the warp and every level after it
+// (100,003 vertices
+// of a power-law graph, 32 levels, up to 22 moved neighbours: the sweep
+// 118 us, so 94; 1,000,000 of a geometric one: 77 us, so 58).  The wait is bounded; false when it ran out or another thread
+// recorded an error (the same in every lane).
+__device__ __forceinline__ bool sweep_group(const SweepArgs &a, const SweepVertex &v, bool has) {
   float hx = v.f.x, hy = v.f.y, lx = v.f.z, ly = v.f.w;
-  const int m = min(v.e1 - v.e0, 4);
-  // the loads of the first (up to) four moved neighbours are issued
-  // together; the terms are added in neighbour order
-  unsigned long long b[4];
+  int c[4] = {v.c[0], v.c[1], v.c[2], v.c[3]};
+  int e = v.e0;
+  bool more = has, wide = true;
+  unsigned long long t0 = 0;
+  for (unsigned int round = 0;; round++) {
+    const int left = more ? v.e1 - e : 0, ask = wide ? left : min(left, 1);
+    unsigned long long b[4];
 #pragma unroll
-  for (int q = 0; q < 4; q++) b[q] = (q < m) ? ld_relaxed_u64(&a.pnew[v.c[q]]) : 0ull;
+    for (int q = 0; q < 4; q++) b[q] = q < ask ? ld_relaxed_u64(&a.pnew[c[q]]) : kUnmoved;
+    int got = 0;
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    if (q < m) {
-      if (!wait_moved(a, v.c[q], b[q])) return false;
-      bh_attract(unpack_pos(b[q]), v.pi, a.W, hx, lx, hy, ly);
+    for (int q = 0; q < 4; q++)
+      if (got == q && b[q] != kUnmoved) {
+        bh_attract(unpack_pos(b[q]), v.pi, a.W, hx, lx, hy, ly);
+        got = q + 1;
+      }
+    if (more && got == left) {  // all are in (left > 4 never equals got)
+      more = false;
+      const float2 np = bh_step(v.pi, hx, lx, hy, ly, a.step);
+      // the force's float-float sums replace f0 (read above, not needed again);
+      // bh_forces_kernel turns them into the FP64 force and |f|^2 in full warps
+      if (a.write_out) a.f0out[v.i] = make_float4(hx, hy, lx, ly);
+      st_relaxed_u64(&a.pnew[v.i], np);  // publishes the position: later levels wait for this word
+    }
+    if (!__any_sync(0xffffffffu, more)) return true;
+    wide = got > 0;
+    if (more && got > 0) {
+      e += got;
+#pragma unroll
+      for (int q = 0; q < 4; q++) c[q] = e + q < v.e1 ? a.early_col[e + q] : 0;
+    }
+    if (!__any_sync(0xffffffffu, got > 0)) {
+      __nanosleep(kSweepSleep);  // fewer polls queued at L2 while the writers work
+      if ((round & 63u) == 63u) {
+        const unsigned long long now = dev_globaltimer();
+        if (t0 == 0) t0 = now;
+        bool quit = ld_volatile_u32(&a.st->code) != 0u;
+        if (!quit && now - t0 > kBarrierTimeoutNs) {
+          dev_record_error(a.st, DEV_TIMEOUT_SWEEP);
+          quit = true;
+        }
+        if (__any_sync(0xffffffffu, quit)) return false;
+      }
     }
   }
-  // more than four (rare): one at a time
-  for (int e = v.e0 + 4; e < v.e1; e++) {
-    const int c = a.early_col[e];
-    unsigned long long bb = ld_relaxed_u64(&a.pnew[c]);
-    if (!wait_moved(a, c, bb)) return false;
-    bh_attract(unpack_pos(bb), v.pi, a.W, hx, lx, hy, ly);
-  }
-  const float2 np = bh_step(v.pi, hx, lx, hy, ly, a.step);
-  // the force's float-float sums replace f0 (read above, not needed again);
-  // bh_forces_kernel turns them into the FP64 force and |f|^2 in full warps
-  if (a.write_out) a.f0out[v.i] = make_float4(hx, hy, lx, ly);
-  st_relaxed_u64(&a.pnew[v.i], np);  // publishes the position: later levels wait for this word
-  return true;
 }
 
 // All dependency levels of an iteration in one launch, without barriers: a
@@ -1607,49 +1675,34 @@ __device__ __forceinline__ bool sweep_vertex(const SweepArgs &a, const SweepVert
 // order, and group G goes to warp G mod W (W warps in the grid, numbered so
 // that consecutive groups land on different SMs): every warp gets about the
 // same number of groups, and takes them in level order.  A warp finishes a
-// level (__syncwarp) before it starts the next, so a slot waits only on slots
+// group before it starts the next, so a slot waits only on slots
 // of lower levels held by other warps or by this warp's finished groups; with
 // every block resident (a cooperative launch) the warp holding the lowest
 // unfinished slot can always proceed, so the sweep cannot deadlock.  A thread
 // loads its next slot's vertex data before it waits on the current slot's
-// neighbours.
+// neighbours.  Bound by the levels: each is a round trip to see the position,
+// the update and the store.  The groups' first slots are a table made with the
+// levels: finding them here (a walk over the levels' ends, 64-bit remainders)
+// took 22 us of the 94 and 10 of the 58.  Blocks of 512 threads are 4 us faster at
+// 100,003 vertices, 11 slower at 1,000,000 and 45 at 3,000,000.
 __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(SweepArgs a) {
   if (!block_status_ok(a.st)) return;
   const int W = gridDim.x * (blockDim.x >> 5);
   const int lane = threadIdx.x & 31;
   const int w = ((int)threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
-  // (lv, j): the warp's current group j of level lv; gb: groups of the levels below lv
-  int lv = 0, j = 0;
-  long long gb = 0;
-  auto first_group = [&](int l, long long base) { return (int)((((long long)w - base) % W + W) % W); };
-  auto settle = [&](int &l, int &jj, long long &base) {
-    while (l < a.levels) {
-      const int lo = a.level_off[l], hi = a.level_off[l + 1];
-      if (lo + 32 * jj < hi) return;
-      base += (hi - lo + 31) / 32;
-      l++;
-      jj = first_group(l, base);
-    }
+  auto load = [&](int g, SweepVertex &v) {  // whether the lane has a vertex in group g
+    if (g >= a.groups) return false;
+    const int t = a.group_start[g] + lane;
+    if (t >= a.group_start[g + 1]) return false;
+    sweep_load(a, t, v);
+    return true;
   };
-  j = first_group(0, 0);
-  settle(lv, j, gb);
-  auto slot = [&](int l, int jj) { return a.level_off[l] + 32 * jj + lane; };
   SweepVertex cur{};
-  bool has = lv < a.levels && slot(lv, j) < a.level_off[lv + 1];
-  if (has) sweep_load(a, slot(lv, j), cur);
-  bool ok = true;
-  while (lv < a.levels) {
-    int nlv = lv, nj = j + W;
-    long long ngb = gb;
-    settle(nlv, nj, ngb);
+  bool has = load(w, cur);
+  for (int g = w; g < a.groups; g += W) {
     SweepVertex nxt{};
-    const bool nhas = nlv < a.levels && slot(nlv, nj) < a.level_off[nlv + 1];
-    if (nhas) sweep_load(a, slot(nlv, nj), nxt);
-    if (has && ok) ok = sweep_vertex(a, cur);
-    if (nlv != lv) __syncwarp();  // the warp's level is done before its next level starts
-    lv = nlv;
-    j = nj;
-    gb = ngb;
+    const bool nhas = load(g + W, nxt);
+    if (!sweep_group(a, cur, has)) return;  // the group is done before the warp's next one starts
     cur = nxt;
     has = nhas;
   }
@@ -1761,7 +1814,7 @@ int bh_build(bl_ctx *ctx, const float2 *pos, double theta, int attract_batch) {
       BL_CUDA(ctx, cudaEventRecord(ctx->ev_fork, st));
       BL_CUDA(ctx, cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
     }
-    unmoved_attraction_kernel<<<nblk(n, 256), 256, 0, side ? ctx->side : st>>>(
+    unmoved_attraction_kernel<<<nblk(n, kAttractThreads), kAttractThreads, 0, side ? ctx->side : st>>>(
         n, ctx->g.rowptr, ctx->g.colids, pos, attract_batch, (float)ctx->weight, s.f0);
     ctx->launches++;
   }
@@ -1915,10 +1968,10 @@ int bh_iteration(bl_ctx *ctx, int batch, double theta, double step, bool want_en
   if (int rc = bh_traverse(ctx, theta, false, batch)) return rc;
   SweepArgs a;
   a.order = ls->order;
-  a.level_off = ls->d_offsets;
+  a.group_start = ls->d_groups;
   a.early_off = ls->early_off;
   a.early_col = ls->early_col;
-  a.levels = ls->levels;
+  a.groups = ls->groups;
   a.f0 = ctx->s.f0;
   a.f0out = ctx->s.f0;
   a.pold = pold;
@@ -2216,16 +2269,20 @@ const LevelSchedule *level_schedule(bl_ctx *ctx, int batch) {
   ls.offsets.assign(ls.levels + 1, 0);
   for (int i = 0; i < n; i++) ls.offsets[lev[i] + 1]++;
   for (int l = 0; l < ls.levels; l++) ls.offsets[l + 1] += ls.offsets[l];
+  std::vector<int> start;  // the sweep's groups: up to 32 slots of one level
+  for (int l = 0; l < ls.levels; l++)
+    for (int t = ls.offsets[l]; t < ls.offsets[l + 1]; t += 32) start.push_back(t);
+  ls.groups = (int)start.size();
+  start.push_back(n);
   std::vector<int> order(std::max(n, 1));
   std::vector<int> fill(ls.offsets.begin(), ls.offsets.end() - 1);
   for (int i = 0; i < n; i++) order[fill[lev[i]]++] = i;
   if (cudaMalloc(&ls.order, order.size() * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&ls.d_offsets, ls.offsets.size() * sizeof(int)) != cudaSuccess) {
+      cudaMalloc(&ls.d_groups, start.size() * sizeof(int)) != cudaSuccess) {
     bl_fail(ctx, -2, "cudaMalloc level schedule");
     return nullptr;
   }
-  if (cudaMemcpy(ls.d_offsets, ls.offsets.data(), ls.offsets.size() * sizeof(int), cudaMemcpyHostToDevice) !=
-      cudaSuccess) {
+  if (cudaMemcpy(ls.d_groups, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
     bl_fail(ctx, -2, "cudaMemcpy level schedule");
     return nullptr;
   }

@@ -161,7 +161,8 @@ struct LevelSchedule {
   int levels = 0;
   std::vector<int> offsets;  // host copy, levels + 1 entries
   int *order = nullptr;      // device: vertices grouped by level
-  int *d_offsets = nullptr;  // device copy of offsets
+  int groups = 0;            // the sweep's: up to 32 slots of one level
+  int *d_groups = nullptr;   // device: first slot of each group, then n
   int *early_off = nullptr;  // per level-order slot: neighbours in earlier batches
   int *early_col = nullptr;
 };
