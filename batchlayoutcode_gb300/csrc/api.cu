@@ -77,7 +77,7 @@ int bl_check_status(bl_ctx *ctx) {
                      : st.code == DEV_TIMEOUT_TREE        ? "tree build wait timed out"
                      : st.code == DEV_FORCE_RANGE         ? "force beyond the fixed-point range (coincident vertices?)"
                      : st.code == DEV_TIMEOUT_MMA         ? "tensor-core MMA completion wait timed out"
-                     : st.code == DEV_TIMEOUT_SWEEP       ? "level sweep wait for a moved neighbour timed out"
+                     : st.code == DEV_TIMEOUT_SWEEP       ? "wait for a moved neighbour timed out"
                                                           : "device error";
   cudaMemset(ctx->s.status, 0, sizeof(DevStatus));
   return bl_fail(ctx, BL_ERR_DEVICE_TIMEOUT,
@@ -175,7 +175,7 @@ void free_ctx(bl_ctx *c) {
   fr(s.bchild); fr(s.brange); fr(s.bdelta); fr(s.qkids); fr(s.qpar); fr(s.qnchild); fr(s.span); fr(s.span_stage); fr(s.ztab); fr(s.chain); fr(s.qcen); fr(s.qbelow); fr(s.startcnt);
   fr(s.startbase); fr(s.nodes); fr(s.nodes_c64); fr(s.nodes_lvl); fr(s.rep);
   fr(s.stats); fr(s.pos_alt); fr(s.f0); fr(s.runs); fr(s.bnode); fr(s.pairs); fr(s.walk_off); fr(s.walk_pairs);
-  fr(s.term_off); fr(s.terms); fr(s.term_tgt); fr(s.greedy_share); fr(s.greedy_pos);
+  fr(s.term_off); fr(s.terms); fr(s.greedy_pos);
   for (auto &ls : c->schedules) {
     fr(ls.order);
     fr(ls.d_groups);

@@ -15,25 +15,18 @@
 // graph instead of once per vertex and iteration: walk_kernel (a warp per
 // vertex, the stack in HBM, each popped row scanned 32 entries at a time,
 // pushes kept in CSR order by a ballot) merges repeated sources in shared
-// memory and stores each vertex's walk as (source, count) pairs, in a count
-// pass and a fill pass around a prefix sum.  An iteration is then a sparse
-// gather over a per-vertex term list (CSR entries, then walk pairs):
-// greedy_iteration_kernel runs all first-phase iterations in one launch of a
-// single thread-block cluster (batches are sequential, so one cluster of up
-// to 16 SMs joined by hardware barriers -- no spin-waits -- does the whole
-// phase).  Each CTA takes a share of every batch with about the same number
-// of terms, sums its targets' terms through warp segmented scans into
-// fixed-point shared-memory accumulators (deterministic), and moves its
-// targets; positions alternate between two arrays by the parity of the
-// number of moves, which keeps the batch's start positions readable while
-// it moves (Jacobi inside the batch) and leaves one cluster barrier per
-// batch to publish the moves (Gauss-Seidel across batches).  The next
-// batch's target positions and first terms are loaded during the batch
-// before.  Positions (8 B per vertex) stay in L2.
+// memory and stores each vertex's walk as (source, count) pairs, in a
+// count pass and a fill pass around a prefix sum.  An iteration is then a
+// sparse gather over a per-vertex term list (CSR entries, then walk pairs):
+// greedy_iteration_kernel runs all first-phase iterations in one persistent
+// launch without barriers.  A warp takes a vertex, a lane a term; a position
+// word is its own ready flag, so a vertex waits only for the sources it reads
+// (Gauss-Seidel across batches, Jacobi inside a batch) and vertices of many
+// batches, and of two iterations, are in work at once.
 //
 // Summation order differs from the reference's (pairs instead of walk
-// order, FP32 terms summed in warp order and 2^-28 fixed point instead of
-// FP64): results agree within FP32 rounding.
+// order, FP32 terms summed exactly in units of 2^-28 instead of in FP64):
+// results agree within FP32 rounding.
 #include <algorithm>
 #include <cstring>
 #include <numeric>
@@ -175,254 +168,328 @@ __global__ void __launch_bounds__(kWalkThreads) walk_kernel(WalkArgs a) {
 
 // Term list of a vertex i, at term_off[i] = rowptr[i] + walk_off[i]: its CSR
 // entries as (neighbour, 0) -- attraction -- then its walk pairs as
-// (source, count) -- count x repulsion -- each with its target i.
+// (source, count) -- count x repulsion.
 __global__ void term_list_kernel(int n, const int *__restrict__ rowptr, const int *__restrict__ colids,
                                  const long long *__restrict__ walk_off, const int2 *__restrict__ walk_pairs,
-                                 int2 *__restrict__ terms, int *__restrict__ term_tgt) {
+                                 int2 *__restrict__ terms) {
   const int warp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (warp >= n) return;
   const int i = warp;
   const int r0 = rowptr[i], r1 = rowptr[i + 1];
   const long long w0 = walk_off[i], w1 = walk_off[i + 1];
   const long long q0 = (long long)r0 + w0;
-  for (int k = r0 + lane; k < r1; k += 32) {
-    terms[q0 + (k - r0)] = make_int2(colids[k], 0);
-    term_tgt[q0 + (k - r0)] = i;
-  }
+  for (int k = r0 + lane; k < r1; k += 32) terms[q0 + (k - r0)] = make_int2(colids[k], 0);
   const long long qa = q0 + (r1 - r0);
-  for (long long k = w0 + lane; k < w1; k += 32) {
-    terms[qa + (k - w0)] = walk_pairs[k];
-    term_tgt[qa + (k - w0)] = i;
-  }
+  for (long long k = w0 + lane; k < w1; k += 32) terms[qa + (k - w0)] = walk_pairs[k];
 }
 
-constexpr int kIterThreads = 512;
-constexpr int kPre = 2;  // terms per thread loaded ahead of each batch
+constexpr int kIterThreads = 896;
+constexpr int kIterWarps = kIterThreads / 32;
+constexpr int kPosBufs = 5;
 
-// Fixed-point force accumulators (units of 2^-28, the minibatch sweep's
-// format): integer atomics are exact and order-free, so the per-target sums
-// do not depend on which warp adds first.  A partial beyond +-2^34 is
-// reported instead of wrapping.
+// Fixed-point force sums (units of 2^-28, the minibatch sweep's format):
+// exact, so they do not depend on the order of the terms.  A term or a lane's
+// sum beyond +-2^34 is reported instead of wrapping.
 constexpr float kFix = 268435456.0f;
 constexpr double kFixInv = 1.0 / 268435456.0;
 constexpr float kFixLimit = 17179869184.0f;
 
+// Batches above this were never taken (they did not fit the shared-memory
+// sums of an earlier form); callers get the same error.
+constexpr size_t kBatchBytes = 2 * sizeof(long long) + 2 * sizeof(float2);
+
+// A position not yet written: both coordinates NaN, all bits set.
+constexpr unsigned long long kNoPos = 0xffffffffffffffffull;
+
 struct IterArgs {
-  int n, batch, nbatches, iterations, energy_last;
+  int n, batch, iterations, energy_last;
   float W;
   double step0, decay;
   const long long *term_off;  // per vertex
   const int2 *terms;
-  const int *term_tgt;
-  const int *share;  // [nbatches][CTAs + 1]: first target (batch-relative) of each CTA's share
-  float2 *pos0, *pos1;  // positions after an even / odd number of moves
+  float2 *buf;         // kPosBufs arrays of n positions: after m moves in array m % kPosBufs
+  unsigned int *done;  // [4]: blocks whose warps have all left iteration k, in word k & 3
   double2 *force;
   double *e;
   DevStatus *st;
 };
 
-__device__ __forceinline__ void cluster_arrive() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+__device__ __forceinline__ unsigned long long ld_word(const float2 *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
 }
 
-__device__ __forceinline__ void cluster_wait() {
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void st_word(float2 *p, unsigned long long b) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
 }
 
-__device__ __forceinline__ unsigned int cluster_rank() {
-  unsigned int r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
+__device__ __forceinline__ float2 word_pos(unsigned long long b) {
+  return make_float2(__uint_as_float((unsigned int)b), __uint_as_float((unsigned int)(b >> 32)));
 }
 
-__device__ __forceinline__ unsigned int cluster_count() {
-  unsigned int r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
+__device__ __forceinline__ unsigned long long pos_word(float2 p) {
+  return (unsigned long long)__float_as_uint(p.x) | ((unsigned long long)__float_as_uint(p.y) << 32);
 }
 
-__device__ __forceinline__ void fix_add_shared(long long *dst, float v, DevStatus *st) {
-  if (!(fabsf(v) < kFixLimit)) {
-    dev_record_error(st, DEV_FORCE_RANGE);
-    return;
+// Array 0: the start; arrays 1 and 2: not written; no warp has left an
+// iteration.  (Arrays 3 and 4 are cleared by iterations 0 and 1.)
+__global__ void greedy_start_kernel(IterArgs a, const float2 *__restrict__ pos) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 4) a.done[i] = 0u;
+  if (i >= a.n) return;
+  unsigned long long b = pos_word(pos[i]);
+  if (b == kNoPos) b = 0x7fffffff7fffffffull;  // a NaN that is not the flag
+  st_word(&a.buf[i], b);
+  st_word(&a.buf[(size_t)a.n + i], kNoPos);
+  st_word(&a.buf[2 * (size_t)a.n + i], kNoPos);
+}
+
+// The sum over the warp of one signed 64-bit value a lane (|v| < 2^62), by
+// three 27-bit limbs; false when it leaves 64 bits.
+__device__ __forceinline__ bool warp_sum_ll(long long v, long long &sum) {
+  const unsigned int lo = __reduce_add_sync(0xffffffffu, (unsigned int)v & 0x7ffffffu);
+  const unsigned int mid = __reduce_add_sync(0xffffffffu, (unsigned int)(v >> 27) & 0x7ffffffu);
+  const int hi = __reduce_add_sync(0xffffffffu, (int)(v >> 54));
+  sum = ((long long)hi << 54) + ((long long)mid << 27) + (long long)lo;
+  return hi > -500 && hi < 500;
+}
+
+// Whether a warp may go on waiting: false once `since` (0: the first call) is
+// too long ago or another warp recorded an error; the same in every lane.
+__device__ __forceinline__ bool keep_waiting(DevStatus *st, unsigned long long &since) {
+  const unsigned long long t = dev_globaltimer();
+  if (since == 0) since = t;
+  bool quit = ld_volatile_u32(&st->code) != 0u;
+  if (!quit && t - since > kBarrierTimeoutNs) {
+    dev_record_error(st, DEV_TIMEOUT_SWEEP);
+    quit = true;
   }
-  atomicAdd(reinterpret_cast<unsigned long long *>(dst), (unsigned long long)__float2ll_rn(v * kFix));
+  return !__any_sync(0xffffffffu, quit);
 }
 
-// One launch = one cluster running every batch of every first-phase
-// iteration.
+// All iterations of the first phase in one cooperative launch.
 //
-// Each CTA owns a share of every batch: a range of consecutive targets whose
-// terms (consecutive in the term list) add up to about 1/CTAs of the batch's
-// terms, so a target's partial sums meet in one CTA's shared memory
-// (warp segmented scans, then fixed-point shared atomics) and the CTA moves
-// its own targets after a CTA barrier.  Jacobi inside the batch without a
-// second cluster barrier: a vertex's position lives in pos0 or pos1 by the
-// parity of the number of times it has moved, so the moves of batch c go to
-// the other array while other CTAs still read the batch's start positions;
-// a reader picks the array from the vertex id (moved once more in this
-// iteration iff it lies before the current batch).  One cluster barrier per
-// batch publishes the moves.  The next batch's share, target positions
-// (staged in shared memory) and first terms are loaded during the batch
-// before (they do not move in it).
+// Task (it, i) moves vertex i in iteration it; warp w of W takes tasks w,
+// w + W, ... in (it, i) order, warps numbered so that consecutive vertices
+// land on different SMs.  A lane holds two terms at a time: it reads its
+// sources' position words, of a vertex in an earlier batch after this
+// iteration's move, of any other before it, and waits (bounded) for those not
+// written yet.  Every word a task waits for is written by a task before it in
+// the order and all blocks are resident, so the first unfinished task can
+// always proceed.  The terms whose words are there are added first, so that
+// only the latest source's term lies between its move and this one.  The lanes' fixed-point sums meet in warp reductions and the
+// new position is one 8-byte store that later tasks see as ready.
+// Positions after m moves live in array m % 5.  A task of iteration it clears
+// its word of array (it + 3) % 5, whose old content (after it - 2 moves) only
+// iterations it - 3 and it - 2 read: a warp enters iteration it when all warps
+// have left it - 2, so at most two iterations are in work, and the words are
+// clear before iteration it + 2 begins to read them.
+// Bound by the dependency chain across the batches (73 links an iteration on
+// the power-law graph below; a link is a load that sees the position, 600-700
+// cycles, the term, the reductions and the store) and, with few links, by
+// instruction issue.  One cluster of 16 blocks with a barrier per batch took
+// 2.6 us a batch whatever it depended on and left 136 SMs idle: nine
+// iterations of 100,000 vertices took 9,200 us, so 1,070 (power law) and 530
+// (geometric).  28 warps a block: 32 spill registers, 24 and 16 take 3 and
+// 11 % longer.
 __global__ void __launch_bounds__(kIterThreads, 1) greedy_iteration_kernel(IterArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  long long *acc = reinterpret_cast<long long *>(smem_raw);                // [batch][2]
-  float2 *tpos = reinterpret_cast<float2 *>(acc + 2 * (size_t)a.batch);  // [2][batch]
-  const unsigned int rank = cluster_rank(), csize = cluster_count();
-  const int tid = threadIdx.x, lane = tid & 31;
-  const bool single = a.nbatches == 1;  // the batch moves its own next targets
-  auto P = [&](int moves) { return (moves & 1) ? a.pos1 : a.pos0; };
-  auto share_of = [&](int c, int &lo, int &hi) {
-    lo = __ldg(&a.share[(size_t)c * (csize + 1) + rank]);
-    hi = __ldg(&a.share[(size_t)c * (csize + 1) + rank + 1]);
-  };
-  for (int t = tid; t < 2 * a.batch; t += kIterThreads) acc[t] = 0;
-  // batch 0: share, staged targets, first terms
-  int t_lo, t_hi;
-  share_of(0, t_lo, t_hi);
-  for (int t = t_lo + tid; t < t_hi; t += kIterThreads) tpos[t] = __ldcg(&a.pos0[t]);
-  int2 pt[kPre];
-  int pg[kPre];
-  long long q0, q1;  // this CTA's terms of the batch
-  auto load_terms = [&](int base, int lo, int hi) {
-    q0 = __ldg(&a.term_off[base + lo]);
-    q1 = __ldg(&a.term_off[base + hi]);
-#pragma unroll
-    for (int j = 0; j < kPre; j++) {
-      const long long q = q0 + (long long)j * kIterThreads + tid;
-      pg[j] = -1;
-      if (q < q1) {
-        pt[j] = __ldg(&a.terms[q]);
-        pg[j] = __ldg(&a.term_tgt[q]);
-      }
-    }
-  };
-  load_terms(0, t_lo, t_hi);
-  cluster_arrive();
-  cluster_wait();
+  __shared__ unsigned int left[4];
+  if (threadIdx.x < 4) left[threadIdx.x] = 0u;
+  if (!block_status_ok(a.st)) return;
+  const int lane = threadIdx.x & 31;
+  const int W = gridDim.x * kIterWarps, w = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
+  const int wrap = W / a.n, rest = W % a.n;  // from a task to the warp's next: iterations, vertices
   double step = a.step0;
-  unsigned int seq = 0;  // batches processed, for the staging buffer parity
-  for (int it = 0; it < a.iterations; it++) {
-    const bool last_it = it == a.iterations - 1;
-    const bool energy_it = a.energy_last && last_it;
-    const float stepf = (float)step;
-    float2 *const pnew = P(it + 1);
-    for (int c = 0; c < a.nbatches; c++, seq++) {
-      const int base = c * a.batch;
-      const int buf = (int)(seq & 1u) * a.batch, nbuf = a.batch - buf;
-      // the next batch: its share now, its target positions (unmoved in this
-      // batch unless there is only one batch) staged at the end
-      const int cn = (c + 1 < a.nbatches) ? c + 1 : 0;
-      const int nbase = cn * a.batch;
-      const int nmoves = (cn > c) ? it : it + 1;  // moves of the next targets by then
-      int n_lo, n_hi;
-      share_of(cn, n_lo, n_hi);
-      float2 stage = make_float2(0.f, 0.f);
-      if (!single && n_lo + tid < n_hi) stage = __ldcg(&P(nmoves)[nbase + n_lo + tid]);
-      // ---- partial forces of this CTA's targets from the batch's start ----
-      // a term's contribution, summed per target over the warp's run of
-      // equal targets (segmented inclusive scan), added by the run's last lane
-      auto add_term = [&](int tg, int2 term, float2 pj) {
-        float fx = 0.f, fy = 0.f;
-        if (tg >= 0) {
-          const float2 pi = tpos[buf + (tg - base)];
-          if (term.y == 0) {
-            attract_pair(MODEL_FR, a.W, pj.x, pj.y, pi.x, pi.y, fx, fy);
-          } else {
-            float rx = 0.f, ry = 0.f;
-            rep_pair(pj.x, pj.y, pi.x, pi.y, rx, ry);
-            fx = (float)term.y * rx;
-            fy = (float)term.y * ry;
+  int entered = 0;  // the iteration the warp is in, its positions before and after the move
+  const float2 *now = a.buf;
+  float2 *next = a.buf + a.n;
+  auto array_after = [&](float2 *p, int m) {  // m arrays on, cyclically
+    return p + (p + m * (size_t)a.n >= a.buf + kPosBufs * (size_t)a.n ? m - kPosBufs : m) * (long long)a.n;
+  };
+  // Leaves iterations until `target` is the current one; false when a wait ran
+  // out or another warp recorded an error.
+  auto enter = [&](int target) {
+    while (entered < target) {
+      __syncwarp();
+      bool ok = true;
+      if (lane == 0) {
+        __threadfence();
+        // the block's last warp tells the others (a warp is at most two
+        // iterations ahead: four words are enough)
+        if (atomicAdd(&left[entered & 3], 1u) % kIterWarps == kIterWarps - 1) {
+          __threadfence();
+          atomicAdd(&a.done[entered & 3], 1u);
+        }
+      }
+      entered++;
+      step = step * a.decay;
+      now = next;
+      next = array_after(next, 1);
+      if (entered >= 2 && entered < a.iterations) {
+        if (lane == 0) {
+          const int k = entered - 2;
+          const unsigned int want = gridDim.x * (unsigned int)(k / 4 + 1);
+          const unsigned long long t0 = dev_globaltimer();
+          for (unsigned int polls = 1; (int)(ld_acquire_gpu(&a.done[k & 3]) - want) < 0; polls++) {
+            __nanosleep(100);
+            if ((polls & 63u) != 0u) continue;
+            if (ld_volatile_u32(&a.st->code) != 0u) ok = false;
+            else if (dev_globaltimer() - t0 > kBarrierTimeoutNs) {
+              dev_record_error(a.st, DEV_TIMEOUT_SWEEP);
+              ok = false;
+            }
+            if (!ok) break;
           }
         }
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const float ux = __shfl_up_sync(0xffffffffu, fx, o);
-          const float uy = __shfl_up_sync(0xffffffffu, fy, o);
-          const int ut = __shfl_up_sync(0xffffffffu, tg, o);
-          if (lane >= o && ut == tg) {
-            fx += ux;
-            fy += uy;
-          }
-        }
-        const int nt = __shfl_down_sync(0xffffffffu, tg, 1);
-        if (tg >= 0 && (lane == 31 || nt != tg)) {
-          fix_add_shared(&acc[2 * (tg - base)], fx, a.st);
-          fix_add_shared(&acc[2 * (tg - base) + 1], fy, a.st);
-        }
-      };
-      auto gather = [&](int tg, int j) {
-        return tg >= 0 ? __ldcg(&P(it + (j < base ? 1 : 0))[j]) : make_float2(0.f, 0.f);
-      };
-      // the loaded-ahead terms: every gather issued before the first use
-      float2 pj[kPre];
-#pragma unroll
-      for (int j = 0; j < kPre; j++) pj[j] = gather(pg[j], pt[j].x);
-#pragma unroll
-      for (int j = 0; j < kPre; j++) add_term(pg[j], pt[j], pj[j]);
-      // the rest of the share (CTA-uniform trip count)
-      for (long long q = q0 + (long long)kPre * kIterThreads; q < q1; q += kIterThreads) {
-        int tg = -1;
-        int2 term = make_int2(0, 0);
-        if (q + tid < q1) {
-          term = __ldg(&a.terms[q + tid]);
-          tg = __ldg(&a.term_tgt[q + tid]);
-        }
-        add_term(tg, term, gather(tg, term.x));
+        if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) return false;
       }
-      __syncthreads();
-      // ---- this CTA's targets move (:1171-1177) into the other array ----
-      for (int t = t_lo + tid; t < t_hi; t += kIterThreads) {
-        const int i = base + t;
-        const long long vx = acc[2 * t], vy = acc[2 * t + 1];
-        acc[2 * t] = 0;
-        acc[2 * t + 1] = 0;
-        const double dfx = (double)vx * kFixInv, dfy = (double)vy * kFixInv;
-        const float2 np = unit_step(tpos[buf + t], dfx, dfy, stepf);
-        pnew[i] = np;
-        if (single) tpos[nbuf + t] = np;  // this CTA's next targets are the same
-        if (last_it) a.force[i] = make_double2(dfx, dfy);
-        if (energy_it) a.e[i] = dfx * dfx + dfy * dfy;
-      }
-      if (!single) {
-        if (n_lo + tid < n_hi) tpos[nbuf + n_lo + tid] = stage;
-        for (int t = n_lo + tid + kIterThreads; t < n_hi; t += kIterThreads)
-          tpos[nbuf + t] = __ldcg(&P(nmoves)[nbase + t]);
-      }
-      cluster_arrive();
-      load_terms(nbase, n_lo, n_hi);  // registers only
-      t_lo = n_lo;
-      t_hi = n_hi;
-      cluster_wait();
     }
-    step = step * a.decay;
+    return true;
+  };
+  int it = w / a.n, i = w % a.n;
+  int off = i % a.batch;  // i's place in its batch
+  const int rest_off = rest % a.batch;
+  // the graph's part of the tasks ahead: offsets two tasks, terms one task
+  int inext = i + rest;
+  if (inext >= a.n) inext -= a.n;
+  struct Terms {
+    const int2 *at;
+    int count;
+  };
+  auto terms_of = [&](int v) {
+    const long long q = __ldg(&a.term_off[v]);
+    return Terms{a.terms + q, (int)(__ldg(&a.term_off[v + 1]) - q)};
+  };
+  auto term = [&](const Terms &t, int k) { return k < t.count ? __ldg(&t.at[k]) : make_int2(-1, 0); };
+  Terms cur = terms_of(i), coming = terms_of(inext);
+  int2 t0 = term(cur, lane), t1 = term(cur, 32 + lane);
+  while (it < a.iterations) {
+    if (!enter(it)) return;
+    const int batch_lo = i - off;
+    // the words of this task, then the graph's part of the tasks ahead
+    auto source = [&](int j) { return (j < batch_lo ? next : now) + j; };
+    unsigned long long bi = ld_word(&now[i]);
+    unsigned long long b0 = t0.x >= 0 ? ld_word(source(t0.x)) : 0ull;
+    unsigned long long b1 = t1.x >= 0 ? ld_word(source(t1.x)) : 0ull;
+    int iahead = inext + rest;
+    if (iahead >= a.n) iahead -= a.n;
+    const Terms ahead = terms_of(iahead);
+    const int2 u0 = term(coming, lane), u1 = term(coming, 32 + lane);
+    // polls until no lane misses its word; false when that takes too long
+    auto wait = [&](unsigned long long &b, const float2 *at) {
+      unsigned long long since = 0;
+      for (unsigned int polls = 1; __any_sync(0xffffffffu, b == kNoPos); polls++) {
+        if (b == kNoPos) b = ld_word(at);
+        if ((polls & 255u) == 0u && !keep_waiting(a.st, since)) return false;
+      }
+      return true;
+    };
+    if (!wait(bi, &now[i])) return;  // its own position before this iteration
+    const float2 pi = word_pos(bi);
+    long long ax = 0, ay = 0;
+    unsigned int wide = 0u;
+    auto add = [&](int count, unsigned long long b) {
+      const float2 pj = word_pos(b);
+      float fx = 0.f, fy = 0.f;
+      if (count == 0) {
+        attract_pair(MODEL_FR, a.W, pj.x, pj.y, pi.x, pi.y, fx, fy);
+      } else {
+        rep_pair(pj.x, pj.y, pi.x, pi.y, fx, fy);
+        fx *= (float)count;
+        fy *= (float)count;
+      }
+      if (!(fmaxf(fabsf(fx), fabsf(fy)) < kFixLimit && fx == fx && fy == fy)) wide = 0x80000000u;
+      ax += __float2ll_rn(fx * kFix);
+      ay += __float2ll_rn(fy * kFix);
+      // the sign of `wide` stays set once a sum leaves 63 bits (|sum| < 2^62
+      // before and |term| <= 2^62 do not wrap)
+      const unsigned int hx = (unsigned int)(ax >> 32), hy = (unsigned int)(ay >> 32);
+      wide |= (hx ^ (hx << 1)) | (hy ^ (hy << 1));
+    };
+    // the terms whose words are there, in any order (the sums are exact); the
+    // others' places are noted: bit k for the lane's k-th term
+    unsigned long long pend = 0ull;
+    for (int k = 0; 64ll * k < cur.count; k++) {
+      const int q = 64 * (k + 1) + lane;
+      const int2 v0 = term(cur, q), v1 = term(cur, q + 32);
+      if (k >= 32) {  // no bits left: wait here
+        if (!wait(b0, source(max(t0.x, 0))) || !wait(b1, source(max(t1.x, 0)))) return;
+      }
+      if (t0.x >= 0) {
+        if (b0 != kNoPos) add(t0.y, b0);
+        else pend |= 1ull << (2 * k);
+      }
+      if (t1.x >= 0) {
+        if (b1 != kNoPos) add(t1.y, b1);
+        else pend |= 2ull << (2 * k);
+      }
+      t0 = v0;
+      t1 = v1;
+      b0 = t0.x >= 0 ? ld_word(source(t0.x)) : 0ull;
+      b1 = t1.x >= 0 ? ld_word(source(t1.x)) : 0ull;
+    }
+    // the rest as they come, each lane its first one
+    if (__any_sync(0xffffffffu, pend != 0ull)) {
+      auto first = [&]() {
+        return pend ? __ldg(&cur.at[32 * (__ffsll((long long)pend) - 1) + lane]) : make_int2(-1, 0);
+      };
+      int2 tm = first();
+      unsigned long long since = 0;
+      for (unsigned int polls = 1; __any_sync(0xffffffffu, tm.x >= 0); polls++) {
+        const unsigned long long b = tm.x >= 0 ? ld_word(source(tm.x)) : kNoPos;
+        if (b != kNoPos) {
+          add(tm.y, b);
+          pend &= pend - 1ull;
+          tm = first();
+        }
+        if ((polls & 255u) == 0u && !keep_waiting(a.st, since)) return;
+      }
+    }
+    long long sx, sy;
+    const bool fits = warp_sum_ll(ax, sx) & warp_sum_ll(ay, sy);
+    if (!__all_sync(0xffffffffu, (int)wide >= 0 && fits)) {
+      if (lane == 0) dev_record_error(a.st, DEV_FORCE_RANGE);
+      return;
+    }
+    // the move (:1171-1177), the same in every lane
+    const float fx = __ll2float_rn(sx) * (float)kFixInv, fy = __ll2float_rn(sy) * (float)kFixInv;
+    const float stepf = (float)step;
+    const float m2 = fmaf(fx, fx, fy * fy);
+    float2 np = pi;
+    if (m2 >= 1.17549435e-38f && m2 <= 3.0e38f) {
+      const float rm = rsqrt_approx(m2);
+      np.x = fmaf(stepf, fx * rm, np.x);
+      np.y = fmaf(stepf, fy * rm, np.y);
+    } else {
+      np = unit_step(pi, (double)sx * kFixInv, (double)sy * kFixInv, stepf);
+    }
+    if (lane == 0) {
+      unsigned long long b = pos_word(np);
+      if (b == kNoPos) b = 0x7fffffff7fffffffull;
+      st_word(&next[i], b);
+      st_word(&array_after(next, 2)[i], kNoPos);
+      if (it == a.iterations - 1) {
+        const double dfx = (double)sx * kFixInv, dfy = (double)sy * kFixInv;
+        a.force[i] = make_double2(dfx, dfy);
+        if (a.energy_last) a.e[i] = dfx * dfx + dfy * dfy;
+      }
+    }
+    off += rest_off;
+    if (off >= a.batch) off -= a.batch;
+    it += wrap;
+    if (inext < i) {  // past the last vertex
+      it++;
+      off = inext % a.batch;
+    }
+    i = inext;
+    inext = iahead;
+    cur = coming;
+    coming = ahead;
+    t0 = u0;
+    t1 = u1;
   }
-}
-
-// Largest cluster (16, else 8, 4, 2, 1 CTAs) of `kernel` with `smem` bytes
-// of dynamic shared memory per CTA that can be scheduled (0: none).
-template <typename Kernel>
-int largest_cluster(Kernel kernel, size_t smem) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (smem) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  for (int c : {16, 8, 4, 2, 1}) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(c);
-    cfg.blockDim = dim3(kIterThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = c;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters >= 1) return c;
-    cudaGetLastError();  // clear a refused size
-  }
-  return 0;
+  enter(a.iterations);
 }
 
 }  // namespace
@@ -546,14 +613,12 @@ int greedy_terms_build(bl_ctx *ctx) {
   std::vector<long long> woff(n + 1);
   BL_CUDA(ctx, cudaMemcpy(woff.data(), ctx->s.walk_off, (size_t)(n + 1) * sizeof(long long), cudaMemcpyDeviceToHost));
   for (int i = 0; i <= n; i++) woff[i] += ctx->h_rowptr[i];
-  ctx->s.h_term_off = woff;
   BL_CUDA(ctx, cudaMalloc(&ctx->s.term_off, (size_t)(n + 1) * sizeof(long long)));
   BL_CUDA(ctx, cudaMemcpy(ctx->s.term_off, woff.data(), (size_t)(n + 1) * sizeof(long long), cudaMemcpyHostToDevice));
-  BL_CUDA(ctx, cudaMalloc(&ctx->s.term_tgt, (size_t)std::max<long long>(total, 1) * sizeof(int)));
   BL_CUDA(ctx, cudaMalloc(&ctx->s.terms, (size_t)std::max<long long>(total, 1) * sizeof(int2)));
   const long long threads = 32LL * n;
   term_list_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(
-      n, ctx->g.rowptr, ctx->g.colids, ctx->s.walk_off, ctx->s.walk_pairs, ctx->s.terms, ctx->s.term_tgt);
+      n, ctx->g.rowptr, ctx->g.colids, ctx->s.walk_off, ctx->s.walk_pairs, ctx->s.terms);
   ctx->launches++;
   BL_CUDA(ctx, cudaGetLastError());
   return 0;
@@ -567,41 +632,15 @@ int greedy_walk_run(bl_ctx *ctx, int batch, int iterations, double step0, double
   if (int rc = greedy_terms_build(ctx)) return rc;
   if (int rc = bl_check_status(ctx)) return rc;
   batch = std::min(batch, n);
-  const size_t smem = (size_t)batch * 2 * sizeof(long long) + (size_t)2 * batch * sizeof(float2);
   int smem_optin = 0;
   cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-  if (smem + 1024 > (size_t)smem_optin)
-    return bl_fail(ctx, BL_ERR_TOO_LARGE, "algo 5: batch too large for the shared-memory accumulators");
-  const int csize = largest_cluster(greedy_iteration_kernel, smem);
-  if (csize < 1) return bl_fail(ctx, BL_ERR_TOO_LARGE, "algo 5: no thread-block cluster fits");
-  const int nbatches = (n + batch - 1) / batch;
-  // each CTA's share of every batch: consecutive targets with about
-  // 1/csize of the batch's terms (graph-only; kept for this batch size)
-  if (ctx->s.greedy_share_key != (long long)batch * 64 + csize) {
-    std::vector<int> share((size_t)nbatches * (csize + 1));
-    const std::vector<long long> &to = ctx->s.h_term_off;
-    for (int c = 0; c < nbatches; c++) {
-      const int base = c * batch, cnt = std::min(batch, n - base);
-      const long long q0 = to[base], T = to[base + cnt] - q0;
-      int t = 0;
-      for (int r = 0; r <= csize; r++) {
-        const long long want = (r == csize) ? T : (T * r + csize - 1) / csize;
-        while (t < cnt && to[base + t] - q0 < want) t++;
-        share[(size_t)c * (csize + 1) + r] = (r == csize) ? cnt : t;
-      }
-    }
-    if (ctx->s.greedy_share) cudaFree(ctx->s.greedy_share);
-    ctx->s.greedy_share = nullptr;
-    ctx->s.greedy_share_key = -1;
-    BL_CUDA(ctx, cudaMalloc(&ctx->s.greedy_share, share.size() * sizeof(int)));
-    BL_CUDA(ctx, cudaMemcpy(ctx->s.greedy_share, share.data(), share.size() * sizeof(int), cudaMemcpyHostToDevice));
-    ctx->s.greedy_share_key = (long long)batch * 64 + csize;
+  if (batch * kBatchBytes + 1024 > (size_t)smem_optin) return bl_fail(ctx, BL_ERR_TOO_LARGE, "algo 5: batch too large");
+  if (!ctx->s.greedy_pos) {
+    BL_CUDA(ctx, cudaMalloc(&ctx->s.greedy_pos, (size_t)kPosBufs * std::max(n, 2) * sizeof(float2) + 4 * sizeof(int)));
   }
-  if (!ctx->s.greedy_pos) BL_CUDA(ctx, cudaMalloc(&ctx->s.greedy_pos, (size_t)std::max(n, 2) * sizeof(float2)));
   IterArgs a;
   a.n = n;
   a.batch = batch;
-  a.nbatches = nbatches;
   a.iterations = iterations;
   a.energy_last = want_energy ? 1 : 0;
   a.W = (float)ctx->weight;
@@ -609,33 +648,25 @@ int greedy_walk_run(bl_ctx *ctx, int batch, int iterations, double step0, double
   a.decay = decay;
   a.term_off = ctx->s.term_off;
   a.terms = ctx->s.terms;
-  a.term_tgt = ctx->s.term_tgt;
-  a.share = ctx->s.greedy_share;
-  a.pos0 = ctx->pos;
-  a.pos1 = ctx->s.greedy_pos;
+  a.buf = ctx->s.greedy_pos;
+  a.done = reinterpret_cast<unsigned int *>(a.buf + (size_t)kPosBufs * std::max(n, 2));
   a.force = ctx->force;
   a.e = ctx->e;
   a.st = ctx->s.status;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(csize);
-  cfg.blockDim = dim3(kIterThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = ctx->stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = csize;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  int occ = 0;
+  BL_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, greedy_iteration_kernel, kIterThreads, 0));
+  if (occ < 1) return bl_fail(ctx, BL_ERR_TOO_LARGE, "algo 5: the iteration kernel cannot be resident");
+  const int grid = std::min(ctx->num_sms, (n + kIterWarps - 1) / kIterWarps);  // no more warps than vertices need
+  greedy_start_kernel<<<(std::max(n, 4) + 255) / 256, 256, 0, ctx->stream>>>(a, ctx->pos);
+  ctx->launches++;
   bl_time_begin(ctx, "greedy_iteration_kernel");
-  BL_CUDA(ctx, cudaLaunchKernelEx(&cfg, greedy_iteration_kernel, a));
+  void *args[] = {&a};
+  BL_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)greedy_iteration_kernel, dim3(grid), dim3(kIterThreads), args, 0,
+                                           ctx->stream));
   bl_time_end(ctx, "greedy_iteration_kernel");
   ctx->launches++;
-  // every vertex moved `iterations` times: an odd count leaves them in pos1
-  if (iterations & 1)
-    BL_CUDA(ctx, cudaMemcpyAsync(ctx->pos, ctx->s.greedy_pos, (size_t)n * sizeof(float2), cudaMemcpyDeviceToDevice,
-                                 ctx->stream));
+  BL_CUDA(ctx, cudaMemcpyAsync(ctx->pos, a.buf + (size_t)(iterations % kPosBufs) * n, (size_t)n * sizeof(float2),
+                               cudaMemcpyDeviceToDevice, ctx->stream));
   if (want_energy) {
     if (int rc = energy_reduce(ctx, energy_out)) return rc;
   } else {
