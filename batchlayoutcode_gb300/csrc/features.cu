@@ -288,14 +288,33 @@ __device__ __forceinline__ double hop2(const unsigned short *dist, int v, int s,
 }
 
 // per block: largest finite distance per pivot
-__global__ void mds_max_kernel(int v0, int v1, const unsigned short *dist, int *part) {
+// The pivot MDS of a slice of graphs: blockIdx.y is the graph of the slice,
+// mds_blocks(n) blocks of blockIdx.x work on its n vertices.  Everything
+// between the distances and the 16 x 16 eigenproblem stays on the device, all
+// graphs at once: with a host reduction (and its synchronisation) after each
+// of three kernels a graph, twelve graphs took 2.3 ms, so they take 1.0 (the
+// eigenproblems included).
+constexpr int kMdsBlocks = 256;
+constexpr int kMdsSlice = 64;        // graphs a launch: bounds the partials' memory
+constexpr int kGram = kP * (kP + 1) / 2;
+constexpr int kMean = kP + 1;        // a graph's column means, then their mean
+
+__host__ __device__ __forceinline__ int mds_blocks(int n) {
+  const int b = (n + 255) / 256;
+  return b < kMdsBlocks ? b : kMdsBlocks;
+}
+
+// hop maxima of every pivot into maxd (zero before)
+__global__ void mds_max_kernel(const int *voff, const unsigned short *dist, int *maxd) {
+  const int g = blockIdx.y, v0 = voff[g], v1 = voff[g + 1], blocks = mds_blocks(v1 - v0);
+  if ((int)blockIdx.x >= blocks) return;
   __shared__ int smax[kP];
   if (threadIdx.x < kP) smax[threadIdx.x] = 0;
   __syncthreads();
   int m[kP];
 #pragma unroll
   for (int s = 0; s < kP; s++) m[s] = 0;
-  for (int v = v0 + blockIdx.x * blockDim.x + threadIdx.x; v < v1; v += gridDim.x * blockDim.x)
+  for (int v = v0 + blockIdx.x * blockDim.x + threadIdx.x; v < v1; v += blocks * blockDim.x)
 #pragma unroll
     for (int s = 0; s < kP; s++) {
       const unsigned short d = dist[(size_t)v * kP + s];
@@ -304,7 +323,7 @@ __global__ void mds_max_kernel(int v0, int v1, const unsigned short *dist, int *
 #pragma unroll
   for (int s = 0; s < kP; s++) atomicMax(&smax[s], m[s]);
   __syncthreads();
-  if (threadIdx.x < kP) part[blockIdx.x * kP + threadIdx.x] = smax[threadIdx.x];
+  if (threadIdx.x < kP) atomicMax(&maxd[g * kP + threadIdx.x], smax[threadIdx.x]);
 }
 
 __device__ void block_sum_doubles(double *vals, int count, double *scratch, double *out) {
@@ -324,27 +343,54 @@ __device__ void block_sum_doubles(double *vals, int count, double *scratch, doub
 }
 
 // per block: column sums of the squared distances
-__global__ void __launch_bounds__(256) mds_colsum_kernel(int v0, int v1, const unsigned short *dist,
-                                                         const int *maxd, double *part) {
+__global__ void __launch_bounds__(256) mds_colsum_kernel(const int *voff, const unsigned short *dist, const int *maxds,
+                                                         double *part) {
+  const int g = blockIdx.y, v0 = voff[g], v1 = voff[g + 1], blocks = mds_blocks(v1 - v0);
+  if ((int)blockIdx.x >= blocks) return;
+  const int *maxd = maxds + g * kP;
   __shared__ double scratch[8 * kP];
   double c[kP];
 #pragma unroll
   for (int s = 0; s < kP; s++) c[s] = 0.0;
-  for (int v = v0 + blockIdx.x * blockDim.x + threadIdx.x; v < v1; v += gridDim.x * blockDim.x)
+  for (int v = v0 + blockIdx.x * blockDim.x + threadIdx.x; v < v1; v += blocks * blockDim.x)
 #pragma unroll
     for (int s = 0; s < kP; s++) c[s] += hop2(dist, v, s, maxd);
-  block_sum_doubles(c, kP, scratch, part + (size_t)blockIdx.x * kP);
+  block_sum_doubles(c, kP, scratch, part + ((size_t)g * kMdsBlocks + blockIdx.x) * kP);
+}
+
+// the means from the blocks' sums, added in block order
+__global__ void mds_mean_kernel(const int *voff, const double *part, double *mean) {
+  const int g = blockIdx.x, n = voff[g + 1] - voff[g], blocks = mds_blocks(n), s = threadIdx.x;
+  __shared__ double m[kP];
+  if (s < kP) {
+    double t = 0.0;
+#pragma unroll 8
+    for (int b = 0; b < blocks; b++) t += part[((size_t)g * kMdsBlocks + b) * kP + s];
+    m[s] = t / n;
+    mean[g * kMean + s] = m[s];
+  }
+  __syncthreads();
+  if (s == 0) {
+    double grand = 0.0;
+    for (int k = 0; k < kP; k++) grand += m[k];
+    mean[g * kMean + kP] = grand / kP;
+  }
 }
 
 // per block: Gram matrix sum_v C_v C_v^T of the double-centred rows
 // C[v][s] = -0.5 (D2[v][s] - r_v - c_s + g), upper triangle (136 values):
 // a tile of 256 rows is staged in shared memory, thread t < 136 owns entry t.
-__global__ void __launch_bounds__(256) mds_gram_kernel(int v0, int v1, const unsigned short *dist, const int *maxd,
-                                                       const double *colmean, double grand, double *part) {
+__global__ void __launch_bounds__(256) mds_gram_kernel(const int *voff, const unsigned short *dist, const int *maxds,
+                                                       const double *mean, double *part) {
+  const int g = blockIdx.y, v0 = voff[g], v1 = voff[g + 1], blocks = mds_blocks(v1 - v0);
+  if ((int)blockIdx.x >= blocks) return;
+  const int *maxd = maxds + g * kP;
+  const double *colmean = mean + g * kMean;
+  const double grand = colmean[kP];
   __shared__ double cbuf[256][kP + 1];
   const int tid = threadIdx.x;
   int pi = 0, pj = 0;
-  if (tid < 136) {
+  if (tid < kGram) {
     int k = tid, i = 0;
     while (k >= kP - i) {
       k -= kP - i;
@@ -354,7 +400,7 @@ __global__ void __launch_bounds__(256) mds_gram_kernel(int v0, int v1, const uns
     pj = i + k;
   }
   double acc = 0.0;
-  for (int base = v0 + blockIdx.x * 256; base < v1; base += gridDim.x * 256) {
+  for (int base = v0 + blockIdx.x * 256; base < v1; base += blocks * 256) {
     const int v = base + tid;
     if (v < v1) {
       double d2[kP], r = 0.0;
@@ -371,29 +417,43 @@ __global__ void __launch_bounds__(256) mds_gram_kernel(int v0, int v1, const uns
       for (int s = 0; s < kP; s++) cbuf[tid][s] = 0.0;
     }
     __syncthreads();
-    if (tid < 136)
+    if (tid < kGram)
       for (int rr = 0; rr < 256; rr++) acc = fma(cbuf[rr][pi], cbuf[rr][pj], acc);
     __syncthreads();
   }
-  if (tid < 136) part[(size_t)blockIdx.x * 136 + tid] = acc;
+  if (tid < kGram) part[((size_t)g * kMdsBlocks + blockIdx.x) * kGram + tid] = acc;
+}
+
+// the Gram matrices from the blocks' sums, added in block order
+__global__ void mds_gram_sum_kernel(const int *voff, const double *part, double *gram) {
+  const int g = blockIdx.x, blocks = mds_blocks(voff[g + 1] - voff[g]), k = threadIdx.x;
+  if (k >= kGram) return;
+  double t = 0.0;
+#pragma unroll 8
+  for (int b = 0; b < blocks; b++) t += part[((size_t)g * kMdsBlocks + b) * kGram + k];
+  gram[g * kGram + k] = t;
 }
 
 struct ProjectArgs {
-  int v0, v1, n_graph;
+  const int *voff;    // of the slice's graphs
   const int *rowptr;  // global CSR
   const int *colids;
   const unsigned short *dist;
   const int *maxd;
-  const double *colmean;
-  double grand;
-  const double *V;  // 16 x 12, column j = eigenvector j
-  double inv_scale;
-  float *features;  // global n x 16
+  const double *mean;  // column means, then their mean
+  const double *V;     // 16 x 12 and the scale's inverse: column j = eigenvector j
+  float *features;     // global n x 16
 };
+constexpr int kProj = kP * 12 + 1;
 
 __global__ void mds_project_kernel(ProjectArgs a) {
-  const int v = a.v0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= a.v1) return;
+  const int g = blockIdx.y, n_graph = a.voff[g + 1] - a.voff[g];
+  const int v = a.voff[g] + blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= a.voff[g + 1]) return;
+  a.maxd += g * kP;
+  a.mean += g * kMean;
+  a.V += (size_t)g * kProj;
+  const double inv_scale = a.V[kP * 12];
   double d2[kP], r = 0.0;
 #pragma unroll
   for (int s = 0; s < kP; s++) {
@@ -403,26 +463,32 @@ __global__ void mds_project_kernel(ProjectArgs a) {
   r *= 1.0 / kP;
   double c[kP];
 #pragma unroll
-  for (int s = 0; s < kP; s++) c[s] = -0.5 * (d2[s] - r - a.colmean[s] + a.grand);
+  for (int s = 0; s < kP; s++) c[s] = -0.5 * (d2[s] - r - a.mean[s] + a.mean[kP]);
   float *f = a.features + (size_t)v * kFeat;
 #pragma unroll
   for (int j = 0; j < 12; j++) {
     double y = 0.0;
 #pragma unroll
     for (int s = 0; s < kP; s++) y = fma(c[s], a.V[s * 12 + j], y);
-    f[j] = (float)(y * a.inv_scale);
+    f[j] = (float)(y * inv_scale);
   }
   const int e0 = a.rowptr[v], e1 = a.rowptr[v + 1];
   const int deg = e1 - e0;
   float m = 0.f;
-  for (int e = e0; e < e1; e++) {
-    const int u = a.colids[e];
-    m += log2f(1.0f + (float)(a.rowptr[u + 1] - a.rowptr[u]));
+  for (int e = e0; e < e1; e += 8) {  // eight neighbours' loads together, added in row order
+    int u[8], d[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) u[q] = e + q < e1 ? a.colids[e + q] : v;
+#pragma unroll
+    for (int q = 0; q < 8; q++) d[q] = a.rowptr[u[q] + 1] - a.rowptr[u[q]];
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      if (e + q < e1) m += log2f(1.0f + (float)d[q]);
   }
   f[12] = log2f(1.0f + (float)deg);
   f[13] = 1.0f / (1.0f + (float)deg);
   f[14] = deg > 0 ? m / (float)deg : 0.0f;
-  f[15] = log2f((float)a.n_graph) / 20.0f;
+  f[15] = log2f((float)n_graph) / 20.0f;
 }
 
 }  // namespace
@@ -514,14 +580,14 @@ int compute_features(bl_ctx *ctx, int num_graphs, const int *voff, int n, const 
   cudaStream_t st = ctx->stream;
   const int P = num_graphs * kP;
   unsigned int *visited = nullptr, *fr0 = nullptr, *fr1 = nullptr, *cnt = nullptr;
-  int *d_piv = nullptr, *d_maxd = nullptr, *d_ipart = nullptr, *wl0 = nullptr, *wl1 = nullptr, *d_voff = nullptr;
-  double *d_dpart = nullptr, *d_colmean = nullptr, *d_V = nullptr;
-  const int kBlocks = 256;
+  int *d_piv = nullptr, *d_maxd = nullptr, *wl0 = nullptr, *wl1 = nullptr, *d_voff = nullptr;
+  double *d_part = nullptr, *d_mean = nullptr, *d_gram = nullptr, *d_V = nullptr;
+  const int slice = std::min(num_graphs, kMdsSlice);
   int rc = 0;
   auto cleanup = [&]() {
     cudaFree(visited); cudaFree(fr0); cudaFree(fr1); cudaFree(cnt); cudaFree(wl0); cudaFree(wl1);
     cudaFree(d_piv); cudaFree(d_maxd); cudaFree(d_voff);
-    cudaFree(d_ipart); cudaFree(d_dpart); cudaFree(d_colmean); cudaFree(d_V);
+    cudaFree(d_part); cudaFree(d_mean); cudaFree(d_gram); cudaFree(d_V);
   };
   auto ck = [&](cudaError_t e, const char *w) {
     if (e != cudaSuccess && !rc) rc = bl_cuda_fail(ctx, e, w);
@@ -541,11 +607,11 @@ int compute_features(bl_ctx *ctx, int num_graphs, const int *voff, int n, const 
   ck(cudaMalloc(&cnt, 4 * sizeof(unsigned int)), "cudaMalloc");
   ck(cudaMalloc(&d_voff, sizeof(int) * (2 * num_graphs + 1)), "cudaMalloc");
   ck(cudaMalloc(&d_piv, sizeof(int) * P), "cudaMalloc");
-  ck(cudaMalloc(&d_maxd, sizeof(int) * kP), "cudaMalloc");
-  ck(cudaMalloc(&d_ipart, sizeof(int) * kBlocks * kP), "cudaMalloc");
-  ck(cudaMalloc(&d_dpart, sizeof(double) * kBlocks * 136), "cudaMalloc");
-  ck(cudaMalloc(&d_colmean, sizeof(double) * kP), "cudaMalloc");
-  ck(cudaMalloc(&d_V, sizeof(double) * kP * 12), "cudaMalloc");
+  ck(cudaMalloc(&d_maxd, sizeof(int) * kP * slice), "cudaMalloc");
+  ck(cudaMalloc(&d_part, sizeof(double) * kMdsBlocks * kGram * (size_t)slice), "cudaMalloc");
+  ck(cudaMalloc(&d_mean, sizeof(double) * kMean * slice), "cudaMalloc");
+  ck(cudaMalloc(&d_gram, sizeof(double) * kGram * slice), "cudaMalloc");
+  ck(cudaMalloc(&d_V, sizeof(double) * kProj * slice), "cudaMalloc");
   if (rc) {
     cleanup();
     return rc;
@@ -607,52 +673,39 @@ int compute_features(bl_ctx *ctx, int num_graphs, const int *voff, int n, const 
   }
   if (!rc) ck(cudaStreamSynchronize(st), "BFS");
   if (!rc) rc = bl_check_status(ctx);
-  std::vector<int> ipart(kBlocks * kP);
-  std::vector<double> dpart(kBlocks * 136);
-  for (int g = 0; g < num_graphs && !rc; g++) {
-    const int v0 = voff[g], v1 = voff[g + 1], ng = v1 - v0;
-    const int blocks = std::max(1, std::min(kBlocks, (ng + 255) / 256));
-    mds_max_kernel<<<blocks, 256, 0, st>>>(v0, v1, d_dist, d_ipart);
-    ck(cudaMemcpyAsync(ipart.data(), d_ipart, sizeof(int) * blocks * kP, cudaMemcpyDeviceToHost, st), "D2H");
+  std::vector<double> gram((size_t)slice * kGram), V12((size_t)slice * kProj);
+  for (int g0 = 0; g0 < num_graphs && !rc; g0 += slice) {
+    const int gs = std::min(slice, num_graphs - g0);
+    const int *vo = d_voff + g0;
+    int widest = 1;
+    for (int g = g0; g < g0 + gs; g++) widest = std::max(widest, mds_blocks(voff[g + 1] - voff[g]));
+    ck(cudaMemsetAsync(d_maxd, 0, sizeof(int) * kP * gs, st), "memset");
+    mds_max_kernel<<<dim3(widest, gs), 256, 0, st>>>(vo, d_dist, d_maxd);
+    mds_colsum_kernel<<<dim3(widest, gs), 256, 0, st>>>(vo, d_dist, d_maxd, d_part);
+    mds_mean_kernel<<<gs, 32, 0, st>>>(vo, d_part, d_mean);
+    mds_gram_kernel<<<dim3(widest, gs), 256, 0, st>>>(vo, d_dist, d_maxd, d_mean, d_part);
+    mds_gram_sum_kernel<<<gs, 256, 0, st>>>(vo, d_part, d_gram);
+    ctx->launches += 5;
+    ck(cudaMemcpyAsync(gram.data(), d_gram, sizeof(double) * kGram * gs, cudaMemcpyDeviceToHost, st), "D2H");
     ck(cudaStreamSynchronize(st), "sync");
-    int maxd[kP] = {0};
-    for (int b = 0; b < blocks; b++)
-      for (int s = 0; s < kP; s++) maxd[s] = std::max(maxd[s], ipart[b * kP + s]);
-    ck(cudaMemcpyAsync(d_maxd, maxd, sizeof(maxd), cudaMemcpyHostToDevice, st), "H2D");
-    mds_colsum_kernel<<<blocks, 256, 0, st>>>(v0, v1, d_dist, d_maxd, d_dpart);
-    ck(cudaMemcpyAsync(dpart.data(), d_dpart, sizeof(double) * blocks * kP, cudaMemcpyDeviceToHost, st), "D2H");
-    ck(cudaStreamSynchronize(st), "sync");
-    double colmean[kP], grand = 0.0;
-    for (int s = 0; s < kP; s++) {
-      double t = 0.0;
-      for (int b = 0; b < blocks; b++) t += dpart[b * kP + s];
-      colmean[s] = t / ng;
-      grand += colmean[s];
+    for (int g = 0; g < gs && !rc; g++) {
+      std::vector<double> S(kP * kP, 0.0), lam, V;
+      const double *t = gram.data() + (size_t)g * kGram;
+      for (int i = 0; i < kP; i++)
+        for (int j = i; j < kP; j++) S[i * kP + j] = S[j * kP + i] = *t++;
+      jacobi_eigen(kP, S, lam, V);
+      for (int s = 0; s < kP; s++)
+        for (int j = 0; j < 12; j++) V12[(size_t)g * kProj + s * 12 + j] = V[s * kP + j];
+      V12[(size_t)g * kProj + kP * 12] = lam[0] > 0 ? 1.0 / std::sqrt(lam[0] / (voff[g0 + g + 1] - voff[g0 + g])) : 0.0;
     }
-    grand /= kP;
-    ck(cudaMemcpyAsync(d_colmean, colmean, sizeof(colmean), cudaMemcpyHostToDevice, st), "H2D");
-    mds_gram_kernel<<<blocks, 256, 0, st>>>(v0, v1, d_dist, d_maxd, d_colmean, grand, d_dpart);
-    ck(cudaMemcpyAsync(dpart.data(), d_dpart, sizeof(double) * blocks * 136, cudaMemcpyDeviceToHost, st), "D2H");
-    ck(cudaStreamSynchronize(st), "sync");
-    std::vector<double> S(kP * kP, 0.0);
-    int k = 0;
-    for (int i = 0; i < kP; i++)
-      for (int j = i; j < kP; j++, k++) {
-        double t = 0.0;
-        for (int b = 0; b < blocks; b++) t += dpart[b * 136 + k];
-        S[i * kP + j] = S[j * kP + i] = t;
-      }
-    std::vector<double> lam, V;
-    jacobi_eigen(kP, S, lam, V);
-    std::vector<double> V12(kP * 12);
-    for (int s = 0; s < kP; s++)
-      for (int j = 0; j < 12; j++) V12[s * 12 + j] = V[s * kP + j];
-    ck(cudaMemcpyAsync(d_V, V12.data(), sizeof(double) * kP * 12, cudaMemcpyHostToDevice, st), "H2D");
-    ProjectArgs pa{v0, v1, ng, d_rowptr, d_colids, d_dist, d_maxd, d_colmean, grand, d_V,
-                   lam[0] > 0 ? 1.0 / std::sqrt(lam[0] / ng) : 0.0, d_features};
-    mds_project_kernel<<<(ng + 255) / 256, 256, 0, st>>>(pa);
-    ctx->launches += 4;
+    ck(cudaMemcpyAsync(d_V, V12.data(), sizeof(double) * kProj * gs, cudaMemcpyHostToDevice, st), "H2D");
+    int most = 1;
+    for (int g = g0; g < g0 + gs; g++) most = std::max(most, (voff[g + 1] - voff[g] + 255) / 256);
+    ProjectArgs pa{vo, d_rowptr, d_colids, d_dist, d_maxd, d_mean, d_V, d_features};
+    mds_project_kernel<<<dim3(most, gs), 256, 0, st>>>(pa);
+    ctx->launches++;
     ck(cudaGetLastError(), "MDS kernels");
+    if (g0 + gs < num_graphs) ck(cudaStreamSynchronize(st), "MDS");  // V12 is filled again
   }
   if (!rc) ck(cudaStreamSynchronize(st), "features");
   cleanup();
