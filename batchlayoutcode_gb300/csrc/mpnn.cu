@@ -320,38 +320,61 @@ struct TopArgs {
   float *part;               // per block: 2 x 64 dWo, then 2 dbo
 };
 
+// In the backward kernels a warp's lanes take 8 rows x 4 pieces of 8 features
+// (row & 7 = lane & 7, piece = lane / 8 + 4 * half): every 32-byte sector of
+// the rows is fetched and written whole, and the 16-byte pieces of 8 rows fill
+// 128 bytes of a core matrix, all banks once.  With a row a thread each
+// instruction touched half sectors of 32 rows, and the weight gradient wrote
+// its transposed tiles two bytes at a time: 207,796 vertices took 43 us here,
+// 67 in the weight gradient (64 features) and 72 in the data gradient, so they
+// take 36, 43 and 53.
 __global__ void __launch_bounds__(kT) mpnn_top_kernel(TopArgs a) {
   __shared__ float s_dxy[kT][2];
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int j = tid >> 6, o = tid & 63;  // this thread's readout gradient entry
   float gw = 0.f, gb = 0.f;
   const int ntiles = (a.n + kT - 1) / kT;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int v = tile * kT + tid;
-    float d0 = 0.f, d1 = 0.f;
-    if (v < a.n) {
-      d0 = a.dxy[2 * (size_t)v];
-      d1 = a.dxy[2 * (size_t)v + 1];
-      float h[64];
+    s_dxy[tid][0] = v < a.n ? a.dxy[2 * (size_t)v] : 0.f;
+    s_dxy[tid][1] = v < a.n ? a.dxy[2 * (size_t)v + 1] : 0.f;
+    __syncthreads();
 #pragma unroll
-      for (int c = 0; c < 8; c++) bf16x8_to_f32(reinterpret_cast<const uint4 *>(a.h3 + (size_t)v * 64)[c], h + 8 * c);
+    for (int half = 0; half < 2; half++) {
+      const int c = (lane >> 3) + 4 * half;
+      float w0[8], w1[8];
 #pragma unroll
-      for (int c = 0; c < 16; c++) {
-        float4 r;
-        float *rr = &r.x;
+      for (int i = 0; i < 8; i++) {
+        w0[i] = a.Wo[8 * c + i];
+        w1[i] = a.Wo[64 + 8 * c + i];
+      }
+      uint4 raw[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const int oo = 4 * c + i;
-          const float g = fmaf(d0, a.Wo[oo], d1 * a.Wo[64 + oo]);
-          rr[i] = h[oo] > 0.f ? g : 0.f;
+      for (int rg = 0; rg < 4; rg++) {
+        const int row = 32 * warp + 8 * rg + (lane & 7);
+        raw[rg] = tile * kT + row < a.n
+                      ? reinterpret_cast<const uint4 *>(a.h3 + (size_t)(tile * kT + row) * 64)[c]
+                      : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int rg = 0; rg < 4; rg++) {
+        const int row = 32 * warp + 8 * rg + (lane & 7);
+        if (tile * kT + row >= a.n) continue;
+        float h[8], r[8];
+        bf16x8_to_f32(raw[rg], h);
+        const float d0 = s_dxy[row][0], d1 = s_dxy[row][1];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const float g = fmaf(d0, w0[i], d1 * w1[i]);
+          r[i] = h[i] > 0.f ? g : 0.f;
         }
-        reinterpret_cast<float4 *>(a.dz + (size_t)v * 64)[c] = r;
+        float4 *out = reinterpret_cast<float4 *>(a.dz + (size_t)(tile * kT + row) * 64 + 8 * c);
+        out[0] = make_float4(r[0], r[1], r[2], r[3]);
+        out[1] = make_float4(r[4], r[5], r[6], r[7]);
       }
     }
-    s_dxy[tid][0] = d0;
-    s_dxy[tid][1] = d1;
-    __syncthreads();
     const int cnt = min(kT, a.n - tile * kT);
+#pragma unroll 16
     for (int r = 0; r < cnt; r++) {
       const float d = s_dxy[r][j];
       gw = fmaf(d, __bfloat162float(a.h3[(size_t)(tile * kT + r) * 64 + o]), gw);
@@ -380,14 +403,17 @@ struct WgradArgs {
 template <int DIN>
 __global__ void __launch_bounds__(kT) mpnn_wgrad_kernel(WgradArgs a) {
   constexpr int K = 2 * DIN;
-  constexpr uint32_t SBO = (kT / 8) * 128;  // K of the MMA = the 128 vertices of a tile
+  constexpr int kPieces = K / 8;  // 16-byte pieces of a vertex's [h | agg]
   extern __shared__ __align__(1024) unsigned char smem[];
+  // K of the MMA = the 128 vertices of a tile; a vertex's features lie next to
+  // each other in memory and in the tiles (rows contiguous), so they are copied
+  // in 16-byte pieces instead of transposed a value at a time
   unsigned char *sA = smem;                 // 128 (k) x 128 (v)
   unsigned char *sB = smem + kT * kT * 2;   // 64 (o) x 128 (v)
   __shared__ uint64_t mbar;
   __shared__ uint32_t tmem_base;
   __shared__ int s_ok;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // rows k >= 2 DIN of A stay zero
   for (int idx = tid; idx < kT * kT * 2 / 16; idx += kT) reinterpret_cast<uint4 *>(sA)[idx] = make_uint4(0, 0, 0, 0);
   if (warp == 0) tc::tmem_alloc(&tmem_base, 64);
@@ -397,42 +423,49 @@ __global__ void __launch_bounds__(kT) mpnn_wgrad_kernel(WgradArgs a) {
   tc::fence_after_sync();
   const uint32_t tmem = tmem_base;
   const uint32_t aBase = tc::smem_addr(sA), bBase = tc::smem_addr(sB);
-  const uint32_t idesc = tc::idesc_bf16_f32(kT, 64);
+  const uint32_t idesc = tc::idesc_bf16_f32(kT, 64) | tc::kMnMajorAB;
   uint32_t phase = 0;
-  float db[64];
+  float db[8][8];  // of the thread's 8 (row, piece) places of a tile
 #pragma unroll
-  for (int o = 0; o < 64; o++) db[o] = 0.f;
+  for (int q = 0; q < 8; q++)
+#pragma unroll
+    for (int i = 0; i < 8; i++) db[q][i] = 0.f;
   bool first = true;
   const int ntiles = (a.n + kT - 1) / kT;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int v = tile * kT + tid;
-    const bool valid = v < a.n;
-    // A^T: element (k, v) ; B: element (o, v)
 #pragma unroll
-    for (int c = 0; c < DIN / 8; c++) {
-      float f[8], g[8];
-      if (valid) {
-        bf16x8_to_f32(reinterpret_cast<const uint4 *>(a.hin + (size_t)v * DIN)[c], f);
-        bf16x8_to_f32(reinterpret_cast<const uint4 *>(a.agg + (size_t)v * DIN)[c], g);
-      } else {
+    for (int cg = 0; cg < kPieces / 4; cg++) {
+      const int c = 4 * cg + (lane >> 3);
+      const __nv_bfloat16 *src = c < DIN / 8 ? a.hin + 8 * c : a.agg + 8 * (c - DIN / 8);
+      uint4 x[4];
 #pragma unroll
-        for (int i = 0; i < 8; i++) f[i] = g[i] = 0.f;
+      for (int rg = 0; rg < 4; rg++) {
+        const int v = tile * kT + 32 * warp + 8 * rg + (lane & 7);
+        x[rg] = v < a.n ? *reinterpret_cast<const uint4 *>(src + (size_t)v * DIN) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        *reinterpret_cast<__nv_bfloat16 *>(sA + tc::kmajor_offset(8 * c + i, tid, kT)) = __float2bfloat16_rn(f[i]);
-        *reinterpret_cast<__nv_bfloat16 *>(sA + tc::kmajor_offset(DIN + 8 * c + i, tid, kT)) =
-            __float2bfloat16_rn(g[i]);
-      }
+      for (int rg = 0; rg < 4; rg++)
+        *reinterpret_cast<uint4 *>(sA + tc::mnmajor_offset(8 * c, 32 * warp + 8 * rg + (lane & 7), kT)) = x[rg];
     }
 #pragma unroll
-    for (int c = 0; c < 16; c++) {
-      float4 d = valid ? reinterpret_cast<const float4 *>(a.dz + (size_t)v * 64)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float dd[4] = {d.x, d.y, d.z, d.w};
+    for (int half = 0; half < 2; half++) {
+      const int c = (lane >> 3) + 4 * half;
+      float d[4][8];
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        db[4 * c + i] += dd[i];
-        *reinterpret_cast<__nv_bfloat16 *>(sB + tc::kmajor_offset(4 * c + i, tid, kT)) = __float2bfloat16_rn(dd[i]);
+      for (int rg = 0; rg < 4; rg++) {
+        const int v = tile * kT + 32 * warp + 8 * rg + (lane & 7);
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 *src = reinterpret_cast<const float4 *>(a.dz + (size_t)v * 64 + 8 * c);
+        const float4 x0 = v < a.n ? src[0] : zero, x1 = v < a.n ? src[1] : zero;
+        d[rg][0] = x0.x; d[rg][1] = x0.y; d[rg][2] = x0.z; d[rg][3] = x0.w;
+        d[rg][4] = x1.x; d[rg][5] = x1.y; d[rg][6] = x1.z; d[rg][7] = x1.w;
+      }
+#pragma unroll
+      for (int rg = 0; rg < 4; rg++) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) db[4 * half + rg][i] += d[rg][i];
+        *reinterpret_cast<uint4 *>(sB + tc::mnmajor_offset(8 * c, 32 * warp + 8 * rg + (lane & 7), 64)) =
+            f32_to_bf16x8(d[rg]);
       }
     }
     tc::fence_smem_to_async();
@@ -441,8 +474,8 @@ __global__ void __launch_bounds__(kT) mpnn_wgrad_kernel(WgradArgs a) {
       tc::fence_after_sync();
 #pragma unroll
       for (int s = 0; s < kT / 16; s++)
-        tc::mma_bf16(tmem, tc::make_desc(aBase + s * 256, 128, SBO), tc::make_desc(bBase + s * 256, 128, SBO),
-                     idesc, (first && s == 0) ? 0u : 1u);
+        tc::mma_bf16(tmem, tc::make_desc(aBase + s * 2 * kT * 16, kT * 16, 128),
+                     tc::make_desc(bBase + s * 2 * 64 * 16, 64 * 16, 128), idesc, (first && s == 0) ? 0u : 1u);
       tc::mma_commit(&mbar);
     }
     first = false;
@@ -469,7 +502,10 @@ __global__ void __launch_bounds__(kT) mpnn_wgrad_kernel(WgradArgs a) {
   __syncthreads();
   float *red = reinterpret_cast<float *>(smem);  // 128 x 64 floats = 32 KB of the A tile
 #pragma unroll
-  for (int o = 0; o < 64; o++) red[o * kT + tid] = db[o];
+  for (int q = 0; q < 8; q++)
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      red[(8 * ((lane >> 3) + 4 * (q >> 2)) + i) * kT + 32 * warp + 8 * (q & 3) + (lane & 7)] = db[q][i];
   __syncthreads();
   if (tid < 64) {
     float s = 0.f;
@@ -492,6 +528,8 @@ struct DgradArgs {
   DevStatus *st;
 };
 
+constexpr int kDgradSmem = kT * 64 * 2 + 128 * 64 * 2 + kT * 36 * 4;
+
 template <int DIN>
 __global__ void __launch_bounds__(kT) mpnn_dgrad_kernel(DgradArgs a) {
   constexpr int N = 2 * DIN;
@@ -502,7 +540,9 @@ __global__ void __launch_bounds__(kT) mpnn_dgrad_kernel(DgradArgs a) {
   __shared__ uint64_t mbar;
   __shared__ uint32_t tmem_base;
   __shared__ int s_ok;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // a warp's 32 rows x 32 columns of the result, rows 36 floats apart (no bank twice)
+  float *stage = reinterpret_cast<float *>(smem + kT * 64 * 2 + N * 64 * 2) + warp * 32 * 36;
   for (int idx = tid; idx < N * 64; idx += kT) {
     const int k = idx / 64, o = idx % 64;
     *reinterpret_cast<__nv_bfloat16 *>(sB + tc::kmajor_offset(k, o, 64)) = a.W[(size_t)o * N + k];
@@ -520,18 +560,22 @@ __global__ void __launch_bounds__(kT) mpnn_dgrad_kernel(DgradArgs a) {
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int v = tile * kT + tid;
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      float f[8];
-      if (v < a.n) {
-        const float4 x0 = reinterpret_cast<const float4 *>(a.dz + (size_t)v * 64)[2 * c];
-        const float4 x1 = reinterpret_cast<const float4 *>(a.dz + (size_t)v * 64)[2 * c + 1];
-        f[0] = x0.x; f[1] = x0.y; f[2] = x0.z; f[3] = x0.w;
-        f[4] = x1.x; f[5] = x1.y; f[6] = x1.z; f[7] = x1.w;
-      } else {
+    for (int half = 0; half < 2; half++) {
+      const int c = (lane >> 3) + 4 * half;
+      float f[4][8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) f[i] = 0.f;
+      for (int rg = 0; rg < 4; rg++) {
+        const int u = tile * kT + 32 * warp + 8 * rg + (lane & 7);
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 *src = reinterpret_cast<const float4 *>(a.dz + (size_t)u * 64 + 8 * c);
+        const float4 x0 = u < a.n ? src[0] : zero, x1 = u < a.n ? src[1] : zero;
+        f[rg][0] = x0.x; f[rg][1] = x0.y; f[rg][2] = x0.z; f[rg][3] = x0.w;
+        f[rg][4] = x1.x; f[rg][5] = x1.y; f[rg][6] = x1.z; f[rg][7] = x1.w;
       }
-      *reinterpret_cast<uint4 *>(sA + tc::kmajor_offset(tid, 8 * c, 64)) = f32_to_bf16x8(f);
+#pragma unroll
+      for (int rg = 0; rg < 4; rg++)
+        *reinterpret_cast<uint4 *>(sA + tc::kmajor_offset(32 * warp + 8 * rg + (lane & 7), 8 * c, 64)) =
+            f32_to_bf16x8(f[rg]);
     }
     tc::fence_smem_to_async();
     __syncthreads();
@@ -546,20 +590,29 @@ __global__ void __launch_bounds__(kT) mpnn_dgrad_kernel(DgradArgs a) {
     const bool ok = tile_mma_wait(&mbar, phase, &s_ok, a.st);
     phase ^= 1u;
     if (!ok) break;
-    float q[N];
+    const int deg = v < a.n ? a.rowptr[v + 1] - a.rowptr[v] : 0;
+    const float inv = deg > 0 ? 1.0f / (float)deg : 0.0f;
+#pragma unroll 1
+    for (int c0 = 0; c0 < N; c0 += 32) {  // 32 columns through the stage, rows written whole
+      float q[32];
+      tc::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + c0, q);
+      tc::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + c0 + 16, q + 16);
+      if (c0 >= DIN)
 #pragma unroll
-    for (int c = 0; c < N / 16; c++) tc::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + 16 * c, q + 16 * c);
-    if (v < a.n) {
-      const int deg = a.rowptr[v + 1] - a.rowptr[v];
-      const float inv = deg > 0 ? 1.0f / (float)deg : 0.0f;
+        for (int i = 0; i < 32; i++) q[i] *= inv;
 #pragma unroll
-      for (int c = 0; c < DIN / 4; c++) {
-        reinterpret_cast<float4 *>(a.P + (size_t)v * DIN)[c] =
-            make_float4(q[4 * c], q[4 * c + 1], q[4 * c + 2], q[4 * c + 3]);
-        reinterpret_cast<float4 *>(a.G + (size_t)v * DIN)[c] =
-            make_float4(q[DIN + 4 * c] * inv, q[DIN + 4 * c + 1] * inv, q[DIN + 4 * c + 2] * inv,
-                        q[DIN + 4 * c + 3] * inv);
+      for (int i = 0; i < 8; i++)
+        *reinterpret_cast<float4 *>(stage + lane * 36 + 4 * i) =
+            make_float4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
+      __syncwarp();
+      float *out = c0 >= DIN ? a.G + (c0 - DIN) : a.P + c0;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const int row = 4 * i + (lane >> 3), u = tile * kT + 32 * warp + row;
+        const float4 x = *reinterpret_cast<const float4 *>(stage + row * 36 + 4 * (lane & 7));
+        if (u < a.n) *reinterpret_cast<float4 *>(out + (size_t)u * DIN + 4 * (lane & 7)) = x;
       }
+      __syncwarp();
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -654,24 +707,37 @@ __global__ void __launch_bounds__(kGatherVerts * 16) mpnn_gather_kernel(
   }
 }
 
-// sum of per-block partials in block order: out[i] = sum_b part[b * len + i];
-// 32 loads in flight (608 partials one after another took 41 us)
-__global__ void __launch_bounds__(64) mpnn_reduce_kernel(const float *__restrict__ part, int blocks, int len,
-                                                         float *__restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= len) return;
+// sum of per-block partials in block order: out[i] = sum_b part[b * len + i].
+// A block takes 32 entries: all its threads fetch 256 partials of each at once
+// and one warp adds them in order from shared memory.  One thread an entry
+// with 32 loads in flight was bound by its round trips: 27 us for 608 partials
+// of 8,256 entries, so 11.
+constexpr int kReduceCols = 32, kReduceRows = 256, kReduceThreads = 256;
+
+__global__ void __launch_bounds__(kReduceThreads) mpnn_reduce_kernel(const float *__restrict__ part, int blocks, int len,
+                                                                     float *__restrict__ out) {
+  __shared__ float rows[kReduceRows][kReduceCols];
+  const int c = threadIdx.x % kReduceCols, g = threadIdx.x / kReduceCols;
+  constexpr int kGroups = kReduceThreads / kReduceCols, kEach = kReduceRows / kGroups;
+  const int i = blockIdx.x * kReduceCols + c;
   float s = 0.f;
-  const float *p = part + i;
-  int b = 0;
-  for (; b + 32 <= blocks; b += 32, p += (size_t)32 * len) {
-    float v[32];
+  for (int b0 = 0; b0 < blocks; b0 += kReduceRows) {
+    float v[kEach];
 #pragma unroll
-    for (int k = 0; k < 32; k++) v[k] = __ldg(p + (size_t)k * len);
+    for (int k = 0; k < kEach; k++) {
+      const int b = b0 + g + k * kGroups;
+      v[k] = i < len && b < blocks ? __ldg(&part[(size_t)b * len + i]) : 0.f;
+    }
+    __syncthreads();  // the rows before are added
 #pragma unroll
-    for (int k = 0; k < 32; k++) s += v[k];
+    for (int k = 0; k < kEach; k++) rows[g + k * kGroups][c] = v[k];
+    __syncthreads();
+    const int m = min(kReduceRows, blocks - b0);
+    if (g == 0)
+#pragma unroll 16
+      for (int r = 0; r < m; r++) s += rows[r][c];
   }
-  for (; b < blocks; b++, p += len) s += __ldg(p);
-  out[i] = s;
+  if (g == 0 && i < len) out[i] = s;
 }
 
 __global__ void to_bf16_kernel(const float *__restrict__ in, __nv_bfloat16 *__restrict__ out, long long n) {
@@ -758,7 +824,7 @@ int ensure_mpnn(bl_ctx *ctx, int n) {
     if (int rc = set_smem(ctx, mpnn_fwd_kernel<64, true>, kT * 128 * 2 + 64 * 128 * 2)) return rc;
     if (int rc = set_smem(ctx, mpnn_wgrad_kernel<16>, kT * kT * 2 + 64 * kT * 2)) return rc;
     if (int rc = set_smem(ctx, mpnn_wgrad_kernel<64>, kT * kT * 2 + 64 * kT * 2)) return rc;
-    if (int rc = set_smem(ctx, mpnn_dgrad_kernel<64>, kT * 64 * 2 + 128 * 64 * 2)) return rc;
+    if (int rc = set_smem(ctx, mpnn_dgrad_kernel<64>, kDgradSmem)) return rc;
   }
   MpnnState &m = *ctx->mpnn;
   if (n > m.cap_n) {
@@ -850,7 +916,7 @@ int mpnn_backward(bl_ctx *ctx, int n, int max_row, const int *d_rowptr, const in
   const int grid = std::min(m.grid, std::max(1, nblk(n, kT)));
   TopArgs t{n, m.dxy, m.h[2], m.params + kOffWo, m.dz, m.part};
   mpnn_top_kernel<<<grid, kT, 0, st>>>(t);
-  mpnn_reduce_kernel<<<nblk(130, 64), 64, 0, st>>>(m.part, grid, 130, m.grad + kOffWo);
+  mpnn_reduce_kernel<<<nblk(130, kReduceCols), kReduceThreads, 0, st>>>(m.part, grid, 130, m.grad + kOffWo);
   ctx->launches += 2;
   for (int l = 2; l >= 0; l--) {
     const int din = l == 0 ? 16 : 64;
@@ -858,12 +924,12 @@ int mpnn_backward(bl_ctx *ctx, int n, int max_row, const int *d_rowptr, const in
     WgradArgs w{n, l == 0 ? m.x : m.h[l - 1], m.agg[l], m.dz, m.part, ctx->s.status};
     if (l == 0) mpnn_wgrad_kernel<16><<<grid, kT, kT * kT * 2 + 64 * kT * 2, st>>>(w);
     else mpnn_wgrad_kernel<64><<<grid, kT, kT * kT * 2 + 64 * kT * 2, st>>>(w);
-    mpnn_reduce_kernel<<<nblk(len, 64), 64, 0, st>>>(m.part, grid, len, m.grad + kOffW[l]);
+    mpnn_reduce_kernel<<<nblk(len, kReduceCols), kReduceThreads, 0, st>>>(m.part, grid, len, m.grad + kOffW[l]);
     ctx->launches += 2;
     BL_CUDA(ctx, cudaGetLastError());
     if (l > 0) {
       DgradArgs d{n, d_rowptr, m.dz, m.wbf + kOffW[l], m.P, m.G, ctx->s.status};
-      mpnn_dgrad_kernel<64><<<grid, kT, kT * 64 * 2 + 128 * 64 * 2, st>>>(d);
+      mpnn_dgrad_kernel<64><<<grid, kT, kDgradSmem, st>>>(d);
       mpnn_gather_kernel<<<nblk(n, kGatherVerts), kGatherVerts * 16, 0, st>>>(
           n, max_row > kLongRow ? 1 : 0, d_rowptr, d_colids, m.P, m.G, m.h[l - 1], m.dz);
       ctx->launches += 2;

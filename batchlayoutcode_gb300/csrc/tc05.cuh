@@ -48,6 +48,17 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// The same operand with its rows (M or N) contiguous instead of K: a core
+// matrix is 8 values of K x 16 bytes (8 rows), element (r, k) of an R-row tile
+// at byte (r / 8) * 128 + (k / 8) * (R / 8) * 128 + (k % 8) * 16 + (r % 8) * 2.
+// The descriptor's stride byte offset steps along the rows (128), its leading
+// byte offset along K (R * 16), and the instruction descriptor says so (bits
+// 15 and 16).
+__host__ __device__ __forceinline__ uint32_t mnmajor_offset(int r, int k, int R) {
+  return (uint32_t)((r >> 3) * 128 + (k >> 3) * (R >> 3) * 128 + (k & 7) * 16 + (r & 7) * 2);
+}
+constexpr uint32_t kMnMajorAB = (1u << 15) | (1u << 16);
+
 // ---- tensor memory --------------------------------------------------------
 // One full warp allocates; the column count is a power of two >= 32.
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t ncols) {
