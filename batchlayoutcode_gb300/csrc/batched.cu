@@ -27,6 +27,8 @@
 #include <climits>
 #include <cmath>
 #include <string>
+#include <functional>
+#include <queue>
 #include <vector>
 
 #include "../../include/batchlayout_gb300.h"
@@ -51,7 +53,7 @@ struct BatchedArgs {
   float W;
   double theta, inv_theta2;  // inv_theta2 = 1 / theta^2, folded into the records
   const BatchedGraph *graphs;
-  const int *order;            // queue order (largest graph first)
+  const int *order;            // queue order (costliest graph first)
   unsigned int *queue;         // next queue slot
   const int *rowptr;           // concatenated local neighbour CSRs
   const int *colids;
@@ -80,16 +82,23 @@ struct BatchedArgs {
 
 namespace {
 
-constexpr int kBThreads = 512;
-constexpr int kBWarps = kBThreads / 32;
+// The device code is compiled for blocks of 512 threads, two to an SM, and of
+// 1,024, one to an SM.  A graph is one block's work: with few graphs the
+// longest sets the time and the larger block shortens it; with many, two
+// smaller blocks an SM overlap their latencies.  Two iterations, ms (512 /
+// 1,024 threads): 192 graphs of 200 to 20,000 vertices 4.1 / 3.1, 304 of 3,000
+// to 4,900 3.9 / 3.1, 1,000 of 200 to 3,000 1.57 / 1.26; but 2,000 of 200 to
+// 400 0.27 / 0.45, 608 of 500 to 1,500 0.51 / 0.55, 304 of 19,000 to 20,000
+// 6.6 / 7.4.  batched_shape() compares the two schedules.
 constexpr int kSortR = 8;  // keys per thread in a sort tile
-constexpr int kSortTile = kBThreads * kSortR;
 constexpr int kMaxBfsLevels = 40;  // digit levels 0..32 need at most 34
 constexpr int kNoKid = INT_MIN;
 constexpr int kMaxBatch = 4096;
 
 // shared memory of the Barnes-Hut path (carved from the dynamic buffer)
+template <int kBThreads>
 struct BhShared {
+  static constexpr int kBWarps = kBThreads / 32;
   unsigned int wcnt[kBWarps][256];
   unsigned int cnt[256];
   unsigned int base[256];
@@ -100,7 +109,9 @@ struct BhShared {
   int trivial;
 };
 
+template <int kBThreads>
 __device__ double block_sum_d(double v, double *red) {
+  constexpr int kBWarps = kBThreads / 32;
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   __syncthreads();
@@ -120,7 +131,9 @@ __device__ double block_sum_d(double v, double *red) {
 }
 
 // exclusive prefix of v over the block; *total = block sum
+template <int kBThreads>
 __device__ int block_scan_excl(int v, int *wsum, int *total) {
+  constexpr int kBWarps = kBThreads / 32;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int x = v;
 #pragma unroll
@@ -143,6 +156,7 @@ __device__ int block_scan_excl(int v, int *wsum, int *total) {
 }
 
 // ---- minibatch graph, entirely inside the block ------------------------------
+template <int kBThreads>
 __device__ void layout_small(const BatchedArgs &a, int g, unsigned char *smem, double *red) {
   const BatchedGraph G = a.graphs[g];
   float2 *fbuf = reinterpret_cast<float2 *>(smem);  // [batch]
@@ -219,7 +233,7 @@ __device__ void layout_small(const BatchedArgs &a, int g, unsigned char *smem, d
     a.xy_out[2 * (size_t)(G.voff + k)] = (double)pos[k].x;
     a.xy_out[2 * (size_t)(G.voff + k) + 1] = (double)pos[k].y;
   }
-  const double e = block_sum_d(e_part, red);
+  const double e = block_sum_d<kBThreads>(e_part, red);
   if (tid == 0) a.energy[g] = e;
 }
 
@@ -254,7 +268,9 @@ __device__ __forceinline__ void write_leaf(const BatchedArgs &a, float4 *nodes, 
   nlvl[idx] = 255;
 }
 
-__device__ void layout_bh(const BatchedArgs &a, int g, BhShared &S, double *red) {
+template <int kBThreads>
+__device__ void layout_bh(const BatchedArgs &a, int g, BhShared<kBThreads> &S, double *red) {
+  constexpr int kBWarps = kBThreads / 32, kSortTile = kBThreads * kSortR;
   const BatchedGraph G = a.graphs[g];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = G.n;
@@ -490,7 +506,7 @@ __device__ void layout_bh(const BatchedArgs &a, int g, BhShared &S, double *red)
           }
         }
         int tot = 0;
-        const int off = block_scan_excl(nc, S.wsum, &tot);
+        const int off = block_scan_excl<kBThreads>(nc, S.wsum, &tot);
         if (q < q1) {
           int kids[4] = {kNoKid, kNoKid, kNoKid, kNoKid};
           if (lv < 32) {
@@ -643,14 +659,15 @@ __device__ void layout_bh(const BatchedArgs &a, int g, BhShared &S, double *red)
     a.xy_out[2 * (size_t)(G.voff + k)] = (double)pos[k].x;
     a.xy_out[2 * (size_t)(G.voff + k) + 1] = (double)pos[k].y;
   }
-  const double e = block_sum_d(e_part, red);
+  const double e = block_sum_d<kBThreads>(e_part, red);
   if (tid == 0) a.energy[g] = e;
 }
 
-__global__ void __launch_bounds__(kBThreads, 2) batched_kernel(BatchedArgs a) {
+template <int kBThreads>
+__global__ void __launch_bounds__(kBThreads, 1024 / kBThreads) batched_kernel(BatchedArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_q;
-  __shared__ double red[kBWarps];
+  __shared__ double red[kBThreads / 32];
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_q = (int)atomicAdd(a.queue, 1u);
@@ -659,10 +676,37 @@ __global__ void __launch_bounds__(kBThreads, 2) batched_kernel(BatchedArgs a) {
     if (q >= a.num_graphs) return;
     const int g = a.order[q];
     const long long t0 = clock64();
-    if (a.graphs[g].algo == kAlgoBH) layout_bh(a, g, *reinterpret_cast<BhShared *>(smem), red);
-    else layout_small(a, g, smem, red);
+    if (a.graphs[g].algo == kAlgoBH) layout_bh<kBThreads>(a, g, *reinterpret_cast<BhShared<kBThreads> *>(smem), red);
+    else layout_small<kBThreads>(a, g, smem, red);
     if (a.cycles && threadIdx.x == 0) a.cycles[g] = (unsigned long long)(clock64() - t0);
   }
+}
+
+// Rough cycles of an iteration by a block of 512 threads that shares its SM,
+// fitted to the sets named at the top: orders the queue and chooses the block
+// size.
+double graph_cost(const BatchedGraph &g) {
+  return g.algo == kAlgoBH ? 300.0 * g.n : 1e4 + 50.0 * g.n + 0.14 * (double)g.n * (double)g.n;
+}
+
+// The same for a block of 1,024 threads alone on its SM, relative to that.
+double wide_factor(const BatchedGraph &g) {
+  if (g.algo == kAlgoBH) return 0.56;
+  return g.n < 128 ? 1.05 : (g.n < 512 ? 0.83 : (g.n < 1536 ? 0.54 : 0.4));
+}
+
+// Time at which `slots` workers that take costs[] in order are done.
+double schedule_end(const std::vector<double> &costs, int slots) {
+  std::priority_queue<double, std::vector<double>, std::greater<double>> free;
+  for (int k = 0; k < slots; k++) free.push(0.0);
+  double end = 0.0;
+  for (double c : costs) {
+    const double t = free.top() + c;
+    free.pop();
+    free.push(t);
+    end = std::max(end, t);
+  }
+  return end;
 }
 
 // size bucket of a minibatch graph for the autotuner
@@ -675,6 +719,8 @@ int size_bucket(int n) { return n < 512 ? 0 : (n < 2048 ? 1 : 2); }
 struct BatchedState {
   int num_graphs = 0, total_v = 0, max_small = 0, max_bh = 0, grid = 0, ws_grid = 0;
   size_t smem = 0;
+  int threads = 512;  // of a block: 512 or 1024
+  double end_pairs = 0.0, end_wide = 0.0;  // estimated ends with either (graph_cost)
   std::vector<BatchedGraph> gs;
   std::vector<int> order;
   int parts[3] = {0, 0, 0};  // autotuned source split per size bucket (0 = not tuned)
@@ -722,7 +768,8 @@ int batched_launch(bl_ctx *ctx, BatchedState &B, int num, const int *d_order, un
   a.cycles = d_cycles;
   a.iterations = iterations;
   BL_CUDA(ctx, cudaMemsetAsync(B.d_queue, 0, sizeof(unsigned int), ctx->stream));
-  batched_kernel<<<std::min(num, B.grid), kBThreads, B.smem, ctx->stream>>>(a);
+  (B.threads == 1024 ? batched_kernel<1024> : batched_kernel<512>)<<<std::min(num, B.grid), B.threads, B.smem,
+                                                                    ctx->stream>>>(a);
   ctx->launches++;
   BL_CUDA(ctx, cudaGetLastError());
   return 0;
@@ -740,17 +787,24 @@ T *carve(char *&p, size_t count) {
 int batched_shape(bl_ctx *ctx, BatchedState &B, int batch) {
   int smem_optin = 0;
   BL_CUDA(ctx, cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-  const size_t smem_small = (size_t)(batch + kBThreads + B.max_small) * sizeof(float2);
-  const size_t smem = std::max(smem_small, sizeof(BhShared));
-  if (smem + 2048 > (size_t)smem_optin)
+  auto need = [&](int threads) {
+    const size_t bh = threads == 1024 ? sizeof(BhShared<1024>) : sizeof(BhShared<512>);
+    return std::max((size_t)(batch + threads + B.max_small) * sizeof(float2), bh);
+  };
+  if (need(512) + 2048 > (size_t)smem_optin)
     return bl_fail(ctx, BL_ERR_TOO_LARGE, "a minibatch graph is too large for one block's shared memory");
-  BL_CUDA(ctx, cudaFuncSetAttribute(batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // 512 or 1,024 threads: the schedule that ends first
+  const int threads = need(1024) + 2048 <= (size_t)smem_optin && B.end_wide < B.end_pairs ? 1024 : 512;
+  const void *kernel = threads == 1024 ? (const void *)batched_kernel<1024> : (const void *)batched_kernel<512>;
+  const size_t smem = need(threads);
+  BL_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int occ = 0;
-  BL_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batched_kernel, kBThreads, smem));
+  BL_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem));
   if (occ < 1) return bl_fail(ctx, BL_ERR_TOO_LARGE, "batched kernel cannot be resident");
   const int grid = std::min(B.num_graphs, ctx->num_sms * occ);
-  if (smem != B.smem || grid != B.grid) B.graph_dirty = true;
+  if (smem != B.smem || grid != B.grid || threads != B.threads) B.graph_dirty = true;
   B.smem = smem;
+  B.threads = threads;
   if (B.max_bh > 0 && grid > B.ws_grid) {
     cudaFree(B.ws);
     B.ws = nullptr;
@@ -911,7 +965,15 @@ int bl_batched_prepare(bl_ctx *ctx, int num_graphs, const int *vertex_offset, co
   // largest graphs first (work grows like n^2 for minibatch graphs)
   B->order.resize(num_graphs);
   for (int g = 0; g < num_graphs; g++) B->order[g] = g;
-  std::stable_sort(B->order.begin(), B->order.end(), [&](int x, int y) { return B->gs[x].n > B->gs[y].n; });
+  std::stable_sort(B->order.begin(), B->order.end(),
+                   [&](int x, int y) { return graph_cost(B->gs[x]) > graph_cost(B->gs[y]); });
+  {
+    std::vector<double> costs(num_graphs);
+    for (int k = 0; k < num_graphs; k++) costs[k] = graph_cost(B->gs[B->order[k]]);
+    B->end_pairs = schedule_end(costs, 2 * ctx->num_sms);
+    for (int k = 0; k < num_graphs; k++) costs[k] *= wide_factor(B->gs[B->order[k]]);
+    B->end_wide = schedule_end(costs, ctx->num_sms);
+  }
   // device buffers
   cudaStream_t st = ctx->stream;
   B->total_v = (int)total_v;
