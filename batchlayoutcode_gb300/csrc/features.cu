@@ -281,10 +281,27 @@ __global__ void __launch_bounds__(kBlockThreads, 1) bfs_block_kernel(BlockBfsArg
 }
 
 // ---- pivot MDS of one graph (vertices [v0, v1)) ---------------------------
-__device__ __forceinline__ double hop2(const unsigned short *dist, int v, int s, const int *maxd) {
-  const unsigned short d = dist[(size_t)v * kP + s];
-  const double h = (d == kUnreached) ? (double)(maxd[s] + 1) : (double)d;
-  return h * h;
+// The squared distance: squared as an integer (at most 65,535 hops) and made a
+// double by its bits above 2^52, one FP64 operation instead of a conversion and
+// a product: FP64 runs at two lanes a cycle and SM here and bounds these kernels.
+__device__ __forceinline__ double hop2(unsigned int d, int s, const int *maxd) {
+  const unsigned int h = d == kUnreached ? (unsigned int)(maxd[s] + 1) : d;
+  return __hiloint2double(0x43300000, (int)(h * h)) - 4503599627370496.0;
+}
+
+// a vertex's 16 hop counts, two loads
+__device__ __forceinline__ void hops(const unsigned short *dist, int v, unsigned int (&d)[kP]) {
+  const uint4 *row = reinterpret_cast<const uint4 *>(dist + (size_t)v * kP);
+  const uint4 x[2] = {row[0], row[1]};
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const unsigned int w[4] = {x[k].x, x[k].y, x[k].z, x[k].w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      d[8 * k + 2 * i] = w[i] & 0xffffu;
+      d[8 * k + 2 * i + 1] = w[i] >> 16;
+    }
+  }
 }
 
 // per block: largest finite distance per pivot
@@ -314,12 +331,14 @@ __global__ void mds_max_kernel(const int *voff, const unsigned short *dist, int 
   int m[kP];
 #pragma unroll
   for (int s = 0; s < kP; s++) m[s] = 0;
-  for (int v = v0 + blockIdx.x * blockDim.x + threadIdx.x; v < v1; v += blocks * blockDim.x)
+  for (int v = v0 + blockIdx.x * blockDim.x + threadIdx.x; v < v1; v += blocks * blockDim.x) {
+    unsigned int h[kP];
+    hops(dist, v, h);
 #pragma unroll
     for (int s = 0; s < kP; s++) {
-      const unsigned short d = dist[(size_t)v * kP + s];
-      if (d != kUnreached) m[s] = max(m[s], (int)d);
+      if (h[s] != kUnreached) m[s] = max(m[s], (int)h[s]);
     }
+  }
 #pragma unroll
   for (int s = 0; s < kP; s++) atomicMax(&smax[s], m[s]);
   __syncthreads();
@@ -352,9 +371,12 @@ __global__ void __launch_bounds__(256) mds_colsum_kernel(const int *voff, const 
   double c[kP];
 #pragma unroll
   for (int s = 0; s < kP; s++) c[s] = 0.0;
-  for (int v = v0 + blockIdx.x * blockDim.x + threadIdx.x; v < v1; v += blocks * blockDim.x)
+  for (int v = v0 + blockIdx.x * blockDim.x + threadIdx.x; v < v1; v += blocks * blockDim.x) {
+    unsigned int h[kP];
+    hops(dist, v, h);
 #pragma unroll
-    for (int s = 0; s < kP; s++) c[s] += hop2(dist, v, s, maxd);
+    for (int s = 0; s < kP; s++) c[s] += hop2(h[s], s, maxd);
+  }
   block_sum_doubles(c, kP, scratch, part + ((size_t)g * kMdsBlocks + blockIdx.x) * kP);
 }
 
@@ -404,14 +426,16 @@ __global__ void __launch_bounds__(256) mds_gram_kernel(const int *voff, const un
     const int v = base + tid;
     if (v < v1) {
       double d2[kP], r = 0.0;
+      unsigned int h[kP];
+      hops(dist, v, h);
 #pragma unroll
       for (int s = 0; s < kP; s++) {
-        d2[s] = hop2(dist, v, s, maxd);
+        d2[s] = hop2(h[s], s, maxd);
         r += d2[s];
       }
       r *= 1.0 / kP;
 #pragma unroll
-      for (int s = 0; s < kP; s++) cbuf[tid][s] = -0.5 * (d2[s] - r - colmean[s] + grand);
+      for (int s = 0; s < kP; s++) cbuf[tid][s] = d2[s] - r - colmean[s] + grand;  // x -0.5 at the end: exact
     } else {
 #pragma unroll
       for (int s = 0; s < kP; s++) cbuf[tid][s] = 0.0;
@@ -421,7 +445,7 @@ __global__ void __launch_bounds__(256) mds_gram_kernel(const int *voff, const un
       for (int rr = 0; rr < 256; rr++) acc = fma(cbuf[rr][pi], cbuf[rr][pj], acc);
     __syncthreads();
   }
-  if (tid < kGram) part[((size_t)g * kMdsBlocks + blockIdx.x) * kGram + tid] = acc;
+  if (tid < kGram) part[((size_t)g * kMdsBlocks + blockIdx.x) * kGram + tid] = 0.25 * acc;
 }
 
 // the Gram matrices from the blocks' sums, added in block order
@@ -453,18 +477,20 @@ __global__ void mds_project_kernel(ProjectArgs a) {
   a.maxd += g * kP;
   a.mean += g * kMean;
   a.V += (size_t)g * kProj;
-  const double inv_scale = a.V[kP * 12];
+  const double inv_scale = -0.5 * a.V[kP * 12];
   double d2[kP], r = 0.0;
+  unsigned int h[kP];
+  hops(a.dist, v, h);
 #pragma unroll
   for (int s = 0; s < kP; s++) {
-    d2[s] = hop2(a.dist, v, s, a.maxd);
+    d2[s] = hop2(h[s], s, a.maxd);
     r += d2[s];
   }
   r *= 1.0 / kP;
   double c[kP];
 #pragma unroll
-  for (int s = 0; s < kP; s++) c[s] = -0.5 * (d2[s] - r - a.mean[s] + a.mean[kP]);
-  float *f = a.features + (size_t)v * kFeat;
+  for (int s = 0; s < kP; s++) c[s] = d2[s] - r - a.mean[s] + a.mean[kP];  // x -0.5 below: exact
+  float f[kFeat];
 #pragma unroll
   for (int j = 0; j < 12; j++) {
     double y = 0.0;
@@ -489,6 +515,9 @@ __global__ void mds_project_kernel(ProjectArgs a) {
   f[13] = 1.0f / (1.0f + (float)deg);
   f[14] = deg > 0 ? m / (float)deg : 0.0f;
   f[15] = log2f((float)n_graph) / 20.0f;
+  float4 *out = reinterpret_cast<float4 *>(a.features + (size_t)v * kFeat);
+#pragma unroll
+  for (int k = 0; k < kFeat / 4; k++) out[k] = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
 }
 
 }  // namespace

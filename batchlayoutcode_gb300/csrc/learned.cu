@@ -43,14 +43,34 @@ __global__ void residual_start_kernel(const float *__restrict__ net, const float
   if (v < n) pos[v] = make_float2(net[2 * v] + feat[(size_t)v * kFeat], net[2 * v + 1] + feat[(size_t)v * kFeat + 1]);
 }
 
-// per block: sum over the CSR entries of |p_v - p_u| (each edge twice)
+// per block: sum over the CSR entries of |p_v - p_u| (each edge twice).  Bound
+// by FP64, so the entries are dealt out in runs of kEdgeRun instead of by row:
+// a warp with a row a lane works as long as its longest row (400,000 vertices
+// of a geometric graph: 205 us, so 81).
+constexpr int kEdgeRun = 8;
+
 __global__ void edge_length_kernel(int n, const int *__restrict__ rowptr, const int *__restrict__ colids,
                                    const float2 *__restrict__ pos, double *part) {
   __shared__ double red[8];
+  const int nnz = rowptr[n];
   double s = 0.0;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    const float2 p = pos[v];
-    for (int e = rowptr[v]; e < rowptr[v + 1]; e++) {
+  for (long long e0 = (long long)kEdgeRun * (blockIdx.x * blockDim.x + threadIdx.x); e0 < nnz;
+       e0 += (long long)kEdgeRun * gridDim.x * blockDim.x) {
+    const int e1 = (int)min(e0 + kEdgeRun, (long long)nnz);
+    int lo = 0, hi = n;  // the row of e0: rowptr[lo] <= e0 < rowptr[hi]
+    while (hi - lo > 1) {
+      const int mid = lo + ((hi - lo) >> 1);
+      if (rowptr[mid] <= e0) lo = mid;
+      else hi = mid;
+    }
+    int end = rowptr[lo + 1];
+    float2 p = pos[lo];
+    for (int e = (int)e0; e < e1; e++) {
+      while (e >= end) {
+        lo++;
+        end = rowptr[lo + 1];
+        p = pos[lo];
+      }
       const float2 q = pos[colids[e]];
       s += sqrt((double)(p.x - q.x) * (p.x - q.x) + (double)(p.y - q.y) * (p.y - q.y));
     }
@@ -67,25 +87,57 @@ __global__ void edge_length_kernel(int n, const int *__restrict__ rowptr, const 
 
 // per block: sum_v A_v . R_v and sum_v |A_v|^2 with A_v the FR attraction
 // sum_u W |p_u - p_v| (p_u - p_v) (algorithms.cpp:1056-1058) and R_v the
-// Barnes-Hut sum of unit vectors towards the cells (BarnesHut.h:69-86)
-__global__ void scale_fit_kernel(int n, const int *__restrict__ rowptr, const int *__restrict__ colids,
-                                 const float2 *__restrict__ pos, const float2 *__restrict__ rep, float W,
-                                 double *part) {
+// Barnes-Hut sum of unit vectors towards the cells (BarnesHut.h:69-86).
+// Bound by FP64: a warp takes 32 consecutive rows and forms the terms of their
+// entries a lane each, kFitEntries at a time, so that the root and the products
+// run in full warps; a lane then adds its row's terms in row order.  With the
+// whole row a lane's, 400,000 vertices of a geometric graph took 272 us, so
+// 155.
+constexpr int kFitEntries = 192, kFitWarps = 8;
+
+__global__ void __launch_bounds__(32 * kFitWarps) scale_fit_kernel(int n, const int *__restrict__ rowptr,
+                                                                   const int *__restrict__ colids,
+                                                                   const float2 *__restrict__ pos,
+                                                                   const float2 *__restrict__ rep, float W,
+                                                                   double *part) {
   __shared__ double red[2][8];
+  __shared__ double2 term[kFitWarps][kFitEntries];
+  __shared__ int first[kFitWarps][33];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double ar = 0.0, aa = 0.0;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    const float2 p = pos[v];
+  for (int v0 = 32 * (blockIdx.x * kFitWarps + warp); v0 < n; v0 += 32 * gridDim.x * kFitWarps) {
+    const int v = v0 + lane, e0 = rowptr[min(v, n)], e1 = rowptr[min(v + 1, n)];
+    __syncwarp();
+    first[warp][lane] = e0;
+    if (lane == 31) first[warp][32] = e1;
+    __syncwarp();
+    const int base = first[warp][0], end = first[warp][32];
     double ax = 0.0, ay = 0.0;
-    for (int e = rowptr[v]; e < rowptr[v + 1]; e++) {
-      const float2 q = pos[colids[e]];
-      const double dx = (double)q.x - p.x, dy = (double)q.y - p.y;
-      const double sc = (double)W * sqrt(dx * dx + dy * dy);
-      ax += sc * dx;
-      ay += sc * dy;
+    for (int c0 = base; c0 < end; c0 += kFitEntries) {
+      const int c1 = min(c0 + kFitEntries, end);
+      for (int e = c0 + lane; e < c1; e += 32) {
+        int lo = 0;  // the row of e: first[lo] <= e < first[lo + 1]
+#pragma unroll
+        for (int h = 16; h > 0; h >>= 1)
+          if (first[warp][lo + h] <= e) lo += h;
+        const float2 p = pos[v0 + lo], q = pos[colids[e]];
+        const double dx = (double)q.x - p.x, dy = (double)q.y - p.y;
+        const double sc = (double)W * sqrt(dx * dx + dy * dy);
+        term[warp][e - c0] = make_double2(sc * dx, sc * dy);
+      }
+      __syncwarp();
+      for (int e = max(e0, c0); e < min(e1, c1); e++) {
+        const double2 t = term[warp][e - c0];
+        ax += t.x;
+        ay += t.y;
+      }
+      __syncwarp();
     }
-    const float2 r = rep[v];
-    ar += ax * r.x + ay * r.y;
-    aa += ax * ax + ay * ay;
+    if (v < n) {
+      const float2 r = rep[v];
+      ar += ax * r.x + ay * r.y;
+      aa += ax * ax + ay * ay;
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     ar += __shfl_xor_sync(0xffffffffu, ar, o);
@@ -326,7 +378,7 @@ double predict_edge_length(const double *sm, int n, double mean_degree) {
 
 }  // namespace
 
-constexpr int kParts = 256;
+constexpr int kEdgeParts = 608;  // blocks of the two kernels over all entries
 
 // Learned coordinates for the context's graph into ctx->pos.
 int learned_init(bl_ctx *ctx, const float *params, const double *scale_model, int seed) {
@@ -355,11 +407,11 @@ int learned_init(bl_ctx *ctx, const float *params, const double *scale_model, in
   if (!rc) {
     residual_start_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(mpnn_output(ctx), d_f, n, ctx->pos);
     double *d_part = nullptr;
-    std::vector<double> part(kParts);
-    if (cudaMalloc(&d_part, sizeof(double) * kParts) != cudaSuccess) rc = bl_fail(ctx, BL_ERR_CUDA, "cudaMalloc");
+    std::vector<double> part(kEdgeParts);
+    if (cudaMalloc(&d_part, sizeof(double) * kEdgeParts) != cudaSuccess) rc = bl_fail(ctx, BL_ERR_CUDA, "cudaMalloc");
     if (!rc) {
-      edge_length_kernel<<<kParts, 256, 0, ctx->stream>>>(n, ctx->g.rowptr, ctx->g.colids, ctx->pos, d_part);
-      if (cudaMemcpyAsync(part.data(), d_part, sizeof(double) * kParts, cudaMemcpyDeviceToHost, ctx->stream) !=
+      edge_length_kernel<<<kEdgeParts, 256, 0, ctx->stream>>>(n, ctx->g.rowptr, ctx->g.colids, ctx->pos, d_part);
+      if (cudaMemcpyAsync(part.data(), d_part, sizeof(double) * kEdgeParts, cudaMemcpyDeviceToHost, ctx->stream) !=
               cudaSuccess ||
           cudaStreamSynchronize(ctx->stream) != cudaSuccess)
         rc = bl_fail(ctx, BL_ERR_CUDA, "learned init");
@@ -383,13 +435,13 @@ int learned_init(bl_ctx *ctx, const float *params, const double *scale_model, in
     if (!rc) rc = bh_traverse(ctx, 1.2, false, 0);
     if (!rc) {
       double *d_p2 = nullptr;
-      std::vector<double> p2(2 * kParts);
-      if (cudaMalloc(&d_p2, sizeof(double) * 2 * kParts) != cudaSuccess) rc = bl_fail(ctx, BL_ERR_CUDA, "cudaMalloc");
+      std::vector<double> p2(2 * kEdgeParts);
+      if (cudaMalloc(&d_p2, sizeof(double) * 2 * kEdgeParts) != cudaSuccess) rc = bl_fail(ctx, BL_ERR_CUDA, "cudaMalloc");
       if (!rc) {
-        scale_fit_kernel<<<kParts, 256, 0, ctx->stream>>>(n, ctx->g.rowptr, ctx->g.colids, ctx->pos, ctx->s.rep,
+        scale_fit_kernel<<<kEdgeParts, 32 * kFitWarps, 0, ctx->stream>>>(n, ctx->g.rowptr, ctx->g.colids, ctx->pos, ctx->s.rep,
                                                           (float)ctx->weight, d_p2);
         ctx->launches++;
-        if (cudaMemcpyAsync(p2.data(), d_p2, sizeof(double) * 2 * kParts, cudaMemcpyDeviceToHost, ctx->stream) !=
+        if (cudaMemcpyAsync(p2.data(), d_p2, sizeof(double) * 2 * kEdgeParts, cudaMemcpyDeviceToHost, ctx->stream) !=
                 cudaSuccess ||
             cudaStreamSynchronize(ctx->stream) != cudaSuccess)
           rc = bl_fail(ctx, BL_ERR_CUDA, "learned init scale");
@@ -397,7 +449,7 @@ int learned_init(bl_ctx *ctx, const float *params, const double *scale_model, in
       cudaFree(d_p2);
       if (!rc) {
         double ar = 0.0, aa = 0.0;
-        for (int b = 0; b < kParts; b++) {
+        for (int b = 0; b < kEdgeParts; b++) {
           ar += p2[2 * b];
           aa += p2[2 * b + 1];
         }
