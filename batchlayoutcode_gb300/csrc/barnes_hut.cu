@@ -586,50 +586,59 @@ __device__ __forceinline__ int kdelta(const u64 *__restrict__ K, int n, int i, i
   return x ? __clzll((long long)x) : 64 + __clz(i ^ j);
 }
 
-// internal node i in [0, n-2]; leaf k encoded as ~k in child links;
-// parent[] holds internal parents of internal nodes (index i) and of leaves
-// (index n-1+k); the root is internal node 0.
-// bnode: the same per internal node packed in 32 bytes for the chain walk,
-// ints {first, last, prefix length, parent, left, right, -, -} (the parent
-// word is written by the parent's thread).
-__global__ void radix_tree_kernel(const u64 *__restrict__ K, int n, int2 *child, int2 *range,
-                                  int *dlt, int *parent, int *bnode) {
+// internal node i in [0, n-2]; leaf k encoded as ~k in child links; the root
+// is internal node 0.  A node is 32 bytes of bnode, ints {first, last, prefix
+// length, left; right, parent, -, -}: its own words are two stores of one
+// sector, the parent word is written by the parent's thread.  range and dlt
+// repeat the first words for the kernels that want only those; leaf_parent[k]
+// is the parent of leaf k.  (With the words stored one by one and a child and a
+// parent array beside them the kernel took 33 us for 1,000,000 points and 76
+// for 3,000,000, so 30 and 72.)
+__global__ void radix_tree_kernel(const u64 *__restrict__ K, int n, int2 *range, int *dlt, int *leaf_parent,
+                                  int *bnode) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
-  const int d = (kdelta(K, n, i, i + 1) - kdelta(K, n, i, i - 1)) >= 0 ? 1 : -1;
-  const int dmin = kdelta(K, n, i, i - d);
+  const u64 ki = K[i];
+  const int dnext = kdelta(K, n, i, i + 1), dprev = kdelta(K, n, i, i - 1);
+  const int d = dnext - dprev >= 0 ? 1 : -1;
+  const int dmin = min(dnext, dprev);
+  // The searches ask whether a prefix with key i is longer than m bits: for
+  // m < 64 whether the keys' difference is below 2^(63 - m), one comparison
+  // where the prefix itself takes a count, a select and the tie's rule (the
+  // searches are bound by issue: 1,000,000 points 41 us, so 33; 3,000,000 101,
+  // so 76).
+  auto longer = [&](int q, int m, u64 lim) {
+    return m < 64 ? (unsigned int)q < (unsigned int)n && (ki ^ K[q]) <= lim : kdelta(K, n, i, q) > m;
+  };
+  auto limit = [](int m) { return m < 0 ? ~0ull : (1ull << (63 - min(m, 63))) - 1ull; };
+  const u64 lmin = limit(dmin);
   int lmax = 2;
-  while (kdelta(K, n, i, i + lmax * d) > dmin) lmax <<= 1;
+  while (longer(i + lmax * d, dmin, lmin)) lmax <<= 1;
   int l = 0;
   for (int t = lmax >> 1; t >= 1; t >>= 1)
-    if (kdelta(K, n, i, i + (l + t) * d) > dmin) l += t;
+    if (longer(i + (l + t) * d, dmin, lmin)) l += t;
   const int j = i + l * d;
   const int dnode = kdelta(K, n, i, j);
+  const u64 lnode = limit(dnode);
   int s = 0;
-  for (int div = 2;; div <<= 1) {
-    const int t = (l + div - 1) / div;
-    if (kdelta(K, n, i, i + (s + t) * d) > dnode) s += t;
-    if (t <= 1) break;
+  for (int t = l; t > 1;) {
+    t = (t + 1) >> 1;  // l / 2, l / 4, ... rounded up
+    if (longer(i + (s + t) * d, dnode, lnode)) s += t;
   }
   const int gamma = i + s * d + min(d, 0);
   const int first = min(i, j), last = max(i, j);
   const int left = (first == gamma) ? ~gamma : gamma;
   const int right = (last == gamma + 1) ? ~(gamma + 1) : gamma + 1;
-  child[i] = make_int2(left, right);
   range[i] = make_int2(first, last);
   dlt[i] = dnode;
-  parent[left >= 0 ? left : (n - 1 + ~left)] = i;
-  parent[right >= 0 ? right : (n - 1 + ~right)] = i;
-  if (i == 0) parent[0] = -1;
   int *b = bnode + 8 * (size_t)i;
-  b[0] = first;
-  b[1] = last;
-  b[2] = dnode;
-  b[4] = left;
-  b[5] = right;
-  if (left >= 0) bnode[8 * (size_t)left + 3] = i;
-  if (right >= 0) bnode[8 * (size_t)right + 3] = i;
-  if (i == 0) b[3] = -1;
+  *reinterpret_cast<int4 *>(b) = make_int4(first, last, dnode, left);
+  b[4] = right;
+  if (i == 0) b[5] = -1;
+  if (left >= 0) bnode[8 * (size_t)left + 5] = i;
+  else leaf_parent[~left] = i;
+  if (right >= 0) bnode[8 * (size_t)right + 5] = i;
+  else leaf_parent[~right] = i;
 }
 
 struct TreeArgs {
@@ -637,7 +646,7 @@ struct TreeArgs {
   const float2 *spos;
   const int2 *range;
   const int *dlt;
-  const int *parent;
+  const int *leaf_parent;
   int4 *qkids;          // quad children of a quad node, kNoChild-padded
   double2 *qcen;
   int *qbelow;
@@ -696,31 +705,35 @@ __global__ void __launch_bounds__(256) chain_kernel(TreeArgs t) {
 
 __device__ __forceinline__ int chain_walk(const TreeArgs &t, int k) {
   int cnt = 0;
-  int cur = t.parent[t.n - 1 + k];
+  int cur = t.leaf_parent[k];
   if (k == 0) t.qpar[0] = -1;  // the root
   const int4 none = make_int4(-1, -1, -1, -1);
-  int4 ra = none, rb = none;  // cur's packed record
+  int4 ra = none;  // cur's packed record
+  int2 rb = make_int2(-1, -1);
+  auto second = [&](int node) { return __ldg(reinterpret_cast<const int2 *>(&t.bnode[2 * node + 1])); };
   if (cur >= 0) {
     ra = __ldg(&t.bnode[2 * cur]);
-    rb = __ldg(&t.bnode[2 * cur + 1]);
+    rb = second(cur);
   }
   // bounded by the tree height: every step moves to a parent.  The parent's
   // record and the children's are loaded together, one round trip a step.
   while (cur >= 0 && ra.x == k) {
-    const int par = ra.w;
-    int4 pa = none, pb = none;
+    const int par = rb.y;
+    int4 pa = none;
+    int2 pb = make_int2(-1, -1);
     if (par >= 0) {
       pa = __ldg(&t.bnode[2 * par]);
-      pb = __ldg(&t.bnode[2 * par + 1]);
+      pb = second(par);
     }
     const int p = ra.z;
-    const int sides[2] = {rb.x, rb.y};
-    int4 ca[2] = {none, none}, cb[2] = {none, none};
+    const int sides[2] = {ra.w, rb.x};
+    int4 ca[2] = {none, none};
+    int2 cb[2];
 #pragma unroll
     for (int h = 0; h < 2; h++)
       if (p < 64 && sides[h] >= 0) {
         ca[h] = __ldg(&t.bnode[2 * sides[h]]);
-        cb[h] = __ldg(&t.bnode[2 * sides[h] + 1]);
+        cb[h] = second(sides[h]);
       }
     // cur is merged into its parent's quad node: the x-bit split of the digit
     // whose y-bit split is the parent, or any split inside a run below its top
@@ -736,8 +749,8 @@ __device__ __forceinline__ int chain_walk(const TreeArgs &t, int k) {
           const int pc = ca[h].z;  // the child's prefix length; its parent is cur
           const bool csub = c > 0 && (pc >= 64 ? p >= 64 : ((pc & 1) && p == pc - 1));
           if (c >= 0 && csub) {
+            kids[m++] = ca[h].w;
             kids[m++] = cb[h].x;
-            kids[m++] = cb[h].y;
           } else {
             kids[m++] = c;
           }
@@ -1732,7 +1745,7 @@ int ensure_bh_scratch(bl_ctx *ctx) {
   if (s.bh_n >= n && s.keys) return 0;
   auto fr = [](void *p) { if (p) cudaFree(p); };
   fr(s.keys); fr(s.keys_alt); fr(s.perm); fr(s.perm_alt); fr(s.hist); fr(s.spos);
-  fr(s.bparent); fr(s.bchild); fr(s.brange); fr(s.bdelta); fr(s.qkids); fr(s.qpar); fr(s.qnchild);
+  fr(s.bparent); fr(s.brange); fr(s.bdelta); fr(s.qkids); fr(s.qpar); fr(s.qnchild);
   fr(s.span); fr(s.span_stage); fr(s.ztab); fr(s.chain); fr(s.qcen);
   fr(s.qbelow); fr(s.startcnt); fr(s.startbase); fr(s.nodes); fr(s.nodes_c64);
   fr(s.nodes_lvl); fr(s.rep); fr(s.f0); fr(s.pos_alt); fr(s.runs); fr(s.bnode); fr(s.pairs);
@@ -1743,8 +1756,7 @@ int ensure_bh_scratch(bl_ctx *ctx) {
   BL_CUDA(ctx, cudaMalloc(&s.perm_alt, m * 4));
   BL_CUDA(ctx, cudaMalloc(&s.pairs, 2 * m * 8));
   BL_CUDA(ctx, cudaMalloc(&s.spos, m * sizeof(float2)));
-  BL_CUDA(ctx, cudaMalloc(&s.bparent, 2 * m * sizeof(int)));
-  BL_CUDA(ctx, cudaMalloc(&s.bchild, m * sizeof(int2)));
+  BL_CUDA(ctx, cudaMalloc(&s.bparent, m * sizeof(int)));
   BL_CUDA(ctx, cudaMalloc(&s.brange, m * sizeof(int2)));
   BL_CUDA(ctx, cudaMalloc(&s.bnode, 2 * m * sizeof(int4)));
   BL_CUDA(ctx, cudaMalloc(&s.bdelta, m * sizeof(int)));
@@ -1857,7 +1869,7 @@ int bh_build(bl_ctx *ctx, const float2 *pos, double theta, int attract_batch) {
   ctx->launches++;
   bl_time_end(ctx, "morton_sort");
   bl_time_begin(ctx, "radix_tree");
-  radix_tree_kernel<<<nblk(n - 1, 256), 256, 0, st>>>(s.keys, n, s.bchild, s.brange, s.bdelta, s.bparent,
+  radix_tree_kernel<<<nblk(n - 1, 256), 256, 0, st>>>(s.keys, n, s.brange, s.bdelta, s.bparent,
                                                        reinterpret_cast<int *>(s.bnode));
   bl_time_end(ctx, "radix_tree");
   TreeArgs t;
@@ -1865,7 +1877,7 @@ int bh_build(bl_ctx *ctx, const float2 *pos, double theta, int attract_batch) {
   t.spos = s.spos;
   t.range = s.brange;
   t.dlt = s.bdelta;
-  t.parent = s.bparent;
+  t.leaf_parent = s.bparent;
   t.qkids = s.qkids;
   t.qcen = s.qcen;
   t.qbelow = s.qbelow;
@@ -2192,20 +2204,22 @@ int bh_canonical_tree(bl_ctx *ctx, int cap, int *lo, int *hi, int *depth, int *n
   if (n < 2) return 0;
   if (int rc = bh_build(ctx, ctx->pos, 1.2)) return rc;  // (theta enters only the records)
   // copy the binary tree back and emit quad nodes in pre-order (host walk)
-  std::vector<int2> child(n - 1), range(n - 1);
-  std::vector<int> dlt(n - 1), parent(2 * n - 1);
+  std::vector<int2> range(n - 1);
+  std::vector<int4> node(2 * (size_t)(n - 1));  // as radix_tree_kernel packs them
+  std::vector<int> dlt(n - 1);
   std::vector<double2> qcen(n - 1);
   cudaStream_t st = ctx->stream;
-  BL_CUDA(ctx, cudaMemcpyAsync(child.data(), ctx->s.bchild, (n - 1) * sizeof(int2), cudaMemcpyDeviceToHost, st));
+  BL_CUDA(ctx, cudaMemcpyAsync(node.data(), ctx->s.bnode, node.size() * sizeof(int4), cudaMemcpyDeviceToHost, st));
   BL_CUDA(ctx, cudaMemcpyAsync(range.data(), ctx->s.brange, (n - 1) * sizeof(int2), cudaMemcpyDeviceToHost, st));
   BL_CUDA(ctx, cudaMemcpyAsync(dlt.data(), ctx->s.bdelta, (n - 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
-  BL_CUDA(ctx, cudaMemcpyAsync(parent.data(), ctx->s.bparent, (2 * n - 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
   BL_CUDA(ctx, cudaMemcpyAsync(qcen.data(), ctx->s.qcen, (n - 1) * sizeof(double2), cudaMemcpyDeviceToHost, st));
   BL_CUDA(ctx, cudaStreamSynchronize(st));
   if (int rc = bl_check_status(ctx)) return rc;
-  auto sub = [&](int node) {
-    if (node <= 0) return false;
-    const int p = dlt[node], pp = dlt[parent[node]];
+  auto left = [&](int v) { return node[2 * (size_t)v].w; };
+  auto right = [&](int v) { return node[2 * (size_t)v + 1].x; };
+  auto sub = [&](int v) {
+    if (v <= 0) return false;
+    const int p = dlt[v], pp = dlt[node[2 * (size_t)v + 1].y];
     if (p >= 64) return pp >= 64;
     return (p & 1) && pp == p - 1;
   };
@@ -2218,11 +2232,11 @@ int bh_canonical_tree(bl_ctx *ctx, int cap, int *lo, int *hi, int *depth, int *n
     if (dlt[v] >= 64) {
       kids.clear();
     } else {
-      const int sides[2] = {child[v].x, child[v].y};
+      const int sides[2] = {left(v), right(v)};
       for (int c : sides) {
         if (c >= 0 && sub(c)) {
-          kids.push_back(child[c].x);
-          kids.push_back(child[c].y);
+          kids.push_back(left(c));
+          kids.push_back(right(c));
         } else {
           kids.push_back(c);
         }

@@ -195,8 +195,7 @@ struct Scratch {
   unsigned int *bbox = nullptr;  // sort: box (ordered-uint floats), arrivals
   double *frame = nullptr;  // {minX, minY, MAXMIN, 1 / MAXMIN}, then the key constants
   float2 *spos = nullptr;        // positions in Morton order
-  int *bparent = nullptr;        // binary radix tree: parent of node (internal i, leaf n-1+k)
-  int2 *bchild = nullptr;        // children of internal node (encoded: >= 0 internal, < 0 leaf ~k)
+  int *bparent = nullptr;        // binary radix tree: parent of leaf k
   int2 *brange = nullptr;        // [first, last] of internal node
   int *bdelta = nullptr;         // common prefix length of internal node
   int4 *qkids = nullptr;         // quad children of a quad node
