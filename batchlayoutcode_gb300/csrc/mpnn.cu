@@ -176,15 +176,17 @@ __global__ void __launch_bounds__(kT) mpnn_fwd_kernel(FwdArgs a) {
 #pragma unroll
       for (int k = 0; k < 8; k++) acc[k] = 0.f;
       const int len = b1 - b0 <= kLongRow ? b1 - b0 : 0;
+      int col[CPL];
+#pragma unroll
+      for (int j = 0; j < CPL; j++) col[j] = first[i][j];
       for (int d = 0; __any_sync(0xffffffffu, d < len); d += 8) {
-        int col[CPL];
+        // the ids of the eight after these come while these rows do (207,796
+        // vertices, the three layers: 258 -> 242 us)
+        int next[CPL];
 #pragma unroll
         for (int j = 0; j < CPL; j++) {
-          col[j] = first[i][j];
-          if (d > 0) {
-            const int e = d + gl + j * LPR;
-            col[j] = e < len ? __ldg(&a.colids[b0 + e]) : 0;
-          }
+          const int e = d + 8 + gl + j * LPR;
+          next[j] = e < len ? __ldg(&a.colids[b0 + e]) : 0;
         }
         uint4 q[8];  // eight rows in flight, summed in row order
 #pragma unroll
@@ -200,6 +202,8 @@ __global__ void __launch_bounds__(kT) mpnn_fwd_kernel(FwdArgs a) {
 #pragma unroll
           for (int x = 0; x < 8; x++) acc[x] += f[x];
         }
+#pragma unroll
+        for (int j = 0; j < CPL; j++) col[j] = next[j];
       }
       *reinterpret_cast<uint4 *>(sA + tc::kmajor_offset(row, gl * 8, K)) = own;
       if (b1 - b0 <= kLongRow) {
