@@ -71,7 +71,7 @@ constexpr int kMoveTile = 32;               // targets a mover handles at a time
 constexpr int kPartLoads = 5;               // partials a P lane loads at a time
 constexpr int kMaxMovers = 32;
 constexpr int kMaxLag = 2;
-constexpr int kExchange = 4;                // exchange slots (two would do)
+constexpr int kExchange = 4;                // slots of the exchange and of the moved counts (two would do)
 constexpr int kNear = 16;                   // staged neighbours in the batch before
 constexpr unsigned int kNearMore = 0x80000000u;
 constexpr int kMaxBatch = 4096;
@@ -82,7 +82,11 @@ constexpr float kForceLimit = 17179869184.0f;  // 2^34
 
 // Control words of a launch (zero before it).
 struct MbControl {
-  unsigned int moved;   // movers that finished a batch, over all batches
+  // movers that stored the new positions of batch q, in word q % kExchange: one
+  // mover's count is at most two batches ahead of another's, so a full word
+  // tells that every mover is done with its batch (one sum over all batches
+  // would not: a mover ahead makes up for one behind)
+  unsigned int moved[kExchange];
   unsigned int stop;    // converged runs: the movers ended
   unsigned int ready;   // movers whose first loads are done
   unsigned int pad;
@@ -321,7 +325,6 @@ __device__ __forceinline__ void sweeper(const MinibatchArgs &a, unsigned char *s
   for (int k = threadIdx.x; k < len; k += kThreads) put_point(slice, k, __ldcg(&a.pos[slo + k]));
   __syncthreads();
   const int nb = a.nbatches, B = a.batch, slots = a.lag + 1, stride = (B + 1) & ~1;
-  const unsigned int M = (unsigned int)a.movers;
   long long left = (a.converged ? LLONG_MAX : (long long)a.iterations * nb) - team;
   // next batch whose new positions this team takes over into the slice
   // (batch numbers modulo 2^32)
@@ -334,16 +337,19 @@ __device__ __forceinline__ void sweeper(const MinibatchArgs &a, unsigned char *s
   float2 p0 = make_float2(0.f, 0.f), p1 = p0;
   bool have = false;
   bool started = false;  // a batch has to have moved
+  // batch q - lag - 1, the last that has to have: its word of `moved`, full at
+  // `target` (0 and a word of a batch before the run at first)
+  int word = (team - a.lag - 1) & (kExchange - 1);
+  unsigned int target = team - a.lag - 1 < 0 ? 0u : (unsigned int)a.movers;
   for (unsigned int q = (unsigned int)team; left > 0; q += 2, left -= 2) {
     const unsigned int need = q - (unsigned int)a.lag;  // batches that have moved
     started = started || (int)need > 0;
     if (tid == 0) {
       int go = 1;
-      const unsigned int target = need * M;
       if (started) {
         Poll w;
 #pragma unroll 1
-        while (!reached(ld_acquire_gpu(&a.ctl->moved), target)) {
+        while (!reached(ld_acquire_gpu(&a.ctl->moved[word]), target)) {
           if ((a.converged && ld_volatile_u32(&a.ctl->stop) != 0u) || !w.again(a.st)) {
             go = 0;
             break;
@@ -351,6 +357,11 @@ __device__ __forceinline__ void sweeper(const MinibatchArgs &a, unsigned char *s
         }
       }
       s_go[team] = go;
+    }
+    word += 2;
+    if (word >= kExchange) {
+      word -= kExchange;
+      target += (unsigned int)a.movers;
     }
     bar_sync(1 + team, kTeam);
     if (!s_go[team]) return;
@@ -960,7 +971,7 @@ __device__ __forceinline__ void mover_critical(const MinibatchArgs &a, const Mov
       bar_sync(kBarPub, kCThreads);
       if (lane == 0) {
         __threadfence();
-        red_add(&a.ctl->moved, 1u);
+        red_add(&a.ctl->moved[q & (kExchange - 1)], 1u);
       }
       if (a.converged || F.last_loop) mover_outputs(a, S, F, m, par, base, t1 - t0, b == nb - 1);
     }
