@@ -488,9 +488,11 @@ constexpr int kCThreads = kCWarps * 32;
 constexpr int kEarlyThreads = kCThreads + (kNWarps + kPWarps) * 32;  // C with N and P
 
 struct MoverFlags {
+  // fail, end and gone are set once and stay: they end waits
   volatile int fail;           // a wait ran out or a force left the range
   volatile unsigned int end;   // batches from this one on do not exist (0: not known yet)
   volatile unsigned int seen;  // batches whose partials all sweepers have stored
+  volatile int gone;           // the watching warp, whose waits are bounded, has returned
   volatile int last[2];        // by parity of the batch: 1 no batch follows, 2 not even this one
   volatile double step;
   volatile float stepf;
@@ -518,10 +520,20 @@ __device__ __forceinline__ bool ring_ready(const MinibatchArgs &a, MoverFlags &F
   return true;
 }
 
+// A lane of team N or P waits until the watching warp has seen `batches`
+// batches' partials.  Bounded by that warp: it ends for a run that is over
+// (end), one that failed (fail), and at the latest when the warp is gone.
+__device__ __forceinline__ void wait_seen(MoverFlags &F, unsigned int batches) {
+#pragma unroll 1
+  while (!reached(F.seen, batches)) {
+    const unsigned int end = F.end;
+    if ((end != 0u && reached(batches, end + 1u)) || F.fail || F.gone) break;
+  }
+}
+
 // One warp: announces in shared memory which batches' partials are complete,
 // a round trip ahead of the team that reads them.
 __device__ __forceinline__ void mover_watch(const MinibatchArgs &a, MoverFlags &F) {
-  if ((threadIdx.x & 31) != 0) return;
   unsigned int q = 0, round = 1;
   for (int slot = 0;; q++) {
     Poll p;
@@ -558,13 +570,7 @@ __device__ __forceinline__ void mover_partials(const MinibatchArgs &a, const Mov
     int fb = b + S.tiles / 2;
     if (fb >= nb) fb -= nb;
     const int nbase = fb * B, ncnt = min(B, a.n - nbase);
-    if (lane == 0) {  // the watching warp bounds this wait
-#pragma unroll 1
-      while (!reached(F.seen, q + 1u)) {
-        const unsigned int end = F.end;
-        if ((end != 0u && reached(q, end)) || F.fail) break;
-      }
-    }
+    if (lane == 0) wait_seen(F, q + 1u);
     __syncwarp();
     __threadfence_block();
 #pragma unroll 1
@@ -669,10 +675,7 @@ __device__ __forceinline__ void mover_neighbours(const MinibatchArgs &a, const M
       int j0 = valid && e < r1 ? __ldg(&a.eff_colids[e]) : -1;
       if (ch == 0) {
         if (!ring_ready(a, F, par, first)) return;
-        if (lane == 0)
-#pragma unroll 1
-          while (!reached(F.seen, q) && !F.fail) {
-          }
+        if (lane == 0) wait_seen(F, q);
         __syncwarp();
         __threadfence_block();
       }
@@ -869,7 +872,9 @@ __device__ __forceinline__ void mover_critical(const MinibatchArgs &a, const Mov
             if (!started && !wait_count(&a.ctl->ready, (unsigned int)a.movers, a.st)) F.fail = 1;
             const int l = (stop || F.fail) ? 2 : (F.last_loop && b == nb - 1) ? 1 : 0;
             F.last[par] = l;
-            if (l) F.end = q + 1u;
+            // (a converged run's end is known since its last iteration's end, a
+            // failed one's waits end by `fail`: what a wait has seen stays)
+            if (l == 1) F.end = q + 1u;
           }
           bar_sync(kBarC, kCThreads);
           last = F.last[par];
@@ -1021,6 +1026,7 @@ __device__ __forceinline__ void mover(const MinibatchArgs &a, unsigned char *sme
     F.fail = 0;
     F.end = 0;
     F.seen = 0;
+    F.gone = 0;
     F.last[0] = F.last[1] = 0;
     F.step = a.step0;
     F.stepf = (float)a.step0;
@@ -1054,7 +1060,12 @@ __device__ __forceinline__ void mover(const MinibatchArgs &a, unsigned char *sme
   if (tid == 0) red_add(&a.ctl->ready, 1u);
   if (tid < kCThreads) mover_critical<kRep>(a, S, F, m);
   else if (tid < kCThreads + kNWarps * 32) mover_neighbours<kRep>(a, S, F, m);
-  else if (tid < kCThreads + (kNWarps + 1) * 32) mover_watch(a, F);
+  else if (tid < kCThreads + (kNWarps + 1) * 32) {
+    if ((tid & 31) == 0) {
+      mover_watch(a, F);
+      F.gone = 1;
+    }
+  }
   else mover_partials(a, S, F, m);
 }
 
