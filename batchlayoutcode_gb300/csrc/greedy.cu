@@ -342,6 +342,9 @@ __global__ void __launch_bounds__(kIterThreads, 1) greedy_iteration_kernel(IterA
             if (!ok) break;
           }
         }
+        // the other lanes' position loads come after lane 0's acquire (a shuffle
+        // orders no memory)
+        __syncwarp();
         if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) return false;
       }
     }
