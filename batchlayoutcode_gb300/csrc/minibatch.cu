@@ -671,8 +671,9 @@ __device__ __forceinline__ void mover_neighbours(const MinibatchArgs &a, const M
         r0 = __ldg(&a.eff_rowptr[base + t]);
         r1 = __ldg(&a.eff_rowptr[base + t + 1]);
       }
+      const int end = valid ? r1 : r0;
       int e = r0 + w;
-      int j0 = valid && e < r1 ? __ldg(&a.eff_colids[e]) : -1;
+      int j0 = e < end ? __ldg(&a.eff_colids[e]) : -1;
       if (ch == 0) {
         if (!ring_ready(a, F, par, first)) return;
         if (lane == 0) wait_seen(F, q);
@@ -685,9 +686,10 @@ __device__ __forceinline__ void mover_neighbours(const MinibatchArgs &a, const M
       const float2 p = valid ? target_at(t) : make_float2(0.f, 0.f);
       Sum2 f = {0ull, 0ull};
 #pragma unroll 1
-      while (j0 >= 0) {
-        const int e1 = e + kNWarps;
-        const int j1 = e1 < r1 ? __ldg(&a.eff_colids[e1]) : -1;
+      for (int j1; e < end; j0 = j1, e += kNWarps) {
+        j1 = e + kNWarps < end ? __ldg(&a.eff_colids[e + kNWarps]) : -1;
+        // a list handed in on the device is not checked: other ids are no neighbours
+        if ((unsigned int)j0 >= (unsigned int)a.n) continue;
         // batch q - d holds j0 as its vertex jt; d > slots: further back
         int d = slots + 1, jt = 0;
         int rel = j0 - w0;
@@ -716,8 +718,6 @@ __device__ __forceinline__ void mover_neighbours(const MinibatchArgs &a, const M
           const float2 v = neighbour_force<kRep>(a.model, W, pj, p);
           f.add(v.x, v.y);
         }
-        j0 = j1;
-        e = e1;
       }
       if (ch + 1 == S.chunks) {  // the next batch's row
         const bool more = t0 + lane < min(ncnt, t0 + S.share);

@@ -368,7 +368,8 @@ int bl_wait_selftest(bl_ctx *ctx, int site, int complete);
  *                             (the CSR rows themselves only when every row is
  *                             sorted ascending without duplicates AND no row
  *                             but the last is empty: an empty row matches the
- *                             next row's first neighbour)
+ *                             next row's first neighbour); an id outside
+ *                             0 .. n - 1 is skipped
  *   d_xy[2n] float32           coordinates, updated in place
  *   d_force[2n], d_vertex_energy[n]  outputs: forces and |f|^2 per vertex
  * stream: cudaStream_t (NULL = default stream); the call returns after the
