@@ -77,7 +77,7 @@ constexpr unsigned int kNearMore = 0x80000000u;
 constexpr int kMaxBatch = 4096;
 
 // A force component beyond +-2^34 (coincident-but-for-rounding vertices) or
-// not a number is reported as an error instead of moving the vertex.
+// not a number is reported as an error; the vertex keeps its position.
 constexpr float kForceLimit = 17179869184.0f;  // 2^34
 
 // Control words of a launch (zero before it).
@@ -960,9 +960,11 @@ __device__ __forceinline__ void mover_critical(const MinibatchArgs &a, const Mov
         } else if (fx != 0.f || fy != 0.f) {
           np = step_fp64(pi, hx, hy, lx, ly, F.step);
         }
+        const bool in_range = fabsf(fx) < kForceLimit && fabsf(fy) < kForceLimit;
+        if (!in_range) np = pi;
         st_relaxed_pair(&a.exchange[(size_t)(q & (kExchange - 1)) * B + t], tagged(np.x, q + 1u), tagged(np.y, q + 1u));
         __stcg(&a.pos[base + t], np);
-        if (!(fabsf(fx) < kForceLimit) || !(fabsf(fy) < kForceLimit)) {
+        if (!in_range) {
           dev_record_error(a.st, DEV_FORCE_RANGE);
           F.fail = 1;
         }
