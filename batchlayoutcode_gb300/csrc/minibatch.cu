@@ -69,10 +69,13 @@ constexpr int kPWarps = 8;                  // mover: sweepers' partials (and on
 constexpr int kRows = 16;                   // sums per target that N and P leave (row kNWarps stays zero)
 constexpr int kMoveTile = 32;               // targets a mover handles at a time
 constexpr int kPartLoads = 5;               // partials a P lane loads at a time
-constexpr int kMaxMovers = 32;
+constexpr int kMaxMovers = 64;              // more than 32 for graphs of long rows only (minibatch_shape)
+constexpr double kDense = 100.0;            // mean row length from which they are considered
 constexpr int kMaxLag = 2;
 constexpr int kExchange = 4;                // slots of the exchange and of the moved counts (two would do)
 constexpr int kNear = 16;                   // staged neighbours in the batch before
+constexpr int kFlatBlock = 64 * kNWarps;    // entries that team N takes at once where it shares them evenly
+constexpr int kFlatJoin = 2 * kFlatBlock;   // more of them: team P takes its part
 constexpr unsigned int kNearMore = 0x80000000u;
 constexpr int kMaxBatch = 4096;
 
@@ -471,6 +474,16 @@ struct Sum2 {
     lo = add2(lo, err);
   }
   __device__ __forceinline__ void add(float x, float y) { add(pack2(x, y)); }
+  __device__ __forceinline__ void merge(Sum2 s) {
+    add(s.hi);
+    lo = add2(lo, s.lo);
+  }
+  __device__ __forceinline__ Sum2 from_xor(int o) const {
+    return Sum2{__shfl_xor_sync(0xffffffffu, hi, o), __shfl_xor_sync(0xffffffffu, lo, o)};
+  }
+  __device__ __forceinline__ Sum2 from_up(int o) const {
+    return Sum2{__shfl_up_sync(0xffffffffu, hi, o), __shfl_up_sync(0xffffffffu, lo, o)};
+  }
 };
 
 struct MoverSmem {
@@ -480,6 +493,7 @@ struct MoverSmem {
   float2 *tile;        // [tiles][stride]: positions of batches q .. q + 2 (q + 1 when late) before they move
   int *near;           // [2][share][kNear]: neighbours in the batch before (unless late)
   unsigned int *mask;  // [2][share]: which of them are set
+  int2 *range;         // [2][share]: where in a long row they are (first above last: not noted; unless late)
   int pairs, stride, share, chunks, tiles;
 };
 
@@ -510,14 +524,13 @@ __device__ __forceinline__ ulonglong2 *rows_of(const MinibatchArgs &a, const Mov
 // The critical team's signal that batch q - 2 (q - 1 when late) is in the
 // ring, which also means that the sums of that batch are used up; false: there
 // is no batch q.
-__device__ __forceinline__ bool ring_ready(const MinibatchArgs &a, MoverFlags &F, int par, bool first) {
+__device__ __forceinline__ bool ring_ready(const MinibatchArgs &a, MoverFlags &F, int par) {
   if (a.late) {
     bar_sync(kBarRing + par, kEarlyThreads);
-  } else if (!first) {
-    bar_sync(kBarRing + (par ^ 1), kEarlyThreads);
-    return F.last[par ^ 1] == 0;
+    return true;
   }
-  return true;
+  bar_sync(kBarRing + (par ^ 1), kEarlyThreads);
+  return F.last[par ^ 1] == 0;
 }
 
 // A lane of team N or P waits until the watching warp has seen `batches`
@@ -555,64 +568,313 @@ __device__ __forceinline__ void mover_watch(const MinibatchArgs &a, MoverFlags &
   }
 }
 
-// Team P: the sweepers' partials of the share, and the positions of batch
-// q + 2 (q + 1 when late) before it moves: N starts on a batch when the
-// critical team has finished the second (first) batch before it.
-__device__ __forceinline__ void mover_partials(const MinibatchArgs &a, const MoverSmem &S, MoverFlags &F, int m) {
-  const int pt = (int)threadIdx.x - (kCWarps + kNWarps + 1) * 32, w = pt >> 5, lane = pt & 31;
-  const int nb = a.nbatches, B = a.batch, slots = a.lag + 1;
-  const bool closed = nb == slots;  // every batch is in the ring
-  const int t0 = m * S.share;
-  int b = 0, slot = 0, tslot = 0, par = 0;
-  unsigned int q = 0;
-  for (bool first = true;; first = false) {
-    const int cnt = min(B, a.n - b * B), t1 = min(cnt, t0 + S.share);
-    int fb = b + S.tiles / 2;
-    if (fb >= nb) fb -= nb;
-    const int nbase = fb * B, ncnt = min(B, a.n - nbase);
-    if (lane == 0) wait_seen(F, q + 1u);
+// Where team N finds the neighbours of batch q = `b` of the iteration: batch
+// q - d holds vertex j as its vertex t; far: in a batch further back, in global
+// memory.
+struct Places {
+  int slot, slots, batch;
+  int w0, w1;  // batches q - slots .. q (cyclically) start at these ids (w1: where they wrap)
+  unsigned int span;
+  float inv_b;
+  int tile;  // where the tile holds the batch's positions before it moves (-1: they are in the ring)
+  __device__ __forceinline__ Places(const MinibatchArgs &a, const MoverSmem &S, int b, int slot_, int tslot)
+      : slot(slot_), slots(a.lag + 1), batch(a.batch) {
+    w0 = (b - slots) * batch;
+    w1 = b < slots ? (a.nbatches + b - slots) * batch : INT_MAX;
+    span = (slots + 1) * batch;
+    inv_b = 1.0f / (float)batch;
+    tile = a.nbatches == slots ? -1 : tslot * S.stride;
+  }
+  __device__ __forceinline__ bool far(int j) const {
+    return (unsigned int)(j - w0) >= span && (unsigned int)(j - w1) >= span;
+  }
+  // of a vertex that is not far
+  __device__ __forceinline__ void find(int j, int &d, int &t) const {
+    const unsigned int rel = (unsigned int)(j - w0) < span ? j - w0 : j - w1;
+    const int k = (int)(((float)rel + 0.5f) * inv_b);  // exact: rel < 2^16
+    d = slots - k;
+    t = (int)rel - k * batch;
+  }
+  __device__ __forceinline__ float2 target(const MoverSmem &S, int t) const {
+    return tile >= 0 ? S.tile[tile + t] : get_point(S.ring + slot * S.pairs, t);
+  }
+  // a position that the mover holds (d <= slots)
+  __device__ __forceinline__ float2 held(const MoverSmem &S, int d, int t) const {
+    if (d == 0) return target(S, t);
+    int ss = slot - d;
+    if (ss < 0) ss += slots;
+    return get_point(S.ring + ss * S.pairs, t);
+  }
+};
+
+// The row of vertex t of batch b when it is in the share that starts at t0, else an empty one.
+__device__ __forceinline__ void row_of(const MinibatchArgs &a, const MoverSmem &S, int b, int t, int t0, int &r0, int &r1) {
+  const int i = b * a.batch + t;
+  const bool valid = t < min(a.batch, t0 + S.share) && i < a.n;
+  r0 = valid ? __ldg(&a.eff_rowptr[i]) : 0;
+  r1 = valid ? __ldg(&a.eff_rowptr[i + 1]) : 0;
+}
+
+// A neighbour in the batch before, vertex jt of it, entry x of the row of
+// staged target t2: the critical team adds it.
+__device__ __forceinline__ void stage_near(const MoverSmem &S, int t2, int x, int jt) {
+  x &= kNear - 1;
+  S.near[t2 * kNear + x] = jt;
+  const unsigned int old = atomicOr(&S.mask[t2], 1u << x);
+  if ((old >> x) & 1u) atomicOr(&S.mask[t2], kNearMore);
+}
+
+// The corrections of a tile of targets in which a row is long (a row a lane,
+// [r0, r1), empty where there is no target, `total` entries in all; the first
+// target is the share's `off`-th): the seven warps share the tile's entries,
+// consecutive in memory, evenly, whatever rows they belong to.  A warp takes 64
+// entries at a time, two consecutive ones a lane, with the ids of the next on
+// their way.  While all 64 are of one row a lane adds its own until the row
+// ends; else a segmented scan over the lanes adds up the rows' parts.  `ready`
+// is called once, before the first position is read; false when it was.
+template <int kRep, typename Ready>
+__device__ __forceinline__ bool neighbours_flat(const MinibatchArgs &a, const MoverSmem &S, int b, int slot, int tslot,
+                                                int par, int off, int r0, int r1, int total, int w, Ready ready) {
+  const int lane = threadIdx.x & 31, parts = total > kFlatJoin ? kNWarps + kPWarps : kNWarps;
+  const Places P(a, S, b, slot, tslot);
+  // the tile's entries and the warp's (unsigned: a few past the end are compared too)
+  const unsigned int e0 = __shfl_sync(0xffffffffu, r0, 0), e1 = e0 + total;
+  const unsigned int each = (total + 64 * parts - 1) / (64 * parts) * 64;
+  unsigned int x0 = e0 + (w > kNWarps ? w - 1 : w) * each;
+  const unsigned int hi = min(e1, x0 + each);
+  int j[2];
+  auto fetch = [&](unsigned int x) {
+    x += 2 * lane;
+#pragma unroll
+    for (int u = 0; u < 2; u++) j[u] = x + u < hi ? __ldg(&a.eff_colids[x + u]) : -1;
+  };
+  fetch(x0);
+  // the rows that have entries, numbered through: lane k holds the first entry
+  // and the target of the k-th (those beyond: behind all entries)
+  unsigned int start = r1 > r0 ? r0 : e1;
+  int target = lane;
+  const unsigned int some = __ballot_sync(0xffffffffu, start < e1);
+  const int nrows = __popc(some);
+  if (some & (some + 1u)) {
+    target = (int)__fns(some, 0, lane + 1);
+    start = __shfl_sync(0xffffffffu, start, target & 31);
+    if (target < 0 || target > 31) start = e1;
+    target &= 31;
+  }
+  if (!ready()) return false;
+  auto rows = [&]() { return rows_of(a, S, par, off / kMoveTile) + w * kMoveTile; };
+  if (w < kNWarps) rows()[lane] = make_ulonglong2(0ull, 0ull);  // (team P's holds its partials)
+  __syncwarp();
+  auto append = [&](int t, Sum2 s) {  // one lane a target
+    ulonglong2 *at = rows() + t;
+    Sum2 z = {at->x, at->y};
+    z.merge(s);
+    *at = make_ulonglong2(z.hi, z.lo);
+  };
+  // the force of entry x of the row of target t, whose position is p where it
+  // is far; nothing where it is staged or no neighbour (an id outside the graph)
+  auto force = [&](bool far, float2 p, int t, int x) {
+    if (!far) {
+      const int id = __float_as_int(p.x);
+      if (id < 0) return make_float2(0.f, 0.f);
+      int d, jt;
+      P.find(id, d, jt);
+      if (d == 1 && !a.late) {
+        const int t2 = par * S.share + off + t;
+        stage_near(S, t2, x, jt);
+        atomicMin(&S.range[t2].x, x);
+        atomicMax(&S.range[t2].y, x);
+        return make_float2(0.f, 0.f);
+      }
+      p = P.held(S, d, jt);
+    }
+    return neighbour_force<kRep>(a.model, a.W, p, P.target(S, (int)blockIdx.x * S.share + off + t));
+  };
+  Sum2 acc = {0ull, 0ull};  // the lane's part of target `cur`
+  int cur = -1;
+  auto flush = [&]() {
+    if (cur < 0) return;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc.merge(acc.from_xor(o));
+    if (lane == 0) append(cur, acc);
     __syncwarp();
-    __threadfence_block();
+    acc.hi = acc.lo = 0ull;
+    cur = -1;
+  };
+#pragma unroll 1
+  for (; x0 < hi; x0 += 64) {
+    bool far[2];
+    float2 p[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const bool known = (unsigned int)j[u] < (unsigned int)a.n;
+      far[u] = known && P.far(j[u]);
+      if (far[u]) p[u] = __ldcg(&a.pos[j[u]]);
+      else p[u].x = __int_as_float(known ? j[u] : -1);
+    }
+    fetch(x0 + 64);
+    // the entries' rows: of those that start behind x0 a bit each
+    const int first = __popc(__ballot_sync(0xffffffffu, start <= x0)) - 1;  // the row of entry x0
+    const unsigned int rel = start - x0;
+    const unsigned int lower = __reduce_or_sync(0xffffffffu, rel - 1u < 31u ? 1u << rel : 0u);
+    const unsigned int upper = __reduce_or_sync(0xffffffffu, rel - 32u < 32u ? 1u << (rel - 32u) : 0u);
+    if ((lower | upper) == 0u) {  // all of one
+      const int t = __shfl_sync(0xffffffffu, target, first);
+      const int x = (int)(x0 + 2 * lane - __shfl_sync(0xffffffffu, start, first));
+      if (cur != t) {
+        flush();
+        cur = t;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const float2 f = force(far[u], p[u], t, x + u);
+        acc.add(f.x, f.y);
+      }
+      continue;
+    }
+    flush();
+    const unsigned long long starts = (unsigned long long)upper << 32 | lower;
+    int row[2], tgt[2];
+    Sum2 s[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      row[u] = first + __popcll(starts << (63 - 2 * lane - u));
+      tgt[u] = __shfl_sync(0xffffffffu, target, row[u]);
+      const float2 f = force(far[u], p[u], tgt[u], (int)(x0 + 2 * lane + u - __shfl_sync(0xffffffffu, start, row[u])));
+      s[u].hi = pack2(f.x, f.y);
+      s[u].lo = 0ull;
+    }
+    // the lane's last row, from its first entry on when that is of the same one
+    Sum2 run = s[1];
+    if (row[0] == row[1]) run.add(s[0].hi);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const Sum2 up = run.from_up(o);
+      if (__shfl_up_sync(0xffffffffu, row[1], o) == row[1] && lane >= o) run.merge(up);
+    }
+    const Sum2 up = run.from_up(1);
+    const int last = __shfl_up_sync(0xffffffffu, row[1], 1), next = __shfl_down_sync(0xffffffffu, row[0], 1);
+    if (row[0] != row[1]) {  // the row that ends with the first entry
+      if (lane > 0 && last == row[0]) s[0].merge(up);
+      append(tgt[0], s[0]);
+    }
+    __syncwarp();
+    // (places behind the last entry are of no row)
+    if ((lane == 31 || next != row[1]) && row[1] < nrows) append(tgt[1], run);
+    __syncwarp();
+  }
+  flush();
+  return true;
+}
+
+// Team P's part of a tile: the sweepers' partials of its targets.
+__device__ __forceinline__ Sum2 partial_sums(const MinibatchArgs &a, const MoverSmem &S, int w, int slot, int t, int t1) {
+  // lane: targets t = 2 (lane % 16) and the next of sweepers 2 w + lane / 16 + 16 k
+  const int lane = threadIdx.x & 31;
+  const float2 *col = a.part + (size_t)slot * a.sweepers * S.stride + t;
+  Sum2 f0 = {0ull, 0ull}, f1 = {0ull, 0ull};
+#pragma unroll 1
+  for (int s0 = w * 2 + (lane >> 4); s0 < a.sweepers; s0 += 2 * kPWarps * kPartLoads) {
+    float4 v[kPartLoads];
+#pragma unroll
+    for (int k = 0; k < kPartLoads; k++) {
+      v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < t1 && s0 + 2 * kPWarps * k < a.sweepers)
+        v[k] = __ldcg(reinterpret_cast<const float4 *>(&col[(size_t)(s0 + 2 * kPWarps * k) * S.stride]));
+    }
+#pragma unroll
+    for (int k = 0; k < kPartLoads; k++) {
+      f0.add(v[k].x, v[k].y);
+      f1.add(v[k].z, v[k].w);
+    }
+  }
+  __syncwarp();
+  // the other half-warp's sweepers: lanes 0-15 keep the first target, 16-31 the second
+  const bool up = lane & 16;
+  Sum2 keep = up ? f1 : f0;
+  const unsigned long long gh = __shfl_xor_sync(0xffffffffu, up ? f0.hi : f1.hi, 16);
+  const unsigned long long gl = __shfl_xor_sync(0xffffffffu, up ? f0.lo : f1.lo, 16);
+  keep.add(gh);
+  keep.lo = add2(keep.lo, gl);
+  return keep;
+}
+
+// Teams N and P, seven and eight warps.
+// P: the sweepers' partials of the share, and the positions of batch q + 2 (q + 1
+// when late) before it moves: N starts on a batch when the critical team has
+// finished the second (first) batch before it.
+// N: the neighbour corrections of the share, those in batch q - 1 staged
+// for the critical team (unless late: the ring holds it then).
+// A row is a lane's, of every seventh entry in each of N's warps, one position
+// in flight: 0.33 us for seven entries of the longest row.  Where that takes
+// longer than the tile's entries shared evenly (neighbours_flat: as 21 entries
+// of a row to start with and as 14 for every kFlatBlock) they are shared, above
+// kFlatJoin by P's warps too.  us a batch, by lanes only / by this rule: power-
+// law graphs of 100,000 vertices and mean degree 10, ids by weight 6.9 / 6.8,
+// ids shuffled 11.9 / 7.1, mean degree 40 shuffled 35 / 7.8; 10,000 vertices of
+// mean degree 65 shuffled 44 / 6.3; 4,096 vertices of 400 neighbours each 28 /
+// 7.8, a grid 3.39 / 3.43.  P looks at its tile's total only: with all rows'
+// lengths the grid took 3.48.
+// What N reads from global memory moved before batch q - lag - 1, which the
+// sweepers saw before they stored the partials of batch q - 1: it waits for
+// the watching warp to have seen those (long since).
+template <int kRep>
+__device__ __forceinline__ void mover_early(const MinibatchArgs &a, const MoverSmem &S, MoverFlags &F, int m) {
+  const int w = (int)(threadIdx.x >> 5) - kCWarps, lane = threadIdx.x & 31;  // N: 0 .., P: kNWarps + 1 ..
+  const bool sums = w > kNWarps;  // team P
+  const int t0 = m * S.share;
+  int b = 0, slot = 0;
+  // N: this lane's row; P: where the tile's rows start (lane 0) and end (the
+  // others); of the share's first tile a batch ahead
+  int r0, r1 = 0;
+  auto rows_of_tile = [&](int off) {
+    if (!sums) {
+      row_of(a, S, b, t0 + off + lane, t0, r0, r1);
+    } else {
+      const int base = b * a.batch, end = min(min(a.batch, a.n - base), min(t0 + S.share, t0 + off + kMoveTile));
+      r0 = __ldg(&a.eff_rowptr[base + (lane == 0 ? min(t0 + off, end) : end)]);
+    }
+  };
+  rows_of_tile(0);
+  for (unsigned int q = 0;; q++) {
+    const int par = (int)(q & 1), tslot = (int)q & (S.tiles - 1);
 #pragma unroll 1
     for (int ch = 0; ch < S.chunks; ch++) {
-      // lane: targets 2 (lane % 16) and the next of sweepers 2 w + lane / 16 + 16 k
-      const int t = t0 + ch * kMoveTile + 2 * (lane & 15);
-      const float2 *col = a.part + (size_t)slot * a.sweepers * S.stride + t;
-      float2 nt[2];
-      if (ch == 0) {
+      const int off = ch * kMoveTile;
+      if (ch > 0) rows_of_tile(off);
+      // waits for the positions (of the share's first tile: the others find them there)
+      auto ready = [&]() {
+        if (ch > 0 || sums) return true;
+        if (!ring_ready(a, F, par)) return false;
+        if (lane == 0) wait_seen(F, q);
+        __syncwarp();
+        __threadfence_block();
+        return true;
+      };
+      if (sums) {
+        const int pt = (int)threadIdx.x - (kCWarps + kNWarps + 1) * 32;
+        int nbase = -1, ncnt = 0;
+        float2 nt[2];
+        if (ch == 0) {
+          if (lane == 0) wait_seen(F, q + 1u);
+          __syncwarp();
+          __threadfence_block();
+          if (a.nbatches > a.lag + 1) {  // (else every batch is in the ring)
+            int fb = b + S.tiles / 2;
+            if (fb >= a.nbatches) fb -= a.nbatches;
+            nbase = fb * a.batch;
+            ncnt = min(a.batch, a.n - nbase);
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
-          const int x = pt + k * kPWarps * 32;
-          nt[k] = x < ncnt && !closed ? __ldcg(&a.pos[nbase + x]) : make_float2(0.f, 0.f);
+            for (int k = 0; k < 2; k++) {
+              const int x = pt + k * kPWarps * 32;
+              if (x < ncnt) nt[k] = __ldcg(&a.pos[nbase + x]);
+            }
+          }
         }
-      }
-      Sum2 f0 = {0ull, 0ull}, f1 = {0ull, 0ull};
-#pragma unroll 1
-      for (int s0 = w * 2 + (lane >> 4); s0 < a.sweepers; s0 += 2 * kPWarps * kPartLoads) {
-        float4 v[kPartLoads];
-#pragma unroll
-        for (int k = 0; k < kPartLoads; k++) {
-          v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (t < t1 && s0 + 2 * kPWarps * k < a.sweepers)
-            v[k] = __ldcg(reinterpret_cast<const float4 *>(&col[(size_t)(s0 + 2 * kPWarps * k) * S.stride]));
-        }
-#pragma unroll
-        for (int k = 0; k < kPartLoads; k++) {
-          f0.add(v[k].x, v[k].y);
-          f1.add(v[k].z, v[k].w);
-        }
-      }
-      __syncwarp();
-      // the other half-warp's sweepers: lanes 0-15 keep the first target, 16-31 the second
-      const bool up = lane & 16;
-      Sum2 keep = up ? f1 : f0;
-      const unsigned long long gh = __shfl_xor_sync(0xffffffffu, up ? f0.hi : f1.hi, 16);
-      const unsigned long long gl = __shfl_xor_sync(0xffffffffu, up ? f0.lo : f1.lo, 16);
-      keep.add(gh);
-      keep.lo = add2(keep.lo, gl);
-      if (ch == 0) {
-        if (!ring_ready(a, F, par, first)) return;
-        if (!closed) {
+        const int t = t0 + off + 2 * (lane & 15);
+        const Sum2 keep = partial_sums(a, S, w - kNWarps - 1, slot, t, min(min(a.batch, a.n - b * a.batch), t0 + S.share));
+        if (ch == 0) {
+          if (!ring_ready(a, F, par)) return;
           float2 *dst = S.tile + ((tslot + S.tiles / 2) & (S.tiles - 1)) * S.stride;
 #pragma unroll
           for (int k = 0; k < 2; k++) {
@@ -622,132 +884,83 @@ __device__ __forceinline__ void mover_partials(const MinibatchArgs &a, const Mov
 #pragma unroll 1
           for (int x = pt + 2 * kPWarps * 32; x < ncnt; x += kPWarps * 32) dst[x] = __ldcg(&a.pos[nbase + x]);
         }
-      }
-      rows_of(a, S, par, ch)[(kNWarps + 1 + w) * kMoveTile + 2 * (lane & 15) + (lane >> 4)] =
-          make_ulonglong2(keep.hi, keep.lo);
-    }
-    bar_arrive(kBarEarly + par, kEarlyThreads);
-    if (a.late && F.last[par]) return;
-    q++;
-    if (++b == nb) b = 0;
-    par ^= 1;
-    if (++slot == slots) slot = 0;
-    tslot = (tslot + 1) & (S.tiles - 1);
-  }
-}
-
-// Team N: the neighbour corrections of the share, those in batch q - 1 staged
-// for the critical team (unless late: the ring holds it then).  What
-// it reads from global memory moved before batch q - lag - 1, which the
-// sweepers saw before they stored the partials of batch q - 1: it waits for
-// the watching warp to have seen those (long since).
-template <int kRep>
-__device__ __forceinline__ void mover_neighbours(const MinibatchArgs &a, const MoverSmem &S, MoverFlags &F, int m) {
-  const int w = (int)(threadIdx.x >> 5) - kCWarps, lane = threadIdx.x & 31;
-  const int nb = a.nbatches, B = a.batch, slots = a.lag + 1;
-  const bool closed = nb == slots;
-  const float W = a.W, inv_b = 1.0f / (float)B;
-  const int t0 = m * S.share;
-  int b = 0, slot = 0, tslot = 0, par = 0;
-  // the next batch's row of this thread's first target
-  int r0 = 0, r1 = 0;
-  if (t0 + lane < min(min(B, a.n), t0 + S.share)) {
-    r0 = __ldg(&a.eff_rowptr[t0 + lane]);
-    r1 = __ldg(&a.eff_rowptr[t0 + lane + 1]);
-  }
-  unsigned int q = 0;
-  for (bool first = true;; first = false, q++) {
-    const int base = b * B, cnt = min(B, a.n - base);
-    const int t1 = min(cnt, t0 + S.share);
-    const int nbb = b + 1 == nb ? 0 : b + 1;
-    const int nbase = nbb * B, ncnt = min(B, a.n - nbase);
-    // batches q - slots .. q (cyclically) start at these ids
-    const int w0 = (b - slots) * B, w1 = (nb + b - slots) * B;
-#pragma unroll 1
-    for (int ch = 0; ch < S.chunks; ch++) {
-      const int t = t0 + ch * kMoveTile + lane;
-      const bool valid = t < t1;
-      if (ch > 0 && valid) {
-        r0 = __ldg(&a.eff_rowptr[base + t]);
-        r1 = __ldg(&a.eff_rowptr[base + t + 1]);
-      }
-      const int end = valid ? r1 : r0;
-      int e = r0 + w;
-      int j0 = e < end ? __ldg(&a.eff_colids[e]) : -1;
-      if (ch == 0) {
-        if (!ring_ready(a, F, par, first)) return;
-        if (lane == 0) wait_seen(F, q);
+        rows_of(a, S, par, ch)[w * kMoveTile + 2 * (lane & 15) + (lane >> 4)] = make_ulonglong2(keep.hi, keep.lo);
         __syncwarp();
-        __threadfence_block();
       }
-      auto target_at = [&](int x) {
-        return closed ? get_point(S.ring + slot * S.pairs, x) : S.tile[tslot * S.stride + x];
-      };
-      const float2 p = valid ? target_at(t) : make_float2(0.f, 0.f);
-      Sum2 f = {0ull, 0ull};
+      if (sums) {
+        if (__shfl_sync(0xffffffffu, r0, 31) - __shfl_sync(0xffffffffu, r0, 0) <= kFlatJoin) continue;
+        row_of(a, S, b, t0 + off + lane, t0, r0, r1);
+      }
+      bool flat = __any_sync(0xffffffffu, r1 - r0 > 5 * kNWarps);
+      int total = 0;
+      if (__builtin_expect(flat, 0)) {
+        total = __reduce_max_sync(0xffffffffu, r1) - __shfl_sync(0xffffffffu, r0, 0);
+        flat = __any_sync(0xffffffffu, r1 - r0 > (3 + 2 * ((total + kFlatBlock - 1) / kFlatBlock)) * kNWarps);
+      }
+      if (__builtin_expect(flat, 0)) {
+        if (!neighbours_flat<kRep>(a, S, b, slot, tslot, par, off, r0, r1, total, w, ready)) return;
+      } else if (!sums) {
+        int e = r0 + w;
+        int j0 = e < r1 ? __ldg(&a.eff_colids[e]) : -1;
+        if (!ready()) return;
+        const Places P(a, S, b, slot, tslot);
+        const float2 p = r0 < r1 ? P.target(S, t0 + off + lane) : make_float2(0.f, 0.f);
+        Sum2 f = {0ull, 0ull};
 #pragma unroll 1
-      for (int j1; e < end; j0 = j1, e += kNWarps) {
-        j1 = e + kNWarps < end ? __ldg(&a.eff_colids[e + kNWarps]) : -1;
-        // a list handed in on the device is not checked: other ids are no neighbours
-        if ((unsigned int)j0 >= (unsigned int)a.n) continue;
-        // batch q - d holds j0 as its vertex jt; d > slots: further back
-        int d = slots + 1, jt = 0;
-        int rel = j0 - w0;
-        if (rel < 0 || rel >= (slots + 1) * B) rel = b < slots ? j0 - w1 : -1;
-        if (rel >= 0) {
-          const int k = (int)(((float)rel + 0.5f) * inv_b);  // exact: rel < 2^16
-          d = slots - k;
-          jt = rel - k * B;
-        }
-        if (d == 1 && !a.late) {  // the batch before: the critical team's
-          const int x = (e - r0) & (kNear - 1), t2 = par * S.share + (t - t0);
-          S.near[t2 * kNear + x] = jt;
-          const unsigned int old = atomicOr(&S.mask[t2], 1u << x);
-          if ((old >> x) & 1u) atomicOr(&S.mask[t2], kNearMore);
-        } else {
+        for (int j1; e < r1; j0 = j1, e += kNWarps) {
+          j1 = e + kNWarps < r1 ? __ldg(&a.eff_colids[e + kNWarps]) : -1;
+          // a list handed in on the device is not checked: other ids are no neighbours
+          if ((unsigned int)j0 >= (unsigned int)a.n) continue;
           float2 pj;
-          if (d > slots) {
+          if (P.far(j0)) {
             pj = __ldcg(&a.pos[j0]);
-          } else if (d == 0) {
-            pj = target_at(jt);
           } else {
-            int ss = slot - d;
-            if (ss < 0) ss += slots;
-            pj = get_point(S.ring + ss * S.pairs, jt);
+            int d, jt;
+            P.find(j0, d, jt);
+            if (d == 1 && !a.late) {  // the batch before: the critical team's
+              stage_near(S, par * S.share + off + lane, e - r0, jt);
+              continue;
+            }
+            pj = P.held(S, d, jt);
           }
-          const float2 v = neighbour_force<kRep>(a.model, W, pj, p);
+          const float2 v = neighbour_force<kRep>(a.model, a.W, pj, p);
           f.add(v.x, v.y);
         }
+        rows_of(a, S, par, ch)[w * kMoveTile + lane] = make_ulonglong2(f.hi, f.lo);
       }
-      if (ch + 1 == S.chunks) {  // the next batch's row
-        const bool more = t0 + lane < min(ncnt, t0 + S.share);
-        r0 = more ? __ldg(&a.eff_rowptr[nbase + t0 + lane]) : 0;
-        r1 = more ? __ldg(&a.eff_rowptr[nbase + t0 + lane + 1]) : 0;
-      }
-      rows_of(a, S, par, ch)[w * kMoveTile + lane] = make_ulonglong2(f.hi, f.lo);
     }
     bar_arrive(kBarEarly + par, kEarlyThreads);
     if (a.late && F.last[par]) return;
-    b = nbb;
-    par ^= 1;
-    if (++slot == slots) slot = 0;
-    tslot = (tslot + 1) & (S.tiles - 1);
+    if (++b == a.nbatches) b = 0;
+    if (++slot > a.lag) slot = 0;
+    rows_of_tile(0);
   }
 }
 
 // A half-warp's sum over the neighbours of vertex i in the batch at `pbase`
-// when there are more than were staged: the row again.
+// when there are more than were staged: its row again, between the first and
+// the last of them where those were noted (`range`), four entries a lane in
+// flight.
 template <int kRep>
-__device__ __noinline__ float2 near_row(const MinibatchArgs &a, const float4 *prev, int pbase, int i, float2 pi) {
-  const int r1 = __ldg(&a.eff_rowptr[i + 1]), pcnt = min(a.batch, a.n - pbase);
+__device__ __noinline__ float2 near_row(const MinibatchArgs &a, const float4 *prev, int pbase, int i, float2 pi,
+                                        int2 range) {
+  const int r0 = __ldg(&a.eff_rowptr[i]), r1 = __ldg(&a.eff_rowptr[i + 1]);
+  const unsigned int pcnt = min(a.batch, a.n - pbase);
+  const int lo = range.x <= range.y ? range.x : 0, hi = range.x <= range.y ? range.y + 1 : r1 - r0;
   float2 f = make_float2(0.f, 0.f);
 #pragma unroll 1
-  for (int e = __ldg(&a.eff_rowptr[i]) + ((int)threadIdx.x & 15); e < r1; e += 16) {
-    const int jt = __ldg(&a.eff_colids[e]) - pbase;
-    if (jt < 0 || jt >= pcnt) continue;
-    const float2 g = neighbour_force<kRep>(a.model, a.W, get_point(prev, jt), pi);
-    f.x += g.x;
-    f.y += g.y;
+  for (int x = lo + ((int)threadIdx.x & 15); x < hi; x += 64) {
+    unsigned int jt[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      jt[u] = x + 16 * u < hi ? (unsigned int)__ldg(&a.eff_colids[r0 + x + 16 * u]) - (unsigned int)pbase : ~0u;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (jt[u] >= pcnt) continue;
+      const float2 g = neighbour_force<kRep>(a.model, a.W, get_point(prev, (int)jt[u]), pi);
+      f.x += g.x;
+      f.y += g.y;
+    }
   }
   return f;
 }
@@ -827,6 +1040,7 @@ __device__ __forceinline__ void mover_critical(const MinibatchArgs &a, const Mov
   const int t0 = m * S.share;
   bool stop = false, started = false;
   int b = 0, slot = 0, tslot = 0;
+  if (!a.late) bar_arrive(kBarRing + 1, kEarlyThreads);  // for batch 0 of the early teams: batch -2 is in the ring
   for (unsigned int q = 0;; q++) {
     const int par = (int)(q & 1);
     const int base = b * B;
@@ -918,7 +1132,7 @@ __device__ __forceinline__ void mover_critical(const MinibatchArgs &a, const Mov
           const float4 *prev = S.ring + (slot == 0 ? slots - 1 : slot - 1) * S.pairs;
           const int pbase = b == 0 ? (nb - 1) * B : base - B;
           if (mask & kNearMore) {
-            const float2 g = near_row<kRep>(a, prev, pbase, base + t, pi);
+            const float2 g = near_row<kRep>(a, prev, pbase, base + t, pi, S.range[x]);
             fx += g.x;
             fy += g.y;
           } else if ((mask >> (lane & 15)) & 1u) {
@@ -927,7 +1141,10 @@ __device__ __forceinline__ void mover_critical(const MinibatchArgs &a, const Mov
             fy += g.y;
           }
           __syncwarp();
-          if ((lane & 15) == 0 && mask != 0u) S.mask[x] = 0u;  // for batch q + 2
+          if ((lane & 15) == 0 && mask != 0u) {  // for batch q + 2
+            S.mask[x] = 0u;
+            S.range[x] = make_int2(INT_MAX, -1);
+          }
         }
       }
       // with N's and P's sums (a row per lane), a fixed tree over the 16 lanes
@@ -1025,6 +1242,7 @@ __device__ __forceinline__ void mover(const MinibatchArgs &a, unsigned char *sme
     S.tile = reinterpret_cast<float2 *>(S.moved + 2 * S.share);
     S.mask = reinterpret_cast<unsigned int *>(S.tile + S.tiles * S.stride);
     S.near = reinterpret_cast<int *>(S.mask + 2 * S.share);
+    S.range = reinterpret_cast<int2 *>(S.near + 2 * S.share * kNear);
     F.fail = 0;
     F.end = 0;
     F.seen = 0;
@@ -1053,7 +1271,10 @@ __device__ __forceinline__ void mover(const MinibatchArgs &a, unsigned char *sme
 #pragma unroll 1
       for (int t = tid; t < min(B, a.n - k * B); t += kThreads) S.tile[k * S.stride + t] = __ldcg(&a.pos[k * B + t]);
 #pragma unroll 1
-  for (int t = tid; t < 2 * S.share; t += kThreads) S.mask[t] = 0u;
+  for (int t = tid; t < 2 * S.share; t += kThreads) {
+    S.mask[t] = 0u;
+    if (!a.late) S.range[t] = make_int2(INT_MAX, -1);
+  }
 #pragma unroll 1
   for (int k = tid; k < (a.late ? 1 : 2) * S.chunks * kMoveTile; k += kThreads)
     S.rows[(k / kMoveTile * kRows + kNWarps) * kMoveTile + k % kMoveTile] = make_ulonglong2(0ull, 0ull);
@@ -1061,14 +1282,11 @@ __device__ __forceinline__ void mover(const MinibatchArgs &a, unsigned char *sme
   // no mover moves a vertex before every mover has its first positions
   if (tid == 0) red_add(&a.ctl->ready, 1u);
   if (tid < kCThreads) mover_critical<kRep>(a, S, F, m);
-  else if (tid < kCThreads + kNWarps * 32) mover_neighbours<kRep>(a, S, F, m);
-  else if (tid < kCThreads + (kNWarps + 1) * 32) {
-    if ((tid & 31) == 0) {
-      mover_watch(a, F);
-      F.gone = 1;
-    }
+  else if (tid / 32 != kCWarps + kNWarps) mover_early<kRep>(a, S, F, m);
+  else if ((tid & 31) == 0) {
+    mover_watch(a, F);
+    F.gone = 1;
   }
-  else mover_partials(a, S, F, m);
 }
 
 template <int kRep>
@@ -1117,7 +1335,7 @@ MinibatchShape shape_of(int n, int batch, int num_sms, int movers, int lag) {
   const size_t mover = (s.lag + 1) * (stride / 2) * sizeof(float4) +
                        (s.late ? 1 : 2) * chunks * kRows * kMoveTile * sizeof(ulonglong2) +
                        2 * share * sizeof(float4) + (s.late ? 2 : 4) * stride * sizeof(float2) +
-                       2 * share * (s.late ? 1 : kNear + 1) * sizeof(int);
+                       2 * share * (s.late ? 1 : kNear + 3) * sizeof(int);
   s.smem = std::max(sweeper, mover);
   s.part_bytes = (size_t)(s.lag + 1) * s.sweepers * stride * sizeof(float2);
   s.exchange_bytes = (size_t)kExchange * batch * sizeof(ulonglong2);
@@ -1132,23 +1350,32 @@ MinibatchShape shape_of(int n, int batch, int num_sms, int movers, int lag) {
 // 9.1 / 5.8 / 6.1; 30,000, batch 1,000 21.5 / 12.0 / 9.8; 90,000, batch 1,000
 // 25.1 / 24.5 / 26.8.  A lag of 2 was best or within 3 % everywhere (4,096
 // vertices 1 / 2 / 3 / 4: 3.7 / 2.9 / 3.1 / 3.3; 31,000: 7.8 / 5.8 / 5.9 /
-// 6.6); a smaller one where shared memory does not hold the batches.  False
-// when a slice does not fit a block's shared memory.
-bool minibatch_shape(int n, int batch, int num_sms, int smem_optin, MinibatchShape &s) {
+// 6.6); a smaller one where shared memory does not hold the batches.
+// Rows (`row`: their mean length, 0 if not known) come beside the chain, or on
+// top of it where they start a batch later: 1 us and 1.3 us for every 960
+// entries of a share.  That matters from some hundred entries a row on, so in a
+// dense graph up to 64 movers, down to four targets each, and every lag are
+// considered; elsewhere rows change nothing.  False when a slice does not fit
+// a block's shared memory.
+bool minibatch_shape(int n, int batch, double row, int num_sms, int smem_optin, MinibatchShape &s) {
   // the largest graph taken: 3.5 million vertices at batch 256, 2.3 million at 4,096
   if ((((n + num_sms - 1) / num_sms + 5) & ~3) * 8LL + 16LL * batch + 44032 > smem_optin) return false;
   bool found = false;
-  for (int lag = 2; lag >= 0 && !found; lag--) {
-    double best = 0.0;
-    for (int movers = kMaxMovers; movers >= 1; movers /= 2) {
-      if (movers > 1 && (movers > (batch + 7) / 8 || movers > num_sms / 4)) continue;
+  const bool dense = row >= kDense;
+  double best = 0.0;
+  for (int lag = 2; lag >= 0 && (!found || dense); lag--) {
+    for (int movers = dense ? kMaxMovers : kMaxMovers / 2; movers >= 1; movers /= 2) {
+      if (movers > 1 && (movers > (dense ? (batch + 3) / 4 : (batch + 7) / 8) || movers > num_sms / (dense ? 2 : 4)))
+        continue;
       const int share = mover_share(batch, movers);
       if (movers < 16 && share > kMoveTile && movers < num_sms / 4) continue;  // several passes a batch
       const MinibatchShape t = shape_of(n, batch, num_sms, movers, lag);
       if (t.smem + 1024 > (size_t)smem_optin) continue;
       const double chain = 2.6 + (double)std::max(t.lag, 1) * batch * share / 15600.0;
       const double sweep = 1.0 + (double)batch * n / (28500.0 * t.sweepers);
-      const double us = t.lag == 0 ? chain + sweep : std::max(chain, sweep);
+      const double rows = dense ? 1.0 + row * share / 740.0 : 0.0;
+      const double us = t.late ? (t.lag == 0 ? chain + sweep : std::max(chain, sweep)) + rows
+                               : std::max(std::max(chain, sweep), rows);
       if (!found || us < best) {
         best = us;
         s = t;
@@ -1186,7 +1413,7 @@ int minibatch_run(bl_ctx *ctx, int model, int batch, int iterations, double step
   int dev_smem_optin = 0;
   cudaDeviceGetAttribute(&dev_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
   MinibatchShape sh;
-  if (!minibatch_shape(n, batch, ctx->num_sms, dev_smem_optin, sh))
+  if (!minibatch_shape(n, batch, (double)ctx->g.nnz / n, ctx->num_sms, dev_smem_optin, sh))
     return bl_fail(ctx, -5, "graph too large for the shared-memory source slices of the minibatch path");
   void (*kernel)(MinibatchArgs) = unit_rep ? minibatch_kernel<REP_UNIT> : minibatch_kernel<REP_INV>;
   const int grid = sh.movers + sh.sweepers;
@@ -1319,7 +1546,7 @@ extern "C" int bl_minibatch_iteration_noalloc(int n, const int *d_rowptr, const 
   cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
   // same blocks and shared-memory sizing as the context path
   MinibatchShape sh;
-  if (!minibatch_shape(n, batch, std::min(num_sms, kNoAllocMaxGrid), smem_optin, sh)) return BL_ERR_TOO_LARGE;
+  if (!minibatch_shape(n, batch, 0.0, std::min(num_sms, kNoAllocMaxGrid), smem_optin, sh)) return BL_ERR_TOO_LARGE;
   const int grid = sh.movers + sh.sweepers;
   if (cudaFuncSetAttribute(minibatch_kernel<REP_INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem) !=
       cudaSuccess)
