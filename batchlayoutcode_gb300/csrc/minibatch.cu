@@ -1354,7 +1354,7 @@ MinibatchShape shape_of(int n, int batch, int num_sms, int movers, int lag) {
 // Rows (`row`: their mean length, 0 if not known) come beside the chain, or on
 // top of it where they start a batch later: 1 us and 1.3 us for every 960
 // entries of a share.  That matters from some hundred entries a row on, so in a
-// dense graph up to 64 movers, down to four targets each, and every lag are
+// dense graph up to 64 movers, down to two targets each, and every lag are
 // considered; elsewhere rows change nothing.  False when a slice does not fit
 // a block's shared memory.
 bool minibatch_shape(int n, int batch, double row, int num_sms, int smem_optin, MinibatchShape &s) {
@@ -1365,7 +1365,7 @@ bool minibatch_shape(int n, int batch, double row, int num_sms, int smem_optin, 
   double best = 0.0;
   for (int lag = 2; lag >= 0 && (!found || dense); lag--) {
     for (int movers = dense ? kMaxMovers : kMaxMovers / 2; movers >= 1; movers /= 2) {
-      if (movers > 1 && (movers > (dense ? (batch + 3) / 4 : (batch + 7) / 8) || movers > num_sms / (dense ? 2 : 4)))
+      if (movers > 1 && (movers > (dense ? (batch + 1) / 2 : (batch + 7) / 8) || movers > num_sms / (dense ? 2 : 4)))
         continue;
       const int share = mover_share(batch, movers);
       if (movers < 16 && share > kMoveTile && movers < num_sms / 4) continue;  // several passes a batch
