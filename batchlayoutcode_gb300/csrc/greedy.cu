@@ -245,6 +245,15 @@ __global__ void greedy_start_kernel(IterArgs a, const float2 *__restrict__ pos) 
   st_word(&a.buf[2 * (size_t)a.n + i], kNoPos);
 }
 
+// The positions after the last move, unless the run ended in an error: then
+// some were never written and the context keeps the start.
+__global__ void greedy_finish_kernel(int n, const float2 *__restrict__ moved, float2 *__restrict__ pos,
+                                     const DevStatus *st) {
+  if (!block_status_ok(st)) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) pos[i] = moved[i];
+}
+
 // The sum over the warp of one signed 64-bit value a lane (|v| < 2^62), by
 // three 27-bit limbs; false when it leaves 64 bits.
 __device__ __forceinline__ bool warp_sum_ll(long long v, long long &sum) {
@@ -668,8 +677,10 @@ int greedy_walk_run(bl_ctx *ctx, int batch, int iterations, double step0, double
                                            ctx->stream));
   bl_time_end(ctx, "greedy_iteration_kernel");
   ctx->launches++;
-  BL_CUDA(ctx, cudaMemcpyAsync(ctx->pos, a.buf + (size_t)(iterations % kPosBufs) * n, (size_t)n * sizeof(float2),
-                               cudaMemcpyDeviceToDevice, ctx->stream));
+  greedy_finish_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(n, a.buf + (size_t)(iterations % kPosBufs) * n,
+                                                                 ctx->pos, ctx->s.status);
+  ctx->launches++;
+  BL_CUDA(ctx, cudaGetLastError());
   if (want_energy) {
     if (int rc = energy_reduce(ctx, energy_out)) return rc;
   } else {

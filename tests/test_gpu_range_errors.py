@@ -67,3 +67,40 @@ def test_all_pairs(n, batch, kind):
         a.nCoordinates = xy
         assert a.run_resident(2, 3, batch, 1.2, 1.0) == e
         assert np.array_equal(a.nCoordinates, got)
+
+
+@pytest.mark.parametrize("kind", ["close", "nan"])
+@pytest.mark.parametrize("n,batch", [(60, 60), (300, 64), (5000, 256)])
+def test_greedy(n, batch, kind):
+    """Algo 5's first phase: the warps wait for position words that a failed
+    warp never writes.  The close pair is joined through two vertices, so that
+    a walk reaches one from the other."""
+    import batchlayoutcode_gb300 as B
+
+    B.build()
+    _, _, xy = layout(n)
+    i, j = 0, n // 2
+    u = np.concatenate([np.arange(n - 1), [i, 1, j - 1]])
+    v = np.concatenate([np.arange(1, n), [1, j - 1, j]])
+    keep = ~((u == i) & (v == j))
+    e = np.unique(np.concatenate([u[keep] * n + v[keep], v[keep] * n + u[keep]]))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(e // n, minlength=n))]).astype(np.int32)
+    ci = (e % n).astype(np.int32)
+    bad = spoiled(xy, kind)
+    with B.Algorithms(rp, ci) as a:
+        off, src, _ = a.greedy_walks()
+        assert kind == "nan" or j in src[off[i]:off[i + 1]] or i in src[off[j]:off[j + 1]]
+        for run in (lambda: a.greedy_iteration(batch, 1.0), lambda: a.run_resident(5, 20, batch, 1.2, 1.0)):
+            a.nCoordinates = bad
+            start = a.nCoordinates
+            with pytest.raises(B.BatchLayoutError) as err:
+                run()
+            assert err.value.code == BL_ERR_DEVICE_TIMEOUT
+            assert np.array_equal(a.nCoordinates, start, equal_nan=True)
+        a.nCoordinates = xy
+        e1 = a.run_resident(5, 6, batch, 1.2, 1.0)
+        got = a.nCoordinates
+    with B.Algorithms(rp, ci) as a:
+        a.nCoordinates = xy
+        assert a.run_resident(5, 6, batch, 1.2, 1.0) == e1
+        assert np.array_equal(a.nCoordinates, got)
