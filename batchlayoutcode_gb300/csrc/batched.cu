@@ -720,7 +720,7 @@ struct BatchedState {
   int num_graphs = 0, total_v = 0, max_small = 0, max_bh = 0, grid = 0, ws_grid = 0;
   size_t smem = 0;
   int threads = 512;  // of a block: 512 or 1024
-  double end_pairs = 0.0, end_wide = 0.0;  // estimated ends with either (graph_cost)
+  double end_pairs = 0.0, end_wide = 0.0;  // estimated ends with two blocks of 512 an SM, one of 1,024 (graph_cost)
   std::vector<BatchedGraph> gs;
   std::vector<int> order;
   int parts[3] = {0, 0, 0};  // autotuned source split per size bucket (0 = not tuned)
@@ -793,8 +793,15 @@ int batched_shape(bl_ctx *ctx, BatchedState &B, int batch) {
   };
   if (need(512) + 2048 > (size_t)smem_optin)
     return bl_fail(ctx, BL_ERR_TOO_LARGE, "a minibatch graph is too large for one block's shared memory");
-  // 512 or 1,024 threads: the schedule that ends first
-  const int threads = need(1024) + 2048 <= (size_t)smem_optin && B.end_wide < B.end_pairs ? 1024 : 512;
+  // 512 or 1,024 threads: the schedule that ends first; the larger where the
+  // shared memory of an all-pairs graph (above some 13,500 vertices) leaves an
+  // SM one block of 512 anyway (15,000 Barnes-Hut graphs of 3,000 vertices and an
+  // all-pairs one of 14,000, two iterations: 49.7 ms by 512, 43.7)
+  int pairs = 0;
+  BL_CUDA(ctx, cudaFuncSetAttribute(batched_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need(512)));
+  BL_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pairs, batched_kernel<512>, 512, need(512)));
+  const bool wide = need(1024) + 2048 <= (size_t)smem_optin && (pairs < 2 || B.end_wide < B.end_pairs);
+  const int threads = wide ? 1024 : 512;
   const void *kernel = threads == 1024 ? (const void *)batched_kernel<1024> : (const void *)batched_kernel<512>;
   const size_t smem = need(threads);
   BL_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -962,7 +969,7 @@ int bl_batched_prepare(bl_ctx *ctx, int num_graphs, const int *vertex_offset, co
     if (erp.size() > (size_t)INT_MAX) return bl_fail(ctx, BL_ERR_TOO_LARGE, "too many graphs");
   }
   if (eci.empty()) eci.push_back(0);
-  // largest graphs first (work grows like n^2 for minibatch graphs)
+  // costliest graphs first
   B->order.resize(num_graphs);
   for (int g = 0; g < num_graphs; g++) B->order[g] = g;
   std::stable_sort(B->order.begin(), B->order.end(),
