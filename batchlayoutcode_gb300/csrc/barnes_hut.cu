@@ -1473,15 +1473,16 @@ __device__ __forceinline__ float4 hub_unmoved_attraction(int v, const int *__res
                                                          float W) {
   const int lane = threadIdx.x & 31;
   const float2 pv = pold[v];
-  const int batch_lo = (v / batch) * batch, e0 = rowptr[v], e1 = rowptr[v + 1];
-  auto column = [&](int e) { return e < e1 ? colids[e] : -1; };
+  const int batch_lo = (v / batch) * batch;
+  const unsigned int e0 = rowptr[v], e1 = rowptr[v + 1];  // (unsigned: two chunks past the end are compared too)
+  auto column = [&](unsigned int e) { return e < e1 ? colids[e] : -1; };
   auto position = [&](int j) { return j >= batch_lo ? pold[j] : pv; };
   float hx = 0.f, lx = 0.f, hy = 0.f, ly = 0.f;
-  int j = column(e0 + lane), jn = e1 - e0 > 32 ? column(e0 + 32 + lane) : -1;
+  int j = column(e0 + lane), jn = column(e0 + 32 + lane);
   float2 p = position(j);
-  for (int e = e0; e < e1; e += 32) {  // positions one chunk ahead, columns two
+  for (unsigned int e = e0; e < e1; e += 32) {  // positions one chunk ahead, columns two
     const float2 pn = position(jn);
-    const int j2 = e1 - e > 64 ? column(e + 64 + lane) : -1;
+    const int j2 = column(e + 64 + lane);
     const float dx = p.x - pv.x, dy = p.y - pv.y;
     const float sc = W * sqrtf(fmaf(dx, dx, dy * dy));
     const unsigned int m = __ballot_sync(0xffffffffu, j >= batch_lo);  // past the row's end j is -1

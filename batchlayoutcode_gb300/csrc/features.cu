@@ -201,7 +201,7 @@ __device__ __forceinline__ void bfs_block(const BlockBfsArgs &a, BlockBfsSmem &S
     const unsigned short d = (unsigned short)min(L, 65534);
     for (int i0 = 0; i0 < 2 * count; i0 += kBlockThreads) {
       const int idx = (i0 + tid) >> 1;
-      int e = 0, e1 = 0;
+      unsigned int e = 0, e1 = 0;  // (unsigned: places behind the last of 2^31 - 1 entries are compared too)
       if (idx < count) {
         const int u = v0 + q[idx];
         e = __ldg(&a.rowptr[u]) + (tid & 1);
@@ -501,15 +501,15 @@ __global__ void mds_project_kernel(ProjectArgs a) {
   const int e0 = a.rowptr[v], e1 = a.rowptr[v + 1];
   const int deg = e1 - e0;
   float m = 0.f;
-  for (int e = e0; e < e1; e += 8) {  // eight neighbours' loads together, added in row order
+  for (int e = 0; e < deg; e += 8) {  // eight neighbours' loads together, added in row order
     int u[8], d[8];
 #pragma unroll
-    for (int q = 0; q < 8; q++) u[q] = e + q < e1 ? a.colids[e + q] : v;
+    for (int q = 0; q < 8; q++) u[q] = e + q < deg ? a.colids[e0 + e + q] : v;
 #pragma unroll
     for (int q = 0; q < 8; q++) d[q] = a.rowptr[u[q] + 1] - a.rowptr[u[q]];
 #pragma unroll
     for (int q = 0; q < 8; q++)
-      if (e + q < e1) m += log2f(1.0f + (float)d[q]);
+      if (e + q < deg) m += log2f(1.0f + (float)d[q]);
   }
   f[12] = log2f(1.0f + (float)deg);
   f[13] = 1.0f / (1.0f + (float)deg);

@@ -111,22 +111,23 @@ __global__ void __launch_bounds__(32 * kFitWarps) scale_fit_kernel(int n, const 
     first[warp][lane] = e0;
     if (lane == 31) first[warp][32] = e1;
     __syncwarp();
-    const int base = first[warp][0], end = first[warp][32];
+    // (unsigned: a step past the last of 2^31 - 1 entries is compared too)
+    const unsigned int base = first[warp][0], end = first[warp][32];
     double ax = 0.0, ay = 0.0;
-    for (int c0 = base; c0 < end; c0 += kFitEntries) {
-      const int c1 = min(c0 + kFitEntries, end);
-      for (int e = c0 + lane; e < c1; e += 32) {
+    for (unsigned int c0 = base; c0 < end; c0 += kFitEntries) {
+      const unsigned int c1 = min(c0 + kFitEntries, end);
+      for (unsigned int e = c0 + lane; e < c1; e += 32) {
         int lo = 0;  // the row of e: first[lo] <= e < first[lo + 1]
 #pragma unroll
         for (int h = 16; h > 0; h >>= 1)
-          if (first[warp][lo + h] <= e) lo += h;
+          if ((unsigned int)first[warp][lo + h] <= e) lo += h;
         const float2 p = pos[v0 + lo], q = pos[colids[e]];
         const double dx = (double)q.x - p.x, dy = (double)q.y - p.y;
         const double sc = (double)W * sqrt(dx * dx + dy * dy);
         term[warp][e - c0] = make_double2(sc * dx, sc * dy);
       }
       __syncwarp();
-      for (int e = max(e0, c0); e < min(e1, c1); e++) {
+      for (unsigned int e = max((unsigned int)e0, c0); e < min((unsigned int)e1, c1); e++) {
         const double2 t = term[warp][e - c0];
         ax += t.x;
         ay += t.y;
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(kFitThreads) join_colids_kernel(FitArgs a) {
   const int4 c = a.echunk[blockIdx.x];
   const int v0 = a.voff[c.x], n = a.voff[c.x + 1] - v0;
   bool bad = false;
-  for (int e = c.y + threadIdx.x; e < c.z; e += kFitThreads) {
+  for (unsigned int e = c.y + threadIdx.x; e < (unsigned int)c.z; e += kFitThreads) {
     const int u = a.colids[e];
     bad |= u < 0 || u >= n;
     a.colids[e] = v0 + u;
@@ -252,18 +253,18 @@ __global__ void __launch_bounds__(kFitThreads) join_colids_kernel(FitArgs a) {
 __global__ void __launch_bounds__(kFitThreads) fit_length_kernel(FitArgs a) {
   const int4 c = a.echunk[blockIdx.x];
   constexpr int kRun = kEdgeChunk / kFitThreads;  // consecutive entries of a thread
-  const int e0 = c.y + threadIdx.x * kRun, e1 = min(e0 + kRun, c.z);
+  const unsigned int e0 = c.y + threadIdx.x * kRun, e1 = min(e0 + kRun, (unsigned int)c.z);
   double s[1] = {0.0};
   if (e0 < e1) {
     int lo = a.voff[c.x], hi = a.voff[c.x + 1];  // the row of e0: rowptr[lo] <= e0 < rowptr[hi]
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if (a.rowptr[mid] <= e0) lo = mid;
+      if ((unsigned int)a.rowptr[mid] <= e0) lo = mid;
       else hi = mid;
     }
-    int end = a.rowptr[lo + 1];
+    unsigned int end = a.rowptr[lo + 1];
     double2 p = a.layout[lo];
-    for (int e = e0; e < e1; e++) {
+    for (unsigned int e = e0; e < e1; e++) {
       while (e >= end) {
         lo++;
         end = a.rowptr[lo + 1];

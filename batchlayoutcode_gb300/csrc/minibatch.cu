@@ -900,15 +900,17 @@ __device__ __forceinline__ void mover_early(const MinibatchArgs &a, const MoverS
       if (__builtin_expect(flat, 0)) {
         if (!neighbours_flat<kRep>(a, S, b, slot, tslot, par, off, r0, r1, total, w, ready)) return;
       } else if (!sums) {
-        int e = r0 + w;
-        int j0 = e < r1 ? __ldg(&a.eff_colids[e]) : -1;
+        // (unsigned: places behind the last of 2^31 - 1 entries are compared too)
+        unsigned int e = r0 + w;
+        const unsigned int end = r1;
+        int j0 = e < end ? __ldg(&a.eff_colids[e]) : -1;
         if (!ready()) return;
         const Places P(a, S, b, slot, tslot);
         const float2 p = r0 < r1 ? P.target(S, t0 + off + lane) : make_float2(0.f, 0.f);
         Sum2 f = {0ull, 0ull};
 #pragma unroll 1
-        for (int j1; e < r1; j0 = j1, e += kNWarps) {
-          j1 = e + kNWarps < r1 ? __ldg(&a.eff_colids[e + kNWarps]) : -1;
+        for (int j1; e < end; j0 = j1, e += kNWarps) {
+          j1 = e + kNWarps < end ? __ldg(&a.eff_colids[e + kNWarps]) : -1;
           // a list handed in on the device is not checked: other ids are no neighbours
           if ((unsigned int)j0 >= (unsigned int)a.n) continue;
           float2 pj;

@@ -221,26 +221,27 @@ __global__ void __launch_bounds__(kT) mpnn_fwd_kernel(FwdArgs a) {
     constexpr int RPG = kLongChunk / kGroups > 0 ? kLongChunk / kGroups : 1, kChunk = kLongChunk;
     for (int x = 0; x < s_nlong; x++) {
       const int row = s_long[x], u = vertex(row);
-      const int b0 = a.rowptr[u], b1 = a.rowptr[u + 1];
+      // (unsigned: a chunk past the last of 2^31 - 1 entries is compared too)
+      const unsigned int b0 = a.rowptr[u], b1 = a.rowptr[u + 1];
       uint4 q[RPG];
-      auto load = [&](int e) {
+      auto load = [&](unsigned int e) {
 #pragma unroll
         for (int k = 0; k < RPG; k++) {
-          const int y = e + gr * RPG + k;
+          const unsigned int y = e + gr * RPG + k;
           q[k] = gr * RPG + k < kChunk && y < b1 ? reinterpret_cast<const uint4 *>(a.hin + (size_t)__ldg(&a.colids[y]) * DIN)[gl]
                         : make_uint4(0, 0, 0, 0);
         }
       };
       float sum = 0.f;
       load(b0);
-      for (int e = b0; e < b1; e += kChunk) {
+      for (unsigned int e = b0; e < b1; e += kChunk) {
 #pragma unroll
         for (int k = 0; k < RPG; k++)
           if (gr * RPG + k < kChunk) *reinterpret_cast<uint4 *>(&s_rows[gr * RPG + k][gl * 8]) = q[k];
         __syncthreads();
         load(e + kChunk);
         if (tid < DIN) {
-          const int m = min(kChunk, b1 - e);
+          const int m = min((unsigned int)kChunk, b1 - e);
 #pragma unroll 8
           for (int k = 0; k < m; k++) sum += __bfloat162float(s_rows[k][tid]);
         }
@@ -684,24 +685,24 @@ __global__ void __launch_bounds__(kGatherVerts * 16) mpnn_gather_kernel(
   constexpr int RPG = kGatherChunk / kGatherVerts;
   for (int x = 0; x < s_nlong; x++) {
     const int u = vertex(s_long[x]);
-    const int r0 = rowptr[u], r1 = rowptr[u + 1];
+    const unsigned int r0 = rowptr[u], r1 = rowptr[u + 1];
     float4 g[RPG];
-    auto load = [&](int e) {
+    auto load = [&](unsigned int e) {
 #pragma unroll
       for (int k = 0; k < RPG; k++) {
-        const int y = e + grp * RPG + k;
+        const unsigned int y = e + grp * RPG + k;
         if (y < r1) g[k] = reinterpret_cast<const float4 *>(G + (size_t)__ldg(&colids[y]) * 64)[c];
       }
     };
     load(r0);
     float4 t = reinterpret_cast<const float4 *>(P + (size_t)u * 64)[c];
-    for (int e = r0; e < r1; e += kGatherChunk) {
+    for (unsigned int e = r0; e < r1; e += kGatherChunk) {
 #pragma unroll
       for (int k = 0; k < RPG; k++) s_rows[grp * RPG + k][c] = g[k];
       __syncthreads();
       load(e + kGatherChunk);
       if (grp == 0) {
-        const int m = min(kGatherChunk, r1 - e);
+        const int m = min((unsigned int)kGatherChunk, r1 - e);
 #pragma unroll 8
         for (int k = 0; k < m; k++) add(t, s_rows[k][c]);
       }
