@@ -591,9 +591,9 @@ __device__ __forceinline__ int kdelta(const u64 *__restrict__ K, int n, int i, i
 // length, left; right, parent, -, -}: its own words are two stores of one
 // sector, the parent word is written by the parent's thread.  range and dlt
 // repeat the first words for the kernels that want only those; leaf_parent[k]
-// is the parent of leaf k.  (With the words stored one by one and a child and a
-// parent array beside them the kernel took 33 us for 1,000,000 points and 76
-// for 3,000,000, so 30 and 72.)
+// is the parent of leaf k.  Bound by issue (the searches): 1,000,000 points 30
+// us, 3,000,000 72; with the words stored one by one and a child and a parent
+// array beside them 33 and 76.
 __global__ void radix_tree_kernel(const u64 *__restrict__ K, int n, int2 *range, int *dlt, int *leaf_parent,
                                   int *bnode) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -604,9 +604,8 @@ __global__ void radix_tree_kernel(const u64 *__restrict__ K, int n, int2 *range,
   const int dmin = min(dnext, dprev);
   // The searches ask whether a prefix with key i is longer than m bits: for
   // m < 64 whether the keys' difference is below 2^(63 - m), one comparison
-  // where the prefix itself takes a count, a select and the tie's rule (the
-  // searches are bound by issue: 1,000,000 points 41 us, so 33; 3,000,000 101,
-  // so 76).
+  // where the prefix itself takes a count, a select and the tie's rule (with
+  // which 1,000,000 points took 8 us more, 3,000,000 25).
   auto longer = [&](int q, int m, u64 lim) {
     return m < 64 ? (unsigned int)q < (unsigned int)n && (ki ^ K[q]) <= lim : kdelta(K, n, i, q) > m;
   };
@@ -1458,13 +1457,14 @@ struct TraverseArgs {
 // sort and the tree; the walk then adds minus the repulsion.
 // A thread takes a row of up to kHubRow neighbours, a warp a longer one: its
 // lanes fetch 32 neighbours at once and form the factors, which every lane
-// then multiplies and adds in CSR order, so the sum is the thread's bit for bit.  A thread alone
-// is bound by its fetches (two dependent L2 round trips per four neighbours):
-// with the longest row at 633 neighbours of 100,003 vertices the
-// kernel took 155 us, longer than the sort and the tree beside it; so 49.  The vertices with long rows often have
-// neighbouring ids, so a block takes groups of 8 vertices from all over the
-// range (8 keep the rows' offsets and the results in whole sectors) and its
-// warps share the long rows among them.
+// then multiplies and adds in CSR order, so the sum is the thread's bit for bit.
+// A thread alone is bound by its fetches, two dependent L2 round trips per four
+// neighbours: 100,003 vertices, the longest row 633 neighbours, 155 us by
+// threads only (longer than the sort and the tree beside it), 49 with the
+// warps.  The vertices with long rows often have neighbouring ids, so a block
+// takes groups of 8 vertices from all over the range (8 keep the rows' offsets
+// and the results in whole sectors) and its warps share the long rows among
+// them.
 constexpr int kHubRow = 32;
 constexpr int kAttractThreads = 256;
 
@@ -1627,12 +1627,12 @@ __device__ __forceinline__ void sweep_load(const SweepArgs &a, int t, SweepVerte
 // each lane loads the words of its next four neighbours (only the first while
 // it waits for that one), takes those that are there and, with the last,
 // publishes its own position.  So a row of many moved neighbours costs a round
-// trip per four of them, all lanes at once; a lane that waited alone and then
-// loaded its neighbours one by one held up the warp and every level after it
-// (100,003 vertices
-// of a power-law graph, 32 levels, up to 22 moved neighbours: the sweep
-// 118 us, so 94; 1,000,000 of a geometric one: 77 us, so 58).  The wait is bounded; false when it ran out or another thread
-// recorded an error (the same in every lane).
+// trip per four of them, all lanes at once; a lane that waits alone and then
+// loads its neighbours one by one holds up the warp and every level after it
+// (the sweep of 100,003 vertices of a power-law graph, 32 levels, up to 22 moved
+// neighbours, 118 us that way, 94 this; of 1,000,000 of a geometric one 77 and
+// 58).  The wait is bounded; false when it ran out or another thread recorded
+// an error (the same in every lane).
 __device__ __forceinline__ bool sweep_group(const SweepArgs &a, const SweepVertex &v, bool has) {
   float hx = v.f.x, hy = v.f.y, lx = v.f.z, ly = v.f.w;
   int c[4] = {v.c[0], v.c[1], v.c[2], v.c[3]};
@@ -1695,10 +1695,11 @@ __device__ __forceinline__ bool sweep_group(const SweepArgs &a, const SweepVerte
 // unfinished slot can always proceed, so the sweep cannot deadlock.  A thread
 // loads its next slot's vertex data before it waits on the current slot's
 // neighbours.  Bound by the levels: each is a round trip to see the position,
-// the update and the store.  The groups' first slots are a table made with the
-// levels: finding them here (a walk over the levels' ends, 64-bit remainders)
-// took 22 us of the 94 and 10 of the 58.  Blocks of 512 threads are 4 us faster at
-// 100,003 vertices, 11 slower at 1,000,000 and 45 at 3,000,000.
+// the update and the store; 72 us for the 100,003 vertices above, 48 for the
+// 1,000,000.  The groups' first slots are a table made with the levels: found
+// here (a walk over the levels' ends, 64-bit remainders) they took 22 and 10 us
+// more.  Blocks of 512 threads are 4 us faster at 100,003 vertices, 11 slower
+// at 1,000,000 and 45 at 3,000,000.
 __global__ void __launch_bounds__(kSweepThreads, 1) sweep_kernel(SweepArgs a) {
   if (!block_status_ok(a.st)) return;
   const int W = gridDim.x * (blockDim.x >> 5);

@@ -83,6 +83,8 @@ struct KeyFrame {
   float ch, cl;
 };
 
+static_assert(sizeof(KeyFrame) <= 12 * sizeof(double), "kept behind the four words of the frame");
+
 __device__ __forceinline__ KeyFrame key_frame(double minX, double minY, double maxmin) {
   KeyFrame f;
   f.minX = minX;
@@ -103,7 +105,6 @@ __device__ __forceinline__ KeyFrame key_frame(double minX, double minY, double m
 // couple of ulp, so unless it lies within 8 ulp of an integer its truncation
 // equals the truncation of the correctly rounded quotient.  Otherwise the
 // exact division decides.
-static_assert(sizeof(KeyFrame) <= 12 * sizeof(double), "kept behind the four words of the frame");
 static __device__ __noinline__ unsigned int quantise_exact(float v, double mn, double maxmin, double inv) {
   if (!(maxmin > 0.0)) return 0u;
   const double a = __dmul_rn(4294967295.0, __dsub_rn(f2d_int(v), mn));
@@ -129,8 +130,8 @@ static __device__ __noinline__ unsigned int quantise_exact(float v, double mn, d
 // Unless the fraction is within 2^-11 of an integer the truncation is
 // therefore the reference's; there (two points in 1,000), below 1 and at the
 // upper end the FP64 form decides.  FP64 runs at 2 lanes a cycle and SM on
-// this part: with three FP64 operations a coordinate the keys of a million
-// points took 19 us, so they take 5.
+// this part: the keys of a million points take 5 us, with three FP64 operations
+// a coordinate 19.
 __device__ __forceinline__ unsigned int quantise(float v, float mn, double mnd, const KeyFrame &f) {
   const float d = __fsub_rn(v, mn);
   const float t = __fsub_rn(d, v);

@@ -304,13 +304,12 @@ __device__ __forceinline__ void hops(const unsigned short *dist, int v, unsigned
   }
 }
 
-// per block: largest finite distance per pivot
 // The pivot MDS of a slice of graphs: blockIdx.y is the graph of the slice,
 // mds_blocks(n) blocks of blockIdx.x work on its n vertices.  Everything
 // between the distances and the 16 x 16 eigenproblem stays on the device, all
-// graphs at once: with a host reduction (and its synchronisation) after each
-// of three kernels a graph, twelve graphs took 2.3 ms, so they take 1.0 (the
-// eigenproblems included).
+// graphs at once: 1.0 ms for twelve graphs, the eigenproblems included (2.3
+// with a host reduction and its synchronisation after each of three kernels a
+// graph).
 constexpr int kMdsBlocks = 256;
 constexpr int kMdsSlice = 64;        // graphs a launch: bounds the partials' memory
 constexpr int kGram = kP * (kP + 1) / 2;

@@ -194,8 +194,10 @@ constexpr float kFix = 268435456.0f;
 constexpr double kFixInv = 1.0 / 268435456.0;
 constexpr float kFixLimit = 17179869184.0f;
 
-// Batches above this were never taken (they did not fit the shared-memory
-// sums of an earlier form); callers get the same error.
+// Batches above some 7,200 (this many bytes a vertex within a block's shared
+// memory) are refused.  Nothing here needs the bound; algo 5's second phase
+// takes 4,096 at most, and a run it cannot end is better refused before the
+// first phase has moved anything.
 constexpr size_t kBatchBytes = 2 * sizeof(long long) + 2 * sizeof(float2);
 
 // A position not yet written: both coordinates NaN, all bits set.
@@ -287,8 +289,9 @@ __device__ __forceinline__ bool keep_waiting(DevStatus *st, unsigned long long &
 // written yet.  Every word a task waits for is written by a task before it in
 // the order and all blocks are resident, so the first unfinished task can
 // always proceed.  The terms whose words are there are added first, so that
-// only the latest source's term lies between its move and this one.  The lanes' fixed-point sums meet in warp reductions and the
-// new position is one 8-byte store that later tasks see as ready.
+// only the latest source's term lies between its move and this one.  The lanes'
+// fixed-point sums meet in warp reductions and the new position is one 8-byte
+// store that later tasks see as ready.
 // Positions after m moves live in array m % 5.  A task of iteration it clears
 // its word of array (it + 3) % 5, whose old content (after it - 2 moves) only
 // iterations it - 3 and it - 2 read: a warp enters iteration it when all warps
@@ -297,9 +300,9 @@ __device__ __forceinline__ bool keep_waiting(DevStatus *st, unsigned long long &
 // Bound by the dependency chain across the batches (73 links an iteration on
 // the power-law graph below; a link is a load that sees the position, 600-700
 // cycles, the term, the reductions and the store) and, with few links, by
-// instruction issue.  One cluster of 16 blocks with a barrier per batch took
-// 2.6 us a batch whatever it depended on and left 136 SMs idle: nine
-// iterations of 100,000 vertices took 9,200 us, so 1,070 (power law) and 530
+// instruction issue.  One cluster of 16 blocks with a barrier a batch takes
+// 2.6 us a batch whatever it depends on and leaves 136 SMs idle: nine
+// iterations of 100,000 vertices 9,200 us, this way 1,070 (power law) and 530
 // (geometric).  28 warps a block: 32 spill registers, 24 and 16 take 3 and
 // 11 % longer.
 __global__ void __launch_bounds__(kIterThreads, 1) greedy_iteration_kernel(IterArgs a) {

@@ -46,7 +46,7 @@ __global__ void residual_start_kernel(const float *__restrict__ net, const float
 // per block: sum over the CSR entries of |p_v - p_u| (each edge twice).  Bound
 // by FP64, so the entries are dealt out in runs of kEdgeRun instead of by row:
 // a warp with a row a lane works as long as its longest row (400,000 vertices
-// of a geometric graph: 205 us, so 81).
+// of a geometric graph: 205 us by rows, 81 by runs).
 constexpr int kEdgeRun = 8;
 
 __global__ void edge_length_kernel(int n, const int *__restrict__ rowptr, const int *__restrict__ colids,
@@ -90,9 +90,8 @@ __global__ void edge_length_kernel(int n, const int *__restrict__ rowptr, const 
 // Barnes-Hut sum of unit vectors towards the cells (BarnesHut.h:69-86).
 // Bound by FP64: a warp takes 32 consecutive rows and forms the terms of their
 // entries a lane each, kFitEntries at a time, so that the root and the products
-// run in full warps; a lane then adds its row's terms in row order.  With the
-// whole row a lane's, 400,000 vertices of a geometric graph took 272 us, so
-// 155.
+// run in full warps; a lane then adds its row's terms in row order: 155 us for
+// 400,000 vertices of a geometric graph, 272 with the whole row a lane's.
 constexpr int kFitEntries = 192, kFitWarps = 8;
 
 __global__ void __launch_bounds__(32 * kFitWarps) scale_fit_kernel(int n, const int *__restrict__ rowptr,
@@ -176,8 +175,8 @@ __global__ void f32_to_bf16_kernel(const float *__restrict__ in, __nv_bfloat16 *
 // graph's shape y = features 0 and 1.  A block takes a chunk of one graph, up
 // to kFitChunk vertices or kEdgeChunk CSR entries (entries, not rows: the long
 // rows of a power-law graph are neighbours).  Sums in FP64 in a fixed order
-// (threads, warps, then chunks).  On the host the joined CSR took 3.5 ms for twelve
-// graphs of 207,796 vertices and the fit with its copies 15.7: so 0.8 and 0.2.
+// (threads, warps, then chunks).  Twelve graphs of 207,796 vertices: the joined
+// CSR 0.8 ms, the fit 0.2 (on the host 3.5, and 15.7 with its copies).
 constexpr int kFitThreads = 256;
 constexpr int kFitChunk = 512;
 constexpr int kEdgeChunk = 4096;

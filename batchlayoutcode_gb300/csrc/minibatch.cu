@@ -27,19 +27,19 @@
 // * Movers (the first M blocks) each move a fixed share of every batch.
 //   Three teams work side by side: P adds up the sweepers' partials, N the
 //   neighbour corrections (remove the repulsion, add the model's attraction
-//   -- the decomposition the reference's own algo 7 uses, :553-579), and the
-//   critical team the pairs with the last `lag` batches; it receives the batch
+//   -- the decomposition the reference's own algo 7 uses, :553-579; of long rows
+//   with P), and the critical team the pairs with the last `lag` batches; it receives the batch
 //   before as 8-byte words {coordinate, batch tag} the other movers write (one
 //   L2 hop, no barrier), moves its share and publishes it the same way.
 //
-// So a batch costs max(sweep, chain) instead of their sum and a grid barrier
-// (one barrier per batch, the form before this one, in brackets).  Bound of
-// the sweep: the MUFU reciprocal, 16 a clock and SM; its loop runs at 14.9
-// pairs a clock, 6.8 us a batch at 100,000 vertices and batch 256 (10.8, of
-// which 6.9 the sweep).  Bound of the chain: instruction latency of about 400
-// dependent instructions and one L2 round trip, 2.9 us a batch at 4,096
-// vertices (5.2), 3.5 at 20,000 and batch 200 (5.4); 31,000 and batch 512 5.9
-// (12.3).  Every sum has a fixed order, so results are deterministic.
+// So a batch costs max(sweep, chain); with a grid barrier a batch it costs their
+// sum and the barrier.  Bound of the sweep: the MUFU reciprocal, 16 a clock and
+// SM; its loop runs at 14.9 pairs a clock.  Bound of the chain: instruction
+// latency of about 400 dependent instructions and one L2 round trip.  us a
+// batch, with a barrier / so: 100,000 vertices and batch 256 10.8 (6.9 of them
+// the sweep) / 6.8; 4,096 vertices 5.2 / 3.0; 20,000 and batch 200 5.4 / 3.5;
+// 31,000 and batch 512 12.3 / 5.8.  Every sum has a fixed order, so results are
+// deterministic.
 //
 // Algorithmic work: 10 flops per ordered pair (2 sub, 3 for |d|^2, 1 rcp,
 // 2 FMA x 2 components counted as 4), n*n pairs per iteration.
@@ -1559,8 +1559,9 @@ extern "C" int bl_minibatch_iteration_noalloc(int n, const int *d_rowptr, const 
       occ < 1 || grid > occ * num_sms)
     return BL_ERR_TOO_LARGE;
   // the scratch: status | energy + loops | control words, exchange, partials.
-  // The first two and the control words and exchange start at zero; every
-  // other value is written before it is read.
+  // The first two and the control words and exchange start at zero.  Partials
+  // may be loaded unwritten (the second of a pair of targets when their number
+  // is odd, those of a batch past the end) and are not used then.
   DevStatus *status = reinterpret_cast<DevStatus *>(base);
   double *energy = reinterpret_cast<double *>(base + sizeof(DevStatus));
   unsigned char *scratch = base + 256;

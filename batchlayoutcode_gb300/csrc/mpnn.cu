@@ -714,9 +714,9 @@ __global__ void __launch_bounds__(kGatherVerts * 16) mpnn_gather_kernel(
 
 // sum of per-block partials in block order: out[i] = sum_b part[b * len + i].
 // A block takes 32 entries: all its threads fetch 256 partials of each at once
-// and one warp adds them in order from shared memory.  One thread an entry
-// with 32 loads in flight was bound by its round trips: 27 us for 608 partials
-// of 8,256 entries, so 11.
+// and one warp adds them in order from shared memory: 11 us for 608 partials of
+// 8,256 entries.  One thread an entry with 32 loads in flight is bound by its
+// round trips (27 us).
 constexpr int kReduceCols = 32, kReduceRows = 256, kReduceThreads = 256;
 
 __global__ void __launch_bounds__(kReduceThreads) mpnn_reduce_kernel(const float *__restrict__ part, int blocks, int len,

@@ -1,14 +1,22 @@
 // waits.cu -- self-test of the library's bounded device waits.
 //
-// Every spin-wait in the layout kernels is bounded: the grid barrier of the
-// cooperative kernels (grid_wait, 2 s of %globaltimer) and the mbarrier wait
-// for tensor-core MMA completion (tc::mbar_wait, 1 s).  When a bound runs out
-// the waiting thread records the site in the context's DevStatus and the
-// kernel returns; the host maps the record to BL_ERR_DEVICE_TIMEOUT.  The two
-// kernels below run exactly those waits with the arrival made or withheld,
-// so a caller (and the tests) can see the timeout path end in an error code
-// with the context still usable.  Nothing here faults or hangs: the withheld
-// arrival only lets the wait run to its limit.
+// Every spin-wait in the layout kernels is bounded.  When a bound runs out the
+// waiting thread records the site in the context's DevStatus and the kernel
+// returns; the host maps the record to BL_ERR_DEVICE_TIMEOUT.  The waits:
+//   grid_wait       grid barrier of the breadth-first start and of the
+//                   device-wide hop distances, 2 s of %globaltimer
+//   tc::mbar_wait   tensor-core MMA completion, 1 s
+//   sort_barrier    grid barrier of the Morton sort, 2 s
+//   Poll            the all-pairs movers' and sweepers' waits, 2 s; the spins on
+//                   the watching warp end with that warp (wait_seen)
+//   enter, keep_waiting   the greedy phase's, 2 s
+//   sweep_group     the Barnes-Hut sweep's, 2 s
+// The two kernels below run the first two with the arrival made or withheld, so
+// a caller (and the tests) can see the timeout path end in an error code with
+// the context still usable.  Nothing here faults or hangs: the withheld arrival
+// only lets the wait run to its limit.  The all-pairs and greedy waits are
+// tested through their other end, an error that another warp recorded (a force
+// out of range).
 #include <algorithm>
 
 #include "../../include/batchlayout_gb300.h"

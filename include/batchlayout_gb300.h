@@ -346,7 +346,7 @@ int bl_learned_layout(bl_ctx *ctx, const float *params, const double *scale_mode
 /* No counterpart in the reference (which has no device waits).  Runs one of
  * the bounded waits the layout kernels use, with its arrival made
  * (complete = 1) or withheld (complete = 0): site 0 the grid barrier of the
- * cooperative kernels (limit 2 s), site 1 the mbarrier wait for tensor-core
+ * breadth-first kernels (limit 2 s), site 1 the mbarrier wait for tensor-core
  * completion (limit 1 s).  A withheld arrival lets the wait run to its limit;
  * the kernel then records the site and returns, and the call returns
  * BL_ERR_DEVICE_TIMEOUT with the reason in bl_last_error -- the path every
