@@ -201,17 +201,17 @@ __device__ __forceinline__ void bfs_block(const BlockBfsArgs &a, BlockBfsSmem &S
     const unsigned short d = (unsigned short)min(L, 65534);
     for (int i0 = 0; i0 < 2 * count; i0 += kBlockThreads) {
       const int idx = (i0 + tid) >> 1;
-      unsigned int e = 0, e1 = 0;  // (unsigned: places behind the last of 2^31 - 1 entries are compared too)
+      int e = 0, left = 0;  // the lane's next entry of its row, entries from there to the row's end
       if (idx < count) {
         const int u = v0 + q[idx];
         e = __ldg(&a.rowptr[u]) + (tid & 1);
-        e1 = __ldg(&a.rowptr[u + 1]);
+        left = __ldg(&a.rowptr[u + 1]) - e;
       }
-      while (__any_sync(0xffffffffu, e < e1)) {
+      while (__any_sync(0xffffffffu, left > 0)) {
         int v[kBlockEdges];
         unsigned int fresh = 0;
 #pragma unroll
-        for (int k = 0; k < kBlockEdges; k++) v[k] = e + 2 * k < e1 ? __ldg(&a.colids[e + 2 * k]) - v0 : -1;
+        for (int k = 0; k < kBlockEdges; k++) v[k] = 2 * k < left ? __ldg(&a.colids[(size_t)(unsigned int)e + 2 * k]) - v0 : -1;
         if (kBits) {
           unsigned int old[kBlockEdges];
 #pragma unroll
@@ -258,7 +258,8 @@ __device__ __forceinline__ void bfs_block(const BlockBfsArgs &a, BlockBfsSmem &S
             slot += __popc(b[k]);
           }
         }
-        e += 2 * kBlockEdges;
+        e = (int)((unsigned int)e + 2 * kBlockEdges);
+        left -= 2 * kBlockEdges;
       }
     }
     __syncthreads();
