@@ -875,8 +875,8 @@ def main():
                 "algorithmic_bytes_per_launch": alg_bytes, "walk_pairs": npairs,
                 "iterations_per_launch": first,
                 "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if pk else "fallback",
-                "note": "one cluster runs the batches in sequence, one cluster barrier per batch; "
-                        "positions stay in L2, so the kernel is bound by barrier and gather latency"}
+                "note": "a warp per vertex and iteration waits only for the positions it reads; they stay in L2, "
+                        "so the kernel is bound by the longest chain of such waits, then by instruction issue"}
     else:
         pairs = float(g.n) * g.n
         avg_s = kern_ms / max(kern_count, 1) / 1e3
