@@ -1739,7 +1739,28 @@ __global__ void bh_forces_kernel(const float4 *__restrict__ ff, int n, double2 *
 
 inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
+// `missing` blocks never arrive; the others wait at the sort's grid barrier.
+__global__ void __launch_bounds__(kSortThreads) sort_barrier_selftest_kernel(SortArgs a, int missing) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if ((int)blockIdx.x >= missing) sort_barrier(a, *reinterpret_cast<SortSmem *>(smem_raw), 1);
+}
+
 }  // namespace
+
+int sort_wait_selftest(bl_ctx *ctx, bool complete) {
+  if (!ctx->s.bbox) return bl_fail(ctx, -7, "no graph loaded");
+  BL_CUDA(ctx, cudaFuncSetAttribute(sort_barrier_selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(SortSmem)));
+  BL_CUDA(ctx, cudaMemsetAsync(ctx->s.bbox, 0xff, 5 * sizeof(unsigned int), ctx->stream));
+  SortArgs a{};
+  a.ctl = ctx->s.bbox;
+  a.st = ctx->s.status;
+  int missing = complete ? 0 : 1;
+  void *args[] = {&a, &missing};
+  BL_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)sort_barrier_selftest_kernel, dim3(8), dim3(kSortThreads),
+                                           args, sizeof(SortSmem), ctx->stream));
+  return 0;
+}
 
 int ensure_bh_scratch(bl_ctx *ctx) {
   const size_t n = (size_t)ctx->g.n;

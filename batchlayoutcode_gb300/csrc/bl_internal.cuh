@@ -283,6 +283,8 @@ void bl_time_end(bl_ctx *ctx, const char *kernel);
 
 // ---- kernels drivers (smu.cu, bh.cu, reduce.cu) ----------------------------
 namespace bl {
+int sort_wait_selftest(bl_ctx *ctx, bool complete);   // bl_wait_selftest's sites 2
+int count_wait_selftest(bl_ctx *ctx, bool complete);  // and 3: launch only
 int minibatch_run(bl_ctx *ctx, int model, int batch, int iterations, double step0,
                   double decay, bool converged, double engt, long long max_loops,
                   double *energy_out, long long *loops_out);

@@ -1388,7 +1388,19 @@ bool minibatch_shape(int n, int batch, double row, int num_sms, int smem_optin, 
   return found;
 }
 
+// One thread waits for the count as the movers do.
+__global__ void count_wait_selftest_kernel(const unsigned int *count, unsigned int target, DevStatus *st) {
+  wait_count(count, target, st);
+}
+
 }  // namespace
+
+int count_wait_selftest(bl_ctx *ctx, bool complete) {
+  // a zero word that nothing counts in
+  count_wait_selftest_kernel<<<1, 1, 0, ctx->stream>>>(&ctx->s.status->pad, complete ? 0u : 1u, ctx->s.status);
+  BL_CUDA(ctx, cudaGetLastError());
+  return 0;
+}
 
 int minibatch_run(bl_ctx *ctx, int model, int batch, int iterations, double step0,
                   double decay, bool converged, double engt, long long max_loops,

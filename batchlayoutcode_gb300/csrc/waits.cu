@@ -11,12 +11,12 @@
 //                   the watching warp end with that warp (wait_seen)
 //   enter, keep_waiting   the greedy phase's, 2 s
 //   sweep_group     the Barnes-Hut sweep's, 2 s
-// The two kernels below run the first two with the arrival made or withheld, so
-// a caller (and the tests) can see the timeout path end in an error code with
-// the context still usable.  Nothing here faults or hangs: the withheld arrival
-// only lets the wait run to its limit.  The all-pairs and greedy waits are
-// tested through their other end, an error that another warp recorded (a force
-// out of range).
+// The kernels below, and two beside sort_barrier and Poll, run the first four
+// with the arrival made or withheld, so a caller (and the tests) can see the
+// timeout path end in an error code with the context still usable.  Nothing here
+// faults or hangs: the withheld arrival only lets the wait run to its limit.  The
+// all-pairs and greedy waits are tested through their other end too, an error
+// that another warp recorded (a force out of range).
 #include <algorithm>
 
 #include "../../include/batchlayout_gb300.h"
@@ -52,10 +52,15 @@ __global__ void mbar_wait_selftest_kernel(DevStatus *st, int arrive) {
 extern "C" int bl_wait_selftest(bl_ctx *ctx, int site, int complete) try {
   using namespace bl;
   if (!ctx) return BL_ERR_ARG;
-  if (site != 0 && site != 1) return bl_fail(ctx, BL_ERR_ARG, "site must be 0 (grid barrier) or 1 (mbarrier)");
+  if (site < 0 || site > 3)
+    return bl_fail(ctx, BL_ERR_ARG, "site must be 0 (grid barrier), 1 (mbarrier), 2 (sort barrier) or 3 (count)");
   BL_CUDA(ctx, cudaSetDevice(ctx->device));
   BL_CUDA(ctx, cudaMemsetAsync(ctx->s.status, 0, sizeof(DevStatus), ctx->stream));
-  if (site == 0) {
+  if (site == 2) {
+    if (int rc = sort_wait_selftest(ctx, complete != 0)) return rc;
+  } else if (site == 3) {
+    if (int rc = count_wait_selftest(ctx, complete != 0)) return rc;
+  } else if (site == 0) {
     const int grid = std::max(2, std::min(ctx->num_sms, 8));
     DevStatus *st = ctx->s.status;
     int missing = complete ? 0 : 1;

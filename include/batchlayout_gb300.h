@@ -347,7 +347,8 @@ int bl_learned_layout(bl_ctx *ctx, const float *params, const double *scale_mode
  * the bounded waits the layout kernels use, with its arrival made
  * (complete = 1) or withheld (complete = 0): site 0 the grid barrier of the
  * breadth-first kernels (limit 2 s), site 1 the mbarrier wait for tensor-core
- * completion (limit 1 s).  A withheld arrival lets the wait run to its limit;
+ * completion (limit 1 s), site 2 the Morton sort's grid barrier and site 3 the
+ * all-pairs movers' wait for a count (2 s each).  A withheld arrival lets the wait run to its limit;
  * the kernel then records the site and returns, and the call returns
  * BL_ERR_DEVICE_TIMEOUT with the reason in bl_last_error -- the path every
  * layout call takes when a device wait runs out.  The context stays usable. */
